@@ -2,13 +2,18 @@
 // one qtensor::operator* (qtensor/qtensor.cpp:652-726) in a single launch.
 //
 // FP64 path: 64x64 CTA tiles, BK=16, 3-stage cp.async pipeline, four warps
-// of 32x32 built from mma.sync m8n8k4 f64 (DMMA).  Operands are gathered
-// through per-pair offset tables (row/column offsets of the strided tensor
-// blocks), so any index permutation of the contraction is handled without a
-// transpose pass; the tables are expanded on the device from the pair
-// descriptors when the plan is built.
+// of 32x32 built from mma.sync m16n8k8 f64 (DMMA), a tile's k range shared by
+// a cluster of CTAs where the plan has few tiles.  Operands are gathered
+// through the strides of the tensor blocks (or per-pair offset tables, where
+// the modes of a row or column do not merge into one stride), so any index
+// permutation of the contraction is handled without a transpose pass; the
+// tables are expanded on the device from the pair descriptors when the plan is
+// built.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cstring>
 #include <functional>
 #include <map>
@@ -24,22 +29,35 @@ constexpr int BM = 64;
 constexpr int BN = 64;
 constexpr int BK = 16;
 constexpr int STAGES = 3;
+constexpr int MT = BM / 32;  // 16-row parts of a warp's tile (2 x THREADS / 64 warps)
 constexpr int THREADS = 128;
-constexpr int SA = BM + 4;  // padded k-rows: conflict-free 8-byte fragment loads
-constexpr int SB = BN + 4;
-constexpr size_t SMEM_BYTES = sizeof(double) * STAGES * BK * (SA + SB);
+constexpr int WN = BN / (THREADS / 64);  // columns of a warp's tile
+constexpr int NT = WN / 8;               // its 8-column parts
+constexpr int STAGE_EL = (BM + BN) * BK;  // elements of a stage: A's rows, then B's
+constexpr size_t SMEM_BYTES = sizeof(double) * STAGES * STAGE_EL;
+constexpr int PAIR_BATCH = 16;   // pair descriptors staged in shared memory at a time
+constexpr int SPLIT_MAX = 8;     // most CTAs (one portable cluster) sharing a tile's k range
 
 struct PairDev {
   int64_t a_off, b_off;
   int32_t m, n, k;
   int32_t rowA, colA, rowB, colB;  // offsets of the tables in the table buffer
   int32_t a_mfast, b_kfast;        // unit stride along m (A) / along k (B)
+  // the stride of A's rows and columns and of B's rows and columns where all
+  // modes merge into one (offset = index * stride); NO_STRIDE: use the table
+  int32_t a_rs, a_ks, b_ks, b_cs;
 };
+constexpr int32_t NO_STRIDE = INT_MIN;
 
 struct TaskDev {
   int32_t out;
   int32_t m0, n0;
   int32_t p_begin, p_end;
+};
+
+struct DTask {  // one output tile of grouped_dgemm
+  int32_t out, m0, n0, p_begin, p_end;
+  int32_t chunks;  // BK-wide k chunks over its pairs
 };
 
 struct OutDev {
@@ -77,143 +95,278 @@ __device__ __forceinline__ void cp_async8(double* smem, const double* gmem, bool
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(saddr), "l"(gmem),
                "r"(src_bytes));
 }
+__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
+  unsigned saddr = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(saddr), "l"(gmem));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+// D += A B, m16n8k8 FP64 (DMMA).  Lane 4g + t holds
+// A[g][t], A[g+8][t], A[g][t+4], A[g+8][t+4]; B[t][g], B[t+4][g];
+// D[g][2t], D[g][2t+1], D[g+8][2t], D[g+8][2t+1].
+__device__ __forceinline__ void dmma_k8(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
   asm volatile(
-      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-      : "+d"(c[0]), "+d"(c[1])
-      : "d"(a), "d"(b));
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+// Element (r, k) of an operand's stage: rows of 64 along m or n (KF false), or
+// rows of 16 along k (KF true), whichever the operand is contiguous in, so a
+// warp's 8-byte copies write consecutive shared memory.  A fragment's lane t
+// takes k = 2t and 2t + 1 (any assignment does, the same for A and B), in KF
+// form with one 16-byte load.  The XOR spreads a fragment load over the banks
+// without padding: a half-warp's 4 rows x 4 k (8-byte loads), a quarter-warp's
+// 2 rows x 4 pairs of k (16-byte loads) touch every bank once.
+template <bool KF, int R>
+__device__ __forceinline__ int stage_at(int r, int k) {
+  return KF ? r * BK + (k ^ ((r & 1) << 3)) : k * R + (r ^ ((k & 6) << 1));
 }
 
-__global__ void __launch_bounds__(THREADS)
-grouped_dgemm(const TaskDev* __restrict__ tasks, const OutDev* __restrict__ outs,
+// rows r and k = kk + 2t, kk + 2t + 1 of a stage
+template <bool KF, int R>
+__device__ __forceinline__ void frag2(const double* st, int r, int kk, int t4, double& lo, double& hi) {
+  if (KF) {
+    const double2 v = *reinterpret_cast<const double2*>(st + stage_at<true, R>(r, kk + 2 * t4));
+    lo = v.x;
+    hi = v.y;
+  } else {
+    lo = st[stage_at<false, R>(r, kk + 2 * t4)];
+    hi = st[stage_at<false, R>(r, kk + 2 * t4 + 1)];
+  }
+}
+
+// one k chunk of a warp's 32x32 tile, k8 (1 or 2) steps of 8; mt / nt: its
+// 16-row and 8-column parts that hold output (FULL: all of them)
+template <bool AKF, bool BKF, bool FULL>
+__device__ __forceinline__ void dgemm_chunk(const double* as, const double* bs, double (&acc)[MT][NT][4], int k8,
+                                            int wm, int wn, int g, int t4, int mt, int nt) {
+#pragma unroll
+  for (int kk = 0; kk < BK; kk += 8) {
+    if (kk >= 8 * k8) break;
+    double a[MT][4], b[NT][2];
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) frag2<AKF, BM>(as, wm + i * 16 + h * 8 + g, kk, t4, a[i][h], a[i][h + 2]);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) frag2<BKF, BN>(bs, wn + j * 8 + g, kk, t4, b[j][0], b[j][1]);
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+        if (FULL || (i < mt && j < nt)) dmma_k8(acc[i][j], a[i], b[j]);
+  }
+}
+
+// One operand's chunk (R rows x BK k) into its stage: 8-byte copies,
+// along the operand's contiguous direction, the thread's other index
+// fixed; rows past the block and k past the pair are zero-filled.  rs / ks:
+// strides, or NO_STRIDE for the table.  The copies of a chunk inside the block
+// need one address addition each.
+template <bool KF, int R>
+__device__ __forceinline__ void load_chunk(double* st, const double* __restrict__ X, const int32_t* __restrict__ tab,
+                                           int row_tab, int k_tab, int32_t rs, int32_t ks, int r0, int rows, int k0,
+                                           int K, int tid) {
+  constexpr int DV = KF ? THREADS / BK : THREADS / R;         // step of the walked index
+  constexpr int NQ = KF ? R / DV : BK / DV;                   // copies per thread
+  const int fi = KF ? k0 + (tid & 15) : r0 + (tid & (R - 1));      // fixed index (k, or row)
+  const int vi = KF ? r0 + (tid >> 4) : k0 + tid / R;      // first walked index (row, or k)
+  const int fn = KF ? K : rows, vn = KF ? rows : K;           // their ends
+  const int32_t fs = KF ? ks : rs, vs = KF ? rs : ks;
+  const bool fv = fi < fn;
+  const double* base = X + (fs != NO_STRIDE ? (int64_t)fi * fs : (int64_t)(fv ? tab[(KF ? k_tab : row_tab) + fi] : 0));
+  auto dst = [&](int q) {
+    return st + (KF ? stage_at<true, R>((tid >> 4) + DV * q, tid & 15) : stage_at<false, R>(tid & (R - 1), tid / R + DV * q));
+  };
+  if (vs != NO_STRIDE) {
+    const double* p = base + (int64_t)vi * vs;
+    const int64_t step = (int64_t)DV * vs;
+    if (r0 + R <= rows && k0 + BK <= K) {  // the whole CTA alike
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        cp_async8(dst(q), p);
+        p += step;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const bool ok = fv && vi + DV * q < vn;
+        cp_async8(dst(q), ok ? p : X, ok);
+        p += step;
+      }
+    }
+  } else {
+    const int32_t* vt = tab + (KF ? row_tab : k_tab) + vi;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const bool ok = fv && vi + DV * q < vn;
+      cp_async8(dst(q), ok ? base + vt[DV * q] : X, ok);
+    }
+  }
+}
+
+// A cluster of CTAs (one, where the plan has tiles enough to fill the GPU)
+// takes one output tile; its CTAs share the tile's k chunks evenly, in order,
+// and add their partial tiles through distributed shared memory, CTA 0's
+// first, so the result does not depend on timing.  The chunks of all pairs of
+// a tile form one stream through the ring: the copies of a pair's first chunks
+// are in flight while the previous pair's last ones are multiplied.
+//
+// Bound by the FP64 tensor pipe (37 TFLOP/s when it is fed from registers); the
+// copies' issue slots and shared-memory wavefronts hide behind it only in part:
+// on the environment update's products (25 GFLOP, blocks of 3 to 545) the pipe is
+// active 75 % of the time, 83 % with the copies left out.  64 x 64 tiles of four
+// warps with four CTAs per SM measured best: 128 x 64 tiles, eight warps per tile
+// or a fourth stage were 3 to 14 % slower.  Measured against offset tables read
+// for every element, padded stages and m8n8k4 fragments: env update at bond
+// dimension 2048 1154 -> 975 us per product; R product at 1400 1110 -> 730 us,
+// where the tile's k range is now shared.
+__global__ void __launch_bounds__(THREADS, 4)
+grouped_dgemm(const DTask* __restrict__ tasks, const OutDev* __restrict__ outs,
               const PairDev* __restrict__ pairs, const int32_t* __restrict__ tab,
               const double* __restrict__ A, const double* __restrict__ B,
-              double* __restrict__ C, double alpha) {
-  extern __shared__ double smem[];
-  double* As = smem;                        // [STAGES][BK][SA]
-  double* Bs = smem + STAGES * BK * SA;     // [STAGES][BK][SB]
-  __shared__ int32_t rowA_s[BM];
-  __shared__ int32_t colB_s[BN];
+              double* __restrict__ C, double alpha, int split) {
+  extern __shared__ double smem[];  // [STAGES][A stage, B stage]
+  __shared__ PairDev sp[PAIR_BATCH];
+  __shared__ int32_t s_meta[STAGES];  // of the chunk in a stage: its 8-wide k steps, and its operands' directions
 
-  const TaskDev task = tasks[blockIdx.x];
+  const DTask task = tasks[blockIdx.x / split];
+  const int rank = blockIdx.x % split;  // its place in the cluster (clusters are consecutive blocks)
   const OutDev out = outs[task.out];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
-  const int wm = (warp & 1) * 32;
-  const int wn = (warp >> 1) * 32;
+  const int wm = (warp & 1) * (BM / 2);
+  const int wn = (warp >> 1) * WN;
   const int g = lane >> 2;  // groupID
   const int t4 = lane & 3;  // thread in group
+  // parts of this warp's tile that hold output
+  const int mt = max(0, min(MT, (out.m - task.m0 - wm + 15) >> 4));
+  const int nt = mt == 0 ? 0 : max(0, min(NT, (out.n - task.n0 - wn + 7) >> 3));
+  const bool full = mt == MT && nt == NT;
 
-  double acc[4][4][2];
+  double acc[MT][NT][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < MT; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
 
-  for (int p = task.p_begin; p < task.p_end; ++p) {
-    const PairDev P = pairs[p];
-    __syncthreads();  // previous pair finished with rowA_s / colB_s / stages
-    if (tid < BM) {
-      int m = task.m0 + tid;
-      rowA_s[tid] = m < P.m ? tab[P.rowA + m] : 0;
-    } else {
-      int n = task.n0 + tid - BM;
-      colB_s[tid - BM] = n < P.n ? tab[P.colB + n] : 0;
-    }
+  // the loader's place in the stream: pair lp (its descriptor in sp), its chunk lc of lnch
+  int lp = task.p_begin, base = task.p_begin, lc = 0, lnch = 0;
+  auto stage_pairs = [&](int from) {  // every thread alike
     __syncthreads();
-    const double* Ab = A + P.a_off;
-    const double* Bb = B + P.b_off;
-    const int K = P.k;
-    const int nchunks = (K + BK - 1) / BK;
-
-    auto load_stage = [&](int chunk, int stage) {
-      const int k0 = chunk * BK;
-      double* as = As + stage * BK * SA;
-      double* bs = Bs + stage * BK * SB;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        int m, k;
-        if (P.a_mfast) {
-          m = tid & 63;
-          k = (tid >> 6) + 2 * r;
-        } else {
-          k = tid & 15;
-          m = (tid >> 4) + 8 * r;
-        }
-        int gk = k0 + k;
-        bool ok = (task.m0 + m < P.m) && (gk < K);
-        const double* src = ok ? Ab + rowA_s[m] + tab[P.colA + gk] : Ab;
-        cp_async8(as + k * SA + m, src, ok);
-      }
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        int n, k;
-        if (P.b_kfast) {
-          k = tid & 15;
-          n = (tid >> 4) + 8 * r;
-        } else {
-          n = tid & 63;
-          k = (tid >> 6) + 2 * r;
-        }
-        int gk = k0 + k;
-        bool ok = (task.n0 + n < P.n) && (gk < K);
-        const double* src = ok ? Bb + tab[P.rowB + gk] + colB_s[n] : Bb;
-        cp_async8(bs + k * SB + n, src, ok);
-      }
-    };
-
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) {
-      if (s < nchunks) load_stage(s, s);
-      cp_async_commit();
+    constexpr int W = sizeof(PairDev) / 4;
+    const int cnt = min(PAIR_BATCH, task.p_end - from) * W;
+    for (int i = tid; i < cnt; i += THREADS)
+      reinterpret_cast<int32_t*>(sp)[i] = reinterpret_cast<const int32_t*>(pairs + from)[i];
+    __syncthreads();
+    base = from;
+  };
+  const int c0 = (int)((int64_t)task.chunks * rank / split), c1 = (int)((int64_t)task.chunks * (rank + 1) / split);
+  const int nch = c1 - c0;
+  if (nch > 0) {
+    stage_pairs(lp);
+    lc = c0;
+    while (true) {  // the pair that holds chunk c0
+      lnch = (sp[lp - base].k + BK - 1) / BK;
+      if (lc < lnch) break;
+      lc -= lnch;
+      if (++lp - base == PAIR_BATCH) stage_pairs(lp);
     }
-    for (int c = 0; c < nchunks; ++c) {
-      cp_async_wait<STAGES - 2>();
-      __syncthreads();
-      const int stage = c % STAGES;
-      const double* as = As + stage * BK * SA;
-      const double* bs = Bs + stage * BK * SB;
-      const int ksteps = min(BK / 4, (K - c * BK + 3) >> 2);
-      for (int kk = 0; kk < ksteps; ++kk) {
-        double af[4], bf[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) af[i] = as[(kk * 4 + t4) * SA + wm + i * 8 + g];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bf[j] = bs[(kk * 4 + t4) * SB + wn + j * 8 + g];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) dmma(acc[i][j], af[i], bf[j]);
-      }
-      const int nxt = c + STAGES - 1;
-      if (nxt < nchunks) load_stage(nxt, nxt % STAGES);
-      cp_async_commit();
-    }
-    cp_async_wait<0>();
   }
+  auto load_next = [&](int stage) {
+    while (lc == lnch) {  // on to the next pair
+      if (++lp - base == PAIR_BATCH) stage_pairs(lp);
+      lnch = (sp[lp - base].k + BK - 1) / BK;
+      lc = 0;
+    }
+    const PairDev& P = sp[lp - base];
+    const int k0 = lc * BK, K = P.k;
+    const bool akf = !P.a_mfast, bkf = P.b_kfast;
+    double* as = smem + stage * STAGE_EL;
+    double* bs = as + BM * BK;
+    if (akf) load_chunk<true, BM>(as, A + P.a_off, tab, P.rowA, P.colA, P.a_rs, P.a_ks, task.m0, P.m, k0, K, tid);
+    else load_chunk<false, BM>(as, A + P.a_off, tab, P.rowA, P.colA, P.a_rs, P.a_ks, task.m0, P.m, k0, K, tid);
+    if (bkf) load_chunk<true, BN>(bs, B + P.b_off, tab, P.colB, P.rowB, P.b_cs, P.b_ks, task.n0, P.n, k0, K, tid);
+    else load_chunk<false, BN>(bs, B + P.b_off, tab, P.colB, P.rowB, P.b_cs, P.b_ks, task.n0, P.n, k0, K, tid);
+    if (tid == 0) s_meta[stage] = (K - k0 > 8 ? 2 : 1) | (akf ? 4 : 0) | (bkf ? 8 : 0);
+    ++lc;
+  };
+
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < nch) load_next(s);
+    cp_async_commit();
+  }
+  for (int c = 0; c < nch; ++c) {
+    cp_async_wait<STAGES - 2>();
+    __syncthreads();
+    const int stage = c % STAGES;
+    const int meta = s_meta[stage];
+    const int k8 = meta & 3;
+    const double* as = smem + stage * STAGE_EL;
+    const double* bs = as + BM * BK;
+    if (full) {
+      switch (meta >> 2) {
+        case 0: dgemm_chunk<false, false, true>(as, bs, acc, k8, wm, wn, g, t4, mt, nt); break;
+        case 1: dgemm_chunk<true, false, true>(as, bs, acc, k8, wm, wn, g, t4, mt, nt); break;
+        case 2: dgemm_chunk<false, true, true>(as, bs, acc, k8, wm, wn, g, t4, mt, nt); break;
+        default: dgemm_chunk<true, true, true>(as, bs, acc, k8, wm, wn, g, t4, mt, nt); break;
+      }
+    } else if (nt > 0) {
+      switch (meta >> 2) {
+        case 0: dgemm_chunk<false, false, false>(as, bs, acc, k8, wm, wn, g, t4, mt, nt); break;
+        case 1: dgemm_chunk<true, false, false>(as, bs, acc, k8, wm, wn, g, t4, mt, nt); break;
+        case 2: dgemm_chunk<false, true, false>(as, bs, acc, k8, wm, wn, g, t4, mt, nt); break;
+        default: dgemm_chunk<true, true, false>(as, bs, acc, k8, wm, wn, g, t4, mt, nt); break;
+      }
+    }
+    if (c + STAGES - 1 < nch) load_next((c + STAGES - 1) % STAGES);
+    cp_async_commit();
+  }
+  cp_async_wait<0>();
 
   // epilogue: C tile = alpha * acc (blocks without pairs get zeros)
   double* Cb = C + out.c_off;
+  if (split == 1) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int m = task.m0 + wm + i * 8 + g;
-    if (m >= out.m) continue;
+    for (int i = 0; i < MT; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        int n = task.n0 + wn + j * 8 + 2 * t4 + e;
-        if (n < out.n) Cb[m + (int64_t)out.ldc * n] = alpha * acc[i][j][e];
-      }
-    }
+        for (int e = 0; e < 4; ++e) {
+          const int m = task.m0 + wm + i * 16 + (e >> 1) * 8 + g;
+          const int n = task.n0 + wn + j * 8 + 2 * t4 + (e & 1);
+          if (m < out.m && n < out.n) Cb[m + (int64_t)out.ldc * n] = alpha * acc[i][j][e];
+        }
+    return;
   }
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __syncthreads();  // the ring is free: this CTA's partial tile goes there, column-major
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        smem[(wm + i * 16 + (e >> 1) * 8 + g) + BM * (wn + j * 8 + 2 * t4 + (e & 1))] = acc[i][j][e];
+  cluster.sync();
+  const int per = BN / split;  // columns this CTA adds up
+  for (int el = tid; el < BM * per; el += THREADS) {
+    const int at = BM * per * rank + el;
+    double s = 0.0;
+    for (int q = 0; q < split; ++q) s += *cluster.map_shared_rank(smem + at, q);
+    const int m = task.m0 + at % BM, n = task.n0 + at / BM;
+    if (m < out.m && n < out.n) Cb[m + (int64_t)out.ldc * n] = alpha * s;
+  }
+  cluster.sync();  // no CTA leaves while another reads its partial tile
 }
 
 // ---------------------------------------------------------------------------
@@ -860,6 +1013,7 @@ struct tt_plan {
   int n_tilesA = 0, n_tilesB = 0;
   int64_t bytesA = 0, bytesB = 0;
   int n_tasks = 0;
+  int split = 1;            // grouped_dgemm: CTAs per output tile
   int n_pairs = 0;
   int n_out = 0;
   double flops = 0.0;
@@ -872,6 +1026,7 @@ struct tt_plan {
   // (keep bits 2 and 3), so that a run of execs allocates them once
   mutable uint8_t* scratch[2] = {nullptr, nullptr};
   TaskDev* d_tasks = nullptr;
+  DTask* d_dtasks = nullptr;  // grouped_dgemm plans, in place of d_tasks
   OutDev* d_outs = nullptr;
   PairDev* d_pairs = nullptr;
   int32_t* d_tab = nullptr;
@@ -930,6 +1085,7 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
   double flops = 0.0;
   std::vector<int> first(n_out + 1, 0);
   std::vector<int64_t> work(n_out, 0);
+  std::vector<int> chunks(n_out, 0);
   for (int ii = 0; ii < n_pairs; ++ii) {
     const tt_block_pair& q = pairs[order[ii]];
     TT_REQUIRE(q.n_m >= 0 && q.n_m <= TT_MAX_MODES && q.n_k >= 0 && q.n_k <= TT_MAX_MODES &&
@@ -982,9 +1138,27 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
     P.a_mfast = (a_m_unit || !a_k_unit) ? 1 : 0;
     bool b_k_unit = q.n_k > 0 && q.b_k_stride[0] == 1;
     P.b_kfast = b_k_unit ? 1 : 0;
+    // the one stride that a dimension's modes merge into, where they do
+    auto merged = [](int nmodes, const int32_t* dims, const int64_t* strides) {
+      int64_t st = 0, next = 0;
+      bool any = false;
+      for (int i = 0; i < nmodes; ++i) {
+        if (dims[i] == 1) continue;
+        if (any && strides[i] != next) return NO_STRIDE;
+        if (!any) st = strides[i];
+        any = true;
+        next = strides[i] * dims[i];
+      }
+      return st >= 0 && st <= INT_MAX ? (int32_t)st : NO_STRIDE;
+    };
+    P.a_rs = merged(q.n_m, q.m_dims, q.a_m_stride);
+    P.a_ks = merged(q.n_k, q.k_dims, q.a_k_stride);
+    P.b_ks = merged(q.n_k, q.k_dims, q.b_k_stride);
+    P.b_cs = merged(q.n_n, q.n_dims, q.b_n_stride);
     hp[ii] = P;
     first[q.out_block + 1]++;
     work[q.out_block] += k;
+    chunks[q.out_block] += (int)((k + BK - 1) / BK);
     flops += 2.0 * (double)m * (double)n * (double)k;
   }
   TT_REQUIRE(tab_len < (1ll << 31), "tt_contract_plan: offset tables too large");
@@ -1145,6 +1319,25 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
   }
   std::vector<TaskDev> tsorted(tasks.size());
   for (size_t i = 0; i < tasks.size(); ++i) tsorted[i] = tasks[torder[i]];
+  const bool dgemm = !tc && !skinny;
+  std::vector<DTask> dtasks;
+  int split = 1;
+  if (dgemm) {
+    int longest = 0;
+    for (const TaskDev& t : tsorted) {
+      dtasks.push_back(DTask{t.out, t.m0, t.n0, t.p_begin, t.p_end, chunks[t.out]});
+      longest = std::max(longest, chunks[t.out]);
+    }
+    // A tile's k range is shared by a cluster while the plan has fewer than two
+    // rounds of CTAs (four fit an SM) and each keeps two chunks of the longest
+    // tile.  R at bond dimension 1400 (420 tiles, k up to 6552): 1110 us whole, 730
+    // in four; stopping at one round 860.  The products of a chain at bond
+    // dimension 128 (34 tiles of at most 12 chunks): 129 us per three products
+    // whole, 123 down to four chunks, 105 down to two.
+    while (split < SPLIT_MAX && (int64_t)dtasks.size() * split < 8 * (int64_t)ctx->num_sms &&
+           longest / (2 * split) >= 2)
+      split *= 2;
+  }
   std::vector<OutDev> ho(n_out);
   for (int o = 0; o < n_out; ++o) ho[o] = OutDev{outs[o].c_off, outs[o].m, outs[o].n, outs[o].ldc};
 
@@ -1201,14 +1394,16 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
   plan->bytesA = bytesA;
   plan->bytesB = bytesB;
   plan->n_tasks = (int)tsorted.size();
+  plan->split = split;
   plan->n_pairs = n_pairs;
   plan->n_out = n_out;
   plan->flops = flops;
-  plan->dev_bytes = (int64_t)(sizeof(TaskDev) * tsorted.size() + sizeof(OutDev) * ho.size() +
+  plan->dev_bytes = (int64_t)((dgemm ? sizeof(DTask) : sizeof(TaskDev)) * tsorted.size() + sizeof(OutDev) * ho.size() +
                               sizeof(PairDev) * hp.size() + sizeof(int32_t) * (size_t)tab_len +
                               sizeof(PackJob) * (ja.size() + jb.size()) + sizeof(PackTile) * (ta.size() + tb.size()) +
                               sizeof(PairTC) * ptc.size());
-  plan->d_tasks = tt::pool_alloc<TaskDev>(ctx, tsorted.size());
+  if (dgemm) plan->d_dtasks = tt::pool_alloc<DTask>(ctx, dtasks.size());
+  else plan->d_tasks = tt::pool_alloc<TaskDev>(ctx, tsorted.size());
   plan->d_outs = tt::pool_alloc<OutDev>(ctx, ho.size());
   plan->d_pairs = tt::pool_alloc<PairDev>(ctx, hp.size());
   plan->d_tab = tt::pool_alloc<int32_t>(ctx, (size_t)tab_len);
@@ -1224,7 +1419,7 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
     tc_ok = (ja.empty() || plan->d_jobsA) && (jb.empty() || plan->d_jobsB) && (ta.empty() || plan->d_tilesA) &&
             (tb.empty() || plan->d_tilesB) && (ptc.empty() || plan->d_pairtc);
   }
-  if (!plan->d_tasks || !plan->d_outs || !plan->d_pairs || !plan->d_tab || !plan->d_status || !d_jobs || !tc_ok) {
+  if ((dgemm ? !plan->d_dtasks : !plan->d_tasks) || !plan->d_outs || !plan->d_pairs || !plan->d_tab || !plan->d_status || !d_jobs || !tc_ok) {
     tt_plan_destroy(ctx, plan);
     tt::pool_free(ctx, d_jobs);
     return tt::fail(TT_ERR_OOM, "tt_contract_plan: device allocation failed");
@@ -1233,7 +1428,8 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
   TT_CUDA(cudaMemsetAsync(plan->d_status, 0, sizeof(int), s));
   lap(3);
   // staged copies: the host vectors may die at return without stalling the stream
-  TT_CUDA(tt::h2d_async(ctx, plan->d_tasks, tsorted.data(), sizeof(TaskDev) * tsorted.size()));
+  if (dgemm) TT_CUDA(tt::h2d_async(ctx, plan->d_dtasks, dtasks.data(), sizeof(DTask) * dtasks.size()));
+  else TT_CUDA(tt::h2d_async(ctx, plan->d_tasks, tsorted.data(), sizeof(TaskDev) * tsorted.size()));
   TT_CUDA(tt::h2d_async(ctx, plan->d_outs, ho.data(), sizeof(OutDev) * ho.size()));
   TT_CUDA(tt::h2d_async(ctx, plan->d_pairs, hp.data(), sizeof(PairDev) * hp.size()));
   TT_CUDA(tt::h2d_async(ctx, d_jobs, jobs.data(), sizeof(TableJob) * jobs.size()));
@@ -1338,9 +1534,23 @@ int tt_contract_exec_keep(tt_ctx* ctx, const tt_plan* plan, const double* A, con
         TT_CUDA(cudaFuncSetAttribute(fns[which], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SK_STAGE_BYTES));
       fns[which]<<<plan->n_tasks, SK_ROWS, dyn, ctx->stream>>>(plan->d_tasks, plan->d_outs, plan->d_pairs,
                                                               plan->d_tab, A, B, C, alpha, staged ? 1 : 0);
-    } else
-      grouped_dgemm<<<plan->n_tasks, THREADS, SMEM_BYTES, ctx->stream>>>(
-          plan->d_tasks, plan->d_outs, plan->d_pairs, plan->d_tab, A, B, C, alpha);
+    } else {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = (unsigned)plan->split;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3((unsigned)plan->n_tasks * (unsigned)plan->split);
+      cfg.blockDim = dim3(THREADS);
+      cfg.dynamicSmemBytes = SMEM_BYTES;
+      cfg.stream = ctx->stream;
+      cfg.attrs = at;
+      cfg.numAttrs = plan->split > 1 ? 1 : 0;
+      TT_CUDA(cudaLaunchKernelEx(&cfg, grouped_dgemm, (const DTask*)plan->d_dtasks, (const OutDev*)plan->d_outs,
+                                 (const PairDev*)plan->d_pairs, (const int32_t*)plan->d_tab, A, B, C, alpha,
+                                 plan->split));
+    }
     TT_LAUNCH_CHECK(ctx);
     return TT_OK;
   }
@@ -1423,6 +1633,7 @@ int tt_plan_destroy(tt_ctx* ctx, tt_plan* plan) {
   if (ctx) {
     tt_plan_release_packed(ctx, plan);
     tt::pool_free(ctx, plan->d_tasks);
+    tt::pool_free(ctx, plan->d_dtasks);
     tt::pool_free(ctx, plan->d_outs);
     tt::pool_free(ctx, plan->d_pairs);
     tt::pool_free(ctx, plan->d_tab);
