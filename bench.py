@@ -753,7 +753,7 @@ def run_c5(args):
                                     "peak": peak_tc, "unit": "TFLOP/s",
                                     "frac": hpts["L*x_and_*R_tflops"] / peak_tc}
             if "mid_gbs" in hpts and hbm:
-                kr["*mid"] = {"bound": "hbm", "kernel": "skinny_dgemm (FP64)", "achieved": hpts["mid_gbs"],
+                kr["*mid"] = {"bound": "hbm", "kernel": "narrow_dgemm (FP64)", "achieved": hpts["mid_gbs"],
                               "peak": hbm, "unit": "GB/s", "frac": hpts["mid_gbs"] / hbm,
                               "peak_source": "MEASURED_PEAKS.json hbm_gbs (copy bandwidth)"}
             arm["kernel_rooflines"] = kr

@@ -195,7 +195,7 @@ int tt_plan_destroy(tt_ctx* ctx, tt_plan* plan);
 /* Device bytes a plan holds (offset tables, tasks, packing jobs). */
 /* Host seconds this thread's planner spent in its stages since the thread
  * started (diagnostic): [0] pair offset tables, [1] the precision choice of
- * the automatic modes, [2] tile tasks and row-stationary chunks, [3]
+ * the automatic modes, [2] tile tasks and narrow chunks, [3]
  * tensor-core packing jobs, [4] device tables, uploads and the rest.  The
  * first min(n, 5) are written. */
 int tt_contract_plan_timers(double* seconds, int n);

@@ -55,8 +55,10 @@ struct TaskDev {
   int32_t p_begin, p_end;
 };
 
-struct DTask {  // one output tile of grouped_dgemm
-  int32_t out, m0, n0, p_begin, p_end;
+struct DTask {  // one output tile of grouped_dgemm, with its output block
+  int64_t c_off;
+  int32_t m, n, ldc;
+  int32_t m0, n0, p_begin, p_end;
   int32_t chunks;  // BK-wide k chunks over its pairs
 };
 
@@ -226,7 +228,7 @@ __device__ __forceinline__ void load_chunk(double* st, const double* __restrict_
 // dimension 2048 1154 -> 975 us per product; R product at 1400 1110 -> 730 us,
 // where the tile's k range is now shared.
 __global__ void __launch_bounds__(THREADS, 4)
-grouped_dgemm(const DTask* __restrict__ tasks, const OutDev* __restrict__ outs,
+grouped_dgemm(const DTask* __restrict__ tasks,
               const PairDev* __restrict__ pairs, const int32_t* __restrict__ tab,
               const double* __restrict__ A, const double* __restrict__ B,
               double* __restrict__ C, double alpha, int split) {
@@ -236,7 +238,6 @@ grouped_dgemm(const DTask* __restrict__ tasks, const OutDev* __restrict__ outs,
 
   const DTask task = tasks[blockIdx.x / split];
   const int rank = blockIdx.x % split;  // its place in the cluster (clusters are consecutive blocks)
-  const OutDev out = outs[task.out];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
@@ -245,8 +246,8 @@ grouped_dgemm(const DTask* __restrict__ tasks, const OutDev* __restrict__ outs,
   const int g = lane >> 2;  // groupID
   const int t4 = lane & 3;  // thread in group
   // parts of this warp's tile that hold output
-  const int mt = max(0, min(MT, (out.m - task.m0 - wm + 15) >> 4));
-  const int nt = mt == 0 ? 0 : max(0, min(NT, (out.n - task.n0 - wn + 7) >> 3));
+  const int mt = max(0, min(MT, (task.m - task.m0 - wm + 15) >> 4));
+  const int nt = mt == 0 ? 0 : max(0, min(NT, (task.n - task.n0 - wn + 7) >> 3));
   const bool full = mt == MT && nt == NT;
 
   double acc[MT][NT][4];
@@ -333,7 +334,7 @@ grouped_dgemm(const DTask* __restrict__ tasks, const OutDev* __restrict__ outs,
   cp_async_wait<0>();
 
   // epilogue: C tile = alpha * acc (blocks without pairs get zeros)
-  double* Cb = C + out.c_off;
+  double* Cb = C + task.c_off;
   if (split == 1) {
 #pragma unroll
     for (int i = 0; i < MT; ++i)
@@ -343,7 +344,7 @@ grouped_dgemm(const DTask* __restrict__ tasks, const OutDev* __restrict__ outs,
         for (int e = 0; e < 4; ++e) {
           const int m = task.m0 + wm + i * 16 + (e >> 1) * 8 + g;
           const int n = task.n0 + wn + j * 8 + 2 * t4 + (e & 1);
-          if (m < out.m && n < out.n) Cb[m + (int64_t)out.ldc * n] = alpha * acc[i][j][e];
+          if (m < task.m && n < task.n) Cb[m + (int64_t)task.ldc * n] = alpha * acc[i][j][e];
         }
     return;
   }
@@ -364,188 +365,209 @@ grouped_dgemm(const DTask* __restrict__ tasks, const OutDev* __restrict__ outs,
     double s = 0.0;
     for (int q = 0; q < split; ++q) s += *cluster.map_shared_rank(smem + at, q);
     const int m = task.m0 + at % BM, n = task.n0 + at / BM;
-    if (m < out.m && n < out.n) Cb[m + (int64_t)out.ldc * n] = alpha * s;
+    if (m < task.m && n < task.n) Cb[m + (int64_t)task.ldc * n] = alpha * s;
   }
   cluster.sync();  // no CTA leaves while another reads its partial tile
 }
 
 // ---------------------------------------------------------------------------
-// Skinny FP64 path: contractions whose output blocks have at most SK_N
-// columns and whose pairs contract at most SK_K elements -- the middle
-// contraction of H_eff*x and of the environment update, (a' b) x (w s1 s2)
-// times (w s1 s2) x (s1' s2' w'), with rows a' b in the hundreds of
-// thousands and k, n the MPO link sector widths.  A 64 x 64 DMMA tile wastes
-// most of its work there, and the contraction is bound by reading T1 and
-// writing T2.  Here a CTA takes SK_ROWS rows of one output block; each
-// thread keeps its row's n outputs in registers across all pairs of the
-// block, with the pair's B (k x n, tiny) staged in shared memory, and reads
-// its A row through the offset tables (coalesced along a unit-stride row
-// mode).  Pairs are summed in the plan's order, as in grouped_dgemm.  The
-// kernel is instantiated for NC = 4, 8, 16, 32 output columns (the plan's
-// widest block rounded up), so a narrow contraction issues no work for
-// columns it does not have and keeps few registers (more CTAs per SM).
-constexpr int SK_N = 32;
-constexpr int SK_K = 64;
-constexpr int SK_ROWS = 256;
-constexpr int64_t SK_STAGE_BYTES = 64 * 1024;  // dynamic shared memory for a task's staged pairs
+// Narrow FP64 path: contractions whose output blocks have at most NR_N columns
+// and whose pairs contract at most NR_K elements -- the middle contraction of
+// H_eff*x and of the environment update, (a' b) x (w s1 s2) times (w s1 s2) x
+// (s1' s2' w'), with rows a' b in the hundreds of thousands and k, n the MPO
+// link sector widths.  It is bound by reading T1 and writing T2.
+//
+// Output blocks that contract the same A blocks (the (s1' s2' w') sectors fed
+// by one set of T1 blocks) form chunks of at most NR_N columns; the A blocks of
+// a chunk, one after another, are its k.  A warp takes 32 rows of a chunk at a
+// time: lane r copies row r of every k to shared memory (8-byte cp.async: 256
+// contiguous bytes per k for a unit row stride), one tile ahead of the one that
+// the m8n8k4 FP64 tensor-core products multiply with the chunk's B (staged once
+// per CTA) into all the chunk's columns.  So T1 crosses HBM once, no column or
+// k is padded by more than a fragment, and after the staging a warp needs no
+// barrier.
+// Measured on the middle contraction (read T1, write T2): bond dimension 3072
+// (2.03 GB) 1131 -> 620 us (1.8 -> 3.3 TB/s), 1400 (0.42 GB) 246 -> 119 us,
+// against a thread per row with the products as FP64 FMAs, 16 columns a time.
+// What is left is instruction issue (IPC 1.7, the tensor pipe 39 % active).
+// Buffers of 16 k with four CTAs per SM measured best: 32 k (three CTAs) 662 us,
+// five CTAs at 96 registers 740 us; A loaded straight into the fragments 853 us.
+constexpr int NR_N = 32;          // columns of a chunk, at most
+constexpr int NR_K = 64;          // k of a pair, at most
+constexpr int NR_KTOT = 256;      // k of a chunk, at most (its B is staged whole)
+constexpr int NR_LD = NR_N + 4;   // row stride of the staged B: a fragment's 4 k on different banks
+constexpr int NR_BUF = 512;       // elements of a warp's A buffer: its rows times 16 k (32 rows) or 64 k (8 rows)
+constexpr int NR_AMAX = 16;       // A blocks of a chunk staged in shared memory, at most
+constexpr int NR_WARPS = 4;
+constexpr int NR_THREADS = 32 * NR_WARPS;
 
-template <int NC>
-__global__ void __launch_bounds__(SK_ROWS)
-skinny_dgemm(const TaskDev* __restrict__ tasks, const OutDev* __restrict__ outs,
-             const PairDev* __restrict__ pairs, const int32_t* __restrict__ tab,
-             const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C,
-             double alpha, int staged) {
-  // staged != 0: every pair's B (k x NC, zero past n) and A column offsets are
-  // staged once for the task (dynamic shared memory sized by the plan), so the
-  // pairs run without barriers; else one pair at a time through sB / sColA
-  extern __shared__ double sk_dyn[];
-  __shared__ double sB[SK_K][NC];
-  __shared__ int32_t sColA[SK_K];
-  const TaskDev task = tasks[blockIdx.x];
-  const OutDev out = outs[task.out];
-  const int r = task.m0 + threadIdx.x;
-  double acc[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) acc[c] = 0.0;
-  if (staged) {
-    double* bst = sk_dyn;
-    int ktot = 0;
-    for (int p = task.p_begin; p < task.p_end; ++p) ktot += pairs[p].k;
-    int32_t* cst = reinterpret_cast<int32_t*>(sk_dyn + (int64_t)ktot * NC);
-    int k0 = 0;
-    for (int p = task.p_begin; p < task.p_end; ++p) {
-      const PairDev P = pairs[p];
-      for (int e = threadIdx.x; e < P.k * NC; e += blockDim.x) {
-        const int kk = e / NC, c = e % NC;
-        bst[(k0 + kk) * NC + c] = c < P.n ? B[P.b_off + tab[P.rowB + kk] + tab[P.colB + c]] : 0.0;
-      }
-      for (int kk = threadIdx.x; kk < P.k; kk += blockDim.x) cst[k0 + kk] = tab[P.colA + kk];
-      k0 += P.k;
-    }
-    __syncthreads();
-    k0 = 0;
-    for (int p = task.p_begin; p < task.p_end; ++p) {
-      const PairDev P = pairs[p];
-      if (r < P.m) {
-        const double* __restrict__ arow = A + P.a_off + tab[P.rowA + r];
-        for (int kk = 0; kk < P.k; ++kk) {
-          const double a = arow[cst[k0 + kk]];
-#pragma unroll
-          for (int c = 0; c < NC; ++c) acc[c] = fma(a, bst[(k0 + kk) * NC + c], acc[c]);
-        }
-      }
-      k0 += P.k;
-    }
-  } else {
-    for (int p = task.p_begin; p < task.p_end; ++p) {
-      const PairDev P = pairs[p];
-      __syncthreads();  // the previous pair's B is no longer read
-      for (int e = threadIdx.x; e < P.k * NC; e += blockDim.x) {
-        const int kk = e / NC, c = e % NC;
-        sB[kk][c] = c < P.n ? B[P.b_off + tab[P.rowB + kk] + tab[P.colB + c]] : 0.0;  // zero past n
-      }
-      for (int kk = threadIdx.x; kk < P.k; kk += blockDim.x) sColA[kk] = tab[P.colA + kk];
-      __syncthreads();
-      if (r < P.m) {
-        const double* __restrict__ arow = A + P.a_off + tab[P.rowA + r];
-        for (int kk = 0; kk < P.k; ++kk) {
-          const double a = arow[sColA[kk]];
-#pragma unroll
-          for (int c = 0; c < NC; ++c) acc[c] = fma(a, sB[kk][c], acc[c]);
-        }
-      }
-    }
-  }
-  if (r < out.m) {
-    double* Cb = C + out.c_off + r;
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-      if (c < out.n) Cb[(int64_t)out.ldc * c] = alpha * acc[c];
-  }
+struct NrChunk {
+  int32_t a_begin, a_end;  // its A blocks in nr_a
+  int32_t ktot;            // and the k of all of them
+  int32_t b_begin, b_end;  // its B blocks in nr_b
+  int32_t c_begin, cols;   // its columns in nr_c
+  int32_t m;               // rows (shared by its output blocks)
+  int32_t d0;              // row r = r0 + d0 r1; 0: rows through the offset tables
+};
+struct NrTask {            // some rows of a chunk
+  NrChunk ch;
+  int32_t row0, tiles, pad;  // first row, and its rows in tiles of RW x NR_WARPS
+};
+struct NrA {               // an A block of a chunk: element (row (r0, r1), k) at off + r0 s0 + r1 s1 + k ks
+  int64_t off;
+  int32_t s0, s1;          // d0 == 0: s0 is the row table
+  int32_t k0, k;           // its first k in the chunk, and how many
+  int32_t ks, pad;
+};
+struct NrB {               // one B block of a chunk: element (k, column) at off + k ks + column cs (or the tables)
+  int64_t off;
+  int32_t k0, c0;          // its first k and column in the chunk
+  int32_t k, n, ks, cs, ktab, ctab;
+};
+
+__device__ __forceinline__ void dmma_k4(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
 }
 
-// Row-stationary form of the skinny path.  Output blocks that read the same
-// A blocks (the same rows, other column sectors: for the middle contraction
-// the (s1' s2' w') sectors fed by one T1 block) are gathered into chunks of
-// at most RS_COLS columns; a task is one chunk's SK_ROWS-row tile.  Each distinct
-// A block of the chunk is read once per row and multiplied into a combined B
-// (k x NC: every pair's B block at its output's columns, zeros elsewhere), so
-// T1 crosses HBM once instead of once per output sector.
-// combined columns per chunk: 16 keeps the accumulators of a 256-row task at
-// about 70 registers a thread (three CTAs per SM); 32 halved the occupancy and
-// ran slower than reading a shared A block twice
-constexpr int RS_COLS = 16;
-struct RsChunk {
-  int32_t a_begin, a_end;  // its distinct A blocks in rs_a
-  int32_t o_begin, o_end;  // its output blocks in rs_o
-  int32_t m;               // rows (shared by the chunk's outputs)
-  int32_t ktot;            // sum of k over its A blocks
-};
-struct RsA {
-  int32_t pair;            // a pair reading this A block (its rowA / colA tables, a_off, k)
-  int32_t e_begin, e_end;  // the pairs of the chunk reading it, in rs_e
-};
-struct RsE {
-  int32_t pair, col;  // a pair and the first combined column of its output
-};
-struct RsO {
-  int32_t out, col;  // an output block and its first combined column
-};
+// elements of one A buffer for chunks of at most ktot k: whole, or NR_BUF at a time
+__host__ __device__ constexpr int narrow_buf(int ktot, int rw) {
+  return rw * ((ktot + 3) & ~3) < NR_BUF ? rw * ((ktot + 3) & ~3) : NR_BUF;
+}
+__host__ __device__ constexpr size_t narrow_smem(int ktot, int rw) {
+  return sizeof(double) * ((size_t)NR_WARPS * 2 * narrow_buf(ktot, rw) + (size_t)((ktot + 3) & ~3) * NR_LD);
+}
 
-template <int NC>
-__global__ void __launch_bounds__(SK_ROWS)
-skinny_rs(const TaskDev* __restrict__ tasks, const RsChunk* __restrict__ chunks, const RsA* __restrict__ ra,
-          const RsE* __restrict__ re, const RsO* __restrict__ ro, const OutDev* __restrict__ outs,
-          const PairDev* __restrict__ pairs, const int32_t* __restrict__ tab, const double* __restrict__ A,
-          const double* __restrict__ B, double* __restrict__ C, double alpha) {
-  extern __shared__ double rs_dyn[];  // ktot x NC combined B, then ktot A column offsets
-  const TaskDev task = tasks[blockIdx.x];
-  const RsChunk ch = chunks[task.out];
-  const int r = task.m0 + threadIdx.x;
-  double* bst = rs_dyn;
-  int32_t* cst = reinterpret_cast<int32_t*>(rs_dyn + (int64_t)ch.ktot * NC);
-  for (int e = threadIdx.x; e < ch.ktot * NC; e += blockDim.x) bst[e] = 0.0;
-  __syncthreads();
-  int k0 = 0;
-  for (int a = ch.a_begin; a < ch.a_end; ++a) {
-    const RsA X = ra[a];
-    const PairDev PA = pairs[X.pair];
-    for (int kk = threadIdx.x; kk < PA.k; kk += blockDim.x) cst[k0 + kk] = tab[PA.colA + kk];
-    for (int q = X.e_begin; q < X.e_end; ++q) {
-      const RsE E = re[q];
-      const PairDev P = pairs[E.pair];
-      for (int e = threadIdx.x; e < P.k * P.n; e += blockDim.x) {
-        const int kk = e / P.n, c = e % P.n;
-        bst[(k0 + kk) * NC + E.col + c] = B[P.b_off + tab[P.rowB + kk] + tab[P.colB + c]];
+// RW: rows of a warp's tile, 32 or 8
+template <int RW>
+__global__ void __launch_bounds__(NR_THREADS, 4)
+narrow_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const NrB* __restrict__ nb,
+             const int64_t* __restrict__ nc, const int32_t* __restrict__ tab, const double* __restrict__ A, const double* __restrict__ B,
+             double* __restrict__ C, double alpha, int abuf) {
+  extern __shared__ double smem[];
+  __shared__ int64_t sc[NR_N];
+  __shared__ NrA sa[NR_AMAX];  // the chunk's A blocks, from the second fetch on
+  const NrTask task = tasks[blockIdx.x];
+  const NrChunk& ch = task.ch;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int ktot = ch.ktot, kz = (ktot + 3) & ~3;
+  constexpr int KB = NR_BUF / RW, MT = RW / 8, ROWS = RW * NR_WARPS, LK = 32 / RW;
+  double* buf = smem + warp * 2 * abuf;      // this warp's two A buffers, [k][RW rows]
+  double* sb = smem + NR_WARPS * 2 * abuf;   // B, [kz][NR_LD]
+  // row r of k in a buffer: a fragment's 4 k x 4 rows on different banks
+  auto at = [](int k, int r) { return RW * k + (RW == 32 ? r ^ ((k & 3) << 2) : r); };
+  const int nblk = ch.a_end - ch.a_begin;
+  if (tid < ch.cols) sc[tid] = nc[ch.c_begin + tid];
+  if (tid < min(nblk, NR_AMAX)) sa[tid] = na[ch.a_begin + tid];
+
+  // tiles of this warp: rows task.row0 + RW (NR_WARPS i + warp), i < tiles
+  const int left = ch.m - task.row0 - RW * warp;
+  const int tiles = left <= 0 ? 0 : min(task.tiles, (left + ROWS - 1) / ROWS);
+  const int nkb = (ktot + KB - 1) / KB;
+  auto row_of = [&](int tile) { return task.row0 + RW * (NR_WARPS * tile + warp); };
+  // copies k [KB kb, ...) of a tile into buffer b; lanes past the last row repeat it
+  const NrA* blocks = na + ch.a_begin;
+  auto fetch = [&](int tile, int kb, int b) {
+    const int row = lane % RW, sub = lane / RW;  // LK k at a time
+    const int r = min(row_of(tile) + row, ch.m - 1);
+    const int r1 = ch.d0 != 0 ? r / ch.d0 : 0, r0 = r - r1 * ch.d0;
+    const int klo = kb * KB, khi = min(klo + KB, ktot);
+    double* dst = buf + b * abuf;
+    for (int q = 0; q < nblk; ++q) {
+      const NrA x = blocks[q];
+      const int lo = max(klo, x.k0), hi = min(khi, x.k0 + x.k);
+      if (lo >= hi) continue;
+      const double* p = A + x.off + (int64_t)(lo + sub - x.k0) * x.ks + (ch.d0 != 0 ? r0 * x.s0 + r1 * x.s1 : tab[x.s0 + r]);
+#pragma unroll 4
+      for (int k = lo - klo + sub; k < hi - klo; k += LK) {
+        cp_async8(dst + at(k, row), p);
+        p += LK * x.ks;
       }
     }
-    k0 += PA.k;
+    const int kend = khi - klo;
+    for (int k = kend + sub; k < ((kend + 3) & ~3); k += LK) dst[at(k, row)] = 0.0;
+  };
+  if (tiles > 0 && nkb > 0) fetch(0, 0, 0);
+  cp_async_commit();
+
+  // the chunk's B: a warp per block, 8 k x 4 columns at a time; zero where there is no column or k
+  for (int k = warp; k < kz; k += NR_WARPS)
+    if (k >= ktot || lane >= ch.cols) sb[k * NR_LD + lane] = 0.0;
+  for (int q = ch.b_begin + warp; q < ch.b_end; q += NR_WARPS) {
+    const NrB E = nb[q];
+    const double* Bp = B + E.off;
+    for (int c = lane >> 3; c < E.n; c += 4)
+      for (int kk = lane & 7; kk < E.k; kk += 8)
+        sb[(E.k0 + kk) * NR_LD + E.c0 + c] = Bp[(E.ks != NO_STRIDE ? kk * E.ks : tab[E.ktab + kk]) +
+                                                (E.cs != NO_STRIDE ? c * E.cs : tab[E.ctab + c])];
   }
   __syncthreads();
-  double acc[NC];
+  if (nblk <= NR_AMAX) blocks = sa;
+
+  const int nt = (ch.cols + 7) >> 3;  // 8-column parts
+  int b = 0;
+  for (int tile = 0; tile < tiles; ++tile) {
+    double acc[MT][4][2];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) acc[c] = 0.0;
-  if (r < ch.m) {
-    k0 = 0;
-    for (int a = ch.a_begin; a < ch.a_end; ++a) {
-      const PairDev PA = pairs[ra[a].pair];
-      const double* __restrict__ arow = A + PA.a_off + tab[PA.rowA + r];
-      for (int kk = 0; kk < PA.k; ++kk) {
-        const double x = arow[cst[k0 + kk]];
+    for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) acc[c] = fma(x, bst[(k0 + kk) * NC + c], acc[c]);
+      for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int kb = 0; kb < nkb; ++kb, b ^= 1) {
+      if (kb + 1 < nkb) fetch(tile, kb + 1, b ^ 1);
+      else if (tile + 1 < tiles) fetch(tile + 1, 0, b ^ 1);
+      cp_async_commit();
+      cp_async_wait<1>();
+      __syncwarp();
+      const int kn = min(KB, ktot - kb * KB);
+      const double* as = buf + b * abuf;
+      const double* bs = sb + (kb * KB + t4) * NR_LD + g;
+#pragma unroll 2
+      for (int k = 0; k < kn; k += 4) {
+        double a[MT];
+#pragma unroll
+        for (int i = 0; i < MT; ++i) a[i] = as[at(k + t4, 8 * i + g)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (j < nt) {
+            const double bv = bs[k * NR_LD + 8 * j];
+#pragma unroll
+            for (int i = 0; i < MT; ++i) dmma_k4(acc[i][j], a[i], bv);
+          }
+        }
       }
-      k0 += PA.k;
+      __syncwarp();  // the buffer is free for the fetch after next
     }
-    for (int o = ch.o_begin; o < ch.o_end; ++o) {
-      const RsO O = ro[o];
-      const OutDev out = outs[O.out];
-      double* Cb = C + out.c_off + r;
+    const int r = row_of(tile) + g;
+    const bool inside = row_of(tile) + RW <= ch.m;
+    if (alpha != 1.0) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
-        if (c >= O.col && c < O.col + out.n) Cb[(int64_t)out.ldc * (c - O.col)] = alpha * acc[c];
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          acc[i][j][0] *= alpha;
+          acc[i][j][1] *= alpha;
+        }
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = 8 * j + 2 * t4 + e;
+        if (c >= ch.cols) continue;
+        double* p = C + sc[c] + r;
+        if (inside) {
+#pragma unroll
+          for (int i = 0; i < MT; ++i) p[8 * i] = acc[i][j][e];
+        } else {
+#pragma unroll
+          for (int i = 0; i < MT; ++i)
+            if (r + 8 * i < ch.m) p[8 * i] = acc[i][j][e];
+        }
+      }
   }
+  cp_async_wait<0>();
 }
 
 // ---------------------------------------------------------------------------
@@ -989,18 +1011,15 @@ double predict_us(const tt_out_block* outs, int n_out, const std::vector<PairDev
 
 struct tt_plan {
   int precision = TT_PREC_FP64;
-  bool skinny = false;      // FP64 plan run by skinny_dgemm (row tasks of SK_ROWS)
-  int skinny_nc = SK_N;     // its widest output block (the kernel instance covers it)
-  int64_t skinny_ktot = 0;  // the largest sum of k over one output block's pairs
-  // row-stationary form of a skinny plan (skinny_rs), when its chunks are valid
-  bool rs = false;
-  int rs_n_tasks = 0, rs_nc = SK_N;
-  int64_t rs_ktot = 0;
-  TaskDev* d_rs_tasks = nullptr;
-  RsChunk* d_rs_chunks = nullptr;
-  RsA* d_rs_a = nullptr;
-  RsE* d_rs_e = nullptr;
-  RsO* d_rs_o = nullptr;
+  char* d_blob = nullptr;  // the device buffer that every array below lies in
+  // narrow FP64 plans (narrow_dgemm)
+  bool narrow = false;
+  int nr_ktot = 0;  // the most k of a chunk
+  int nr_rw = 32;   // rows of a warp's tile
+  NrTask* d_nr_tasks = nullptr;
+  NrA* d_nr_a = nullptr;
+  NrB* d_nr_b = nullptr;
+  int64_t* d_nr_c = nullptr;
   int* d_status = nullptr;  // tensor-core path: TT_OK or TT_ERR_TIMEOUT
   // tensor-core path: packing jobs and tiles of the unique A / B blocks, the
   // pairs in packed form, and the packed sizes (buffers are taken from the
@@ -1035,7 +1054,7 @@ struct tt_plan {
 extern "C" {
 
 // Host seconds of the planner's stages on this thread (tt_contract_plan_timers):
-// pair tables, precision choice, tile tasks and the row-stationary chunks,
+// pair tables, precision choice, tile tasks and the narrow chunks,
 // tensor-core packing jobs, device tables and uploads.
 static thread_local double g_plan_stage_s[5];
 struct PlanLap {
@@ -1080,7 +1099,7 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
   std::vector<TableJob> jobs;
   jobs.reserve(4 * (size_t)n_pairs);
   int64_t tab_len = 0;
-  std::map<std::vector<int64_t>, int32_t> tab_of;  // table contents -> its offset
+  std::map<std::vector<int64_t>, int32_t> tab_of;  // table contents -> its number in jobs
   std::vector<int64_t> tab_key;
   double flops = 0.0;
   std::vector<int> first(n_out + 1, 0);
@@ -1105,7 +1124,9 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
     P.n = (int)n;
     P.k = (int)k;
     // an offset table is a function of (length, dims, strides) alone: pairs
-    // that address the same rows or columns of a block share one table
+    // that address the same rows or columns of a block share one.  rowA ..
+    // colB are table numbers until the path is chosen; only the tables that it
+    // reads are then laid out
     auto add_job = [&](int len, int nmodes, const int32_t* dims, const int64_t* strides) {
       tab_key.assign({(int64_t)len, (int64_t)nmodes});
       for (int i = 0; i < nmodes; ++i) {
@@ -1116,17 +1137,17 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
       if (hit != tab_of.end()) return hit->second;
       TableJob J;
       memset(&J, 0, sizeof(J));
-      J.dst = (int32_t)tab_len;
+      J.dst = -1;
       J.len = len;
       J.nmodes = nmodes;
       for (int i = 0; i < nmodes; ++i) {
         J.dims[i] = dims[i];
         J.strides[i] = strides[i];
       }
+      const int32_t id = (int32_t)jobs.size();
       jobs.push_back(J);
-      tab_len += len;
-      tab_of.emplace(tab_key, J.dst);
-      return J.dst;
+      tab_of.emplace(tab_key, id);
+      return id;
     };
     P.rowA = add_job((int)m, q.n_m, q.m_dims, q.a_m_stride);
     P.colA = add_job((int)k, q.n_k, q.k_dims, q.a_k_stride);
@@ -1161,7 +1182,6 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
     chunks[q.out_block] += (int)((k + BK - 1) / BK);
     flops += 2.0 * (double)m * (double)n * (double)k;
   }
-  TT_REQUIRE(tab_len < (1ll << 31), "tt_contract_plan: offset tables too large");
   lap(0);
   for (int o = 0; o < n_out; ++o) first[o + 1] += first[o];
   // FP64 unless the tensor-core form is predicted clearly (20 %) faster: the
@@ -1171,161 +1191,203 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
     precision = TT_PREC_FP64;
   lap(1);
   const bool tc = precision != TT_PREC_FP64;
-  // FP64 plans whose output blocks are at most SK_N wide and whose pairs
-  // contract at most SK_K elements run on the skinny kernel
-  bool skinny = !tc && n_pairs > 0;
-  for (int o = 0; o < n_out && skinny; ++o) skinny = outs[o].n <= SK_N;
-  for (int i = 0; i < n_pairs && skinny; ++i) skinny = hp[i].k <= SK_K && hp[i].n <= SK_N;
-  const int tile_m = tc ? TC_BM : (skinny ? SK_ROWS : BM), tile_n = tc ? TC_BN : (skinny ? SK_N : BN);
-  // tile tasks, longest first (LPT) so heavy blocks start early
-  std::vector<TaskDev> tasks;
-  std::vector<int64_t> tcost;
-  for (int o = 0; o < n_out; ++o) {
+  // FP64 plans whose output blocks are at most NR_N wide and whose pairs
+  // contract at most NR_K elements (NR_KTOT over a block) run on the narrow kernel
+  bool narrow = !tc && n_pairs > 0;
+  for (int o = 0; o < n_out && narrow; ++o) narrow = outs[o].n <= NR_N;
+  for (int i = 0; i < n_pairs && narrow; ++i) narrow = hp[i].k <= NR_K && hp[i].n <= NR_N;
+  for (int o = 0; o < n_out && narrow; ++o) narrow = work[o] <= NR_KTOT;
+  for (int o = 0; o < n_out; ++o)
     TT_REQUIRE(outs[o].m >= 0 && outs[o].n >= 0 && outs[o].ldc >= outs[o].m,
                "tt_contract_plan: bad output block");
-    for (int m0 = 0; m0 < outs[o].m; m0 += tile_m)
-      for (int n0 = 0; n0 < outs[o].n; n0 += tile_n) {
-        TaskDev t{o, m0, n0, first[o], first[o + 1]};
-        tasks.push_back(t);
-        tcost.push_back(work[o] + 1);
+  // tile tasks, longest first (LPT) so heavy blocks start early
+  const int tile_m = tc ? TC_BM : BM, tile_n = tc ? TC_BN : BN;
+  std::vector<TaskDev> tsorted;
+  int nr_rw = 32;
+  std::vector<NrTask> nr_tasks;
+  std::vector<NrChunk> nr_chunks;
+  std::vector<NrA> nr_a;
+  std::vector<NrB> nr_b;
+  std::vector<int64_t> nr_c;
+  if (!narrow) {
+    std::vector<int> oorder(n_out);
+    std::iota(oorder.begin(), oorder.end(), 0);
+    std::stable_sort(oorder.begin(), oorder.end(), [&](int x, int y) { return work[x] > work[y]; });
+    for (int o : oorder)
+      for (int m0 = 0; m0 < outs[o].m; m0 += tile_m)
+        for (int n0 = 0; n0 < outs[o].n; n0 += tile_n) tsorted.push_back(TaskDev{o, m0, n0, first[o], first[o + 1]});
+  } else {
+    // chunks: output blocks whose pairs read the same A blocks the same way
+    // (an offset table stands for its modes and strides), so that every k of a
+    // chunk belongs to every one of its columns
+    std::map<std::vector<int64_t>, std::vector<int>> by_a;  // (rows, A blocks in order) -> output blocks
+    std::vector<std::vector<int>> opairs(n_out);             // an output block's pairs in that order
+    std::vector<int64_t> sig;
+    for (int o = 0; o < n_out; ++o) {
+      if (outs[o].m == 0 || outs[o].n == 0) continue;
+      std::vector<int>& op = opairs[o];
+      for (int i = first[o]; i < first[o + 1]; ++i) op.push_back(i);
+      auto key = [&](int i) { return std::make_pair(std::make_pair(hp[i].a_off, hp[i].rowA), std::make_pair(hp[i].colA, hp[i].k)); };
+      std::stable_sort(op.begin(), op.end(), [&](int x, int y) { return key(x) < key(y); });
+      sig.assign(1, outs[o].m);
+      for (int i : op) sig.insert(sig.end(), {hp[i].a_off, hp[i].rowA, hp[i].colA, hp[i].k});
+      by_a[sig].push_back(o);
+    }
+    // the two strides (first extent d0) that a pair's row modes merge into;
+    // d0 = 0 when they do not
+    struct Rows {
+      int64_t d0, s0, s1;
+    };
+    auto rows_of = [&](int i) {
+      const tt_block_pair& q = pairs[order[i]];
+      Rows r{1, 0, 0};
+      int groups = 0;
+      int64_t next = 0;
+      for (int d = 0; d < q.n_m; ++d) {
+        const int64_t e = q.m_dims[d], st = q.a_m_stride[d];
+        if (e == 1) continue;
+        if (groups > 0 && st == next) {
+          if (groups == 1) r.d0 *= e;
+        } else if (groups == 0) {
+          r.d0 = e;
+          r.s0 = st;
+          groups = 1;
+        } else if (groups == 1) {
+          r.s1 = st;
+          groups = 2;
+        } else {
+          return Rows{0, 0, 0};
+        }
+        next = st * e;
       }
-  }
-  std::vector<int> torder(tasks.size());
-  std::iota(torder.begin(), torder.end(), 0);
-  bool rs_ok = false;
-  std::vector<RsChunk> rs_chunks;
-  std::vector<RsA> rs_a;
-  std::vector<RsE> rs_e;
-  std::vector<RsO> rs_o;
-  std::vector<TaskDev> rs_tasks;
-  int64_t rs_ktot = 0;
-  if (skinny) {
-    // The skinny kernel is bound by reading A, and every output block that
-    // shares A's blocks (the same rows, other column sectors) reads them
-    // again.  Tasks of such output blocks are interleaved by row tile, so the
-    // CTAs that run together read the same A rows and all but the first read
-    // hit L2.  Groups: output blocks linked through a shared A block
-    // (union-find on the pairs' A offsets), heaviest group first.
-    std::vector<int> parent(n_out);
-    std::iota(parent.begin(), parent.end(), 0);
-    auto root = [&](int o) {
-      int r = o;
-      while (parent[r] != r) r = parent[r];
-      while (parent[o] != r) {  // path compression
-        const int up = parent[o];
-        parent[o] = r;
-        o = up;
-      }
+      if (groups <= 1) r.s1 = -1;  // any d0 will do: s1 = s0 d0
       return r;
     };
-    std::unordered_map<int64_t, int> owner;
-    for (int o = 0; o < n_out; ++o)
-      for (int i = first[o]; i < first[o + 1]; ++i) {
-        auto it = owner.emplace(hp[i].a_off, o).first;
-        const int ra = root(it->second), rb = root(o);
-        if (ra != rb) parent[rb] = ra;
-      }
-    std::vector<int> groot(n_out);
-    for (int o = 0; o < n_out; ++o) groot[o] = root(o);
-    std::vector<int64_t> gcost(n_out, 0);
-    for (int o = 0; o < n_out; ++o) gcost[groot[o]] += work[o] + 1;
-    // row-stationary chunks (skinny_rs): a group's outputs in order, at most
-    // SK_N combined columns each; valid when the group's outputs share their
-    // rows and every A block is read through the same tables by all its pairs
-    rs_ok = true;
-    std::unordered_map<int64_t, int> a_first;  // a_off -> first pair reading it
-    for (int i = 0; i < n_pairs && rs_ok; ++i) {
-      auto it = a_first.emplace(hp[i].a_off, i).first;
-      const tt_block_pair& x = pairs[order[it->second]];
-      const tt_block_pair& y = pairs[order[i]];
-      rs_ok = hp[i].m == hp[it->second].m && hp[i].k == hp[it->second].k && x.n_m == y.n_m && x.n_k == y.n_k;
-      for (int d = 0; d < x.n_m && rs_ok; ++d)
-        rs_ok = x.m_dims[d] == y.m_dims[d] && x.a_m_stride[d] == y.a_m_stride[d];
-      for (int d = 0; d < x.n_k && rs_ok; ++d)
-        rs_ok = x.k_dims[d] == y.k_dims[d] && x.a_k_stride[d] == y.a_k_stride[d];
-    }
-    std::vector<std::vector<int>> members(n_out);
-    for (int o = 0; o < n_out; ++o) members[groot[o]].push_back(o);
-    for (int g = 0; g < n_out && rs_ok; ++g)
-      for (int o : members[g]) rs_ok = rs_ok && outs[o].m == outs[members[g][0]].m;
-    std::vector<int> gorder;
-    for (int g = 0; g < n_out; ++g)
-      if (!members[g].empty()) gorder.push_back(g);
-    std::stable_sort(gorder.begin(), gorder.end(), [&](int a, int b) { return gcost[a] > gcost[b]; });
-    for (int g : gorder) {
-      if (!rs_ok) break;
-      size_t c0 = rs_chunks.size();
-      auto open_chunk = [&]() {
-        RsChunk c{(int32_t)rs_a.size(), (int32_t)rs_a.size(), (int32_t)rs_o.size(), (int32_t)rs_o.size(),
-                  (int32_t)outs[members[g][0]].m, 0};
-        rs_chunks.push_back(c);
-      };
-      open_chunk();
-      int cols = 0;
-      std::unordered_map<int64_t, int> a_slot;  // a_off -> index in rs_a within the chunk
-      std::vector<std::vector<RsE>> ents;       // per rs_a entry of the chunk
-      auto close_chunk = [&]() {
-        RsChunk& c = rs_chunks.back();
-        for (size_t i = 0; i < ents.size(); ++i) {
-          rs_a[c.a_begin + i].e_begin = (int32_t)rs_e.size();
-          rs_e.insert(rs_e.end(), ents[i].begin(), ents[i].end());
-          rs_a[c.a_begin + i].e_end = (int32_t)rs_e.size();
-          c.ktot += hp[rs_a[c.a_begin + i].pair].k;
-        }
-        c.a_end = (int32_t)rs_a.size();
-        c.o_end = (int32_t)rs_o.size();
-        ents.clear();
-        a_slot.clear();
-      };
-      for (int o : members[g]) {
-        if (cols + outs[o].n > RS_COLS && cols > 0) {
-          close_chunk();
-          open_chunk();
-          cols = 0;
-        }
-        rs_o.push_back(RsO{o, cols});
-        for (int i = first[o]; i < first[o + 1]; ++i) {
-          auto it = a_slot.find(hp[i].a_off);
-          if (it == a_slot.end()) {
-            it = a_slot.emplace(hp[i].a_off, (int)ents.size()).first;
-            rs_a.push_back(RsA{i, 0, 0});
-            ents.emplace_back();
+    std::vector<std::pair<int64_t, std::vector<int>>> groups;  // the chunks of one signature, and their cost
+    for (auto& kv : by_a) {
+      const std::vector<int>& os = kv.second;
+      std::vector<int> ids;
+      int64_t cost = 0;
+      for (size_t x = 0; x < os.size();) {
+        NrChunk c{(int32_t)nr_a.size(), 0, 0, (int32_t)nr_b.size(), 0, (int32_t)nr_c.size(), 0, outs[os[x]].m, 0};
+        size_t y = x;
+        for (; y < os.size() && c.cols + outs[os[y]].n <= NR_N; ++y) {
+          int32_t k0 = 0;
+          for (int i : opairs[os[y]]) {
+            const PairDev& P = hp[i];
+            nr_b.push_back(NrB{P.b_off, k0, c.cols, P.k, P.n, P.b_ks, P.b_cs, P.rowB, P.colB});
+            k0 += hp[i].k;
           }
-          ents[it->second].push_back(RsE{i, cols});
+          for (int n = 0; n < outs[os[y]].n; ++n) nr_c.push_back(outs[os[y]].c_off + (int64_t)outs[os[y]].ldc * n);
+          c.cols += outs[os[y]].n;
         }
-        cols += outs[o].n;
+        c.b_end = (int32_t)nr_b.size();
+        const std::vector<int>& op = opairs[os[x]];
+        std::vector<Rows> rw;
+        int64_t d0 = 0;
+        bool two = true;
+        for (int i : op) {
+          rw.push_back(rows_of(i));
+          if (rw.back().d0 == 0) two = false;
+          if (rw.back().s1 >= 0) {
+            two = two && (d0 == 0 || d0 == rw.back().d0);
+            d0 = rw.back().d0;
+          }
+        }
+        if (d0 == 0) d0 = c.m;
+        for (size_t u = 0; u < op.size(); ++u) {
+          const int64_t s1 = rw[u].s1 < 0 ? rw[u].s0 * d0 : rw[u].s1;
+          two = two && rw[u].s0 >= 0 && rw[u].s0 <= INT_MAX && s1 >= 0 && s1 <= INT_MAX;
+        }
+        c.d0 = two ? (int32_t)d0 : 0;
+        for (size_t u = 0; u < op.size(); ++u) {
+          const PairDev& P = hp[op[u]];
+          const tt_block_pair& q = pairs[order[op[u]]];
+          NrA x{P.a_off, two ? (int32_t)rw[u].s0 : P.rowA, 0, c.ktot, P.k, P.a_ks, 0};
+          if (two) x.s1 = (int32_t)(rw[u].s1 < 0 ? rw[u].s0 * d0 : rw[u].s1);
+          if (P.a_ks != NO_STRIDE) {
+            nr_a.push_back(x);
+          } else {  // k modes that do not merge: one entry per k
+            x.k = 1;
+            x.ks = 0;
+            for (int k = 0; k < P.k; ++k, ++x.k0) {
+              x.off = P.a_off;
+              int rem = k;
+              for (int d = 0; d < q.n_k; ++d) {
+                x.off += (int64_t)(rem % q.k_dims[d]) * q.a_k_stride[d];
+                rem /= q.k_dims[d];
+              }
+              nr_a.push_back(x);
+            }
+          }
+          c.ktot += P.k;
+        }
+        c.a_end = (int32_t)nr_a.size();
+        cost += (int64_t)c.m * (c.ktot + c.cols);
+        ids.push_back((int)nr_chunks.size());
+        nr_chunks.push_back(c);
+        x = y;
       }
-      close_chunk();
-      // tasks: the group's row tiles, its chunks interleaved within a tile
-      const int m = outs[members[g][0]].m;
-      for (int m0 = 0; m0 < m; m0 += SK_ROWS)
-        for (size_t c = c0; c < rs_chunks.size(); ++c) rs_tasks.push_back(TaskDev{(int32_t)c, m0, 0, 0, 0});
+      groups.emplace_back(cost, std::move(ids));
     }
-    for (const RsChunk& c : rs_chunks) rs_ktot = std::max<int64_t>(rs_ktot, c.ktot);
-    for (const RsO& x : rs_o) rs_ok = rs_ok && outs[x.out].n <= RS_COLS;  // every chunk fits its instance
-    if (rs_ok) rs_ok = rs_ktot * (int64_t)(RS_COLS * sizeof(double) + sizeof(int32_t)) <= SK_STAGE_BYTES;
-    // the per-pair skinny kernel (no row-stationary chunks): tasks of a group
-    // interleaved by row tile, heaviest group first; with the chunks, the
-    // tile tasks are not run and stay in their plain order
-    if (!rs_ok)
-      std::stable_sort(torder.begin(), torder.end(), [&](int a, int b) {
-        const int ga = groot[tasks[a].out], gb = groot[tasks[b].out];
-        if (ga != gb) return gcost[ga] != gcost[gb] ? gcost[ga] > gcost[gb] : ga < gb;
-        if (tasks[a].m0 != tasks[b].m0) return tasks[a].m0 < tasks[b].m0;
-        return tasks[a].out < tasks[b].out;
-      });
-  } else {
-    std::stable_sort(torder.begin(), torder.end(), [&](int a, int b) { return tcost[a] > tcost[b]; });
+    std::stable_sort(groups.begin(), groups.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+    // rows per CTA: enough tiles to pay for staging B, but eight CTAs per SM and
+    // more while there are rows (at bond dimension 1400 2857 us per two products
+    // with this bound, 2894 with sixteen tiles as soon as there are four CTAs)
+    // (of 128 rows).  With fewer than four of them per SM the kernel is a chain of
+    // latencies: 8 rows to a warp then, all of their k in flight at once (a sweep
+    // of 48 sites at bond dimension 200: 220 -> 210 ms, with the bound at one, two,
+    // four or eight per SM)
+    int64_t all = 0;
+    for (const NrChunk& c : nr_chunks) all += (c.m + 127) / 128;
+    nr_rw = all < 4 * (int64_t)ctx->num_sms ? 8 : 32;
+    const int rows = nr_rw * NR_WARPS;
+    const int tiles = (int)std::max<int64_t>(1, std::min<int64_t>(16, all / (8 * (int64_t)ctx->num_sms)));
+    for (const auto& gr : groups) {
+      const int m = nr_chunks[gr.second[0]].m;
+      for (int row0 = 0; row0 < m; row0 += tiles * rows)
+        for (int id : gr.second)
+          nr_tasks.push_back(NrTask{nr_chunks[id], row0, std::min(tiles, (m - row0 + rows - 1) / rows), 0});
+    }
   }
-  std::vector<TaskDev> tsorted(tasks.size());
-  for (size_t i = 0; i < tasks.size(); ++i) tsorted[i] = tasks[torder[i]];
-  const bool dgemm = !tc && !skinny;
+  // the offset tables that this path reads, back to back (elsewhere strides serve)
+  {
+    auto need = [&](int32_t& id, bool used) {
+      if (!used) {
+        id = 0;
+        return;
+      }
+      TableJob& J = jobs[id];
+      if (J.dst < 0) {
+        J.dst = (int32_t)tab_len;
+        tab_len += J.len;
+      }
+      id = J.dst;
+    };
+    for (const NrChunk& c : nr_chunks)
+      if (c.d0 == 0)
+        for (int i = c.a_begin; i < c.a_end; ++i) need(nr_a[i].s0, true);
+    for (NrB& x : nr_b) {
+      need(x.ktab, x.ks == NO_STRIDE);
+      need(x.ctab, x.cs == NO_STRIDE);
+    }
+    for (PairDev& P : hp) {
+      need(P.rowA, tc || (!narrow && P.a_rs == NO_STRIDE));
+      need(P.colA, tc || (!narrow && P.a_ks == NO_STRIDE));
+      need(P.rowB, tc || (!narrow && P.b_ks == NO_STRIDE));
+      need(P.colB, tc || (!narrow && P.b_cs == NO_STRIDE));
+      TT_REQUIRE(tab_len < (1ll << 31), "tt_contract_plan: offset tables too large");
+    }
+    jobs.erase(std::remove_if(jobs.begin(), jobs.end(), [](const TableJob& J) { return J.dst < 0; }), jobs.end());
+  }
+  const bool dgemm = !tc && !narrow;
   std::vector<DTask> dtasks;
   int split = 1;
   if (dgemm) {
     int longest = 0;
     for (const TaskDev& t : tsorted) {
-      dtasks.push_back(DTask{t.out, t.m0, t.n0, t.p_begin, t.p_end, chunks[t.out]});
+      const tt_out_block& o = outs[t.out];
+      dtasks.push_back(DTask{o.c_off, o.m, o.n, o.ldc, t.m0, t.n0, t.p_begin, t.p_end, chunks[t.out]});
       longest = std::max(longest, chunks[t.out]);
     }
     // A tile's k range is shared by a cluster while the plan has fewer than two
@@ -1378,98 +1440,80 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
 
   tt_plan* plan = new tt_plan();
   plan->precision = precision;
-  plan->skinny = skinny;
-  if (skinny) {
-    int wmax = 1;
-    for (int o = 0; o < n_out; ++o) wmax = std::max(wmax, outs[o].n);
-    plan->skinny_nc = wmax;
-    for (int o = 0; o < n_out; ++o) {
-      int64_t kt = 0;
-      for (int i = first[o]; i < first[o + 1]; ++i) kt += hp[i].k;
-      plan->skinny_ktot = std::max(plan->skinny_ktot, kt);
-    }
-  }
+  plan->narrow = narrow;
+  plan->nr_rw = nr_rw;
+  for (const NrChunk& c : nr_chunks) plan->nr_ktot = std::max(plan->nr_ktot, c.ktot);
   plan->n_tilesA = (int)ta.size();
   plan->n_tilesB = (int)tb.size();
   plan->bytesA = bytesA;
   plan->bytesB = bytesB;
-  plan->n_tasks = (int)tsorted.size();
+  plan->n_tasks = narrow ? (int)nr_tasks.size() : (int)tsorted.size();
   plan->split = split;
   plan->n_pairs = n_pairs;
   plan->n_out = n_out;
   plan->flops = flops;
-  plan->dev_bytes = (int64_t)((dgemm ? sizeof(DTask) : sizeof(TaskDev)) * tsorted.size() + sizeof(OutDev) * ho.size() +
-                              sizeof(PairDev) * hp.size() + sizeof(int32_t) * (size_t)tab_len +
-                              sizeof(PackJob) * (ja.size() + jb.size()) + sizeof(PackTile) * (ta.size() + tb.size()) +
-                              sizeof(PairTC) * ptc.size());
-  if (dgemm) plan->d_dtasks = tt::pool_alloc<DTask>(ctx, dtasks.size());
-  else plan->d_tasks = tt::pool_alloc<TaskDev>(ctx, tsorted.size());
-  plan->d_outs = tt::pool_alloc<OutDev>(ctx, ho.size());
-  plan->d_pairs = tt::pool_alloc<PairDev>(ctx, hp.size());
-  plan->d_tab = tt::pool_alloc<int32_t>(ctx, (size_t)tab_len);
-  plan->d_status = tt::pool_alloc<int>(ctx, 1);
-  TableJob* d_jobs = tt::pool_alloc<TableJob>(ctx, jobs.size());
-  bool tc_ok = true;
-  if (tc) {
-    plan->d_jobsA = tt::pool_alloc<PackJob>(ctx, ja.size());
-    plan->d_jobsB = tt::pool_alloc<PackJob>(ctx, jb.size());
-    plan->d_tilesA = tt::pool_alloc<PackTile>(ctx, ta.size());
-    plan->d_tilesB = tt::pool_alloc<PackTile>(ctx, tb.size());
-    plan->d_pairtc = tt::pool_alloc<PairTC>(ctx, ptc.size());
-    tc_ok = (ja.empty() || plan->d_jobsA) && (jb.empty() || plan->d_jobsB) && (ta.empty() || plan->d_tilesA) &&
-            (tb.empty() || plan->d_tilesB) && (ptc.empty() || plan->d_pairtc);
+  // the plan's arrays in one device buffer, filled by one staged copy (the host
+  // vectors may die at return without stalling the stream); the offset tables
+  // and the status word, where the path has them, follow it
+  std::vector<char> blob;
+  auto put = [&](const auto& v) {
+    const size_t at = blob.size();
+    blob.resize((at + v.size() * sizeof(v[0]) + 15) & ~(size_t)15);
+    if (!v.empty()) memcpy(blob.data() + at, v.data(), v.size() * sizeof(v[0]));
+    return at;
+  };
+  size_t at_tasks = 0, at_outs = 0, at_pairs = 0, at_a = 0, at_b = 0, at_c = 0, at_ja = 0, at_jb = 0, at_ta = 0, at_tb = 0,
+         at_ptc = 0;
+  if (dgemm) {
+    at_tasks = put(dtasks);
+    at_pairs = put(hp);
+  } else if (narrow) {
+    at_tasks = put(nr_tasks);
+    at_a = put(nr_a);
+    at_b = put(nr_b);
+    at_c = put(nr_c);
+  } else {
+    at_tasks = put(tsorted);
+    at_outs = put(ho);
+    at_ja = put(ja);
+    at_jb = put(jb);
+    at_ta = put(ta);
+    at_tb = put(tb);
+    at_ptc = put(ptc);
   }
-  if ((dgemm ? !plan->d_dtasks : !plan->d_tasks) || !plan->d_outs || !plan->d_pairs || !plan->d_tab || !plan->d_status || !d_jobs || !tc_ok) {
+  const size_t at_jobs = put(jobs);
+  const size_t at_status = blob.size(), at_tab = at_status + 16;
+  const size_t total = at_tab + sizeof(int32_t) * (size_t)tab_len;
+  plan->dev_bytes = (int64_t)total;
+  plan->d_blob = tt::pool_alloc<char>(ctx, total);
+  if (!plan->d_blob) {
     tt_plan_destroy(ctx, plan);
-    tt::pool_free(ctx, d_jobs);
     return tt::fail(TT_ERR_OOM, "tt_contract_plan: device allocation failed");
   }
+  blob.resize(at_tab, 0);  // the status word starts as TT_OK
+  char* d = plan->d_blob;
+  if (dgemm) plan->d_dtasks = reinterpret_cast<DTask*>(d + at_tasks);
+  else if (narrow) plan->d_nr_tasks = reinterpret_cast<NrTask*>(d + at_tasks);
+  else plan->d_tasks = reinterpret_cast<TaskDev*>(d + at_tasks);
+  plan->d_outs = reinterpret_cast<OutDev*>(d + at_outs);
+  plan->d_pairs = reinterpret_cast<PairDev*>(d + at_pairs);
+  plan->d_nr_a = reinterpret_cast<NrA*>(d + at_a);
+  plan->d_nr_b = reinterpret_cast<NrB*>(d + at_b);
+  plan->d_nr_c = reinterpret_cast<int64_t*>(d + at_c);
+  plan->d_jobsA = reinterpret_cast<PackJob*>(d + at_ja);
+  plan->d_jobsB = reinterpret_cast<PackJob*>(d + at_jb);
+  plan->d_tilesA = reinterpret_cast<PackTile*>(d + at_ta);
+  plan->d_tilesB = reinterpret_cast<PackTile*>(d + at_tb);
+  plan->d_pairtc = reinterpret_cast<PairTC*>(d + at_ptc);
+  plan->d_status = reinterpret_cast<int*>(d + at_status);
+  plan->d_tab = reinterpret_cast<int32_t*>(d + at_tab);
   cudaStream_t s = ctx->stream;
-  TT_CUDA(cudaMemsetAsync(plan->d_status, 0, sizeof(int), s));
   lap(3);
-  // staged copies: the host vectors may die at return without stalling the stream
-  if (dgemm) TT_CUDA(tt::h2d_async(ctx, plan->d_dtasks, dtasks.data(), sizeof(DTask) * dtasks.size()));
-  else TT_CUDA(tt::h2d_async(ctx, plan->d_tasks, tsorted.data(), sizeof(TaskDev) * tsorted.size()));
-  TT_CUDA(tt::h2d_async(ctx, plan->d_outs, ho.data(), sizeof(OutDev) * ho.size()));
-  TT_CUDA(tt::h2d_async(ctx, plan->d_pairs, hp.data(), sizeof(PairDev) * hp.size()));
-  TT_CUDA(tt::h2d_async(ctx, d_jobs, jobs.data(), sizeof(TableJob) * jobs.size()));
-  if (tc) {
-    TT_CUDA(tt::h2d_async(ctx, plan->d_jobsA, ja.data(), sizeof(PackJob) * ja.size()));
-    TT_CUDA(tt::h2d_async(ctx, plan->d_jobsB, jb.data(), sizeof(PackJob) * jb.size()));
-    TT_CUDA(tt::h2d_async(ctx, plan->d_tilesA, ta.data(), sizeof(PackTile) * ta.size()));
-    TT_CUDA(tt::h2d_async(ctx, plan->d_tilesB, tb.data(), sizeof(PackTile) * tb.size()));
-    TT_CUDA(tt::h2d_async(ctx, plan->d_pairtc, ptc.data(), sizeof(PairTC) * ptc.size()));
-  }
+  TT_CUDA(tt::h2d_async(ctx, d, blob.data(), blob.size()));
   if (!jobs.empty()) {
-    expand_tables<<<(unsigned)jobs.size(), 128, 0, s>>>(d_jobs, (int)jobs.size(), plan->d_tab);
+    expand_tables<<<(unsigned)jobs.size(), 128, 0, s>>>(reinterpret_cast<const TableJob*>(d + at_jobs), (int)jobs.size(),
+                                                        plan->d_tab);
     TT_LAUNCH_CHECK(ctx);
-  }
-  tt::pool_free(ctx, d_jobs);  // stream-ordered: freed after expand_tables ran
-  if (rs_ok && !rs_tasks.empty()) {
-    plan->d_rs_tasks = tt::pool_alloc<TaskDev>(ctx, rs_tasks.size());
-    plan->d_rs_chunks = tt::pool_alloc<RsChunk>(ctx, rs_chunks.size());
-    plan->d_rs_a = tt::pool_alloc<RsA>(ctx, rs_a.size());
-    plan->d_rs_e = tt::pool_alloc<RsE>(ctx, rs_e.size());
-    plan->d_rs_o = tt::pool_alloc<RsO>(ctx, rs_o.size());
-    if (plan->d_rs_tasks && plan->d_rs_chunks && plan->d_rs_a && plan->d_rs_e && plan->d_rs_o) {
-      TT_CUDA(tt::h2d_async(ctx, plan->d_rs_tasks, rs_tasks.data(), sizeof(TaskDev) * rs_tasks.size()));
-      TT_CUDA(tt::h2d_async(ctx, plan->d_rs_chunks, rs_chunks.data(), sizeof(RsChunk) * rs_chunks.size()));
-      TT_CUDA(tt::h2d_async(ctx, plan->d_rs_a, rs_a.data(), sizeof(RsA) * rs_a.size()));
-      TT_CUDA(tt::h2d_async(ctx, plan->d_rs_e, rs_e.data(), sizeof(RsE) * rs_e.size()));
-      TT_CUDA(tt::h2d_async(ctx, plan->d_rs_o, rs_o.data(), sizeof(RsO) * rs_o.size()));
-      plan->rs = true;
-      plan->rs_n_tasks = (int)rs_tasks.size();
-      plan->rs_ktot = rs_ktot;
-      int wmax = 1;
-      for (const RsChunk& c : rs_chunks) {
-        int w = 0;
-        for (int o = c.o_begin; o < c.o_end; ++o) w += outs[rs_o[o].out].n;
-        wmax = std::max(wmax, w);
-      }
-      plan->rs_nc = wmax;
-      plan->dev_bytes += (int64_t)(sizeof(TaskDev) * rs_tasks.size() + sizeof(RsChunk) * rs_chunks.size() +
-                                   sizeof(RsA) * rs_a.size() + sizeof(RsE) * rs_e.size() + sizeof(RsO) * rs_o.size());
-    }
   }
   *plan_out = plan;
   return TT_OK;
@@ -1500,40 +1544,21 @@ int tt_contract_exec_keep(tt_ctx* ctx, const tt_plan* plan, const double* A, con
   if (tt::first_on_device(attr_set, ctx->device)) {
     TT_CUDA(cudaFuncSetAttribute(grouped_dgemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)SMEM_BYTES));
+    TT_CUDA(cudaFuncSetAttribute(narrow_dgemm<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)narrow_smem(NR_KTOT, 8)));
+    TT_CUDA(cudaFuncSetAttribute(narrow_dgemm<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)narrow_smem(NR_KTOT, 32)));
     TT_CUDA(cudaFuncSetAttribute(grouped_tc_persist<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)TC_BULK_SMEM));
     TT_CUDA(cudaFuncSetAttribute(grouped_tc_persist<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)TC_BULK_SMEM));
   }
   if (plan->precision == TT_PREC_FP64) {
-    if (plan->rs) {
-      const int nc = plan->rs_nc <= 4 ? 4 : plan->rs_nc <= 8 ? 8 : plan->rs_nc <= 16 ? 16 : 32;
-      const size_t dyn = (size_t)(plan->rs_ktot * (int64_t)(nc * sizeof(double) + sizeof(int32_t)));
-      using RsFn = void (*)(const TaskDev*, const RsChunk*, const RsA*, const RsE*, const RsO*, const OutDev*,
-                            const PairDev*, const int32_t*, const double*, const double*, double*, double);
-      const int which = nc == 4 ? 0 : nc == 8 ? 1 : nc == 16 ? 2 : 3;
-      const RsFn fns[4] = {skinny_rs<4>, skinny_rs<8>, skinny_rs<16>, skinny_rs<32>};
-      static thread_local uint64_t rs_attr[4] = {0, 0, 0, 0};  // per instance, per host thread and device
-      if (tt::first_on_device(rs_attr[which], ctx->device))
-        TT_CUDA(cudaFuncSetAttribute(fns[which], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SK_STAGE_BYTES));
-      fns[which]<<<plan->rs_n_tasks, SK_ROWS, dyn, ctx->stream>>>(
-          plan->d_rs_tasks, plan->d_rs_chunks, plan->d_rs_a, plan->d_rs_e, plan->d_rs_o, plan->d_outs,
-          plan->d_pairs, plan->d_tab, A, B, C, alpha);
-    } else if (plan->skinny) {
-      const int nc = plan->skinny_nc <= 4 ? 4 : plan->skinny_nc <= 8 ? 8 : plan->skinny_nc <= 16 ? 16 : 32;
-      // every pair of a task staged at once when the widest task fits
-      const int64_t need = plan->skinny_ktot * (int64_t)(nc * sizeof(double) + sizeof(int32_t));
-      const bool staged = need <= SK_STAGE_BYTES;
-      const size_t dyn = staged ? (size_t)need : 0;
-      using SkinnyFn = void (*)(const TaskDev*, const OutDev*, const PairDev*, const int32_t*, const double*,
-                                const double*, double*, double, int);
-      const int which = nc == 4 ? 0 : nc == 8 ? 1 : nc == 16 ? 2 : 3;
-      const SkinnyFn fns[4] = {skinny_dgemm<4>, skinny_dgemm<8>, skinny_dgemm<16>, skinny_dgemm<32>};
-      static thread_local uint64_t attr[4] = {0, 0, 0, 0};  // per instance, per host thread and device
-      if (tt::first_on_device(attr[which], ctx->device))
-        TT_CUDA(cudaFuncSetAttribute(fns[which], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SK_STAGE_BYTES));
-      fns[which]<<<plan->n_tasks, SK_ROWS, dyn, ctx->stream>>>(plan->d_tasks, plan->d_outs, plan->d_pairs,
-                                                              plan->d_tab, A, B, C, alpha, staged ? 1 : 0);
+    if (plan->narrow) {
+      const auto fn = plan->nr_rw == 8 ? narrow_dgemm<8> : narrow_dgemm<32>;
+      fn<<<plan->n_tasks, NR_THREADS, narrow_smem(plan->nr_ktot, plan->nr_rw), ctx->stream>>>(
+          plan->d_nr_tasks, plan->d_nr_a, plan->d_nr_b, plan->d_nr_c, plan->d_tab, A, B, C, alpha,
+          narrow_buf(plan->nr_ktot, plan->nr_rw));
     } else {
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute at[1];
@@ -1547,7 +1572,7 @@ int tt_contract_exec_keep(tt_ctx* ctx, const tt_plan* plan, const double* A, con
       cfg.stream = ctx->stream;
       cfg.attrs = at;
       cfg.numAttrs = plan->split > 1 ? 1 : 0;
-      TT_CUDA(cudaLaunchKernelEx(&cfg, grouped_dgemm, (const DTask*)plan->d_dtasks, (const OutDev*)plan->d_outs,
+      TT_CUDA(cudaLaunchKernelEx(&cfg, grouped_dgemm, (const DTask*)plan->d_dtasks,
                                  (const PairDev*)plan->d_pairs, (const int32_t*)plan->d_tab, A, B, C, alpha,
                                  plan->split));
     }
@@ -1632,22 +1657,7 @@ int tt_plan_destroy(tt_ctx* ctx, tt_plan* plan) {
   if (!plan) return TT_OK;
   if (ctx) {
     tt_plan_release_packed(ctx, plan);
-    tt::pool_free(ctx, plan->d_tasks);
-    tt::pool_free(ctx, plan->d_dtasks);
-    tt::pool_free(ctx, plan->d_outs);
-    tt::pool_free(ctx, plan->d_pairs);
-    tt::pool_free(ctx, plan->d_tab);
-    tt::pool_free(ctx, plan->d_status);
-    tt::pool_free(ctx, plan->d_jobsA);
-    tt::pool_free(ctx, plan->d_jobsB);
-    tt::pool_free(ctx, plan->d_tilesA);
-    tt::pool_free(ctx, plan->d_tilesB);
-    tt::pool_free(ctx, plan->d_pairtc);
-    tt::pool_free(ctx, plan->d_rs_tasks);
-    tt::pool_free(ctx, plan->d_rs_chunks);
-    tt::pool_free(ctx, plan->d_rs_a);
-    tt::pool_free(ctx, plan->d_rs_e);
-    tt::pool_free(ctx, plan->d_rs_o);
+    tt::pool_free(ctx, plan->d_blob);
   }
   delete plan;
   return TT_OK;
