@@ -1697,6 +1697,7 @@ trsm_rows(const EigDev* __restrict__ probs, const VecTask* __restrict__ tasks, d
     const int pb = min(CH_PB, m - p0);
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     double rx[PER], rl[PER];
+    __syncthreads();  // the previous panel's columns, solved by the first warp, are read below
     if (p0 > 0) load(p0, pb, 0, rx, rl);
     for (int k0 = 0; k0 < p0; k0 += CH_PB) {
       __syncthreads();
