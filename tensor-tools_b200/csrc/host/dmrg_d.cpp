@@ -470,11 +470,18 @@ double tensor_davidson(big_dtensor& A, dtensor& x, int m, int max_restart, doubl
   for (int i = 0; i < max_restart; ++i) {
     for (int j = 0; j < m; ++j) {
       v[j] = x;
-      for (int k = j - 1; k >= 0; --k) {
-        double alpha = v[k].inner_product(v[j]);
-        v[j].add(v[k], -alpha);
-      }
-      v[j].normalize();
+      auto project = [&]() {
+        for (int k = j - 1; k >= 0; --k) {
+          double alpha = v[k].inner_product(v[j]);
+          v[j].add(v[k], -alpha);
+        }
+        return v[j].normalize();
+      };
+      // x is a unit vector: a small remainder is mostly the cancellation's
+      // rounding and has to be projected again, or the projected matrix belongs
+      // to a basis that is not orthonormal (a converged residual is nearly
+      // parallel to v[0]; the Ritz value then came out up to 5e-3 too high)
+      if (project() < 0.1 && j > 0) project();
       va[j] = A.product(v[j]);
       if (stats) stats->matvecs++;
       int l = j;
