@@ -3,23 +3,24 @@
 // the host can apply the truncation rule of :1290-1300), then eigenvectors
 // only for the states that are kept.
 //
-// Phase 1 (tt_sym_eigvals_batched), one CTA per sector:
-//   Householder reduction to tridiagonal form T = Q^T G Q (Golub & Van Loan,
-//   "Matrix Computations", 4th ed., alg. 8.3.1), reflectors kept below the
-//   subdiagonal of G; then every eigenvalue of T by bisection on Sturm
-//   sequence counts (ibid. sec. 8.4.1), one thread per eigenvalue.
-// Phase 2 (tt_sym_eigvecs_batched), one CTA per sector:
-//   inverse iteration on T - lambda I (tridiagonal LU with partial pivoting,
-//   tiny pivots replaced by eps*||T||), one thread per wanted eigenvector;
-//   classical Gram-Schmidt applied twice inside clusters of close eigenvalues
-//   (gap <= 1e-3 ||T||, the clustering rule of LAPACK's inverse iteration);
-//   back-transformation z = Q y with the stored reflectors.
-// The matrix sits in shared memory when n <= 160, otherwise in global memory.
+// Phase 1 (tt_sym_eigvals_batched): Householder reduction to tridiagonal form
+//   T = Q^T G Q (Golub & Van Loan, "Matrix Computations", 4th ed., alg. 8.3.1),
+//   reflectors kept below the subdiagonal of G -- sectors with n <= SN by one
+//   CTA each with the matrix in shared memory, larger ones by a cluster of CTAs;
+//   then every eigenvalue of every T by bisection on Sturm sequence counts
+//   (ibid. sec. 8.4.1), spread over the GPU.
+// Phase 2 (tt_sym_eigvecs_batched): inverse iteration on T - lambda I
+//   (tridiagonal LU with partial pivoting, tiny pivots replaced by eps*||T||),
+//   orthogonalisation inside clusters of close eigenvalues (gap <= 1e-3 ||T||,
+//   the clustering rule of LAPACK's inverse iteration) and back-transformation
+//   z = Q y with the stored reflectors -- one CTA per sector with n <= SN, GPU-wide
+//   kernels batched over the larger ones.
 #include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "tt_internal.h"
@@ -27,7 +28,8 @@
 namespace {
 
 constexpr int TT = 512;          // threads per CTA
-constexpr int SM_N = 160;        // full n x n FP64 matrix in shared memory up to this size
+constexpr int SN = 128;          // sectors up to this size: one CTA, matrix in shared memory
+constexpr int SB = SN / 32;      // row chunks of 32 of such a sector
 constexpr int MAX_N = 4096;
 constexpr int INV_ITERS = 3;
 
@@ -56,199 +58,222 @@ __device__ double block_reduce(double v, double* red, bool is_max) {
   return red[32];
 }
 
-// number of eigenvalues of T (diag d, squared offdiag e2) that are < x: the
-// sign changes of the Sturm sequence p_i = (d_i - x) p_{i-1} - e2_{i-1} p_{i-2}
-// of leading principal minors (Golub & Van Loan, "Matrix Computations", 4th
-// ed., sec. 8.4.1), counted as LAPACK's dlaebz counts the non-positive pivots
-// q_i = p_i / p_{i-1} of T - x I -- without its division per step: a pivot
-// with |q_i| <= pivmin is replaced by a tiny negative one (here p_i = -p_{i-1}
-// 2^-200, which steers the next step as q = -pivmin does), and the pair
-// (p_{i-1}, p_i) is rescaled by a power of two when p_i leaves [2^-400, 2^400]
-__device__ int sturm_count(const double* d, const double* e2, int n, double x, double pivmin) {
-  double pm = 1.0;
-  double p = d[0] - x;
-  if (fabs(p) <= pivmin) p = -pivmin;
-  int c = p <= 0.0;
-  for (int i = 1; i < n; ++i) {
-    double pn = fma(d[i] - x, p, -e2[i - 1] * pm);
-    if (fabs(pn) <= pivmin * fabs(p)) pn = -p * 0x1p-200;
-    c += (pn < 0.0) != (p < 0.0);
-    const double a = fabs(pn);
-    if (a > 0x1p400 || a < 0x1p-400) {
-      int ex;
-      frexp(pn, &ex);
-      const double sc = ldexp(1.0, -ex);
-      pn *= sc;
-      p *= sc;
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// number of eigenvalues of T that are < x: the sign changes of the Sturm
+// sequence p_i = (d_i - x) p_{i-1} - e2_{i-1} p_{i-2} of leading principal
+// minors (Golub & Van Loan, "Matrix Computations", 4th ed., sec. 8.4.1).
+// de[i] = (d_i, e2_{i-1}) of T scaled to a norm in [1/2, 1), padded to a
+// multiple of 8 with (4, 0), which keep the sign.  Off-diagonals are floored at
+// 2^-60 (their squares at STURM_E2), far below the rounding of T, so a vanishing
+// minor is followed by one of the opposite sign of the one before it and needs
+// no test of its own; a step then is one dependent FMA, and the pair (p_{i-1},
+// p_i), which shrinks by at most 2^-480 and grows by at most 3^8 over 8 steps,
+// is rescaled by a power of two every 8 steps when it has left 2^+-300.
+constexpr double STURM_E2 = 0x1p-120;
+__device__ __forceinline__ int sturm_count(const double2* de, int npad, double x) {
+  double pm = 0.0, p = 1.0;
+  int c = 0;
+  for (int i = 0; i < npad; i += 8) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const double2 t = de[i + u];
+      const double pn = fma(t.x - x, p, -(t.y * pm));
+      c += (unsigned)(__double2hiint(pn) ^ __double2hiint(p)) >> 31;
+      pm = p;
+      p = pn;
     }
-    pm = p;
-    p = pn;
+    const int ex = max(__double2hiint(p) & 0x7fffffff, __double2hiint(pm) & 0x7fffffff) >> 20;
+    if (ex > 1023 + 300 || ex < 1023 - 300) {
+      const double sc = __hiloint2double((2046 - ex) << 20, 0);
+      p *= sc;
+      pm *= sc;
+    }
   }
   return c;
 }
 
-__global__ void __launch_bounds__(TT)
-tridiag_eigvals(const EigDev* __restrict__ probs, double* G, double* Tg, double* W, const double* Amat) {
+// ---------------------------------------------------------------------------
+// Sectors with n <= SN: tridiagonalisation by one CTA, matrix in shared memory.
+//
+// A column costs two barriers.  Every warp forms the reflector v of column k
+// for itself (same data, same order: rows lane + 32 b in registers, a private
+// copy in shared memory for the column factors), then takes its share of the
+// trailing columns in one pass that applies the previous reflector's rank-2
+// update and accumulates A22 v of the new one, so the matrix is read and
+// written once per column.  After barrier 1 thread r sums row r of A22 v over
+// the warps; after barrier 2 every warp forms w on its own rows.
+//
+// Bound by the latency of that chain (square root, two reciprocals, two warp
+// sums, two barriers: 1.5 us a column), not by its shared-memory traffic.
+// Measured with the eigenvalues by the kernel below, against five barriers a
+// column, indices by division and a bisection per CTA: a block SVD at bond
+// dimension 75 (n <= 36) 153 -> 54 + 22 us, at 512 (n <= 75) 385 -> 127 us.  It
+// stops at 128: its working arrays and a 128 x 128 matrix take 197 KB.
+// doubles of shared memory
+__host__ __device__ constexpr int64_t small_smem(int n, int nw) { return (int64_t)n * n + 4 * (int64_t)nw * n + n; }
+constexpr int small_threads(int nmax) { return nmax <= 32 ? 256 : 512; }
+
+__global__ void __launch_bounds__(TT, 1)
+tridiag_small(const EigDev* __restrict__ probs, double* G, double* Tg, double* W, const double* Amat) {
   extern __shared__ double sm[];
-  __shared__ double red[33];
-  __shared__ double s_beta, s_tau, s_scale;
+  __shared__ double dots[SB], red[33];
+  // the cluster kernel that may follow reads nothing of this one's
+  asm volatile("griddepcontrol.launch_dependents;");
   const EigDev P = probs[blockIdx.x];
   const int n = P.n;
-  const int tid = threadIdx.x;
-  double* Wp = W + P.w_off;
-  double* dg = Tg + 3 * P.w_off;  // d[n], e[n], tau[n]
-  double* eg = dg + n;
-  double* tg = eg + n;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   if (n <= 0) return;
   if (P.flags & TT_EIG_ROW_1X2) {
     if (tid == 0) {
-      double a = Amat[P.a_off], b = Amat[P.a_off + 1];
-      Wp[0] = a * a + b * b;
-      Wp[1] = 0.0;
+      const double a = Amat[P.a_off], b = Amat[P.a_off + 1];
+      W[P.w_off] = a * a + b * b;
+      W[P.w_off + 1] = 0.0;
     }
     return;
   }
-  const bool in_smem = n <= SM_N;
+  double* dg = Tg + 3 * P.w_off;  // d[n], e[n], tau[n]
+  double* eg = dg + n;
+  double* tg = eg + n;
   double* Gp = G + P.g_off;
-  double* A = in_smem ? sm : Gp;
-  double* v = in_smem ? sm + SM_N * SM_N : sm;
-  double* p = v + n;
-  double* d = p + n;    // diag
-  double* e2 = d + n;   // offdiag squared
-  const int lda = n;
-  if (in_smem)
-    for (int i = tid; i < n * n; i += blockDim.x) A[i] = Gp[i];
-  __syncthreads();
-
-  for (int k = 0; k + 2 < n; ++k) {
-    const int m = n - k - 1;  // length of x = A[k+1:n, k]
-    double loc = 0.0;
-    for (int i = 1 + tid; i < m; i += blockDim.x) {
-      double t = A[(k + 1 + i) + lda * k];
-      loc += t * t;
-    }
-    const double sigma = block_reduce(loc, red, false);
-    if (tid == 0) {
-      double alpha = A[(k + 1) + lda * k];
-      if (sigma == 0.0) {
-        s_tau = 0.0;
-        s_beta = alpha;
-        s_scale = 0.0;
-      } else {
-        double mu = sqrt(alpha * alpha + sigma);
-        double beta = alpha <= 0.0 ? mu : -mu;
-        s_tau = (beta - alpha) / beta;
-        s_scale = 1.0 / (alpha - beta);
-        s_beta = beta;
-      }
-      tg[k] = s_tau;
-      eg[k] = s_beta;
-    }
-    __syncthreads();
-    const double tau = s_tau;
-    if (tau == 0.0) continue;  // column already reduced
-    // v = [1, x[1:] * scale]; keep v[1:] below the subdiagonal for phase 2
-    for (int i = tid; i < m; i += blockDim.x) {
-      double vi = (i == 0) ? 1.0 : A[(k + 1 + i) + lda * k] * s_scale;
-      v[i] = vi;
-      if (i > 0) A[(k + 1 + i) + lda * k] = vi;
-    }
-    __syncthreads();
-    // p = tau * A22 v, one warp per row (A22 symmetric: read the column)
-    const int warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
-    for (int r = warp; r < m; r += nw) {
-      const double* col = A + (k + 1) + lda * (k + 1 + r);
-      double s = 0.0;
-      for (int c = lane; c < m; c += 32) s += col[c] * v[c];
+  double* A = sm;                            // [n][n]
+  double* part = A + n * n;                  // [nw][n]: A22 v by warp
+  double* vold = part + nw * n + warp * n;   // this warp's copies: the previous v,
+  double* vnew = vold + nw * n;              // the new one,
+  double* wold = vnew + nw * n;              // and the previous w
+  double* ps = part + 4 * nw * n;            // [n]: p = tau A22 v
+  // squares of the entries must neither overflow nor vanish: a matrix far from
+  // 1 is scaled by a power of two (T is scaled back; the reflectors do not care)
+  double amax = 0.0;
+  for (int i = tid; i < n * n; i += blockDim.x) {
+    const double g = Gp[i];
+    A[i] = g;
+    amax = fmax(amax, fabs(g));
+  }
+  for (int i = lane; i < n; i += 32) vold[i] = wold[i] = 0.0;
+  amax = block_reduce(amax, red, true);
+  double isc = 1.0;
+  if (amax > 0.0 && isfinite(amax) && (amax < 0x1p-300 || amax > 0x1p300)) {
+    int ex;
+    frexp(amax, &ex);
+    ex = max(ex, -1000);
+    isc = ldexp(1.0, ex);
+    for (int i = tid; i < n * n; i += blockDim.x) A[i] = ldexp(A[i], -ex);
+  }
+  double vo[SB], wo[SB];  // the previous v, w on the rows lane + 32 b
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-      if (lane == 0) p[r] = tau * s;
-    }
-    __syncthreads();
-    loc = 0.0;
-    for (int i = tid; i < m; i += blockDim.x) loc += v[i] * p[i];
-    const double K = 0.5 * tau * block_reduce(loc, red, false);
-    for (int i = tid; i < m; i += blockDim.x) p[i] -= K * v[i];  // w
-    __syncthreads();
-    // A22 -= v w^T + w v^T
-    for (int e = tid; e < m * m; e += blockDim.x) {
-      int r = e % m, c = e / m;
-      A[(k + 1 + r) + lda * (k + 1 + c)] -= v[r] * p[c] + p[r] * v[c];
-    }
-    __syncthreads();
-  }
-  // T: diagonal, offdiagonal (the last one is A[n-1,n-2])
-  for (int i = tid; i < n; i += blockDim.x) {
-    double di = A[i + lda * i];
-    d[i] = di;
-    dg[i] = di;
-  }
-  if (tid == 0) {
-    if (n >= 2) eg[n - 2] = A[(n - 1) + lda * (n - 2)];
-    eg[n - 1] = 0.0;
-    tg[n - 1] = 0.0;
-    if (n >= 2) tg[n - 2] = 0.0;
-  }
+  for (int b = 0; b < SB; ++b) vo[b] = wo[b] = 0.0;
   __syncthreads();
-  for (int i = tid; i < n - 1; i += blockDim.x) e2[i] = eg[i] * eg[i];
-  if (in_smem) {  // phase 2 reads the reflectors from G
-    for (int i = tid; i < n * n; i += blockDim.x) Gp[i] = A[i];
-  }
-  __syncthreads();
-  // Gershgorin bounds and the pivot floor of the Sturm recurrence
-  double lo_loc = DBL_MAX, hi_loc = -DBL_MAX, e2max = 0.0;
-  for (int i = tid; i < n; i += blockDim.x) {
-    double r = (i > 0 ? fabs(eg[i - 1]) : 0.0) + (i < n - 1 ? fabs(eg[i]) : 0.0);
-    lo_loc = fmin(lo_loc, d[i] - r);
-    hi_loc = fmax(hi_loc, d[i] + r);
-    if (i < n - 1) e2max = fmax(e2max, e2[i]);
-  }
-  const double gu = block_reduce(hi_loc, red, true);
-  const double gl = -block_reduce(-lo_loc, red, true);
-  const double emax = block_reduce(e2max, red, true);
-  const double bnorm = fmax(fabs(gl), fabs(gu));
-  const double pivmin = DBL_MIN * fmax(1.0, emax);
-  const double atol = 4.0 * DBL_EPSILON * bnorm + 2.0 * pivmin;
-  if (bnorm == 0.0) {  // T == 0: every eigenvalue is exactly zero
-    for (int j = tid; j < n; j += blockDim.x) Wp[j] = 0.0;
-    return;
-  }
-  // Bisection for the j-th smallest eigenvalue, two levels per round: three
-  // lanes of a group evaluate the Sturm count at the midpoint and at the
-  // midpoints of both halves, so a round takes the same two steps (same
-  // points, same tests) as two rounds of plain bisection.
-  auto open_interval = [&](double lo, double hi) {
-    return hi - lo > fmax(atol, 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)));
-  };
-  const int lane = tid & 31, wid = tid >> 5, nwarp = blockDim.x >> 5;
-  const int grp = lane < 30 ? lane / 3 : 0, sub = lane % 3;
-  for (int base = wid * 10; base < n; base += nwarp * 10) {
-    const int j = base + grp;
-    const bool active = lane < 30 && j < n;
-    double lo = gl - atol, hi = gu + atol;
-    int it = 0;
-    bool work = active && open_interval(lo, hi);
-    while (__any_sync(0xffffffffu, work)) {
-      const double mid = 0.5 * (lo + hi), lm = 0.5 * (lo + mid), rm = 0.5 * (mid + hi);
-      const double x = sub == 0 ? mid : (sub == 1 ? lm : rm);
-      const int c = work ? sturm_count(d, e2, n, x, pivmin) : 0;
-      const int cm = __shfl_sync(0xffffffffu, c, 3 * grp);
-      const int cl = __shfl_sync(0xffffffffu, c, 3 * grp + 1);
-      const int cr = __shfl_sync(0xffffffffu, c, 3 * grp + 2);
-      if (work) {
-        const bool left = cm > j;
-        if (left) hi = mid; else lo = mid;
-        ++it;
-        if (it < 128 && open_interval(lo, hi)) {
-          const double x2 = left ? lm : rm;
-          if ((left ? cl : cr) > j) hi = x2; else lo = x2;
-          ++it;
+  for (int k = 0; k + 2 < n; ++k) {
+    // column k as the previous reflector leaves it, and its own reflector
+    const double vk = vold[k], wk = wold[k];
+    double x[SB], sig = 0.0;
+#pragma unroll
+    for (int b = 0; b < SB; ++b) {
+      const int r = lane + 32 * b;
+      x[b] = 0.0;
+      if (r >= k && r < n) x[b] = A[r + n * k] - vo[b] * wk - wo[b] * vk;
+      if (r >= k + 2) sig += x[b] * x[b];
+    }
+    const double sigma = warp_sum(sig);
+    auto row = [&](int i) {  // x of row i, to every lane
+      double t = x[0];
+#pragma unroll
+      for (int b = 1; b < SB; ++b)
+        if ((i >> 5) == b) t = x[b];
+      return __shfl_sync(0xffffffffu, t, i & 31);
+    };
+    const double dk = row(k), alpha = row(k + 1);
+    double tau = 0.0, beta = alpha, scale = 0.0;
+    if (sigma != 0.0) {
+      const double mu = sqrt(alpha * alpha + sigma);
+      beta = alpha <= 0.0 ? mu : -mu;
+      tau = (beta - alpha) / beta;
+      scale = 1.0 / (alpha - beta);
+    }
+    double vn[SB], pr[SB];
+#pragma unroll
+    for (int b = 0; b < SB; ++b) {
+      const int r = lane + 32 * b;
+      vn[b] = r == k + 1 ? 1.0 : (r >= k + 2 ? x[b] * scale : 0.0);
+      pr[b] = 0.0;
+      if (r < n) vnew[r] = vn[b];
+    }
+    __syncwarp();
+    for (int c = k + 1 + warp; c < n; c += nw) {
+      const double vc = vold[c], wc = wold[c], nc = vnew[c];
+      double* col = A + n * c;
+#pragma unroll
+      for (int b = 0; b < SB; ++b) {
+        const int r = lane + 32 * b;
+        if (r > k && r < n) {
+          const double t = fma(-wo[b], vc, fma(-vo[b], wc, col[r]));
+          col[r] = t;
+          pr[b] = fma(t, nc, pr[b]);
         }
-        work = it < 128 && open_interval(lo, hi);
       }
     }
-    if (active && sub == 0) Wp[n - 1 - j] = 0.5 * (lo + hi);  // descending order
+#pragma unroll
+    for (int b = 0; b < SB; ++b)
+      if (lane + 32 * b < n) part[warp * n + lane + 32 * b] = pr[b];
+    __syncthreads();  // 1
+    if (warp < SB) {
+      double p = 0.0, v = 0.0;
+      if (tid > k && tid < n) {
+        for (int w = 0; w < nw; ++w) p += part[w * n + tid];
+        p *= tau;
+        v = vnew[tid];
+        ps[tid] = p;
+      }
+      const double d = warp_sum(v * p);
+      if (lane == 0) dots[warp] = d;
+    }
+    if (warp == nw - 1) {  // the reflector, for phase 2, and T
+#pragma unroll
+      for (int b = 0; b < SB; ++b) {
+        const int r = lane + 32 * b;
+        if (r >= k + 2 && r < n) A[r + n * k] = vn[b];
+      }
+      if (lane == 0) {
+        dg[k] = dk * isc;
+        eg[k] = beta * isc;
+        tg[k] = tau;
+      }
+    }
+    __syncthreads();  // 2
+    double K = dots[0];
+#pragma unroll
+    for (int b = 1; b < SB; ++b) K += dots[b];
+    K *= 0.5 * tau;
+#pragma unroll
+    for (int b = 0; b < SB; ++b) {
+      const int r = lane + 32 * b;
+      vo[b] = vn[b];
+      wo[b] = r > k && r < n ? ps[r] - K * vn[b] : 0.0;
+      if (r < n) wold[r] = wo[b];
+    }
+    double* t = vold;
+    vold = vnew;
+    vnew = t;
+    __syncwarp();
   }
+  __syncthreads();
+  if (tid == 0) {  // the last 2 x 2 block
+    const int i = n - 2, j = n - 1;
+    if (n >= 2) {
+      dg[i] = (A[i + n * i] - 2.0 * vold[i] * wold[i]) * isc;
+      eg[i] = (A[j + n * i] - vold[j] * wold[i] - wold[j] * vold[i]) * isc;
+      tg[i] = 0.0;
+    }
+    dg[j] = (A[j + n * j] - 2.0 * vold[j] * wold[j]) * isc;
+    eg[j] = 0.0;
+    tg[j] = 0.0;
+  }
+  for (int i = tid; i < n * n; i += blockDim.x) Gp[i] = A[i];
 }
 
 // solve (T - lambda I) y = b in place (y holds b on entry); U holds 3n scratch
@@ -434,24 +459,68 @@ __device__ __forceinline__ double hash_unit(uint64_t z) {
   return (double)(z >> 11) * 0x1.0p-53 * 2.0 - 1.0;
 }
 
-__global__ void __launch_bounds__(TT)
-tridiag_eigvecs(const EigDev* __restrict__ probs, const double* G, const double* Tg, const double* W, double* Zg,
-                double* work, const double* Amat, int smem_cap) {
-  extern __shared__ double zsm[];  // n*nvec eigenvector block + n reflector, when they fit
+// ---------------------------------------------------------------------------
+// Eigenvectors of the sectors with n <= SN, one CTA each.
+//
+// (a) Inverse iteration, one thread per vector: T - lambda I is factored once
+//     (one reciprocal per step; the row exchange is kept in the last bit of the
+//     multiplier, which the factorisation itself uses too), the INV_ITERS solves
+//     then are substitutions only.
+// (b) Gram-Schmidt inside clusters, right-looking and twice: once vector j is
+//     final, every warp takes it out of its share of the later members, so a
+//     vector costs one barrier.  A vector that the first pass has left less than
+//     half of had collapsed onto earlier ones: it is iterated once more from its
+//     remainder and projected again.
+// (c) Back-transformation z = H_0 H_1 ... H_{n-3} y, four vectors at a time in a
+//     warp's registers, without barriers; then the gauge.
+// All three are chains of latencies.  Measured against a factorisation per solve,
+// Gram-Schmidt vector by vector with eight barriers each and two barriers per
+// reflector: at bond dimension 75 (n <= 36) 108 -> 52 us, at 512 (n <= 75) 282 ->
+// 116 us.
+// Solve with the factors of (T - lambda I): y = the solution for y * scale;
+// returns its squared norm.  Entry i of the factors is at [i * st].
+__device__ __forceinline__ double small_solve(int n, double scale, double* y, const double* u0, const double* u1,
+                                              const double* u2, const double* ml, int st) {
+  double bi = y[0] * scale;
+#pragma unroll 4
+  for (int i = 0; i + 1 < n; ++i) {
+    const double bn = y[i + 1] * scale, m = ml[i * st];
+    const bool sw = __double2loint(m) & 1;
+    const double top = sw ? bn : bi, low = sw ? bi : bn;
+    y[i] = top;
+    bi = fma(-m, top, low);
+  }
+  double x1 = 0.0, x2 = 0.0, ss = 0.0;
+  double s = bi;
+#pragma unroll 4
+  for (int i = n - 1; i >= 0; --i) {
+    if (i < n - 1) s = y[i] - u1[i * st] * x1 - u2[i * st] * x2;
+    const double xi = s * u0[i * st];
+    y[i] = xi;
+    ss = fma(xi, xi, ss);
+    x2 = x1;
+    x1 = xi;
+  }
+  return ss;
+}
+
+__host__ __device__ constexpr int64_t small_vec_smem(int n, int nvec) { return 4 * (int64_t)n + (int64_t)nvec * (n | 1); }
+
+__global__ void __launch_bounds__(TT, 1)
+eigvecs_small(const EigDev* __restrict__ probs, const double* G, const double* Tg, const double* W, double* Zg,
+              double* work, const double* Amat, int64_t cap) {
+  extern __shared__ double zsm[];
   __shared__ double red[33];
-  __shared__ double coef[MAX_N / 2];
-  __shared__ int cstart[MAX_N / 2];
+  __shared__ double coef[SN];
+  __shared__ unsigned begins[SB];  // bit j: vector j begins a cluster
+  // the GPU-wide kernel that may follow reads nothing of this one's
+  asm volatile("griddepcontrol.launch_dependents;");
   const EigDev P = probs[blockIdx.x];
-  const int n = P.n, nvec = P.nvec;
-  const int tid = threadIdx.x;
-  if (n <= 0 || nvec <= 0) return;
-  double* Zout = Zg + P.g_off;  // n x nvec, leading dimension n
-  // the iterations run on a shared-memory copy when it fits
-  const bool in_smem = (int64_t)n * nvec + n <= (int64_t)smem_cap;
-  double* Z = in_smem ? zsm : Zout;
-  double* vk = in_smem ? zsm + (int64_t)n * nvec : nullptr;
+  const int n = P.n, cnt = P.nvec;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  if (n <= 0 || cnt <= 0) return;
+  double* Zout = Zg + P.g_off;  // n x cnt, leading dimension n
   if (P.flags & TT_EIG_ROW_1X2) {
-    Z = Zout;
     if (tid == 0) {
       double a = Amat[P.a_off], b = Amat[P.a_off + 1];
       double dd = sqrt(a * a + b * b), z0, z1;
@@ -462,143 +531,249 @@ tridiag_eigvecs(const EigDev* __restrict__ probs, const double* G, const double*
       } else {
         z0 = z1 = 1.0 / sqrt(2.0);
       }
-      Z[0] = z0;
-      Z[1] = z1;
-      if (nvec > 1) {
-        Z[2] = -z1;
-        Z[3] = z0;
+      Zout[0] = z0;
+      Zout[1] = z1;
+      if (cnt > 1) {
+        Zout[2] = -z1;
+        Zout[3] = z0;
       }
     }
     return;
   }
-  const double* d = Tg + 3 * P.w_off;
-  const double* e = d + n;
-  const double* tau = e + n;
-  const double* lam = W + P.w_off;  // descending
+  const double* tau = Tg + 3 * P.w_off + 2 * n;
   const double* Gp = G + P.g_off;
-  // 3n scratch per eigenvector (3 n*n per problem in global memory), in shared
-  // memory after the eigenvectors and the reflector when it fits
-  const bool u_smem = in_smem && 4 * (int64_t)n * nvec + n <= (int64_t)smem_cap;
-  double* U = u_smem ? zsm + (int64_t)n * nvec + n : work + 3 * P.g_off;
-  // ||T||_1 for the pivot floor and the cluster tolerance
+  const int ld = n | 1;  // odd: the threads' vectors lie on different banks
+  double* d = zsm;
+  double* e = d + n;
+  double* lam = e + n;    // descending
+  double* Z = lam + 2 * n;  // [cnt][ld]
+  // the factors, per vector: in shared memory when they fit, else interleaved
+  // in the work area and (u2) in the output
+  const bool fits = small_vec_smem(n, cnt) + 4 * (int64_t)cnt * ld <= cap;
+  double* u0 = fits ? Z + (int64_t)cnt * ld : work + 3 * P.g_off;
+  double* u1 = u0 + (int64_t)cnt * (fits ? ld : n);
+  double* ml = u1 + (int64_t)cnt * (fits ? ld : n);
+  double* u2 = fits ? ml + (int64_t)cnt * ld : Zout;
+  const int st = fits ? 1 : cnt, sv = fits ? ld : 1;  // from entry to entry, from vector to vector
+  for (int i = tid; i < n; i += blockDim.x) {
+    d[i] = Tg[3 * P.w_off + i];
+    e[i] = i + 1 < n ? Tg[3 * P.w_off + n + i] : 0.0;
+    if (i < cnt) lam[i] = W[P.w_off + i];
+  }
+  __syncthreads();
   double loc = 0.0;
-  for (int i = tid; i < n; i += blockDim.x)
-    loc = fmax(loc, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < n ? fabs(e[i]) : 0.0));
-  const double tnorm = block_reduce(loc, red, true);
-  // pivot floor; a (numerically) zero T takes 1 so that b / tiny cannot overflow
-  const double tiny = tnorm > 1e-250 ? fmax(DBL_EPSILON * tnorm, DBL_MIN) : 1.0;
+  for (int i = tid; i < n; i += blockDim.x) loc = fmax(loc, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + fabs(e[i]));
+  double tnorm = block_reduce(loc, red, true);
+  if (tnorm > 0.0 && isfinite(tnorm)) {  // a norm in [1/2, 1), so that no solution overflows when it is squared
+    int ex;
+    frexp(tnorm, &ex);
+    tnorm = ldexp(tnorm, -ex);
+    for (int i = tid; i < n; i += blockDim.x) {
+      d[i] = ldexp(d[i], -ex);
+      e[i] = ldexp(e[i], -ex);
+      if (i < cnt) lam[i] = ldexp(lam[i], -ex);
+    }
+    __syncthreads();
+  }
+  // pivot floor; a zero T takes 1 so that b / tiny cannot overflow
+  const double tiny = tnorm > 0.0 ? DBL_EPSILON * tnorm : 1.0;
   const double ortol = 1e-3 * tnorm;
-  // (a) inverse iteration, one thread per eigenvector
-  for (int j = tid; j < nvec; j += blockDim.x) {
-    double* y = Z + (int64_t)n * j;
+  auto clamped = [&](double p) { return fabs(p) < tiny ? (p < 0.0 ? -tiny : tiny) : p; };
+  auto solve = [&](int j, double scale) {
+    return small_solve(n, scale, Z + (int64_t)ld * j, u0 + (int64_t)sv * j, u1 + (int64_t)sv * j, u2 + (int64_t)sv * j,
+                       ml + (int64_t)sv * j, st);
+  };
+  if (tid < SB * 32) {
+    const bool first = tid < cnt && (tid == 0 || lam[tid - 1] - lam[tid] > ortol);
+    const unsigned m = __ballot_sync(0xffffffffu, first);
+    if (lane == 0) begins[warp] = m;
+  }
+  // (a)
+  if (tid < cnt) {
+    const int j = tid;
+    double* y = Z + (int64_t)ld * j;
+    double* f0 = u0 + (int64_t)sv * j;
+    double* f1 = u1 + (int64_t)sv * j;
+    double* f2 = u2 + (int64_t)sv * j;
+    double* fm = ml + (int64_t)sv * j;
+    const double lj = lam[j];
+    double di = d[0] - lj, si = e[0];
+    for (int i = 0; i + 1 < n; ++i) {
+      const double ci = e[i], an = d[i + 1] - lj, bn = e[i + 1];
+      const bool sw = fabs(di) < fabs(ci);
+      if (!sw && di == 0.0) di = tiny;
+      const double piv = sw ? ci : di, r = 1.0 / piv;
+      double m = (sw ? di : ci) * r;
+      m = __hiloint2double(__double2hiint(m), (__double2loint(m) & ~1) | (sw ? 1 : 0));
+      f0[i * st] = fabs(piv) < tiny ? 1.0 / clamped(piv) : r;
+      f1[i * st] = sw ? an : si;
+      f2[i * st] = sw ? bn : 0.0;
+      fm[i * st] = m;
+      di = sw ? si - m * an : an - m * si;
+      si = sw ? -m * bn : bn;
+    }
+    f0[(n - 1) * st] = 1.0 / clamped(di);
+    f1[(n - 1) * st] = f2[(n - 1) * st] = 0.0;
     for (int i = 0; i < n; ++i) y[i] = hash_unit(((uint64_t)P.g_off << 20) ^ ((uint64_t)j << 32) ^ (uint64_t)i);
-    for (int it = 0; it < INV_ITERS; ++it) {
-      tri_solve(d, e, n, lam[j], tiny, y, U + (int64_t)3 * n * j, 1);
+    double scale = 1.0;
+    for (int it = 0; it < INV_ITERS; ++it) scale = 1.0 / sqrt(solve(j, scale));
+    for (int i = 0; i < n; ++i) y[i] *= scale;
+  }
+  __syncthreads();
+  // (b)
+  auto next_begin = [&](int j) {  // the first vector after j that begins a cluster (cnt: none)
+    for (int w = (j + 1) >> 5; w < SB; ++w) {
+      const unsigned m = begins[w] & (w == (j + 1) >> 5 ? 0xffffffffu << ((j + 1) & 31) : 0xffffffffu);
+      if (m) return 32 * w + __ffs(m) - 1;
+    }
+    return cnt;
+  };
+  auto dot = [&](const double* a, const double* b) {
+    double s = 0.0;
+    for (int i = lane; i < n; i += 32) s += a[i] * b[i];
+    return warp_sum(s);
+  };
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int c0 = 0; c0 < cnt;) {
+      const int c1 = next_begin(c0);
+      for (int j = c0; j < c1 && c1 - c0 > 1; ++j) {
+        double* y = Z + (int64_t)ld * j;
+        double nn = dot(y, y);  // every warp alike
+        if (pass == 0 && j > c0 && !(nn > 0.25)) {
+          for (int tries = 0; tries < 5; ++tries) {
+            __syncthreads();
+            if (tid == 0) {
+              const double nrm = sqrt(nn);
+              if (!(nrm > 0.0))
+                for (int i = 0; i < n; ++i) y[i] = hash_unit((uint64_t)(j * 7919 + i + tries));
+              solve(j, nrm > 0.0 ? 1.0 / nrm : 1.0);
+            }
+            __syncthreads();
+            for (int r = 0; r < 2; ++r) {
+              for (int k = c0 + warp; k < j; k += nw) {
+                const double* z = Z + (int64_t)ld * k;
+                const double q = dot(z, y) / dot(z, z);
+                if (lane == 0) coef[k] = q;
+              }
+              __syncthreads();
+              if (tid < n) {
+                double s = y[tid];
+                for (int k = c0; k < j; ++k) s -= coef[k] * Z[(int64_t)ld * k + tid];
+                y[tid] = s;
+              }
+              __syncthreads();
+            }
+            nn = dot(y, y);
+            if (nn > 0.25) break;
+          }
+          __syncthreads();
+          const double inv = nn > 0.0 ? 1.0 / sqrt(nn) : 0.0;
+          if (tid < n) y[tid] *= inv;
+          __syncthreads();
+          nn = dot(y, y);
+        }
+        if (j + 1 == c1) continue;
+        const double inv = nn > 0.0 ? 1.0 / nn : 0.0;
+        for (int k = j + 1 + warp; k < c1; k += nw) {
+          double* z = Z + (int64_t)ld * k;
+          const double q = dot(y, z) * inv;
+          for (int i = lane; i < n; i += 32) z[i] -= q * y[i];
+        }
+        __syncthreads();
+      }
+      c0 = c1;
+    }
+  }
+  __syncthreads();
+  // (c)
+  constexpr int VB = 4;
+  for (int t0 = VB * warp; t0 < cnt; t0 += VB * nw) {
+    double y[VB][SB];
+#pragma unroll
+    for (int u = 0; u < VB; ++u) {
       double s = 0.0;
-      for (int i = 0; i < n; ++i) s += y[i] * y[i];
-      double inv = 1.0 / sqrt(s);
-      for (int i = 0; i < n; ++i) y[i] *= inv;
-    }
-  }
-  // cluster starts: j begins a new cluster when lam[j-1] - lam[j] > ortol
-  if (tid == 0) {
-    int c = 0;
-    for (int j = 0; j < nvec; ++j) {
-      if (j == 0 || lam[j - 1] - lam[j] > ortol) c = j;
-      cstart[j < MAX_N / 2 ? j : MAX_N / 2 - 1] = c;
-    }
-  }
-  __syncthreads();
-  // (b) Gram-Schmidt twice against the earlier members of the cluster
-  for (int j = 1; j < nvec && j < MAX_N / 2; ++j) {
-    const int c0 = cstart[j];
-    if (c0 == j) continue;
-    double* y = Z + (int64_t)n * j;
-    for (int pass = 0; pass < 6; ++pass) {
-      for (int r = 0; r < 2; ++r) {
-        const int nk = j - c0;
-        const int warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
-        for (int k = warp; k < nk; k += nw) {
-          const double* yk = Z + (int64_t)n * (c0 + k);
-          double s = 0.0;
-          for (int i = lane; i < n; i += 32) s += yk[i] * y[i];
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-          if (lane == 0) coef[k] = s;
-        }
-        __syncthreads();
-        for (int i = tid; i < n; i += blockDim.x) {
-          double s = y[i];
-          for (int k = 0; k < nk; ++k) s -= coef[k] * Z[(int64_t)n * (c0 + k) + i];
-          y[i] = s;
-        }
-        __syncthreads();
+      for (int b = 0; b < SB; ++b) {
+        const int r = lane + 32 * b;
+        y[u][b] = t0 + u < cnt && r < n ? Z[(int64_t)ld * (t0 + u) + r] : 0.0;
+        s += y[u][b] * y[u][b];
       }
-      loc = 0.0;
-      for (int i = tid; i < n; i += blockDim.x) loc += y[i] * y[i];
-      double nrm = sqrt(block_reduce(loc, red, false));
-      if (nrm > 0.5 || pass == 5) {
-        double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
-        for (int i = tid; i < n; i += blockDim.x) y[i] *= inv;
-        __syncthreads();
-        break;
-      }
-      // the iterate had collapsed onto earlier vectors: one more inverse
-      // iteration from the orthogonal remainder, then orthogonalise again
-      if (tid == 0) {
-        double inv = nrm > 0.0 ? 1.0 / nrm : 1.0;
-        for (int i = 0; i < n; ++i) y[i] = nrm > 0.0 ? y[i] * inv : hash_unit((uint64_t)(j * 7919 + i + pass));
-        tri_solve(d, e, n, lam[j], tiny, y, U + (int64_t)3 * n * j, 1);
-      }
-      __syncthreads();
-    }
-  }
-  __syncthreads();
-  // (c) back-transformation z = H_0 H_1 ... H_{n-3} y, last reflector first
-  for (int k = n - 3; k >= 0; --k) {
-    const double tk = tau[k];
-    if (tk == 0.0) continue;
-    const int m = n - k - 1;
-    const int warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
-    const double* refl = Gp + (k + 1) + (int64_t)n * k;  // v[1:] = refl[1:], v[0] = 1
-    if (vk) {
-      for (int i = tid; i < m; i += blockDim.x) vk[i] = (i == 0) ? 1.0 : refl[i];
-      __syncthreads();
-      refl = vk;
-    }
-    for (int j = warp; j < nvec; j += nw) {
-      const double* y = Z + (int64_t)n * j + (k + 1);
-      double s = (lane == 0) ? y[0] : 0.0;  // v_0 = 1
-      for (int i = 1 + lane; i < m; i += 32) s += refl[i] * y[i];
+      s = warp_sum(s);
+      const double inv = s > 0.0 ? 1.0 / sqrt(s) : 0.0;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-      if (lane == 0) coef[j] = tk * s;
+      for (int b = 0; b < SB; ++b) y[u][b] *= inv;
     }
-    __syncthreads();
-    for (int el = tid; el < m * nvec; el += blockDim.x) {
-      int i = el % m, j = el / m;
-      double vi = (i == 0) ? 1.0 : refl[i];
-      Z[(int64_t)n * j + k + 1 + i] -= vi * coef[j];
+    double vnx[SB], tnx = 0.0;  // the next reflector, loaded one step ahead
+    auto load = [&](int k) {
+#pragma unroll
+      for (int b = 0; b < SB; ++b) {
+        const int r = lane + 32 * b;
+        vnx[b] = k >= 0 && r >= k + 1 && r < n ? (r == k + 1 ? 1.0 : Gp[r + n * k]) : 0.0;
+      }
+      tnx = k >= 0 ? tau[k] : 0.0;
+    };
+    load(n - 3);
+    for (int k = n - 3; k >= 0; --k) {
+      double v[SB];
+#pragma unroll
+      for (int b = 0; b < SB; ++b) v[b] = vnx[b];
+      const double tk = tnx;
+      load(k - 1);
+      double s[VB];
+#pragma unroll
+      for (int u = 0; u < VB; ++u) {
+        s[u] = 0.0;
+#pragma unroll
+        for (int b = 0; b < SB; ++b) s[u] = fma(v[b], y[u][b], s[u]);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < VB; ++u) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+#pragma unroll
+      for (int u = 0; u < VB; ++u)
+#pragma unroll
+        for (int b = 0; b < SB; ++b) y[u][b] = fma(-tk * s[u], v[b], y[u][b]);
     }
-    __syncthreads();
-  }
-  // deterministic gauge: the largest-magnitude entry of each vector is positive
-  for (int j = tid; j < nvec; j += blockDim.x) {
-    double* y = Z + (int64_t)n * j;
-    int imax = 0;
-    for (int i = 1; i < n; ++i)
-      if (fabs(y[i]) > fabs(y[imax])) imax = i;
-    if (y[imax] < 0.0)
-      for (int i = 0; i < n; ++i) y[i] = -y[i];
-  }
-  if (in_smem) {
-    __syncthreads();
-    for (int64_t i = tid; i < (int64_t)n * nvec; i += blockDim.x) Zout[i] = Z[i];
+    // deterministic gauge: the largest-magnitude entry (first on ties) is positive
+#pragma unroll
+    for (int u = 0; u < VB; ++u) {
+      double best = -1.0;
+      int bi = n;
+      bool neg = false;
+#pragma unroll
+      for (int b = 0; b < SB; ++b) {
+        const int r = lane + 32 * b;
+        const double m = fabs(y[u][b]);
+        if (r < n && m > best) {
+          best = m;
+          bi = r;
+          neg = y[u][b] < 0.0;
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        const bool on = __shfl_xor_sync(0xffffffffu, (int)neg, o);
+        if (ob > best || (ob == best && oi < bi)) {
+          best = ob;
+          bi = oi;
+          neg = on;
+        }
+      }
+      if (t0 + u < cnt)
+#pragma unroll
+        for (int b = 0; b < SB; ++b) {
+          const int r = lane + 32 * b;
+          if (r < n) Zout[r + (int64_t)n * (t0 + u)] = neg ? -y[u][b] : y[u][b];
+        }
+    }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Sectors with n > SM_N: one thread-block cluster (CL CTAs, distributed shared
+// Sectors with n > SN: one thread-block cluster (CL CTAs, distributed shared
 // memory) per sector, so a large density matrix is reduced by CL SMs at once
 // instead of one SM streaming it from L2.
 //
@@ -686,12 +861,6 @@ __device__ __forceinline__ int first_owned(int from, int rank, int CL) {
   return from <= rank ? 0 : (from - rank + CL - 1) / CL;
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // acc[k] (k < 16) summed over the 32 lanes of the warp, lane L receiving the
 // sum of index L % 16: a butterfly sum across the half-warps, then a
 // reduce-scatter (31 shuffles for 16 sums)
@@ -727,7 +896,6 @@ tridiag_eigvals_cluster(const EigDev* __restrict__ probs, double* G, double* Tg,
   if (n <= 0) return;  // the same problem for the whole cluster
   const int nb = P.nb;
   double* Gp = G + P.g_off;
-  double* Wp = W + P.w_off;
   double* dg = Tg + 3 * P.w_off;
   double* eg = dg + n;
   double* tg = eg + n;
@@ -1098,19 +1266,23 @@ tridiag_eigvals_cluster(const EigDev* __restrict__ probs, double* G, double* Tg,
   }
   __threadfence();
   cluster.sync();  // also the last access of another CTA's shared memory
+  // launched alongside tridiag_small: complete only when that is
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Bisection for the cluster-sized sectors after their tridiagonalisation,
-// spread over the GPU: a CTA of BS_THREADS threads takes BS_PER eigenvalues
-// of one problem, with the problem's d and e^2 in shared memory.  Sixteen
-// lanes serve one eigenvalue: in a round they count at the 15 points that
-// four successive halvings of the current interval can probe (the nodes of a
-// four-level bisection tree, each computed by the same chain of midpoints
-// that plain bisection would compute), then every lane of the group walks
-// the tree with the shared counts.  The intervals, the stopping rule and so
-// the eigenvalues are bit for bit those of plain bisection; a round advances
-// four halvings instead of one, so an eigenvalue takes about 13 rounds of
-// Sturm chains instead of 50.
+// Bisection for every sector after its tridiagonalisation, spread over the
+// GPU: a CTA of BS_THREADS threads takes BS_PER eigenvalues of one problem, with
+// the problem's d and e^2 in shared memory, scaled by a power of two to a norm in
+// [1/2, 1).  Sixteen lanes serve one eigenvalue: in a round they count at the 15
+// points that four successive halvings of the current interval can probe (the
+// nodes of a four-level bisection tree, each computed by the same chain of
+// midpoints that plain bisection would compute), then every lane of the group
+// walks the tree with the shared counts.  The intervals and the stopping rule
+// are those of plain bisection; a round advances four halvings instead of one,
+// so an eigenvalue takes about 13 rounds of Sturm chains instead of 50.
+// Bound by the FP64 pipe where there are many eigenvalues (three operations a
+// step and lane), by the chain of FMAs where there are few.  All sectors of a
+// block SVD at bond dimension 3072: 1977 (those above 160 only) -> 626 us.
 constexpr int BS_THREADS = 128;
 constexpr int BS_LANES = 16;  // lanes per eigenvalue: 15 probes, one idle
 constexpr int BS_LEVELS = 4;  // halvings per round
@@ -1127,30 +1299,34 @@ bisect_sectors(const EigDev* __restrict__ probs, const VecTaskB* __restrict__ ta
   const double* eg = dg + n;
   double* Wp = W + P.w_off;
   const int tid = threadIdx.x, lane = tid & 31;
-  double* d = bs_sm;
-  double* e2 = bs_sm + n;
-  for (int i = tid; i < n; i += blockDim.x) {
-    d[i] = dg[i];
-    e2[i] = i < n - 1 ? eg[i] * eg[i] : 0.0;
-  }
-  __syncthreads();
-  double lo_loc = DBL_MAX, hi_loc = -DBL_MAX, e2max = 0.0;
+  double2* de = reinterpret_cast<double2*>(bs_sm);
+  const int npad = (n + 7) & ~7;
+  // Gershgorin bounds
+  double lo_loc = DBL_MAX, hi_loc = -DBL_MAX;
   for (int i = tid; i < n; i += blockDim.x) {
     const double r = (i > 0 ? fabs(eg[i - 1]) : 0.0) + (i < n - 1 ? fabs(eg[i]) : 0.0);
-    lo_loc = fmin(lo_loc, d[i] - r);
-    hi_loc = fmax(hi_loc, d[i] + r);
-    if (i < n - 1) e2max = fmax(e2max, e2[i]);
+    lo_loc = fmin(lo_loc, dg[i] - r);
+    hi_loc = fmax(hi_loc, dg[i] + r);
   }
-  const double gu = block_reduce(hi_loc, red, true);
-  const double gl = -block_reduce(-lo_loc, red, true);
-  const double emax = block_reduce(e2max, red, true);
-  const double bnorm = fmax(fabs(gl), fabs(gu));
-  const double pivmin = DBL_MIN * fmax(1.0, emax);
-  const double atol = 4.0 * DBL_EPSILON * bnorm + 2.0 * pivmin;
-  if (bnorm == 0.0) {
-    for (int j = tk.j0 + tid; j < min(n, tk.j0 + BS_PER); j += blockDim.x) Wp[n - 1 - j] = 0.0;
+  double gu = block_reduce(hi_loc, red, true);
+  double gl = -block_reduce(-lo_loc, red, true);
+  double bnorm = fmax(fabs(gl), fabs(gu));
+  if (!(bnorm > 0.0) || !isfinite(bnorm)) {  // T == 0: every eigenvalue is exactly zero (not finite: passed on)
+    for (int j = tk.j0 + tid; j < min(n, tk.j0 + BS_PER); j += blockDim.x) Wp[n - 1 - j] = bnorm;
     return;
   }
+  int ex;
+  frexp(bnorm, &ex);
+  const double sc = ldexp(1.0, -max(ex, -1000)), isc = ldexp(1.0, max(ex, -1000));
+  gu *= sc;
+  gl *= sc;
+  bnorm *= sc;
+  for (int i = tid; i < npad; i += blockDim.x) {
+    const double ei = i > 0 && i < n ? eg[i - 1] * sc : 0.0;
+    de[i] = i < n ? make_double2(dg[i] * sc, i > 0 ? fmax(ei * ei, STURM_E2) : 0.0) : make_double2(4.0, 0.0);
+  }
+  __syncthreads();
+  const double atol = 4.0 * DBL_EPSILON * bnorm;
   auto open_interval = [&](double lo, double hi) {
     return hi - lo > fmax(atol, 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)));
   };
@@ -1174,7 +1350,7 @@ bisect_sectors(const EigDev* __restrict__ probs, const VecTaskB* __restrict__ ta
         if (p < pos) { b = m; pos -= half; } else { a = m; pos += half; }
         half >>= 1;
       }
-      c = sturm_count(d, e2, n, 0.5 * (a + b), pivmin);
+      c = sturm_count(de, npad, 0.5 * (a + b));
     }
     // every lane of the group walks the same path with the group's counts
     int pos = ROOT, half = ROOT >> 1;
@@ -1192,7 +1368,7 @@ bisect_sectors(const EigDev* __restrict__ probs, const VecTaskB* __restrict__ ta
     }
     if (work) work = it < 128 && open_interval(lo, hi);
   }
-  if (active && sub == 0) Wp[n - 1 - j] = 0.5 * (lo + hi);
+  if (active && sub == 0) Wp[n - 1 - j] = 0.5 * (lo + hi) * isc;
 }
 
 __global__ void __launch_bounds__(TT)
@@ -1511,6 +1687,8 @@ inv_iter_batched(const EigDev* __restrict__ probs, const VecTask* __restrict__ t
     }
     for (; i < n; ++i) z[i] = y[(int64_t)i * cnt] * inv;
   }
+  // launched alongside eigvecs_small: complete only when that is
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // (2a) Gram matrix, lower 64 x 64 tiles (a >= b): G[r + m c] = sum_i Z[i, r] Z[i, c],
@@ -1924,16 +2102,15 @@ std::vector<EigDev> to_dev(const tt_eig_problem* probs, int n_probs, const int* 
   return hp;
 }
 
-size_t vals_smem() { return sizeof(double) * ((size_t)SM_N * SM_N + 4 * (size_t)SM_N); }
-constexpr int64_t kVecsSmemCap = 25 * 1024;  // doubles (200 KB) of eigenvectors + reflector in shared memory
+constexpr int64_t kVecsSmemCap = 28 * 1024;  // doubles (224 KB) of dynamic shared memory of eigvecs_small
 
-// Sectors above the shared-memory size of the one-CTA kernels go to the cluster kernels.
-bool is_big(const EigDev& e) { return e.n > SM_N && !(e.flags & TT_EIG_ROW_1X2); }
+// Sectors above the size of the one-CTA kernels go to the cluster kernels.
+bool is_big(const EigDev& e) { return e.n > SN && !(e.flags & TT_EIG_ROW_1X2); }
 
 // Cluster size and shared-memory caps of the cluster kernels on this thread's
 // device: 16 CTAs per cluster when the device can co-schedule that many with
-// the full shared-memory carve-out, else 8, else none (the one-CTA kernels
-// take every problem).
+// the full shared-memory carve-out, else 8, else none (an error for sectors that
+// need them).
 struct ClusterPlan {
   int device = -1;
   int cl = 0;
@@ -2004,25 +2181,42 @@ const ClusterPlan& cluster_plan(tt_ctx* ctx) {
   return cp;
 }
 
-// One cluster of `cl` CTAs per problem; `need` doubles of dynamic shared memory.
+// A launch in clusters of `cl` CTAs (0: none) with `smem` bytes of dynamic
+// shared memory.  With `beside` it may start while the launch before it still
+// runs (that one says so, and this one ends with a wait for it).
 template <class... Args>
-cudaError_t launch_cluster(tt_ctx* ctx, int cl, int n_probs, int64_t need, const void* kernel, Args... args) {
+cudaError_t launch(tt_ctx* ctx, int grid, int block, int cl, size_t smem, bool beside, const void* kernel,
+                   Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = cl;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)(cl * n_probs));
-  cfg.blockDim = dim3(TT);
-  cfg.dynamicSmemBytes = (size_t)(need * 8);
+  cudaLaunchAttribute at[2];
+  unsigned na = 0;
+  if (cl > 0) {
+    at[na].id = cudaLaunchAttributeClusterDimension;
+    at[na].val.clusterDim.x = cl;
+    at[na].val.clusterDim.y = 1;
+    at[na++].val.clusterDim.z = 1;
+  }
+  if (beside) {
+    at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[na++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = na;
   void* argv[] = {(void*)&args...};
   const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, argv);
   tt::count_launch(ctx);
   return e;
+}
+
+// One cluster of `cl` CTAs per problem; `need` doubles of dynamic shared memory.
+template <class... Args>
+cudaError_t launch_cluster(tt_ctx* ctx, int cl, int n_probs, int64_t need, bool beside, const void* kernel,
+                           Args... args) {
+  return launch(ctx, cl * n_probs, TT, cl, (size_t)(need * 8), beside, kernel, args...);
 }
 
 }  // namespace
@@ -2040,25 +2234,18 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
   }
   std::vector<EigDev> all = to_dev(probs, n_probs, nullptr);
   const ClusterPlan& cp = cluster_plan(ctx);
-  std::vector<EigDev> small, big;
-  for (const EigDev& e : all) (cp.cl > 0 && is_big(e) ? big : small).push_back(e);
-  EigDev* dp = tt::pool_alloc<EigDev>(ctx, all.size());
-  if (!dp) return tt::fail(TT_ERR_OOM, "tt_sym_eigvals_batched: allocation failed");
-  small.insert(small.end(), big.begin(), big.end());  // small problems first, then the cluster ones
-  TT_CUDA(tt::h2d_async(ctx, dp, small.data(), sizeof(EigDev) * small.size()));
-  const int n_small = (int)(small.size() - big.size());
-  static thread_local uint64_t attr = 0;  // per host thread and device
-  if (tt::first_on_device(attr, ctx->device))
-    TT_CUDA(cudaFuncSetAttribute(tridiag_eigvals, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vals_smem()));
-  if (n_small > 0) {
-    tridiag_eigvals<<<n_small, TT, vals_smem(), ctx->stream>>>(dp, G, T, w, A);
-    TT_LAUNCH_CHECK(ctx);
+  std::vector<EigDev> hp, big;  // small problems first, then the cluster ones
+  int nsmall_max = 1;
+  for (const EigDev& e : all) {
+    (is_big(e) ? big : hp).push_back(e);
+    if (!is_big(e)) nsmall_max = std::max(nsmall_max, e.n);
   }
-  double* vw = nullptr;
+  const int n_small = (int)hp.size();
+  int64_t need = 0, scratch = 0;
   if (!big.empty()) {
+    TT_REQUIRE(cp.cl > 0, "tt_sym_eigvals_batched: no thread-block clusters for sectors of this size");
     // panel width per problem: the widest whose shared memory fits; the
     // panel scratch (n x 2nb per problem) lives in the pool
-    int64_t need = 0, scratch = 0;
     for (EigDev& e : big) {
       e.nb = PNB_MAX;
       while (e.nb > 8 && blocked_smem(e.n, e.nb, cp.cl) > cp.vals_cap) e.nb /= 2;
@@ -2067,32 +2254,49 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
       scratch += (int64_t)e.n * 2 * e.nb;
     }
     TT_REQUIRE(need <= cp.vals_cap, "tt_sym_eigvals_batched: sector too large for the cluster eigensolver");
-    vw = tt::pool_alloc<double>(ctx, (size_t)scratch);
-    if (!vw) return tt::fail(TT_ERR_OOM, "tt_sym_eigvals_batched: allocation failed");
-    TT_CUDA(tt::h2d_async(ctx, dp + n_small, big.data(), sizeof(EigDev) * big.size()));
-    TT_CUDA(launch_cluster(ctx, cp.cl, (int)big.size(), need, (const void*)tridiag_eigvals_cluster,
+  }
+  hp.insert(hp.end(), big.begin(), big.end());
+  // every sector's eigenvalues, BS_PER per CTA over the whole GPU
+  std::vector<VecTaskB> bt;
+  int nmax = 1;
+  for (int p = 0; p < (int)hp.size(); ++p) {
+    if (hp[p].flags & TT_EIG_ROW_1X2) continue;
+    nmax = std::max(nmax, hp[p].n);
+    for (int j0 = 0; j0 < hp[p].n; j0 += BS_PER) bt.push_back(VecTaskB{p, j0});
+  }
+  // problems, bisection tasks and the panel scratch in one buffer
+  const size_t pb = sizeof(EigDev) * hp.size(), tb = (sizeof(VecTaskB) * bt.size() + 15) & ~(size_t)15;
+  std::vector<char> host(pb + tb);
+  std::memcpy(host.data(), hp.data(), pb);
+  if (!bt.empty()) std::memcpy(host.data() + pb, bt.data(), sizeof(VecTaskB) * bt.size());
+  char* buf = tt::pool_alloc<char>(ctx, pb + tb + sizeof(double) * (size_t)scratch);
+  if (!buf) return tt::fail(TT_ERR_OOM, "tt_sym_eigvals_batched: allocation failed");
+  TT_CUDA(tt::h2d_async(ctx, buf, host.data(), host.size()));
+  const EigDev* dp = reinterpret_cast<const EigDev*>(buf);
+  const VecTaskB* d_bt = reinterpret_cast<const VecTaskB*>(buf + pb);
+  double* vw = reinterpret_cast<double*>(buf + pb + tb);
+  static thread_local uint64_t attr = 0;  // per host thread and device
+  if (tt::first_on_device(attr, ctx->device)) {
+    TT_CUDA(cudaFuncSetAttribute(tridiag_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double) * small_smem(SN, TT / 32))));
+    TT_CUDA(cudaFuncSetAttribute(bisect_sectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double2) * MAX_N)));
+  }
+  if (n_small > 0) {
+    const int threads = small_threads(nsmall_max);
+    tridiag_small<<<n_small, threads, sizeof(double) * (size_t)small_smem(nsmall_max, threads / 32), ctx->stream>>>(
+        dp, G, T, w, A);
+    TT_LAUNCH_CHECK(ctx);
+  }
+  if (!big.empty())
+    TT_CUDA(launch_cluster(ctx, cp.cl, (int)big.size(), need, n_small > 0, (const void*)tridiag_eigvals_cluster,
                            dp + n_small, G, T, w, vw));
-    // their eigenvalues, BS_PER per CTA over the whole GPU
-    std::vector<VecTaskB> bt;
-    int nmax = 0;
-    for (size_t b = 0; b < big.size(); ++b) {
-      nmax = std::max(nmax, big[b].n);
-      for (int j0 = 0; j0 < big[b].n; j0 += BS_PER) bt.push_back(VecTaskB{n_small + (int32_t)b, j0});
-    }
-    VecTaskB* d_bt = tt::pool_alloc<VecTaskB>(ctx, bt.size());
-    if (!d_bt) return tt::fail(TT_ERR_OOM, "tt_sym_eigvals_batched: allocation failed");
-    TT_CUDA(tt::h2d_async(ctx, d_bt, bt.data(), sizeof(VecTaskB) * bt.size()));
-    const size_t bs_smem = sizeof(double) * 2 * (size_t)nmax;
-    static thread_local uint64_t bs_attr = 0;
-    if (tt::first_on_device(bs_attr, ctx->device))
-      TT_CUDA(cudaFuncSetAttribute(bisect_sectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(sizeof(double) * 2 * MAX_N)));
+  if (!bt.empty()) {
+    const size_t bs_smem = sizeof(double2) * (size_t)((nmax + 7) & ~7);
     bisect_sectors<<<(unsigned)bt.size(), BS_THREADS, bs_smem, ctx->stream>>>(dp, d_bt, T, w);
     TT_LAUNCH_CHECK(ctx);
-    tt::pool_free(ctx, d_bt);
   }
-  tt::pool_free(ctx, vw);
-  tt::pool_free(ctx, dp);
+  tt::pool_free(ctx, buf);
   return TT_OK;
 }
 
@@ -2120,74 +2324,77 @@ int tt_sym_eigvecs_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
   }
   std::vector<EigDev> all = to_dev(probs, n_probs, nvec);
   const ClusterPlan& cp = cluster_plan(ctx);
-  std::vector<EigDev> small, big;
-  for (const EigDev& e : all) (cp.cl > 0 && is_big(e) ? big : small).push_back(e);
-  EigDev* dp = tt::pool_alloc<EigDev>(ctx, all.size());
-  if (!dp) return tt::fail(TT_ERR_OOM, "tt_sym_eigvecs_batched: allocation failed");
-  const int n_small = (int)small.size();
-  small.insert(small.end(), big.begin(), big.end());
-  TT_CUDA(tt::h2d_async(ctx, dp, small.data(), sizeof(EigDev) * small.size()));
-  // shared memory for the largest problem that fits (the others iterate in global memory)
+  std::vector<EigDev> hp, big;  // small problems first, then the cluster ones
+  int nsmall_max = 1;
+  for (const EigDev& e : all) {
+    (is_big(e) ? big : hp).push_back(e);
+    if (!is_big(e)) nsmall_max = std::max(nsmall_max, e.n);
+  }
+  TT_REQUIRE(big.empty() || cp.cl > 0, "tt_sym_eigvecs_batched: no thread-block clusters for sectors of this size");
+  const int n_small = (int)hp.size(), nbig = (int)big.size();
+  hp.insert(hp.end(), big.begin(), big.end());
+  std::vector<VecTask> iv, ts, ap;
+  std::vector<TileTask> gm, wy;
+  for (int p = 0; p < nbig; ++p) {
+    const EigDev& e = big[p];
+    for (int j = 0; j < e.nvec; j += IV_THREADS) iv.push_back(VecTask{p, j});
+    const int nt = (e.nvec + GT - 1) / GT;
+    for (int a = 0; a < nt; ++a)
+      for (int b = 0; b <= a; ++b) gm.push_back(TileTask{p, a, b});
+    if (e.nvec > 0) {
+      for (int i = 0; i < e.n; i += TS_ROWS) ts.push_back(VecTask{p, i});
+      for (int k = 0; k * BT_NB < e.n - 2; ++k) wy.push_back(TileTask{p, k, 0});
+      for (int j = 0; j < e.nvec; j += BT_VB) ap.push_back(VecTask{p, j});
+    }
+  }
+  // problems, task lists and the (zero) flags in one buffer, one copy
+  std::vector<char> host;
+  auto put = [&](const auto& v) {
+    const size_t at = host.size();
+    host.resize((at + v.size() * sizeof(v[0]) + 15) & ~(size_t)15);
+    if (!v.empty()) std::memcpy(host.data() + at, v.data(), v.size() * sizeof(v[0]));
+    return at;
+  };
+  put(hp);
+  const size_t at_iv = put(iv), at_ts = put(ts), at_ap = put(ap), at_gm = put(gm), at_wy = put(wy);
+  const size_t at_flags = put(std::vector<int>((size_t)nbig + 1, 0));
+  char* buf = tt::pool_alloc<char>(ctx, host.size());
+  if (!buf) return tt::fail(TT_ERR_OOM, "tt_sym_eigvecs_batched: allocation failed");
+  TT_CUDA(tt::h2d_async(ctx, buf, host.data(), host.size()));
+  const EigDev* dp = reinterpret_cast<const EigDev*>(buf);
+  const EigDev* db = dp + n_small;
+  const VecTask* d_iv = reinterpret_cast<const VecTask*>(buf + at_iv);
+  const VecTask* d_ts = reinterpret_cast<const VecTask*>(buf + at_ts);
+  const VecTask* d_ap = reinterpret_cast<const VecTask*>(buf + at_ap);
+  const TileTask* d_gm = reinterpret_cast<const TileTask*>(buf + at_gm);
+  const TileTask* d_wy = reinterpret_cast<const TileTask*>(buf + at_wy);
+  int* flags = reinterpret_cast<int*>(buf + at_flags);
+  // shared memory for the largest problem whose factors fit, or its vectors alone
   int64_t need = 0;
   for (int i = 0; i < n_small; ++i) {
-    const EigDev& e = small[i];
-    const int64_t with_u = 4 * (int64_t)e.n * e.nvec + e.n;  // Z, reflector and LU scratch
-    const int64_t z_only = (int64_t)e.n * e.nvec + e.n;
-    if (with_u <= kVecsSmemCap) need = std::max(need, with_u);
-    else if (z_only <= kVecsSmemCap) need = std::max(need, z_only);
+    const EigDev& e = hp[i];
+    const int64_t vecs = small_vec_smem(e.n, e.nvec), all5 = vecs + 4 * (int64_t)e.nvec * (e.n | 1);
+    need = std::max(need, all5 <= kVecsSmemCap ? all5 : vecs);
   }
   static thread_local uint64_t attr = 0;  // per host thread and device
   if (tt::first_on_device(attr, ctx->device))
-    TT_CUDA(cudaFuncSetAttribute(tridiag_eigvecs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    TT_CUDA(cudaFuncSetAttribute(eigvecs_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(double) * kVecsSmemCap)));
   if (n_small > 0) {
-    tridiag_eigvecs<<<n_small, TT, sizeof(double) * (size_t)need, ctx->stream>>>(dp, G, T, w, Z, work, A,
-                                                                                  (int)need);
+    eigvecs_small<<<n_small, small_threads(nsmall_max), sizeof(double) * (size_t)need, ctx->stream>>>(
+        dp, G, T, w, Z, work, A, need);
     TT_LAUNCH_CHECK(ctx);
   }
   if (!big.empty()) {
     // the GPU-wide path: inverse iteration, CholeskyQR2, compact-WY
     // back-transformation; problems it flags are redone by the cluster kernel
-    const int nbig = (int)big.size();
-    std::vector<VecTask> iv, ts, ap;
-    std::vector<TileTask> gm, wy;
-    for (int p = 0; p < nbig; ++p) {
-      const EigDev& e = big[p];
-      for (int j = 0; j < e.nvec; j += IV_THREADS) iv.push_back(VecTask{p, j});
-      const int nt = (e.nvec + GT - 1) / GT;
-      for (int a = 0; a < nt; ++a)
-        for (int b = 0; b <= a; ++b) gm.push_back(TileTask{p, a, b});
-      if (e.nvec > 0) {
-        for (int i = 0; i < e.n; i += TS_ROWS) ts.push_back(VecTask{p, i});
-        for (int k = 0; k * BT_NB < e.n - 2; ++k) wy.push_back(TileTask{p, k, 0});
-        for (int j = 0; j < e.nvec; j += BT_VB) ap.push_back(VecTask{p, j});
-      }
-    }
-    const size_t bytes = sizeof(int) * nbig + sizeof(VecTask) * (iv.size() + ts.size() + ap.size()) +
-                         sizeof(TileTask) * (gm.size() + wy.size()) + 64;
-    char* buf = tt::pool_alloc<char>(ctx, bytes);
-    if (!buf) return tt::fail(TT_ERR_OOM, "tt_sym_eigvecs_batched: allocation failed");
-    int* flags = reinterpret_cast<int*>(buf);
-    VecTask* d_iv = reinterpret_cast<VecTask*>(buf + ((sizeof(int) * nbig + 15) & ~(size_t)15));
-    VecTask* d_ts = d_iv + iv.size();
-    VecTask* d_ap = d_ts + ts.size();
-    TileTask* d_gm = reinterpret_cast<TileTask*>(d_ap + ap.size());
-    TileTask* d_wy = d_gm + gm.size();
-    TT_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * nbig, ctx->stream));
-    TT_CUDA(tt::h2d_async(ctx, d_iv, iv.data(), sizeof(VecTask) * iv.size()));
-    TT_CUDA(tt::h2d_async(ctx, d_ts, ts.data(), sizeof(VecTask) * ts.size()));
-    TT_CUDA(tt::h2d_async(ctx, d_ap, ap.data(), sizeof(VecTask) * ap.size()));
-    TT_CUDA(tt::h2d_async(ctx, d_gm, gm.data(), sizeof(TileTask) * gm.size()));
-    TT_CUDA(tt::h2d_async(ctx, d_wy, wy.data(), sizeof(TileTask) * wy.size()));
-    const EigDev* db = dp + n_small;
-    if (!iv.empty()) {
-      inv_iter_batched<<<(unsigned)iv.size(), IV_THREADS, 0, ctx->stream>>>(db, d_iv, T, w, Z, work);
-      TT_LAUNCH_CHECK(ctx);
-    }
+    if (!iv.empty())
+      TT_CUDA(launch(ctx, (int)iv.size(), IV_THREADS, 0, 0, n_small > 0, (const void*)inv_iter_batched, db, d_iv, T, w,
+                     Z, work));
     for (int pass = 0; pass < 2 && !gm.empty(); ++pass) {
       gram_tiles<<<(unsigned)gm.size(), 256, 0, ctx->stream>>>(db, d_gm, Z, work, flags);
       TT_LAUNCH_CHECK(ctx);
-      TT_CUDA(launch_cluster(ctx, cp.cl, nbig, 0, (const void*)chol_cluster, db, work, flags, pass == 0 ? 1 : 0));
+      TT_CUDA(launch_cluster(ctx, cp.cl, nbig, 0, false, (const void*)chol_cluster, db, work, flags, pass == 0 ? 1 : 0));
       trsm_rows<<<(unsigned)ts.size(), 256, 0, ctx->stream>>>(db, d_ts, Z, work, flags);
       TT_LAUNCH_CHECK(ctx);
     }
@@ -2204,11 +2411,10 @@ int tt_sym_eigvecs_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
       const int64_t full = q * e.n + extra;
       needc = std::max(needc, full <= cp.vecs_cap ? full : extra);
     }
-    TT_CUDA(launch_cluster(ctx, cp.cl, nbig, needc, (const void*)tridiag_eigvecs_cluster, db, G, T, w, Z, work,
+    TT_CUDA(launch_cluster(ctx, cp.cl, nbig, needc, false, (const void*)tridiag_eigvecs_cluster, db, G, T, w, Z, work,
                            (int)needc, (const int*)flags));
-    tt::pool_free(ctx, buf);
   }
-  tt::pool_free(ctx, dp);
+  tt::pool_free(ctx, buf);
   return TT_OK;
 }
 
