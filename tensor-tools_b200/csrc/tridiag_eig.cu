@@ -35,8 +35,8 @@ constexpr int INV_ITERS = 3;
 
 struct EigDev {
   int64_t g_off, w_off, a_off;
-  int32_t n, flags, nvec, nb;  // nb: panel width of the blocked cluster reduction
-  int64_t s_off;               // its n x 2nb panel scratch (blocked cluster reduction)
+  int32_t n, flags, nvec, pad;
+  int64_t s_off;               // its columns in the scratch of the cluster reduction
 };
 
 __device__ double block_reduce(double v, double* red, bool is_max) {
@@ -777,37 +777,24 @@ eigvecs_small(const EigDev* __restrict__ probs, const double* G, const double* T
 // memory) per sector, so a large density matrix is reduced by CL SMs at once
 // instead of one SM streaming it from L2.
 //
-// Phase 1 is the blocked Householder tridiagonalisation of LAPACK's dsytrd /
-// dlatrd (Golub & Van Loan, "Matrix Computations", 4th ed., sec. 8.3.1 with
-// the panel form of sec. 5.1.7): the reflectors of a panel of nb columns are
-// formed one by one against the matrix as it stood at the start of the
-// panel, corrected on the fly by the panel's V and W (A22 v - V W^T v -
-// W V^T v), and the trailing matrix receives the rank-2nb update
-// A -= V W^T + W V^T once per panel.  Only the lower triangle is read or
-// updated.  Index c (row or column) belongs to CTA c % CL.  Per column j,
-// two cluster barriers:
-//   1. the owners of rows >= j bring column j up to date and push it to
-//      every CTA (barrier A);
-//   2. every CTA forms the same reflector from the whole column (same data,
-//      same reduction order), keeps v, and pushes its partial V^T v, W^T v;
-//   3. every CTA runs A22 v over the lower triangle of its own columns: one
-//      warp per block of 64 rows, each lane two rows, columns 16 at a time;
-//      an element A[i,c] (i >= c) adds A[i,c] v_i to the dot of column c and,
-//      below the diagonal, A[i,c] v_c to row i.  The column dots are summed
-//      across the lanes by a butterfly reduce-scatter (lane k ends with
-//      column k % 16), the row sums go to the row's owner (a slot per
-//      sender), and the CTA's share of v^T A22 v to every CTA (barrier B);
-//   4. every CTA completes p = A22 v on its own rows (own dot + the pushed row
-//      sums, in CTA order), w' = tau (p - V W^T v - W V^T v) and
-//      w = w' - (tau/2)(w'.v) v with w'.v = tau (v^T A22 v - 2 (V^T v).(W^T v));
-//      the panel's rows, which every CTA needs, have their row sums and
-//      column dots pushed to every CTA.
-// Every CTA sums pushed partials in CTA order, so every decision and scalar
-// is the same in every CTA.  The trailing update goes through a global
-// n x 2nb scratch (two barriers per panel): m8n8k4 FP64 tensor-core (DMMA)
-// products of 32 rows x 16 own columns per warp, the rows' [V W] read from
-// the scratch and the columns' from shared memory.  The eigenvalues follow by
-// bisection in a separate, GPU-wide launch (bisect_sectors).
+// Phase 1: Householder tridiagonalisation with the rank-2 updates of up to nb
+// reflectors pending (Golub & Van Loan, "Matrix Computations", 4th ed., sec.
+// 8.3.1).  CTA q owns the columns c % CL == q, whole (both triangles), in shared
+// memory when they fit, else in a scratch of its own in L2; every CTA holds the
+// pending v and w on all rows.  So CTA q forms (A0 v)_c of its own columns c
+// without help, A0 the matrix as of the last flush, and one exchange per column
+// is enough: to every CTA go, for every own column c, (A0 v)_c and -- the matrix
+// is symmetric -- the entry A0[k+1, c] of the next column, and the CTA's shares of
+// v^T A0 v and of the pending V^T v and W^T v.  After the cluster barrier every
+// CTA forms for itself, on all rows and from the same data,
+//   p = A0 v - V (W^T v) - W (V^T v),  w = tau p - (tau^2 / 2)(v^T p) v,
+//   x = A0[:, k+1] - V W[k+1]^T - W V[k+1]^T   (this reflector included),
+// and from x the next reflector: one block-wide reduction (sigma) and one
+// barrier (v is complete) before the next products.  When nb reflectors are
+// pending, the products' pass over the own columns applies them on the way.
+// What a CTA pushes for column k + 1 may arrive while another still reads what it
+// got for column k, so the arrays pushed to are double (by parity); where two do
+// not fit (n above about 3300) a second barrier per column follows instead.
 //
 // Phase 2: CTA r owns eigenvectors [r q, r q + q), q = ceil(nvec / CL).
 // Inverse iteration runs one thread per vector.  Gram-Schmidt (twice, inside
@@ -825,27 +812,43 @@ namespace cgx = cooperative_groups;
 
 constexpr int CL_STAGE = 4;  // reflectors staged per round of the back-transformation
 constexpr int CL_MAX = 16;   // largest cluster the kernels are launched with
-constexpr int PNB_MAX = 32;  // widest panel of the blocked reduction
 constexpr int NWARP = TT / 32;
+constexpr int NB_MAX = 16;   // pending reflectors of the cluster reduction, at most
+constexpr int CR_THREADS = 256;  // its threads per CTA
+constexpr int CR_STAGE = 64;     // columns between its layouts (a multiple of CL_MAX)
 struct VecTaskB {
   int32_t prob, j0;  // problem (index into the problem array) and first eigenvalue
 };
 
-// doubles of dynamic shared memory of the blocked cluster reduction
-__host__ __device__ inline int64_t blocked_smem(int n, int nb, int CL) {
-  const int64_t nloc = (n + CL - 1) / CL;
-  return 2 * (int64_t)nb * nloc        // V, W of the panel on the own rows
-         + 2 * nloc                    // the own rows of the current and the next column
-         + (int64_t)CL * nloc          // the pushed column, then v, owner-major
-         + (int64_t)CL * nloc          // this CTA's row sums of A22 v, owner-major
-         + (int64_t)CL * nloc          // pushed row sums of A22 v on the own rows, per sender
-         + (int64_t)NWARP * nloc       // per-warp column dots
-         + CL_MAX * 2 * (int64_t)nb    // pushed V^T v, W^T v partials
-         + CL_MAX                      // pushed v^T A22 v partials
-         + CL_MAX * (int64_t)nb        // pushed row sums on the panel's rows
-         + nb                          // pushed column dots of the panel's rows
-         + 2 * (int64_t)nb * nb        // V, W on the panel's rows
-         + 2 * (int64_t)nb;            // V^T v, W^T v
+__device__ __host__ __forceinline__ int first_owned(int from, int rank, int CL) {
+  // smallest l with rank + CL * l >= from
+  return from <= rank ? 0 : (from - rank + CL - 1) / CL;
+}
+
+// Shared memory of the cluster reduction, in doubles, for the n rows and columns
+// that are left: nb pending reflectors (v, w) on all rows and (w, v) on the own
+// columns, the current v, the pushed pairs (once or twice), the pushed partial
+// sums, and the own columns when they are resident.
+constexpr int CLR_MISC = 2 * CL_MAX * 2 * NB_MAX + 2 * CL_MAX * NWARP + NWARP * 2 * NB_MAX;
+struct ClusterLayout {
+  int nb;           // pending reflectors (0: does not fit)
+  bool resident;    // own columns in shared memory
+  bool twice;       // double push buffers
+  int64_t doubles;  // in all
+};
+__host__ __device__ inline int cl_ld(int n) { return (n + 2) & ~1; }  // rows of a column: even, at least one of padding
+__host__ __device__ inline ClusterLayout cluster_layout(int n, int CL, int64_t cap) {
+  const int64_t ld = cl_ld(n), nloc = (n + CL - 1) / CL;
+  for (int form = 0; form < 3; ++form) {  // resident; in L2; in L2 with single push buffers
+    const bool resident = form == 0, twice = form < 2;
+    const int64_t fixed = CLR_MISC + ld + (twice ? 4 : 2) * ld + (resident ? nloc * ld : 0);
+    int64_t nb = fixed < cap ? (cap - fixed) / (2 * (ld + nloc)) : 0;
+    if (nb > NB_MAX) nb = NB_MAX;
+    // resident columns pay when a few reflectors still fit beside them
+    if (nb < (resident ? 6 : 1)) continue;
+    return ClusterLayout{(int)nb, resident, twice, fixed + nb * 2 * (ld + nloc)};
+  }
+  return ClusterLayout{0, false, false, 0};
 }
 
 // D += A B for one m8n8k4 FP64 tile (DMMA): A 8x4 row fragment (lane L holds
@@ -856,416 +859,389 @@ __device__ __forceinline__ void dmma_tr(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-__device__ __forceinline__ int first_owned(int from, int rank, int CL) {
-  // smallest l with rank + CL * l >= from
-  return from <= rank ? 0 : (from - rank + CL - 1) / CL;
-}
-
-// acc[k] (k < 16) summed over the 32 lanes of the warp, lane L receiving the
-// sum of index L % 16: a butterfly sum across the half-warps, then a
-// reduce-scatter (31 shuffles for 16 sums)
-__device__ __forceinline__ double warp_reduce_scatter16(double (&acc)[16], int lane) {
+// The pending reflectors applied to the own columns l >= lf, rows from rs (even) on:
+// A -= V W^T + W V^T on the FP64 tensor path, a warp per 32 rows x 16 columns as the
+// transposed product (a lane's pair of results is two rows of a column: 16-byte
+// accesses).  vw: (v, w)
+// on all rows; wv: (w, v) on the own columns.
+template <int NW>
+__device__ __noinline__ void cluster_flush(double* cols, int ld, int rend, int lf, int lown, int rs, int np,
+                                           const double2* vw, int ldv, const double2* wv, int ldw, int warp, int lane) {
+  const int g = lane >> 2, t4 = lane & 3;
+  const int ncb = (lown - lf + 15) >> 4, nrt = (rend - rs + 31) >> 5;
+  const double* va = reinterpret_cast<const double*>(vw) + (t4 & 1);
+  const double* vb = reinterpret_cast<const double*>(wv) + (t4 & 1);
+  // columns and rows past the end read a valid element, which is not stored
+  auto tile = [&](int task, bool store, double (&acc)[2][4][2]) {
+    const int r0 = rs + 32 * (task / ncb) + 2 * t4, lb = lf + 16 * (task % ncb) + g;
 #pragma unroll
-  for (int k = 0; k < 16; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 16);
+    for (int b = 0; b < 2; ++b) {
+      const int l = lb + 8 * b;
+      double* col = cols + (int64_t)min(l, lown - 1) * ld;
 #pragma unroll
-  for (int s = 8; s >= 1; s >>= 1) {
-    const bool up = (lane & s) != 0;
-#pragma unroll
-    for (int k = 0; k < s; ++k) {
-      const double send = up ? acc[k] : acc[k + s];
-      const double keep = up ? acc[k + s] : acc[k];
-      acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + 8 * i;
+        if (!store) {
+          const double2 x = *reinterpret_cast<const double2*>(col + min(r, rend - 2));
+          acc[b][i][0] = x.x;
+          acc[b][i][1] = x.y;
+        } else if (r < rend && l < lown) {
+          *reinterpret_cast<double2*>(col + r) = make_double2(acc[b][i][0], acc[b][i][1]);
+        }
+      }
     }
+  };
+  const int tasks = ncb * nrt;
+  auto update = [&](int task, double (&acc)[2][4][2]) {
+    const int r0 = rs + 32 * (task / ncb) + g, lb = lf + 16 * (task % ncb) + g;
+    for (int t0 = 0; t0 < np; t0 += 2) {
+      const int t = min(t0 + (t4 >> 1), np - 1);
+      const bool in = t0 + (t4 >> 1) < np;
+      double af[2], bf[4];
+#pragma unroll
+      for (int b = 0; b < 2; ++b) af[b] = in ? -vb[2 * (t * ldw + min(lb + 8 * b, lown - 1))] : 0.0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) bf[i] = in ? va[2 * ((int64_t)t * ldv + min(r0 + 8 * i, rend - 1))] : 0.0;
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dmma_tr(acc[b][i], af[b], bf[i]);
+    }
+    tile(task, true, acc);
+  };
+  // two tiles in turn, so that one is in flight while the other is updated
+  double t0[2][4][2], t1[2][4][2];
+  int task = warp;
+  if (task < tasks) tile(task, false, t0);
+  if (task + NW < tasks) tile(task + NW, false, t1);
+  for (; task < tasks; task += 2 * NW) {
+    update(task, t0);
+    if (task + 2 * NW < tasks) tile(task + 2 * NW, false, t0);
+    if (task + NW < tasks) update(task + NW, t1);
+    if (task + 3 * NW < tasks) tile(task + 3 * NW, false, t1);
   }
-  return acc[0];
 }
 
-__global__ void __launch_bounds__(TT)
-tridiag_eigvals_cluster(const EigDev* __restrict__ probs, double* G, double* Tg, double* W, double* VWg) {
-  extern __shared__ double sm[];
-  __shared__ double red[33];
-  __shared__ double s_K;
-  __shared__ double vw_part[NWARP * 2 * PNB_MAX];  // per-warp V^T v, W^T v sums
+// One pass over the own columns l >= lf of a CTA: A0[:, c] . v over the rows from
+// rs on (even), pushed with A0[row, c] to every CTA; returns this warp's share of
+// v^T A0 v.  A warp takes two columns at a time, 64 U rows of each per step.
+template <int NW, int U>
+__device__ __forceinline__ double cluster_pass(const double* cols, int ld, int rend, int lf, int lown,
+                                               int rank, int CL, int rs, int row, const double* vcur, double2* push,
+                                               int warp, int lane) {
+  cgx::cluster_group cluster = cgx::this_cluster();
+  double share = 0.0;
+  auto load = [&](int l, int rc, double2 (&a)[2][U]) {
+    const double* q0 = cols + (int64_t)l * ld + rc + 2 * lane;
+    const double* q1 = l + 1 < lown ? q0 + ld : q0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = rc + 2 * lane + 64 * u < rend;
+      a[0][u] = in ? *reinterpret_cast<const double2*>(q0 + 64 * u) : make_double2(0.0, 0.0);
+      a[1][u] = in ? *reinterpret_cast<const double2*>(q1 + 64 * u) : make_double2(0.0, 0.0);
+    }
+  };
+  auto emit = [&](int l, double s) {
+    const int c = rank + CL * l;
+    const double2 out = make_double2(s, cols[(int64_t)l * ld + row]);
+    if (lane < CL) *cluster.map_shared_rank(push + c, lane) = out;
+    share += s * vcur[c];
+  };
+  double s0 = 0.0, s1 = 0.0;
+  auto use = [&](int l, int rc, const double2 (&a)[2][U]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = rc + 2 * lane + 64 * u;
+      const double2 v = r < rend ? *reinterpret_cast<const double2*>(vcur + r) : make_double2(0.0, 0.0);
+      s0 = fma(a[0][u].x, v.x, fma(a[0][u].y, v.y, s0));
+      s1 = fma(a[1][u].x, v.x, fma(a[1][u].y, v.y, s1));
+    }
+    if (rc + 64 * U < rend) return;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    }
+    emit(l, s0);
+    if (l + 1 < lown) emit(l + 1, s1);
+    s0 = s1 = 0.0;
+  };
+  // two steps in turn, so that one is in flight while the other is used
+  int l0 = lf + 2 * warp, r0 = rs, l1 = l0, r1 = r0;
+  auto after = [&](int l, int rc, int& ln, int& rn) {  // the step after (l, rc)
+    ln = l;
+    rn = rc + 64 * U;
+    if (rn >= rend) {
+      ln = l + 2 * NW;
+      rn = rs;
+    }
+  };
+  double2 b0[2][U], b1[2][U];
+  if (l0 < lown) load(l0, r0, b0);
+  after(l0, r0, l1, r1);
+  if (l1 < lown) load(l1, r1, b1);
+  while (l0 < lown) {
+    use(l0, r0, b0);
+    after(l1, r1, l0, r0);
+    if (l0 < lown) load(l0, r0, b0);
+    if (l1 >= lown) break;
+    use(l1, r1, b1);
+    after(l0, r0, l1, r1);
+    if (l1 < lown) load(l1, r1, b1);
+  }
+  return share;
+}
 
+// RPT: rows of a thread, at least n / CR_THREADS.  256 threads: what every warp
+// does for itself costs half of what it would with 512, and 255 registers a thread
+// hold two steps of loads (eight columns' worth spilled, and a spill goes to L2
+// beside 220 KB of shared memory: 10 ms more at n = 1471).
+//
+// Measured with clocks in the kernel, n = 1471 (17 ms in all): the pass over the
+// own columns 8 (their reads from L2 while they do not fit), flushes 3.7, rows 2.1,
+// cluster barrier 1.4, the reflector 1.3.  Against the blocked
+// reduction with two barriers per column, panels of 32 and the row sums of a lower
+// triangle exchanged: block SVD's reduction at bond dimension 3072 (n <= 1471)
+// 22.3 -> 17.2 ms, at 512 (n <= 245, columns resident) 2.33 -> 0.79 ms.
+template <int RPT>
+__global__ void __launch_bounds__(CR_THREADS, 1)
+tridiag_eigvals_cluster(const EigDev* __restrict__ probs, double* G, double* Tg, double* scratch,
+                        int64_t cap) {
+  extern __shared__ double sm[];
+  constexpr int NT = CR_THREADS, NW = NT / 32, U = 4;
+  __shared__ double red[NW], s_x[2];
   cgx::cluster_group cluster = cgx::this_cluster();
   const int CL = (int)cluster.num_blocks();
   const int rank = (int)cluster.block_rank();
   const EigDev P = probs[blockIdx.x / CL];
   const int n = P.n;
-  const int tid = threadIdx.x;
-  if (n <= 0) return;  // the same problem for the whole cluster
-  const int nb = P.nb;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double* Gp = G + P.g_off;
   double* dg = Tg + 3 * P.w_off;
   double* eg = dg + n;
   double* tg = eg + n;
-  double* VW = VWg + P.s_off;  // n x 2nb, row-major: [i][t] = V(i, t), [i][nb + t] = W(i, t)
-  const int warp = tid >> 5, lane = tid & 31;
-  const int nloc = (n + CL - 1) / CL;
-  int lown = 0;  // own indices c = rank + CL l, l < lown
-  while (lown < nloc && rank + CL * lown < n) ++lown;
-  double* Vl = sm;                            // [nb][nloc]
-  double* Wl = Vl + (int64_t)nb * nloc;       // [nb][nloc]
-  double* xc = Wl + (int64_t)nb * nloc;       // [2][nloc]: own rows of a column, by parity of jj
-  // Vectors over all rows are kept owner-major: row i = r + CL l at [r nloc + l],
-  // so what one CTA pushes to another is contiguous on both sides
-  const int lg = __ffs(CL) - 1;  // CL is a power of two
-  auto om = [&](int i) { return ((i & (CL - 1)) * nloc) + (i >> lg); };
-  double* xo = xc + 2 * nloc;                 // [CL][nloc]: column j as pushed, then v
-  double* yl = xo + (int64_t)CL * nloc;       // [CL][nloc]: this CTA's row sums of A22 v
-  double* yb = yl + (int64_t)CL * nloc;       // [CL][nloc]: row sums of A22 v on the own rows, by sender
-  double* dw = yb + (int64_t)CL * nloc;       // [NWARP][nloc]: column dots by warp
-  double* r2 = dw + (int64_t)NWARP * nloc;    // [CL_MAX][2nb]: V^T v, W^T v partials by sender
-  double* r3 = r2 + CL_MAX * 2 * nb;          // [CL_MAX]: v^T A22 v partials by sender
-  double* yp = r3 + CL_MAX;                   // [CL_MAX][nb]: row sums on the panel's rows by sender
-  double* dp = yp + CL_MAX * nb;              // [nb]: column dots of the panel's rows
-  double* Vp = dp + nb;                       // [nb][nb]: Vp[t nb + s] = v_t[k0 + s]
-  double* Wq = Vp + nb * nb;                  // [nb][nb]: Wq[t nb + s] = w_t[k0 + s]
-  double* cvt = Wq + nb * nb;                 // [nb]: V^T v
-  double* cwt = cvt + nb;                     // [nb]: W^T v
-  for (int k0 = 0; k0 + 2 < n; k0 += nb) {
-    const int nbe = min(nb, n - 2 - k0);  // reflector columns k0 .. k0 + nbe - 1
-    for (int jj = 0; jj < nbe; ++jj) {
-      const int j = k0 + jj;
-      double* xcur = xc + (jj & 1) * nloc;
-      // ---- 1: column j on the own rows >= j, pushed to every CTA ----
-      const int l1 = first_owned(j, rank, CL);
-      {
-        // four threads per row, each summing a quarter of the panel's terms
-        // (the loop bound is the same for the whole warp: the shuffles need it)
-        const int sub = tid & 3;
-        for (int base = l1 + (warp << 3); base < lown; base += blockDim.x >> 2) {
-          const int l = base + (lane >> 2);
-          const bool act = l < lown;
-          double corr = 0.0;
-          if (act)
-#pragma unroll 1
-            for (int t = sub; t < jj; t += 4)
-              corr += Vl[t * nloc + l] * Wq[t * nb + jj] + Wl[t * nloc + l] * Vp[t * nb + jj];
-          corr += __shfl_xor_sync(0xffffffffu, corr, 1);
-          corr += __shfl_xor_sync(0xffffffffu, corr, 2);
-          if (act && sub == 0) xcur[l] = (jj == 0 ? Gp[(rank + CL * l) + (int64_t)n * j] : xcur[l]) - corr;
-        }
-      }
+  const int rend = cl_ld(n);  // end of the (zero-padded) rows
+  const int nloc = (n + CL - 1) / CL, lg = __ffs(CL) - 1;  // CL is a power of two
+  const int lown = first_owned(n, rank, CL);  // own columns c = rank + CL l, l < lown
+  double* gcols = scratch + P.s_off + (int64_t)rank * nloc * rend;  // the own columns in L2, [lown][rend]
+  // Shared memory, laid out for the rows and columns from o on (a multiple of CL)
+  // and again every CR_STAGE columns: the fewer are left, the more reflectors may
+  // be pending, until the own columns fit as well.  All pointers take the absolute
+  // row r or own column l.
+  int o = 0, nb = 0, ldv = 0, ldw = 0, ldc = rend;
+  bool resident = false, twice = true;
+  double2 *vw = nullptr, *push = nullptr, *part = nullptr, *ab = nullptr, *wv = nullptr;
+  double *vcur = nullptr, *vav = nullptr, *cols = nullptr;
+  auto lay_out = [&](int from) {
+    const ClusterLayout L = cluster_layout(n - from, CL, cap);
+    o = from;
+    nb = L.nb;
+    twice = L.twice;
+    resident = L.resident;
+    ldv = rend - o;
+    ldw = nloc - o / CL;
+    vw = reinterpret_cast<double2*>(sm) - o;                     // [nb][ldv]: (v, w)
+    vcur = sm + (int64_t)nb * 2 * ldv - o;                       // [ldv]
+    push = reinterpret_cast<double2*>(vcur + o + ldv) - o;       // [1 or 2][ldv]: (A0 v, A0[:, k + 1])
+    part = push + o + (twice ? 2 : 1) * ldv;                     // [2][CL_MAX][NB_MAX]: shares of (W^T v, V^T v)
+    vav = reinterpret_cast<double*>(part + 2 * CL_MAX * NB_MAX);  // [2][CL_MAX][NW]: shares of v^T A0 v
+    ab = reinterpret_cast<double2*>(vav + 2 * CL_MAX * NWARP) + warp * NB_MAX;  // this warp's (W^T v, V^T v)
+    wv = reinterpret_cast<double2*>(reinterpret_cast<double*>(part) + CLR_MISC) - o / CL;  // [nb][ldw]: (w, v) on the own columns
+    ldc = resident ? ldv : rend;
+    cols = resident ? reinterpret_cast<double*>(wv + o / CL + nb * ldw) - (int64_t)(o / CL) * ldc - o : gcols;
+  };
+  lay_out(0);
+  for (int l = warp; l < lown; l += NW)
+    for (int r = lane; r < rend; r += 32)
+      cols[(int64_t)l * ldc + r] = r < n ? Gp[r + (int64_t)n * (rank + CL * l)] : 0.0;
+  auto zero_padding = [&]() {
+    for (int i = tid; i < nb * (rend - n); i += NT)
+      vw[(int64_t)(i / (rend - n)) * ldv + n + i % (rend - n)] = make_double2(0.0, 0.0);
+    if (tid < rend - n) vcur[n + tid] = 0.0;
+  };
+  zero_padding();
+  double x[RPT];  // the next column on the rows tid + TT i
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) x[i] = tid + NT * i < n ? Gp[tid + NT * i] : 0.0;
+  __threadfence_block();
+  cluster.sync();  // column 0 is read; its owner overwrites it
+  int np = 0, par = 0;
+  for (int k = 0; k + 2 < n; ++k) {
+    if (!resident && k > 0 && k % CR_STAGE == 0) {  // lay out again (x stays in registers)
       __syncthreads();
-      for (int e = tid; e < (lown - l1) * CL; e += blockDim.x) {
-        const int q = e / (lown - l1), l = l1 + e % (lown - l1);
-        *cluster.map_shared_rank(xo + rank * nloc + l, q) = xcur[l];
-      }
-      cluster.sync();  // A
-      // ---- 2: the reflector (same in every CTA), v kept, V^T v and W^T v partials ----
-      const double alpha = xo[om(j + 1)];  // read before the reduction's barriers, overwritten below
-      double part = 0.0;
-      for (int i = j + 2 + tid; i < n; i += blockDim.x) part += xo[om(i)] * xo[om(i)];
-      const double sigma = block_reduce(part, red, false);
-      double tau = 0.0, beta = alpha, scale = 0.0;
-      if (sigma != 0.0) {
-        const double mu = sqrt(alpha * alpha + sigma);
-        beta = alpha <= 0.0 ? mu : -mu;
-        tau = (beta - alpha) / beta;
-        scale = 1.0 / (alpha - beta);
-      }
-      if (rank == j % CL && tid == 0) {
-        dg[j] = xo[om(j)];
-        tg[j] = tau;
-        eg[j] = beta;
-      }
-      for (int i = j + 1 + tid; i < n; i += blockDim.x) xo[om(i)] = i == j + 1 ? 1.0 : xo[om(i)] * scale;
-      __syncthreads();
-      for (int l = tid; l < lown; l += blockDim.x) {
-        const int i = rank + CL * l;
-        const double vi = i >= j + 1 ? xo[rank * nloc + l] : 0.0;
-        Vl[jj * nloc + l] = vi;
-        Wl[jj * nloc + l] = 0.0;
-        if (i >= j + 2) Gp[i + (int64_t)n * j] = vi;  // reflector kept below the subdiagonal for phase 2
-      }
-      for (int s = tid; s < nb; s += blockDim.x) {
-        const int row = k0 + s;
-        Vp[jj * nb + s] = row >= j + 1 && row < n ? xo[om(row)] : 0.0;
-      }
-      __syncthreads();
-      const int lf = first_owned(j + 1, rank, CL);
-      // V^T v and W^T v partials over the own rows >= j + 1: lane t of each
-      // warp sums column t over every NWARP-th row, the warps' sums are added
-      // in warp order and pushed to every CTA
-      if (jj > 0) {
-        double sv = 0.0, sw = 0.0;
-        if (lane < jj)
-          for (int l = lf + warp; l < lown; l += NWARP) {
-            const double v = Vl[jj * nloc + l];
-            sv += Vl[lane * nloc + l] * v;
-            sw += Wl[lane * nloc + l] * v;
-          }
-        vw_part[warp * 2 * PNB_MAX + lane] = sv;
-        vw_part[warp * 2 * PNB_MAX + PNB_MAX + lane] = sw;
-        __syncthreads();
-        if (tid < 2 * PNB_MAX) {
-          const int t = tid & (PNB_MAX - 1);
-          if (t < jj) {
-            double a = 0.0;
-            for (int w = 0; w < NWARP; ++w) a += vw_part[w * 2 * PNB_MAX + tid];
-            const int slot = rank * 2 * nb + (tid < PNB_MAX ? t : nb + t);
-            for (int q = 0; q < CL; ++q) *cluster.map_shared_rank(r2 + slot, q) = a;
-          }
-        }
-      }
-      // ---- 3: p = A22 v from the lower triangle of the own columns ----
-      if (jj + 1 < nbe)  // the next column's own rows: unchanged until its step 1
-        for (int l = lf + tid; l < lown; l += blockDim.x)
-          xc[((jj + 1) & 1) * nloc + l] = Gp[(rank + CL * l) + (int64_t)n * (j + 1)];
-      double kp = 0.0;  // this thread's share of v^T A22 v
-      if (tau != 0.0) {
-        for (int l = lf + lane; l < lown; l += 32) dw[warp * nloc + l] = 0.0;
-        __syncwarp();
-        // blocks of 64 rows from row j + 1, two rows per lane (i0 = rb + lane,
-        // i1 = i0 + 32); the longest (last) blocks are dealt first and back and
-        // forth, so the warps' shares come out even
-        const int nrb = (n - j - 1 + 63) / 64;
-        const int64_t cstep = (int64_t)n * CL;  // from one own column to the next
-        for (int round = 0; round * NWARP < nrb; ++round) {
-          const int o = round * NWARP + ((round & 1) ? NWARP - 1 - warp : warp);
-          if (o >= nrb) continue;
-          const int rb = j + 1 + 64 * (nrb - 1 - o);
-          const int i0 = rb + lane, i1 = i0 + 32;
-          const double v0 = i0 < n ? xo[om(i0)] : 0.0, v1 = i1 < n ? xo[om(i1)] : 0.0;
-          // rows past the end read row n - 1 (weighted by v = 0, sums discarded)
-          const double* g0 = Gp + min(i0, n - 1) + (int64_t)n * rank;
-          const double* g1 = Gp + min(i1, n - 1) + (int64_t)n * rank;
-          const int le = first_owned(min(n, rb + 64), rank, CL);  // own columns c < the block's end
-          const int lfull = min(le, first_owned(rb, rank, CL));   // own columns c < rb: no masking
-          double y0 = 0.0, y1 = 0.0;
-          int lt = lf;
-          for (; lt + 16 <= lfull; lt += 16) {
-            double acc[16];
+      if (np > 0) cluster_flush<NW>(cols, ldc, rend, first_owned(k, rank, CL), lown, k, np, vw, ldv, wv, ldw, warp, lane);
+      np = 0;
+      cluster.sync();  // nobody reads the old layout any more
+      lay_out(k);
+      if (resident)
+        for (int l = o / CL + warp; l < lown; l += NW)
+          for (int r = o + lane; r < rend; r += 32) cols[(int64_t)l * ldc + r] = gcols[(int64_t)l * rend + r];
+      zero_padding();
+      cluster.sync();  // the new one is ready to be pushed to
+    }
+    // ---- the reflector of column k (every CTA alike) ----
+    double sig = 0.0;
 #pragma unroll
-            for (int h = 0; h < 16; h += 8) {  // eight columns' loads in flight at a time
-              double a0[8], a1[8];
+    for (int i = 0; i < RPT; ++i) {
+      const int r = tid + NT * i;
+      if (r >= k + 2 && r < n) sig += x[i] * x[i];
+      if (r == k) s_x[0] = x[i];
+      if (r == k + 1) s_x[1] = x[i];
+    }
+    sig = warp_sum(sig);
+    if (lane == 0) red[warp] = sig;
+    __syncthreads();
+    double part_s[NW];
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                a0[k] = g0[(lt + h + k) * cstep];
-                a1[k] = g1[(lt + h + k) * cstep];
-              }
+    for (int w = 0; w < NW; ++w) part_s[w] = red[w];
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                const double vc = xo[rank * nloc + lt + h + k];
-                y0 = fma(a0[k], vc, y0);
-                y1 = fma(a1[k], vc, y1);
-                acc[h + k] = fma(a1[k], v1, a0[k] * v0);
-              }
-            }
-            const double d = warp_reduce_scatter16(acc, lane);
-            if (lane < 16) dw[warp * nloc + lt + lane] += d;
-          }
-          for (; lt < le; lt += 16) {  // the rest, masked: the block's diagonal part and a short tail
-            double acc[16];
+    for (int o = NW / 2; o > 0; o >>= 1)
 #pragma unroll
-            for (int h = 0; h < 16; h += 8) {
-              double a0[8], a1[8];
+      for (int w = 0; w < o; ++w) part_s[w] += part_s[w + o];
+    const double sigma = part_s[0], alpha = s_x[1];
+    // beta = -sign(alpha) |(alpha, sigma)|, tau = (beta - alpha) / beta, v = x / (alpha - beta)
+    double tau = 0.0, beta = alpha, scale = 0.0;
+    if (sigma != 0.0) {
+      const double s2 = fma(alpha, alpha, sigma), ri = rsqrt(s2), mu = s2 * ri;
+      beta = alpha <= 0.0 ? mu : -mu;
+      tau = fma(fabs(alpha), ri, 1.0);
+      scale = 1.0 / (alpha - beta);
+    }
+    const bool owner = rank == k % CL;
+    if (owner && tid == 0) {
+      dg[k] = s_x[0];
+      eg[k] = beta;
+      tg[k] = tau;
+    }
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                const int c = rank + CL * (lt + h + k);
-                const bool cv = lt + h + k < le;
-                a0[k] = cv && i0 >= c ? g0[(lt + h + k) * cstep] : 0.0;
-                a1[k] = cv && i1 >= c ? g1[(lt + h + k) * cstep] : 0.0;
-              }
-#pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                const int c = rank + CL * (lt + h + k);
-                const double vc = lt + h + k < le ? xo[rank * nloc + lt + h + k] : 0.0;
-                y0 = fma(i0 > c ? a0[k] : 0.0, vc, y0);
-                y1 = fma(i1 > c ? a1[k] : 0.0, vc, y1);
-                acc[h + k] = fma(a1[k], v1, a0[k] * v0);
-              }
-            }
-            const double d = warp_reduce_scatter16(acc, lane);
-            if (lane < 16 && lt + lane < le) dw[warp * nloc + lt + lane] += d;
-          }
-          if (i0 < n) {
-            yl[om(i0)] = y0;
-            kp += v0 * y0;
-          }
-          if (i1 < n) {
-            yl[om(i1)] = y1;
-            kp += v1 * y1;
-          }
-        }
+    for (int i = 0; i < RPT; ++i) {
+      const int r = tid + NT * i;
+      if (r >= k && r < n) {
+        const double v = r == k + 1 ? 1.0 : (r == k ? 0.0 : x[i] * scale);
+        vcur[r] = v;
+        if (owner && r >= k + 2) Gp[r + (int64_t)n * k] = v;  // kept below the subdiagonal for phase 2
       }
-      __syncthreads();
-      if (tau != 0.0) {
-        // the row sums to their owners (rows below j + 1 and beyond n ride
-        // along unread), those of the panel's rows to every CTA
-        const int lmin = (j + 1) >> lg, cnt = nloc - lmin;
-        for (int e = tid; e < CL * cnt; e += blockDim.x) {
-          const int d = e / cnt, l = lmin + e % cnt;
-          *cluster.map_shared_rank(yb + rank * nloc + l, d) = yl[d * nloc + l];
-        }
-        for (int e = tid; e < CL * nb; e += blockDim.x) {
-          const int q = e / nb, s = e % nb, row = k0 + s;
-          if (row >= j + 1 && row < n) *cluster.map_shared_rank(yp + rank * nb + s, q) = yl[om(row)];
-        }
-      }
-      if (tau != 0.0)
-        for (int l = lf + tid; l < lown; l += blockDim.x) {
-          double d = 0.0;
-          for (int w = 0; w < NWARP; ++w) d += dw[w * nloc + l];
-          dw[l] = d;  // the column's dot, kept in warp 0's row
-          const int c = rank + CL * l;
-          kp += xo[rank * nloc + l] * d;
-          if (c < k0 + nb)
-            for (int q = 0; q < CL; ++q) *cluster.map_shared_rank(dp + (c - k0), q) = d;
-        }
-      const double vav_part = block_reduce(kp, red, false);
-      if (tid < CL) *cluster.map_shared_rank(r3 + rank, tid) = vav_part;
-      cluster.sync();  // B
-      // ---- 4: w on the own rows and on the panel's rows ----
-      if (warp == 0) {  // V^T v, W^T v and the scalar K = (tau/2) w'.v, one lane per panel column
-        double a = 0.0, b = 0.0;
-        if (lane < jj)
-          for (int q = 0; q < CL; ++q) {
-            a += r2[q * 2 * nb + lane];
-            b += r2[q * 2 * nb + nb + lane];
-          }
-        if (lane < jj) {
-          cvt[lane] = a;
-          cwt[lane] = b;
-        }
-        const double cc = warp_sum(a * b);
-        if (lane == 0) {
-          double vav = 0.0;
-          for (int q = 0; q < CL; ++q) vav += r3[q];
-          s_K = 0.5 * tau * tau * (vav - 2.0 * cc);
-        }
-      }
-      __syncthreads();
-      if (tau != 0.0) {
-        const double K = s_K;
-        // own rows: four threads per row, each summing a quarter of the terms
-        // (the loop bound is the same for the whole warp: the shuffles need it)
-        const int sub = tid & 3;
-        for (int base = lf + (warp << 3); base < lown; base += blockDim.x >> 2) {
-          const int l = base + (lane >> 2);
-          const bool act = l < lown;
-          double p = 0.0, corr = 0.0;
-          if (act) {
-#pragma unroll 1
-            for (int q = sub; q < CL; q += 4) p += yb[q * nloc + l];
-#pragma unroll 1
-            for (int t = sub; t < jj; t += 4) corr += Vl[t * nloc + l] * cwt[t] + Wl[t * nloc + l] * cvt[t];
-          }
-          p += __shfl_xor_sync(0xffffffffu, p, 1);
-          p += __shfl_xor_sync(0xffffffffu, p, 2);
-          corr += __shfl_xor_sync(0xffffffffu, corr, 1);
-          corr += __shfl_xor_sync(0xffffffffu, corr, 2);
-          if (act && sub == 0) Wl[jj * nloc + l] = tau * (dw[l] + p - corr) - K * Vl[jj * nloc + l];
-        }
-        // the panel's rows: sixteen threads per row
-        const int s = tid >> 4, sub16 = tid & 15;
-        if (s < nb) {
-          const int row = k0 + s;
-          const bool live = row >= j + 1 && row < n;
-          double p = 0.0, corr = 0.0;
-          if (live) {
-            for (int q = sub16; q < CL; q += 16) p += yp[q * nb + s];
-            for (int t = sub16; t < jj; t += 16) corr += Vp[t * nb + s] * cwt[t] + Wq[t * nb + s] * cvt[t];
-          }
-#pragma unroll
-          for (int o = 1; o < 16; o <<= 1) {
-            p += __shfl_xor_sync(0xffffffffu, p, o);
-            corr += __shfl_xor_sync(0xffffffffu, corr, o);
-          }
-          if (sub16 == 0) Wq[jj * nb + s] = live ? tau * (dp[s] + p - corr) - K * Vp[jj * nb + s] : 0.0;
-        }
-      } else {
-        for (int s = tid; s < nb; s += blockDim.x) Wq[jj * nb + s] = 0.0;
-      }
+    }
+    __syncthreads();
+    // ---- the shares of the pending V^T v and W^T v, and A0 v on the own columns ----
+    const bool flush = np == nb;
+    double2* pushed = push + (twice ? par * ldv : 0);
+    double2* mypart = part + par * CL_MAX * NB_MAX;
+    double* myvav = vav + par * CL_MAX * NWARP;
+    const int lf = first_owned(k + 1, rank, CL), rs = (k + 1) & ~1;
+    if (flush) {
+      cluster_flush<NW>(cols, ldc, rend, lf, lown, rs, np, vw, ldv, wv, ldw, warp, lane);
+      np = 0;
       __syncthreads();
     }
-    // ---- trailing update A[k1:, k1:] -= V W^T + W V^T (lower triangle) through the global scratch ----
-    const int k1 = k0 + nbe;
-    for (int e = tid; e < lown * 2 * nbe; e += blockDim.x) {
-      const int l = e / (2 * nbe), t2 = e - l * 2 * nbe;
-      const int i = rank + CL * l;
-      if (i < k1) continue;
-      const int t = t2 < nbe ? t2 : t2 - nbe;
-      VW[(int64_t)i * 2 * nb + (t2 < nbe ? t : nb + t)] = (t2 < nbe ? Vl : Wl)[t * nloc + l];
+    for (int t = warp; t < np; t += NW) {
+      const double2* p = vw + (int64_t)t * ldv;
+      const int seg = (n - k - 1 + CL - 1) / CL, r0 = k + 1 + rank * seg, r1 = min(n, r0 + seg);
+      double a = 0.0, b = 0.0;
+      for (int r = r0 + lane; r < r1; r += 32) {
+        const double2 y = p[r];
+        const double v = vcur[r];
+        a = fma(y.y, v, a);
+        b = fma(y.x, v, b);
+      }
+      a = warp_sum(a);
+      b = warp_sum(b);
+      if (lane < CL) *cluster.map_shared_rank(mypart + rank * NB_MAX + t, lane) = make_double2(a, b);
     }
-    __threadfence();
+    const double share = cluster_pass<NW, U>(cols, ldc, rend, lf, lown, rank, CL, rs, k + 1, vcur, pushed, warp, lane);
+    if (lane < CL) *cluster.map_shared_rank(myvav + rank * NW + warp, lane) = share;
     cluster.sync();
-    // DMMA (m8n8k4 f64) tiles: a warp takes 32 rows x 16 own columns and runs
-    // P = V W^T + W V^T over the panel's k, the rows' [V W] fragments read
-    // straight from the scratch (no shared staging, no barrier per tile); the
-    // lower triangle of its block then receives A -= P
-    const int lf = first_owned(k1, rank, CL);
-    const int nbe4 = (nbe + 3) & ~3;
-    const int gr = lane >> 2, gk = lane & 3;
-    const int nrt = (n - k1 + 31) >> 5;                 // 32-row tiles
-    const int ncb = (first_owned(n, rank, CL) - lf + 15) >> 4;  // 16-column blocks
-    for (int task = warp; task < nrt * ncb; task += NWARP) {
-      const int i0 = k1 + 32 * (task / ncb), lb = lf + 16 * (task % ncb);
-      if (rank + CL * lb > i0 + 31) continue;  // the block lies above the diagonal
-      const int le = min(first_owned(min(n, i0 + 32), rank, CL), lb + 16);
-      double acc[4][2][2];
+    // ---- w and the next column, on all rows (every CTA alike; the sums by every warp for itself) ----
+    const int t = lane & 15, half = lane >> 4;  // two lanes per pending reflector, each every other CTA's share
+    double a = 0.0, b = 0.0, s = 0.0;
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-#pragma unroll
-      for (int part = 0; part < 2; ++part) {
-        // part 0: V (rows) x W (columns); part 1: W x V
-        const int xo0 = part ? nb : 0;
-        const double* Y = part ? Vl : Wl;
-#pragma unroll 1
-        for (int t = 0; t < nbe4; t += 4) {
-          const int k = t + gk;
-          const bool kv = k < nbe;
-          double af[4], bf[2];
-#pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            const int i = i0 + 8 * a + gr;
-            af[a] = kv && i < n ? VW[(int64_t)i * 2 * nb + xo0 + k] : 0.0;
-          }
-#pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            const int l = lb + 8 * b + gr;
-            bf[b] = kv && l < le ? Y[k * nloc + l] : 0.0;
-          }
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) dmma_tr(acc[a][b], af[a], bf[b]);
-        }
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const int i = i0 + 8 * a + gr;
-#pragma unroll
-        for (int b = 0; b < 2; ++b)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int l = lb + 8 * b + 2 * gk + e;
-            const int c = rank + CL * l;
-            if (i < n && l < le && i >= c) Gp[(int64_t)n * c + i] -= acc[a][b][e];
-          }
+    for (int u = 0; u < CL_MAX / 2; ++u) {
+      const int q = 2 * u + half;
+      if (t < np && q < CL) {
+        const double2 y = mypart[q * NB_MAX + t];
+        a += y.x;
+        b += y.y;
       }
     }
-    __threadfence();
-    cluster.sync();
+#pragma unroll
+    for (int u = 0; u < CL_MAX * NW / 32; ++u)
+      if (lane + 32 * u < CL * NW) s += myvav[lane + 32 * u];
+    a += __shfl_xor_sync(0xffffffffu, a, 16);
+    b += __shfl_xor_sync(0xffffffffu, b, 16);
+    double pc = 0.0;  // V (W^T v) + W (V^T v) at row k + 1
+    if (lane < np) {
+      const double2 y = vw[(int64_t)lane * ldv + k + 1];
+      pc = fma(y.x, a, y.y * b);
+      s = fma(-2.0 * a, b, s);
+      ab[lane] = make_double2(a, b);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+      pc += __shfl_xor_sync(0xffffffffu, pc, o);
+    }
+    const double K = 0.5 * tau * tau * s;
+    const double wk1 = tau * (pushed[k + 1].x - pc) - K;  // w at row k + 1, where v is 1
+    __syncwarp();
+    double p[RPT];
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      const int r = tid + NT * i;
+      const double2 y = r > k && r < n ? pushed[r] : make_double2(0.0, 0.0);
+      p[i] = y.x;
+      x[i] = y.y;
+    }
+    for (int u = 0; u < np; ++u) {
+      const double2 f = vw[(int64_t)u * ldv + k + 1], q = ab[u];
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        const int r = tid + NT * i;
+        if (r > k && r < n) {
+          const double2 z = vw[(int64_t)u * ldv + r];
+          p[i] = fma(-z.x, q.x, fma(-z.y, q.y, p[i]));
+          x[i] = fma(-z.x, f.y, fma(-z.y, f.x, x[i]));
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      const int r = tid + NT * i;
+      if (r > k && r < n) {
+        const double v = vcur[r];
+        const double w = tau * p[i] - K * v;
+        x[i] = x[i] - v * wk1 - w;
+        vw[(int64_t)np * ldv + r] = make_double2(v, w);
+        if ((r & (CL - 1)) == rank) wv[np * ldw + (r >> lg)] = make_double2(w, v);
+      }
+    }
+    ++np;
+    par ^= 1;
+    if (!twice) cluster.sync();  // the pushed pairs are read before the next ones arrive
   }
-  // T: the last two diagonal entries and the last off-diagonal A[n-1, n-2]
-  if (tid == 0) {
-    if (rank == (n - 2) % CL) {
-      dg[n - 2] = Gp[(n - 2) + (int64_t)n * (n - 2)];
-      eg[n - 2] = Gp[(n - 1) + (int64_t)n * (n - 2)];
+  // T: the last 2 x 2 block
+  __syncthreads();
+  if (rank == 0) {
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      const int r = tid + NT * i;
+      if (r == n - 2) dg[n - 2] = x[i];
+      if (r == n - 1) eg[n - 2] = x[i];
     }
-    if (rank == (n - 1) % CL) dg[n - 1] = Gp[(n - 1) + (int64_t)n * (n - 1)];
-    if (rank == 0) {
+    if (tid == 0) {
       eg[n - 1] = 0.0;
       tg[n - 1] = 0.0;
       tg[n - 2] = 0.0;
     }
   }
-  __threadfence();
-  cluster.sync();  // also the last access of another CTA's shared memory
+  if (rank == (n - 1) % CL && tid == 0) {
+    double t = cols[(int64_t)(lown - 1) * ldc + n - 1];
+    for (int q = 0; q < np; ++q) {
+      const double2 z = vw[(int64_t)q * ldv + n - 1];
+      t -= 2.0 * z.x * z.y;
+    }
+    dg[n - 1] = t;
+  }
+  cluster.sync();  // the last access of another CTA's shared memory
   // launched alongside tridiag_small: complete only when that is
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -2111,6 +2087,14 @@ bool is_big(const EigDev& e) { return e.n > SN && !(e.flags & TT_EIG_ROW_1X2); }
 // device: 16 CTAs per cluster when the device can co-schedule that many with
 // the full shared-memory carve-out, else 8, else none (an error for sectors that
 // need them).
+// The cluster reduction for sectors of up to n states
+const void* vals_kernel(int n) {
+  return n <= 2 * CR_THREADS   ? (const void*)tridiag_eigvals_cluster<2>
+         : n <= 4 * CR_THREADS ? (const void*)tridiag_eigvals_cluster<4>
+         : n <= 8 * CR_THREADS ? (const void*)tridiag_eigvals_cluster<8>
+                               : (const void*)tridiag_eigvals_cluster<16>;
+}
+
 struct ClusterPlan {
   int device = -1;
   int cl = 0;
@@ -2128,7 +2112,7 @@ const ClusterPlan& cluster_plan(tt_ctx* ctx) {
     return cp;
   }
   cudaFuncAttributes fa, fb;
-  if (cudaFuncGetAttributes(&fa, tridiag_eigvals_cluster) != cudaSuccess ||
+  if (cudaFuncGetAttributes(&fa, vals_kernel(MAX_N)) != cudaSuccess ||
       cudaFuncGetAttributes(&fb, tridiag_eigvecs_cluster) != cudaSuccess) {
     cudaGetLastError();
     return cp;
@@ -2136,9 +2120,11 @@ const ClusterPlan& cluster_plan(tt_ctx* ctx) {
   const int64_t va = ((int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024) / 8;
   const int64_t vb = ((int64_t)optin - (int64_t)fb.sharedSizeBytes - 1024) / 8;
   if (vb < 6 * MAX_N) return cp;
-  const void* kernels[2] = {(const void*)tridiag_eigvals_cluster, (const void*)tridiag_eigvecs_cluster};
-  const int64_t caps[2] = {va, vb};
-  for (int k = 0; k < 2; ++k) {
+  constexpr int NK = 5;
+  const void* kernels[NK] = {vals_kernel(1), vals_kernel(4 * CR_THREADS), vals_kernel(8 * CR_THREADS), vals_kernel(MAX_N),
+                             (const void*)tridiag_eigvecs_cluster};
+  const int64_t caps[NK] = {va, va, va, va, vb};
+  for (int k = 0; k < NK; ++k) {
     if (cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(caps[k] * 8)) !=
             cudaSuccess ||
         cudaFuncSetAttribute(kernels[k], cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
@@ -2151,8 +2137,8 @@ const ClusterPlan& cluster_plan(tt_ctx* ctx) {
     return cp;
   }
   for (int cl : {CL_MAX, 8}) {
-    bool ok = blocked_smem(MAX_N, 8, cl) <= va;  // the largest sector fits at the narrowest panel
-    for (int k = 0; k < 2 && ok; ++k) {
+    bool ok = cluster_layout(MAX_N, cl, va).nb > 0;  // the largest sector fits
+    for (int k = 0; k < NK && ok; ++k) {
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute at[1];
       at[0].id = cudaLaunchAttributeClusterDimension;
@@ -2160,7 +2146,7 @@ const ClusterPlan& cluster_plan(tt_ctx* ctx) {
       at[0].val.clusterDim.y = 1;
       at[0].val.clusterDim.z = 1;
       cfg.gridDim = dim3(cl);
-      cfg.blockDim = dim3(TT);
+      cfg.blockDim = dim3(k + 1 < NK ? CR_THREADS : TT);
       cfg.dynamicSmemBytes = (size_t)(caps[k] * 8);
       cfg.attrs = at;
       cfg.numAttrs = 1;
@@ -2214,9 +2200,8 @@ cudaError_t launch(tt_ctx* ctx, int grid, int block, int cl, size_t smem, bool b
 
 // One cluster of `cl` CTAs per problem; `need` doubles of dynamic shared memory.
 template <class... Args>
-cudaError_t launch_cluster(tt_ctx* ctx, int cl, int n_probs, int64_t need, bool beside, const void* kernel,
-                           Args... args) {
-  return launch(ctx, cl * n_probs, TT, cl, (size_t)(need * 8), beside, kernel, args...);
+cudaError_t launch_cluster(tt_ctx* ctx, int cl, int n_probs, int64_t need, const void* kernel, Args... args) {
+  return launch(ctx, cl * n_probs, TT, cl, (size_t)(need * 8), false, kernel, args...);
 }
 
 }  // namespace
@@ -2242,18 +2227,18 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
   }
   const int n_small = (int)hp.size();
   int64_t need = 0, scratch = 0;
+  int nbig_max = 0;
   if (!big.empty()) {
     TT_REQUIRE(cp.cl > 0, "tt_sym_eigvals_batched: no thread-block clusters for sectors of this size");
-    // panel width per problem: the widest whose shared memory fits; the
-    // panel scratch (n x 2nb per problem) lives in the pool
     for (EigDev& e : big) {
-      e.nb = PNB_MAX;
-      while (e.nb > 8 && blocked_smem(e.n, e.nb, cp.cl) > cp.vals_cap) e.nb /= 2;
-      need = std::max(need, blocked_smem(e.n, e.nb, cp.cl));
+      const ClusterLayout L = cluster_layout(e.n, cp.cl, cp.vals_cap);
+      TT_REQUIRE(L.nb > 0, "tt_sym_eigvals_batched: sector too large for the cluster eigensolver");
+      // the layouts of later stages take what there is
+      need = std::max(need, L.resident ? L.doubles : cp.vals_cap);
       e.s_off = scratch;
-      scratch += (int64_t)e.n * 2 * e.nb;
+      nbig_max = std::max(nbig_max, e.n);
+      scratch += (int64_t)cp.cl * ((e.n + cp.cl - 1) / cp.cl) * cl_ld(e.n);
     }
-    TT_REQUIRE(need <= cp.vals_cap, "tt_sym_eigvals_batched: sector too large for the cluster eigensolver");
   }
   hp.insert(hp.end(), big.begin(), big.end());
   // every sector's eigenvalues, BS_PER per CTA over the whole GPU
@@ -2264,7 +2249,7 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
     nmax = std::max(nmax, hp[p].n);
     for (int j0 = 0; j0 < hp[p].n; j0 += BS_PER) bt.push_back(VecTaskB{p, j0});
   }
-  // problems, bisection tasks and the panel scratch in one buffer
+  // problems, bisection tasks and the columns' scratch in one buffer
   const size_t pb = sizeof(EigDev) * hp.size(), tb = (sizeof(VecTaskB) * bt.size() + 15) & ~(size_t)15;
   std::vector<char> host(pb + tb);
   std::memcpy(host.data(), hp.data(), pb);
@@ -2274,7 +2259,7 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
   TT_CUDA(tt::h2d_async(ctx, buf, host.data(), host.size()));
   const EigDev* dp = reinterpret_cast<const EigDev*>(buf);
   const VecTaskB* d_bt = reinterpret_cast<const VecTaskB*>(buf + pb);
-  double* vw = reinterpret_cast<double*>(buf + pb + tb);
+  double* cols = reinterpret_cast<double*>(buf + pb + tb);
   static thread_local uint64_t attr = 0;  // per host thread and device
   if (tt::first_on_device(attr, ctx->device)) {
     TT_CUDA(cudaFuncSetAttribute(tridiag_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2288,9 +2273,10 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
         dp, G, T, w, A);
     TT_LAUNCH_CHECK(ctx);
   }
-  if (!big.empty())
-    TT_CUDA(launch_cluster(ctx, cp.cl, (int)big.size(), need, n_small > 0, (const void*)tridiag_eigvals_cluster,
-                           dp + n_small, G, T, w, vw));
+  if (!big.empty()) {
+    TT_CUDA(launch(ctx, cp.cl * (int)big.size(), CR_THREADS, cp.cl, (size_t)(need * 8), n_small > 0,
+                   vals_kernel(nbig_max), dp + n_small, G, T, cols, need));
+  }
   if (!bt.empty()) {
     const size_t bs_smem = sizeof(double2) * (size_t)((nmax + 7) & ~7);
     bisect_sectors<<<(unsigned)bt.size(), BS_THREADS, bs_smem, ctx->stream>>>(dp, d_bt, T, w);
@@ -2394,7 +2380,7 @@ int tt_sym_eigvecs_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
     for (int pass = 0; pass < 2 && !gm.empty(); ++pass) {
       gram_tiles<<<(unsigned)gm.size(), 256, 0, ctx->stream>>>(db, d_gm, Z, work, flags);
       TT_LAUNCH_CHECK(ctx);
-      TT_CUDA(launch_cluster(ctx, cp.cl, nbig, 0, false, (const void*)chol_cluster, db, work, flags, pass == 0 ? 1 : 0));
+      TT_CUDA(launch_cluster(ctx, cp.cl, nbig, 0, (const void*)chol_cluster, db, work, flags, pass == 0 ? 1 : 0));
       trsm_rows<<<(unsigned)ts.size(), 256, 0, ctx->stream>>>(db, d_ts, Z, work, flags);
       TT_LAUNCH_CHECK(ctx);
     }
@@ -2411,7 +2397,7 @@ int tt_sym_eigvecs_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
       const int64_t full = q * e.n + extra;
       needc = std::max(needc, full <= cp.vecs_cap ? full : extra);
     }
-    TT_CUDA(launch_cluster(ctx, cp.cl, nbig, needc, false, (const void*)tridiag_eigvecs_cluster, db, G, T, w, Z, work,
+    TT_CUDA(launch_cluster(ctx, cp.cl, nbig, needc, (const void*)tridiag_eigvecs_cluster, db, G, T, w, Z, work,
                            (int)needc, (const int*)flags));
   }
   tt::pool_free(ctx, buf);
