@@ -322,6 +322,24 @@ int tt_dav_gs_refill(tt_ctx* ctx, tt_dav_state* st, int ii, int ni, int maxsize,
                      const double* const* xs, double* y, int nranges, const int64_t* d_ranges, uint64_t seed,
                      const double* d_gsnorm, double* d_dots);
 int tt_dav_refill_flag(tt_dav_state* st, const int** d_flag);
+/* All of one iteration between two products in one launch, for vectors of up
+ * to TT_DAV_STEP_MAX elements (more are faster with the calls above): the new
+ * row of the projected matrix from vs[0..ii] and vas[0..ii] (HOST arrays of
+ * device pointers), its lowest eigenpair, the Ritz vector to x (ii >= 1), the
+ * test, and the next basis vector to q.  Steps after the loop has ended are
+ * no-ops; step 0 starts a new loop.  tt_dav_read as above. */
+#define TT_DAV_STEP_MAX 262144
+int tt_dav_step(tt_ctx* ctx, tt_dav_state* st, int ii, int maxiter, double tol, int maxsize, int64_t n,
+                const double* const* vs, const double* const* vas, double* x, double* q, int nranges,
+                const int64_t* d_ranges, uint64_t seed);
+/* The same for step j of a restart of the dense loop (linalg/
+ * tensor_davidson.cpp:74-184): writes the next basis vector to vs[j + 1], or,
+ * for j = m - 1, the Ritz vector to x and, normalised, to vs[0].
+ * tt_dav_read_dense synchronises and returns the Ritz value and the norm of
+ * the residual. */
+int tt_dav_step_dense(tt_ctx* ctx, tt_dav_state* st, int j, int m, int high, int64_t n, double* const* vs,
+                      const double* const* vas, const double* D, double* x);
+int tt_dav_read_dense(tt_ctx* ctx, const tt_dav_state* st, double* eval, double* r_norm);
 
 /* ---- strided copies ------------------------------------------------------
  * dst[dst_off + sum_i j_i*dst_stride[i]] = src[src_off + sum_i j_i*src_stride[i]]

@@ -14,6 +14,8 @@
 #include <cstddef>
 #include <cstring>
 
+#include <cooperative_groups.h>
+
 #include "tt_internal.h"
 
 struct tt_dav_state {
@@ -29,111 +31,129 @@ struct tt_dav_state {
   double evals[TT_DAV_MAX];
   double coef_x[TT_DAV_MAX];      // Ritz vector:   x = sum_k coef_x[k] v[k]
   double coef_q[TT_DAV_MAX + 1];  // residual:      q = sum_k coef_q[k] va[k] + coef_q[ii+1] x
+  double H[TT_DAV_MAX][TT_DAV_MAX];  // the projected matrix of the one-launch steps (lower triangle)
 };
 
 namespace {
+
+namespace cgx = cooperative_groups;
+
+constexpr int DLD = TT_DAV_MAX + 1;
+struct DiagShared {
+  double A[TT_DAV_MAX * DLD], V[TT_DAV_MAX * DLD];  // element (i, j) at i + DLD j
+  double cs[TT_DAV_MAX / 2], sn[TT_DAV_MAX / 2];
+  int pp[TT_DAV_MAX / 2], qq[TT_DAV_MAX / 2];
+  int order[TT_DAV_MAX];
+};
 
 // DIAG (linalg/lapack_wrapper.cpp:40-54, dsyev semantics) for one warp:
 // parallel cyclic Jacobi with the round-robin ordering (every round rotates
 // n/2 disjoint index pairs at once; Golub & Van Loan, "Matrix Computations",
 // 4th ed., sec. 8.5.5), stopping when the off-diagonal mass falls below
-// 1e-32 of the total, as the host DIAG does.  Eigenvalues ascending in ev,
-// eigenvectors in the columns of M (column-major, n x n).  All 32 lanes call it.
-__device__ void dav_diag_warp(int n, double* M, double* ev) {
-  __shared__ double A[TT_DAV_MAX * TT_DAV_MAX], V[TT_DAV_MAX * TT_DAV_MAX];
-  __shared__ double cs[TT_DAV_MAX / 2], sn[TT_DAV_MAX / 2];
-  __shared__ int pp[TT_DAV_MAX / 2], qq[TT_DAV_MAX / 2];
-  __shared__ int order[TT_DAV_MAX];
+// 1e-32 of the total, as the host DIAG does.  On entry S.A holds the n x n
+// matrix; eigenvalues ascending in ev, the eigenvector of ev[j] in column
+// S.order[j] of S.V.  All 32 lanes call it.
+//
+// A chain of latencies: a round is the rotations (two rsqrt in a row in place
+// of three divisions and two square roots: cos 2t = |d| / r and sin 2t = h / r
+// with d = a_qq - a_pp, h = 2 a_pq, r = |(d, h)|), then one pass that applies
+// them to both sides of the 2 x 2 blocks and to V.  An odd n is padded with a
+// zero row and column, which no rotation touches.
+__device__ void dav_diag_warp(int n, DiagShared& S, double* ev) {
   const int lane = threadIdx.x & 31;
-  for (int i = lane; i < n * n; i += 32) {
-    A[i] = M[i];
-    V[i] = (i % n == i / n) ? 1.0 : 0.0;
+  const int N = n + (n & 1), npair = N / 2;
+  // scaled by a power of two, so that no square leaves the range
+  double mx = 0.0;
+  for (int i = lane; i < n * n; i += 32) mx = fmax(mx, fabs(S.A[i % n + DLD * (i / n)]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const int ex = mx > 0.0 && mx < HUGE_VAL ? ilogb(mx) : 0;
+  double fro = 0.0;
+  for (int e = lane; e < N * N; e += 32) {
+    const int i = e % N, j = e / N;
+    const double a = i < n && j < n ? scalbn(S.A[i + DLD * j], -ex) : 0.0;
+    S.A[i + DLD * j] = a;
+    S.V[i + DLD * j] = i == j ? 1.0 : 0.0;
+    fro = fma(a, a, fro);
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
   __syncwarp();
-  const int N = n + (n & 1);  // even number of players; index n is a bye when n is odd
-  const int npair = N / 2;
+  double off = 0.0;
   for (int sweep = 0; sweep < 100; ++sweep) {
-    double off = 0.0, fro = 0.0;
-    for (int i = lane; i < n * n; i += 32) {
-      const double a2 = A[i] * A[i];
-      fro += a2;
-      if (i % n != i / n) off += a2;
+    off = 0.0;
+    for (int e = lane; e < n * n; e += 32) {
+      const int i = e % n, j = e / n;
+      const double a = S.A[i + DLD * j];
+      if (i != j) off = fma(a, a, off);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      off += __shfl_down_sync(0xffffffffu, off, o);
-      fro += __shfl_down_sync(0xffffffffu, fro, o);
-    }
-    off = __shfl_sync(0xffffffffu, off, 0);  // lane 0's sums decide for the whole warp
-    fro = __shfl_sync(0xffffffffu, fro, 0);
-    if (off <= 1e-32 * fro || off == 0.0) break;
+    for (int o = 16; o > 0; o >>= 1) off += __shfl_xor_sync(0xffffffffu, off, o);
+    if (!(off > 1e-32 * fro)) break;  // the same sums on every lane
     for (int r = 0; r < N - 1; ++r) {
       if (lane < npair) {
         // round-robin: player 0 fixed, the others rotate by r
-        auto player = [&](int i) { return i == 0 ? 0 : ((i - 1 + r) % (N - 1)) + 1; };
-        int a = player(lane), b = player(N - 1 - lane);
-        int p = a < b ? a : b, q = a < b ? b : a;
+        auto player = [&](int i) {
+          int k = i - 1 + r;
+          if (k >= N - 1) k -= N - 1;
+          return i == 0 ? 0 : k + 1;
+        };
+        const int a = player(lane), b = player(N - 1 - lane);
+        const int p = a < b ? a : b, q = a < b ? b : a;
+        const double apq = S.A[p + DLD * q], d = S.A[q + DLD * q] - S.A[p + DLD * p], h = 2.0 * apq;
+        const double r2 = fma(d, d, h * h);
         double c = 1.0, sv = 0.0;
-        if (q < n) {
-          const double apq = A[p + n * q];
-          if (apq != 0.0) {
-            const double tau = (A[q + n * q] - A[p + n * p]) / (2.0 * apq);
-            const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-            c = 1.0 / sqrt(1.0 + t * t);
-            sv = t * c;
-          }
-        } else {
-          q = p;  // bye: identity rotation
+        if (apq != 0.0 && r2 > 0.0) {
+          const double ri = rsqrt(r2), c2 = fma(0.5 * fabs(d), ri, 0.5), ic = rsqrt(c2);
+          c = c2 * ic;
+          sv = 0.5 * h * ri * ic;
+          if (d < 0.0) sv = -sv;
         }
-        pp[lane] = p;
-        qq[lane] = q;
-        cs[lane] = c;
-        sn[lane] = sv;
+        S.pp[lane] = p;
+        S.qq[lane] = q;
+        S.cs[lane] = c;
+        S.sn[lane] = sv;
       }
       __syncwarp();
-      // A <- A J and V <- V J (columns p, q of every pair), then A <- J^T A (rows)
-      for (int it = lane; it < npair * n; it += 32) {
-        const int t = it / n, k = it % n;
-        const int p = pp[t], q = qq[t];
-        if (p == q || sn[t] == 0.0) continue;
-        const double c = cs[t], sv = sn[t];
-        const double akp = A[k + n * p], akq = A[k + n * q];
-        A[k + n * p] = c * akp - sv * akq;
-        A[k + n * q] = sv * akp + c * akq;
-        const double vkp = V[k + n * p], vkq = V[k + n * q];
-        V[k + n * p] = c * vkp - sv * vkq;
-        V[k + n * q] = sv * vkp + c * vkq;
+      // A <- J^T A J by the 2 x 2 blocks (pair s, pair t), V <- V J
+      for (int it = lane; it < npair * (npair + N); it += 32) {
+        const int t = it % npair, u = it / npair;
+        const int p = S.pp[t], q = S.qq[t];
+        const double c = S.cs[t], sv = S.sn[t];
+        if (u < npair) {
+          const int ps = S.pp[u], qs = S.qq[u];
+          const double cu = S.cs[u], su = S.sn[u];
+          double *a0 = S.A + DLD * p, *a1 = S.A + DLD * q;
+          const double a = a0[ps], b = a1[ps], e = a0[qs], f = a1[qs];
+          const double x0 = c * a - sv * b, x1 = sv * a + c * b, y0 = c * e - sv * f, y1 = sv * e + c * f;
+          a0[ps] = cu * x0 - su * y0;
+          a1[ps] = u == t && sv != 0.0 ? 0.0 : cu * x1 - su * y1;
+          a0[qs] = u == t && sv != 0.0 ? 0.0 : su * x0 + cu * y0;
+          a1[qs] = su * x1 + cu * y1;
+        } else {
+          const int k = u - npair;
+          const double vp = S.V[k + DLD * p], vq = S.V[k + DLD * q];
+          S.V[k + DLD * p] = c * vp - sv * vq;
+          S.V[k + DLD * q] = sv * vp + c * vq;
+        }
       }
-      __syncwarp();
-      for (int it = lane; it < npair * n; it += 32) {
-        const int t = it / n, k = it % n;
-        const int p = pp[t], q = qq[t];
-        if (p == q || sn[t] == 0.0) continue;
-        const double c = cs[t], sv = sn[t];
-        const double apk = A[p + n * k], aqk = A[q + n * k];
-        A[p + n * k] = c * apk - sv * aqk;
-        A[q + n * k] = sv * apk + c * aqk;
-      }
-      __syncwarp();
-      if (lane < npair && pp[lane] != qq[lane] && sn[lane] != 0.0) A[pp[lane] + n * qq[lane]] = A[qq[lane] + n * pp[lane]] = 0.0;
       __syncwarp();
     }
   }
-  if (lane == 0) {  // stable insertion sort by eigenvalue
-    for (int i = 0; i < n; ++i) order[i] = i;
-    for (int i = 1; i < n; ++i) {
-      const int o = order[i];
-      int j = i - 1;
-      while (j >= 0 && A[order[j] + n * order[j]] > A[o + n * o]) {
-        order[j + 1] = order[j];
-        --j;
-      }
-      order[j + 1] = o;
+  if (lane < n) {  // rank by eigenvalue, the first index first on ties
+    const double a = S.A[lane + DLD * lane];
+    int rank = 0;
+    for (int i = 0; i < n; ++i) {
+      const double b = S.A[i + DLD * i];
+      rank += (b < a || (b == a && i < lane)) ? 1 : 0;
     }
+    if (!(off == off)) {  // a NaN in the matrix: everything is
+      rank = lane;
+      for (int i = 0; i < n; ++i) S.V[i + DLD * lane] = off;
+    }
+    S.order[rank] = lane;
+    ev[rank] = off == off ? scalbn(a, ex) : off;
   }
-  __syncwarp();
-  for (int j = lane; j < n; j += 32) ev[j] = A[order[j] + n * order[j]];
-  for (int i = lane; i < n * n; i += 32) M[i] = V[(i % n) + n * order[i / n]];
   __syncwarp();
 }
 
@@ -168,16 +188,16 @@ __global__ void dav_ritz_kernel(tt_dav_state* st, int ii) {
       Mn[mi + mj * (ni + 1)] = M[mi + mj * ni];
     }
   }
+  __shared__ DiagShared S;
+  for (int e = lane; e < ni * ni; e += 32) S.A[e % ni + DLD * (e / ni)] = M[e];
   __syncwarp();
-  dav_diag_warp(ni, M, st->evals);
+  dav_diag_warp(ni, S, st->evals);
+  const double* vec = S.V + DLD * S.order[0];
+  const double sgn = (vec[0] < 0.0) ? -1.0 : 1.0;  // sign stabilisation (:265-268)
+  if (lane <= ii) st->coef_x[lane] = st->coef_q[lane] = sgn * vec[lane];
   if (lane == 0) {
     const double lam = st->evals[0];
     st->lambda = lam;
-    const double sgn = (M[0] < 0.0) ? -1.0 : 1.0;  // sign stabilisation (:265-268)
-    for (int k = 0; k <= ii; ++k) {
-      st->coef_x[k] = sgn * M[k];
-      st->coef_q[k] = sgn * M[k];
-    }
     st->coef_q[ii + 1] = -lam;
   }
 }
@@ -305,6 +325,269 @@ dav_refill_kernel(tt_dav_state* st, int ii, int ni, int maxsize, int64_t n, Refi
   }
 }
 
+// ---- one Davidson iteration in one launch ------------------------------------
+//
+// Everything between two products of the Davidson loops: the new row of the
+// projected matrix, its diagonalisation, Ritz vector and residual, the test, and
+// the next basis vector (linalg/tensor_davidson.cpp:193-347 for block-sparse
+// states; DENSE: :74-184, with the diagonal preconditioner and restarts).  One
+// cluster of up to 16 CTAs walks the vectors, which are in L2; the sums go through
+// the CTAs' shared memory, and every CTA adds them up in the same order and takes
+// the same decisions for itself.
+//
+// At these sizes (a chain's bond) a launch that does almost nothing costs the host
+// and the device about 3 us each, and an iteration took twelve of them.
+constexpr int DS_T = 512, DS_W = DS_T / 32, DS_CL = 16;
+
+struct DavStep {
+  const double* v[TT_DAV_MAX];   // basis vectors 0..ii
+  const double* va[TT_DAV_MAX];  // their products
+  const double* y;               // va[ii]
+  double* x;                     // Ritz vector
+  double* q;                     // residual, then the next basis vector
+  const double* D;               // DENSE: the diagonal of the operator
+  double* v0;                    // DENSE, last of a restart: v[0] <- x / |x|
+  const int64_t* ranges;         // where a random refill may draw
+  uint64_t seed;
+  int64_t n;
+  double tol;
+  int ii, maxiter, maxsize, nranges, high, last;
+};
+
+template <int N>
+struct StepSums {
+  double red[DS_W][N], part[2][DS_CL][N], tot[N];
+};
+
+// tot[j] = the cluster's sum of acc[j], j < cnt, on every thread after the call
+template <int N>
+__device__ __forceinline__ void step_sum(double (&acc)[N], int cnt, StepSums<N>& S, int& par, int rank, int CL) {
+  cgx::cluster_group cluster = cgx::this_cluster();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if (j < cnt) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+      if (lane == 0) S.red[warp][j] = acc[j];
+    }
+  }
+  __syncthreads();
+  for (int j = warp; j < cnt; j += DS_W) {
+    double s = S.red[lane & (DS_W - 1)][j];
+#pragma unroll
+    for (int o = DS_W / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane < CL) *cluster.map_shared_rank(&S.part[par][rank][j], lane) = s;
+  }
+  cluster.sync();
+  for (int j = warp; j < cnt; j += DS_W) {
+    double s = lane < CL ? S.part[par][lane][j] : 0.0;
+#pragma unroll
+    for (int o = DS_CL / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) S.tot[j] = s;
+  }
+  __syncthreads();
+  par ^= 1;  // the next sums may arrive while these are still read elsewhere
+}
+
+template <int NV, bool DENSE>
+__global__ void __launch_bounds__(DS_T, 1) dav_step_kernel(tt_dav_state* st, const __grid_constant__ DavStep P) {
+  constexpr int N = NV + 3, U = NV <= 4 ? 4 : NV <= 8 ? 2 : 1;  // sums; elements in flight
+  __shared__ StepSums<N> S;
+  __shared__ DiagShared J;
+  __shared__ double ev[TT_DAV_MAX], coef[NV];
+  const int ii = P.ii, nv = ii + 1;
+  if (!DENSE && ii > 0 && st->done) return;  // the whole cluster alike: written by an earlier launch
+  const double last_lambda = ii > 0 ? st->last_lambda : 1000.0;
+  cgx::cluster_group cluster = cgx::this_cluster();
+  cluster.sync();  // every CTA has started (and read the state) before one is written to
+  const int CL = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x;
+  const bool writer = rank == 0 && tid == 0;
+  const int64_t n = P.n, e0 = rank * DS_T + tid, step = (int64_t)CL * DS_T;
+  int par = 0;
+  double acc[N];
+  auto clear = [&]() {
+#pragma unroll
+    for (int j = 0; j < N; ++j) acc[j] = 0.0;
+  };
+  // f(e, the basis vectors' element e), U elements in flight
+  auto walk = [&](auto pre, auto f) {
+    for (int64_t e = e0; e < n; e += U * step) {
+      double a[U][NV], b[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t i = e + u * step;
+        b[u] = i < n ? pre(i) : 0.0;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) a[u][j] = j < nv && i < n ? P.v[j][i] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (e + u * step < n) f(e + u * step, a[u], b[u]);
+    }
+  };
+  auto overlaps = [&](double b, const double (&a)[NV]) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) acc[j] = fma(a[j], b, acc[j]);
+  };
+  // ---- the new row of the projected matrix ----
+  clear();
+  walk([&](int64_t i) { return P.y[i]; }, [&](int64_t, const double (&a)[NV], double b) { overlaps(b, a); });
+  step_sum(acc, nv, S, par, rank, CL);
+  // ---- its lowest (highest) eigenpair ----
+  if (tid < 32) {
+    for (int e = tid; e < nv * nv; e += 32) {
+      const int i = e % nv, j = e / nv, hi = i > j ? i : j, lo = i > j ? j : i;
+      J.A[i + DLD * j] = hi == ii ? S.tot[lo] : st->H[hi][lo];
+    }
+    __syncwarp();
+    dav_diag_warp(nv, J, ev);
+    const int which = DENSE && P.high ? ii : 0;
+    const double* vec = J.V + DLD * J.order[which];
+    const double sgn = !DENSE && vec[0] < 0.0 ? -1.0 : 1.0;  // sign stabilisation (:265-268)
+    if (tid < nv) {
+      coef[tid] = sgn * vec[tid];
+      if (rank == 0) st->H[ii][tid] = S.tot[tid];
+    }
+  }
+  __syncthreads();
+  const double lambda = ev[DENSE && P.high ? ii : 0];
+  // ---- Ritz vector, residual, its norm and its overlaps with the basis ----
+  clear();
+  for (int64_t e = e0; e < n; e += U * step) {
+    double a[U][NV], b[U][NV], d[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = e + u * step;
+      d[u] = DENSE && i < n ? P.D[i] : 0.0;
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        a[u][j] = j < nv && i < n ? P.v[j][i] : 0.0;
+        b[u][j] = j < nv && i < n ? P.va[j][i] : 0.0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = e + u * step;
+      if (i >= n) continue;
+      double xs = 0.0, qs = 0.0;
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const double c = j < nv ? coef[j] : 0.0;
+        xs = fma(c, a[u][j], xs);
+        qs = fma(c, b[u][j], qs);
+      }
+      qs = fma(-lambda, xs, qs);
+      acc[NV] = fma(qs, qs, acc[NV]);
+      if (DENSE) {
+        if (d[u] != lambda) qs /= d[u] - lambda;  // elemWiseDivide (:25-36)
+        acc[NV + 1] = fma(qs, qs, acc[NV + 1]);
+        acc[NV + 2] = fma(xs, xs, acc[NV + 2]);
+      }
+      overlaps(qs, a[u]);
+      if (DENSE ? P.last : ii > 0) P.x[i] = xs;
+      if (!DENSE || !P.last) P.q[i] = qs;
+    }
+  }
+  step_sum(acc, N, S, par, rank, CL);
+  const double qnorm = sqrt(S.tot[NV]);
+  double inv = 1.0;
+  if (DENSE) {
+    if (writer) {
+      st->lambda = lambda;
+      st->qnorm = qnorm;
+    }
+    if (P.last) {
+      inv = 1.0 / sqrt(S.tot[NV + 2]);
+      for (int64_t i = e0; i < n; i += step) P.v0[i] = P.x[i] * inv;
+      return;
+    }
+    inv = 1.0 / sqrt(S.tot[NV + 1]);
+  } else {
+    const bool converged =
+        (qnorm < P.tol && fabs(lambda - last_lambda) < P.tol) || qnorm < fmax(1e-12, P.tol * 1e-3);
+    const bool ends = qnorm < 1e-20 || (converged && ii >= 1) || ii == P.maxiter;
+    if (writer) {
+      st->lambda = lambda;
+      st->last_lambda = lambda;
+      st->qnorm = qnorm;
+      st->iters = ii;
+      st->done = ends;
+      st->final_ii = ends ? ii : -1;
+      if (ii == 0) {
+        st->fail_ii = -1;
+        st->randomized = 0;
+      }
+    }
+    if (ends) return;
+  }
+  // ---- Gram-Schmidt: q <- scale q - sum_j (scale o_j) v_j and its norm ----
+  auto project = [&](double scale) {
+    double o[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) o[j] = j < nv ? scale * S.tot[j] : 0.0;
+    double norm2 = 0.0;
+    walk([&](int64_t i) { return P.q[i]; },
+         [&](int64_t i, const double (&a)[NV], double b) {
+           b *= scale;
+#pragma unroll
+           for (int j = 0; j < NV; ++j) b = fma(-o[j], a[j], b);
+           P.q[i] = b;
+           norm2 = fma(b, b, norm2);
+         });
+    clear();
+    acc[0] = norm2;
+    step_sum(acc, 1, S, par, rank, CL);
+    return sqrt(S.tot[0]);
+  };
+  double g = project(inv);
+  if (DENSE) {
+    // q was a unit vector: a small remainder is mostly the cancellation's rounding
+    // and is projected again
+    if (g < 0.1) {
+      clear();
+      walk([&](int64_t i) { return P.q[i]; }, [&](int64_t, const double (&a)[NV], double b) { overlaps(b, a); });
+      step_sum(acc, nv, S, par, rank, CL);
+      g = project(1.0 / g);
+    }
+  } else if (!(g >= 1e-10)) {
+    // Gram-Schmidt failure (:298-316): random numbers on the blocks of the vector
+    // before, projected once more; the loop ends when the vectors already span the
+    // problem or that fails too
+    if (nv < P.maxsize) {
+      clear();
+      walk([&](int64_t) { return 0.0; },
+           [&](int64_t i, const double (&a)[NV], double) {
+             int lo = 0, hi = P.nranges;  // is i inside one of the sorted [begin, end) ranges?
+             while (lo < hi) {
+               const int mid = (lo + hi) >> 1;
+               if (P.ranges[2 * mid + 1] <= i) lo = mid + 1; else hi = mid;
+             }
+             double v = 0.0;
+             if (lo < P.nranges && P.ranges[2 * lo] <= i)
+               v = (double)(rf_mix(P.seed ^ (uint64_t)i * 0xD1B54A32D192ED03ull) >> 11) * 0x1.0p-53;
+             P.q[i] = v;
+             overlaps(v, a);
+           });
+      step_sum(acc, nv, S, par, rank, CL);
+      g = project(1.0);
+      if (writer) st->randomized++;
+    }
+    if (!(g >= 1e-10)) {
+      if (writer) {
+        st->done = 1;
+        st->final_ii = ii;
+        st->fail_ii = ii;
+      }
+      return;
+    }
+  }
+  if (!DENSE && writer) st->gsnorm = g;
+  inv = 1.0 / g;
+  for (int64_t i = e0; i < n; i += step) P.q[i] *= inv;
+}
+
 }  // namespace
 
 extern "C" {
@@ -374,6 +657,93 @@ int tt_dav_gs_refill(tt_ctx* ctx, tt_dav_state* st, int ii, int ni, int maxsize,
   dav_refill_kernel<<<nb, RF_THREADS, 0, ctx->stream>>>(st, ii, ni, maxsize, n, v, y, nranges, d_ranges, seed,
                                                         d_gsnorm, part, d_dots, ctx->d_ticket);
   TT_LAUNCH_CHECK(ctx);
+  return TT_OK;
+}
+
+extern "C++" {
+template <bool DENSE>
+static int launch_step(tt_ctx* ctx, tt_dav_state* st, const DavStep& P) {
+  const int nv = P.ii + 1;
+  const void* kernel = nv <= 4   ? (const void*)dav_step_kernel<4, DENSE>
+                       : nv <= 8 ? (const void*)dav_step_kernel<8, DENSE>
+                                 : (const void*)dav_step_kernel<TT_DAV_MAX, DENSE>;
+  int cl = 1;
+  while (cl < DS_CL && (int64_t)cl * DS_T * 2 < P.n) cl *= 2;
+  if (cl > 8) {
+    static thread_local uint64_t attr[3] = {0, 0, 0};  // per host thread and device
+    if (tt::first_on_device(attr[nv <= 4 ? 0 : nv <= 8 ? 1 : 2], ctx->device))
+      TT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = cl;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)cl);
+  cfg.blockDim = dim3(DS_T);
+  cfg.stream = ctx->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  void* argv[] = {(void*)&st, (void*)&P};
+  TT_CUDA(cudaLaunchKernelExC(&cfg, kernel, argv));
+  TT_LAUNCH_CHECK(ctx);
+  return TT_OK;
+}
+}  // extern "C++"
+
+int tt_dav_step(tt_ctx* ctx, tt_dav_state* st, int ii, int maxiter, double tol, int maxsize, int64_t n,
+                const double* const* vs, const double* const* vas, double* x, double* q, int nranges,
+                const int64_t* d_ranges, uint64_t seed) {
+  TT_REQUIRE(ctx && st && vs && vas && x && q && (nranges == 0 || d_ranges), "tt_dav_step: null argument");
+  TT_REQUIRE(ii >= 0 && ii <= maxiter && maxiter + 2 <= TT_DAV_MAX && n >= 1, "tt_dav_step: bad argument");
+  DavStep P = {};
+  for (int j = 0; j <= ii; ++j) {
+    P.v[j] = vs[j];
+    P.va[j] = vas[j];
+  }
+  P.y = vas[ii];
+  P.x = x;
+  P.q = q;
+  P.ranges = d_ranges;
+  P.nranges = nranges;
+  P.seed = seed;
+  P.n = n;
+  P.tol = tol;
+  P.ii = ii;
+  P.maxiter = maxiter;
+  P.maxsize = maxsize;
+  return launch_step<false>(ctx, st, P);
+}
+
+int tt_dav_step_dense(tt_ctx* ctx, tt_dav_state* st, int j, int m, int high, int64_t n, double* const* vs,
+                      const double* const* vas, const double* D, double* x) {
+  TT_REQUIRE(ctx && st && vs && vas && D && x, "tt_dav_step_dense: null argument");
+  TT_REQUIRE(j >= 0 && j < m && m <= TT_DAV_MAX && n >= 1, "tt_dav_step_dense: bad argument");
+  DavStep P = {};
+  for (int k = 0; k <= j; ++k) {
+    P.v[k] = vs[k];
+    P.va[k] = vas[k];
+  }
+  P.y = vas[j];
+  P.x = x;
+  P.last = j == m - 1;
+  P.q = P.last ? nullptr : vs[j + 1];
+  P.v0 = vs[0];
+  P.D = D;
+  P.n = n;
+  P.ii = j;
+  P.high = high;
+  return launch_step<true>(ctx, st, P);
+}
+
+int tt_dav_read_dense(tt_ctx* ctx, const tt_dav_state* st, double* eval, double* r_norm) {
+  TT_REQUIRE(ctx && st && eval && r_norm, "tt_dav_read_dense: null argument");
+  double h[3];
+  static_assert(offsetof(tt_dav_state, qnorm) == offsetof(tt_dav_state, lambda) + 2 * sizeof(double), "read at once");
+  int rc = tt_memcpy_d2h(ctx, h, &st->lambda, sizeof(h));
+  if (rc != TT_OK) return rc;
+  *eval = h[0];
+  *r_norm = h[2];
   return TT_OK;
 }
 

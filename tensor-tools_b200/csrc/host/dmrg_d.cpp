@@ -459,9 +459,45 @@ size_t big_dtensor::size() const {
 }
 
 // ---- restarted Davidson (tensor_davidson.cpp:74-184) ----------------------------
+// Device-resident form for vectors that one launch per step handles: the host
+// enqueues a restart and reads the Ritz value and the residual's norm once at its
+// end (17 reads and 60 vector operations before).
+static double davidson_device(big_dtensor& A, dtensor& x, int m, int max_restart, double tol, char mode,
+                              DavidsonStats* stats) {
+  if (!rt().dav) check(tt_dav_state_create(ctx(), &rt().dav), "davidson state");
+  const int64_t n = x.size;
+  dtensor D = A.diagonal();
+  DevPtr d = aligned(x, D);
+  std::vector<dtensor> v(m, x);  // in x's index order
+  std::vector<double*> pv;
+  for (auto& t : v) pv.push_back(t.data->get());
+  v[0].normalize();
+  DevPtr u = dev_alloc(n);
+  double eval = 0.0, r_norm = 0.0;
+  for (int i = 0; i < max_restart; ++i) {
+    std::vector<DevPtr> va;
+    std::vector<const double*> pa;
+    for (int j = 0; j < m; ++j) {
+      va.push_back(aligned(x, A.product(v[j])));
+      pa.push_back(va.back()->get());
+      if (stats) stats->matvecs++;
+      check(tt_dav_step_dense(ctx(), rt().dav, j, m, mode == 'S' ? 0 : 1, n, pv.data(), pa.data(), d->get(),
+                              u->get()),
+            "davidson step");
+    }
+    check(tt_dav_read_dense(ctx(), rt().dav, &eval, &r_norm), "davidson read");
+    if (stats) stats->iters++;
+    if (r_norm < tol) break;
+  }
+  x.data = u;
+  return eval;
+}
+
 double tensor_davidson(big_dtensor& A, dtensor& x, int m, int max_restart, double tol, char mode,
                        DavidsonStats* stats) {
   if (!(m >= 1 && max_restart >= 1 && tol > 0)) throw std::runtime_error("tensor_davidson: bad arguments");
+  if (x.size >= 1 && x.size <= TT_DAV_STEP_MAX && m <= TT_DAV_MAX)
+    return davidson_device(A, x, m, max_restart, tol, mode, stats);
   std::vector<dtensor> v(m), va(m);
   dtensor D = A.diagonal();
   std::vector<double> M((size_t)(m + 1) * (m + 1), 0.0), Mnext((size_t)(m + 1) * (m + 1), 0.0), evals(m, 0.0);

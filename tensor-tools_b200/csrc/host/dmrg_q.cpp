@@ -456,73 +456,111 @@ static bool davidson_device(big_qtensor& A, qtensor& x, int max_restart, double 
   eng.pack(x, v[0].d->get());
   v[0].p = eng.x_presence();
   va[0] = product(v[0]);
-  {
-    const double* p0 = v[0].d->get();
-    check(tt_vec_multidot(ctx(), n, 1, &p0, va[0].d->get(), scalar_slot(0)), "initial energy");
-  }
-  check(tt_dav_begin(ctx(), st, scalar_slot(0)), "davidson begin");
-  for (int ii = 0; ii < actual_maxiter + 1; ++ii) {
-    const int ni = ii + 1;
-    KVec q = newvec();
-    if (ii == 0) {
-      lincomb(q, {va[0].d->get(), v[0].d->get()}, coef_q, 1.0, 0);
-      q.p = por(va[0].p, v[0].p);
-    } else {
-      check(tt_dav_ritz(ctx(), st, ii), "davidson ritz");
-      KVec xn = newvec();
-      std::vector<const double*> vv, vq;
-      Presence px(v[0].p.size(), 0), pq(v[0].p.size(), 0);
-      for (int k = 0; k <= ii; ++k) {
-        vv.push_back(v[k].d->get());
-        px = por(px, v[k].p);
-        vq.push_back(va[k].d->get());
-        pq = por(pq, va[k].p);
-      }
-      check(tt_vec_ritz_residual_dev(ctx(), n, ii + 1, vv.data(), vq.data(), coef_x, coef_q, xn.d->get(),
-                                     q.d->get()),
-            "ritz vector and residual");
-      xn.p = px;
-      q.p = por(pq, px);
-      xs[ii] = xn;
-    }
-    check(tt_vec_nrm2(ctx(), n, q.d->get(), scalar_slot(kQnormSlot)), "residual norm");
-    check(tt_dav_converged(ctx(), st, ii, actual_maxiter, tol, scalar_slot(kQnormSlot)), "davidson test");
-    v[ni] = q;
-    if (ii == actual_maxiter) break;
-    // one Gram-Schmidt pass (:285-320) with device-side overlaps and norm
-    std::vector<const double*> vs;
-    for (int k = 0; k < ni; ++k) {
-      vs.push_back(v[k].d->get());
-      v[ni].p = por(v[ni].p, v[k].p);
-    }
-    check(tt_vec_multidot(ctx(), n, ni, vs.data(), v[ni].d->get(), scalar_slot(0)), "GS overlaps");
-    check(tt_vec_project_nrm2_dev(ctx(), n, ni, vs.data(), scalar_slot(0), v[ni].d->get(), scalar_slot(kNormSlot)),
-          "GS update and norm");
-    {
-      // Gram-Schmidt failure (:298-316) handled on the device: a random
-      // refill on the blocks of v[ni-1] and one more projection, both no-ops
-      // unless the norm just computed is below 1e-10
-      std::vector<int64_t> ranges;
+  if (n <= TT_DAV_STEP_MAX) {
+    // one launch per iteration.  Which blocks a vector has does not depend on
+    // the numbers, so the element ranges of every possible refill (the blocks of
+    // the vector before) go up in one copy.
+    std::vector<int64_t> ranges, first(1, 0);
+    Presence px = v[0].p, pq = va[0].p;
+    xs[0].p = px;
+    for (int ii = 0; ii < actual_maxiter; ++ii) {
       for (unsigned b = 0; b < eng.ublocks.size(); ++b)
-        if (v[ni - 1].p[b]) {
+        if (v[ii].p[b]) {
           ranges.push_back(eng.ublocks[b].off);
           ranges.push_back(eng.ublocks[b].off + eng.ublocks[b].size);
         }
-      refill_ranges.emplace_back((int64_t)ranges.size() + 1);  // one int64 per 8-byte slot
-      int64_t* dr = reinterpret_cast<int64_t*>(refill_ranges.back().get());
-      if (!ranges.empty()) check(tt_memcpy_h2d(ctx(), dr, ranges.data(), sizeof(int64_t) * ranges.size()), "ranges");
-      check(tt_dav_gs_refill(ctx(), st, ii, ni, maxsize, n, vs.data(), v[ni].d->get(), (int)ranges.size() / 2, dr,
-                             rt().rng_counter++, scalar_slot(kNormSlot), scalar_slot(0)),
-            "GS refill");
-      check(tt_vec_project_nrm2_dev_if(ctx(), n, ni, vs.data(), scalar_slot(0), v[ni].d->get(),
-                                       scalar_slot(kNormSlot), refill_flag),
-            "GS refill projection");
+      first.push_back((int64_t)ranges.size() / 2);
+      v[ii + 1].p = por(pq, px);
+      px = por(px, v[ii + 1].p);
+      pq = por(pq, eng.product_presence(v[ii + 1].p));
+      xs[ii + 1].p = px;
     }
-    check(tt_vec_scal_inv_dev(ctx(), n, scalar_slot(kNormSlot), v[ni].d->get()), "GS scale");
-    va[ni] = product(v[ni]);
-    vs.push_back(v[ni].d->get());
-    check(tt_vec_multidot(ctx(), n, ni + 1, vs.data(), va[ni].d->get(), scalar_slot(0)), "M row");
-    check(tt_dav_add_row(ctx(), st, ii, scalar_slot(0), scalar_slot(kNormSlot)), "davidson row");
+    refill_ranges.emplace_back((int64_t)ranges.size() + 1);  // one int64 per 8-byte slot
+    int64_t* dr = reinterpret_cast<int64_t*>(refill_ranges.back().get());
+    if (!ranges.empty()) check(tt_memcpy_h2d(ctx(), dr, ranges.data(), sizeof(int64_t) * ranges.size()), "ranges");
+    KVec xn = newvec();
+    std::vector<const double*> pv, pa;
+    for (int ii = 0; ii < actual_maxiter + 1; ++ii) {
+      pv.push_back(v[ii].d->get());
+      pa.push_back(va[ii].d->get());
+      const bool more = ii < actual_maxiter;
+      v[ii + 1].d = dev_alloc(n);
+      check(tt_dav_step(ctx(), st, ii, actual_maxiter, tol, maxsize, n, pv.data(), pa.data(), xn.d->get(),
+                        v[ii + 1].d->get(), more ? (int)(first[ii + 1] - first[ii]) : 0,
+                        more ? dr + 2 * first[ii] : nullptr, more ? rt().rng_counter++ : 0),
+            "davidson step");
+      if (more) va[ii + 1] = product(v[ii + 1]);
+      xs[ii].d = xn.d;
+    }
+  } else {
+    {
+      const double* p0 = v[0].d->get();
+      check(tt_vec_multidot(ctx(), n, 1, &p0, va[0].d->get(), scalar_slot(0)), "initial energy");
+    }
+    check(tt_dav_begin(ctx(), st, scalar_slot(0)), "davidson begin");
+    for (int ii = 0; ii < actual_maxiter + 1; ++ii) {
+      const int ni = ii + 1;
+      KVec q = newvec();
+      if (ii == 0) {
+        lincomb(q, {va[0].d->get(), v[0].d->get()}, coef_q, 1.0, 0);
+        q.p = por(va[0].p, v[0].p);
+      } else {
+        check(tt_dav_ritz(ctx(), st, ii), "davidson ritz");
+        KVec xn = newvec();
+        std::vector<const double*> vv, vq;
+        Presence px(v[0].p.size(), 0), pq(v[0].p.size(), 0);
+        for (int k = 0; k <= ii; ++k) {
+          vv.push_back(v[k].d->get());
+          px = por(px, v[k].p);
+          vq.push_back(va[k].d->get());
+          pq = por(pq, va[k].p);
+        }
+        check(tt_vec_ritz_residual_dev(ctx(), n, ii + 1, vv.data(), vq.data(), coef_x, coef_q, xn.d->get(),
+                                       q.d->get()),
+              "ritz vector and residual");
+        xn.p = px;
+        q.p = por(pq, px);
+        xs[ii] = xn;
+      }
+      check(tt_vec_nrm2(ctx(), n, q.d->get(), scalar_slot(kQnormSlot)), "residual norm");
+      check(tt_dav_converged(ctx(), st, ii, actual_maxiter, tol, scalar_slot(kQnormSlot)), "davidson test");
+      v[ni] = q;
+      if (ii == actual_maxiter) break;
+      // one Gram-Schmidt pass (:285-320) with device-side overlaps and norm
+      std::vector<const double*> vs;
+      for (int k = 0; k < ni; ++k) {
+        vs.push_back(v[k].d->get());
+        v[ni].p = por(v[ni].p, v[k].p);
+      }
+      check(tt_vec_multidot(ctx(), n, ni, vs.data(), v[ni].d->get(), scalar_slot(0)), "GS overlaps");
+      check(tt_vec_project_nrm2_dev(ctx(), n, ni, vs.data(), scalar_slot(0), v[ni].d->get(), scalar_slot(kNormSlot)),
+            "GS update and norm");
+      {
+        // Gram-Schmidt failure (:298-316) handled on the device: a random
+        // refill on the blocks of v[ni-1] and one more projection, both no-ops
+        // unless the norm just computed is below 1e-10
+        std::vector<int64_t> ranges;
+        for (unsigned b = 0; b < eng.ublocks.size(); ++b)
+          if (v[ni - 1].p[b]) {
+            ranges.push_back(eng.ublocks[b].off);
+            ranges.push_back(eng.ublocks[b].off + eng.ublocks[b].size);
+          }
+        refill_ranges.emplace_back((int64_t)ranges.size() + 1);  // one int64 per 8-byte slot
+        int64_t* dr = reinterpret_cast<int64_t*>(refill_ranges.back().get());
+        if (!ranges.empty()) check(tt_memcpy_h2d(ctx(), dr, ranges.data(), sizeof(int64_t) * ranges.size()), "ranges");
+        check(tt_dav_gs_refill(ctx(), st, ii, ni, maxsize, n, vs.data(), v[ni].d->get(), (int)ranges.size() / 2, dr,
+                               rt().rng_counter++, scalar_slot(kNormSlot), scalar_slot(0)),
+              "GS refill");
+        check(tt_vec_project_nrm2_dev_if(ctx(), n, ni, vs.data(), scalar_slot(0), v[ni].d->get(),
+                                         scalar_slot(kNormSlot), refill_flag),
+              "GS refill projection");
+      }
+      check(tt_vec_scal_inv_dev(ctx(), n, scalar_slot(kNormSlot), v[ni].d->get()), "GS scale");
+      va[ni] = product(v[ni]);
+      vs.push_back(v[ni].d->get());
+      check(tt_vec_multidot(ctx(), n, ni + 1, vs.data(), va[ni].d->get(), scalar_slot(0)), "M row");
+      check(tt_dav_add_row(ctx(), st, ii, scalar_slot(0), scalar_slot(kNormSlot)), "davidson row");
+    }
   }
   tt_dav_result res;
   check(tt_dav_read(ctx(), st, &res), "davidson read");  // the call's one synchronisation
