@@ -189,6 +189,11 @@ int tt_contract_exec(tt_ctx* ctx, const tt_plan* plan, const double* A,
  * ignore keep. */
 int tt_contract_exec_keep(tt_ctx* ctx, const tt_plan* plan, const double* A, const double* B, double* C,
                           double alpha, int keep);
+/* The same with the device's clock (ns, %globaltimer) written to *d_stamp when the
+ * work before it has ended; for plans with tt_plan_stamps(plan) != 0 (FP64, not empty). */
+int tt_plan_stamps(const tt_plan* plan);
+int tt_contract_exec_stamped(tt_ctx* ctx, const tt_plan* plan, const double* A, const double* B, double* C,
+                             double alpha, int keep, uint64_t* d_stamp);
 int tt_plan_release_packed(tt_ctx* ctx, const tt_plan* plan);
 int tt_plan_destroy(tt_ctx* ctx, tt_plan* plan);
 /* Algorithmic work of one exec: sum over pairs of 2*m*n*k. */
@@ -339,6 +344,11 @@ int tt_dav_step(tt_ctx* ctx, tt_dav_state* st, int ii, int maxiter, double tol, 
  * the residual. */
 int tt_dav_step_dense(tt_ctx* ctx, tt_dav_state* st, int j, int m, int high, int64_t n, double* const* vs,
                       const double* const* vas, const double* D, double* x);
+/* Device clocks of a loop of steps: slots 0..2 of product i may be given to its
+ * three contractions (tt_contract_exec_stamped); slot 3 is written by step i.
+ * tt_dav_read_stamped returns them (TT_DAV_MAX x 4) with the result. */
+int tt_dav_stamp_slots(tt_dav_state* st, int i, uint64_t** d_slots);
+int tt_dav_read_stamped(tt_ctx* ctx, const tt_dav_state* st, tt_dav_result* out, uint64_t* stamps);
 int tt_dav_read_dense(tt_ctx* ctx, const tt_dav_state* st, double* eval, double* r_norm);
 
 /* ---- strided copies ------------------------------------------------------

@@ -26,7 +26,9 @@ struct tt_dav_state {
   int refill;      // 1 while the current new vector is a random refill to orthogonalise
   int randomized;  // random refills in this call
   int cur;       // which of buf[0], buf[1] holds M (the other holds Mnext)
-  double lambda, last_lambda, qnorm, gsnorm;
+  double lambda;
+  unsigned long long stamps[TT_DAV_MAX][4];
+  double last_lambda, qnorm, gsnorm;
   double buf[2][TT_DAV_MAX * TT_DAV_MAX];
   double evals[TT_DAV_MAX];
   double coef_x[TT_DAV_MAX];      // Ritz vector:   x = sum_k coef_x[k] v[k]
@@ -397,6 +399,13 @@ __global__ void __launch_bounds__(DS_T, 1) dav_step_kernel(tt_dav_state* st, con
   __shared__ DiagShared J;
   __shared__ double ev[TT_DAV_MAX], coef[NV];
   const int ii = P.ii, nv = ii + 1;
+  // as after_previous in contract.cu: may start when the blocks of the product before it have ended
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!DENSE && blockIdx.x == 0 && threadIdx.x == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    st->stamps[ii][3] = t;
+  }
   if (!DENSE && ii > 0 && st->done) return;  // the whole cluster alike: written by an earlier launch
   const double last_lambda = ii > 0 ? st->last_lambda : 1000.0;
   cgx::cluster_group cluster = cgx::this_cluster();
@@ -495,7 +504,7 @@ __global__ void __launch_bounds__(DS_T, 1) dav_step_kernel(tt_dav_state* st, con
   double inv = 1.0;
   if (DENSE) {
     if (writer) {
-      st->lambda = lambda;
+      st->last_lambda = lambda;
       st->qnorm = qnorm;
     }
     if (P.last) {
@@ -675,15 +684,17 @@ static int launch_step(tt_ctx* ctx, tt_dav_state* st, const DavStep& P) {
       TT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   }
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = cl;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cl;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = dim3((unsigned)cl);
   cfg.blockDim = dim3(DS_T);
   cfg.stream = ctx->stream;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
   void* argv[] = {(void*)&st, (void*)&P};
   TT_CUDA(cudaLaunchKernelExC(&cfg, kernel, argv));
   TT_LAUNCH_CHECK(ctx);
@@ -738,12 +749,12 @@ int tt_dav_step_dense(tt_ctx* ctx, tt_dav_state* st, int j, int m, int high, int
 
 int tt_dav_read_dense(tt_ctx* ctx, const tt_dav_state* st, double* eval, double* r_norm) {
   TT_REQUIRE(ctx && st && eval && r_norm, "tt_dav_read_dense: null argument");
-  double h[3];
-  static_assert(offsetof(tt_dav_state, qnorm) == offsetof(tt_dav_state, lambda) + 2 * sizeof(double), "read at once");
-  int rc = tt_memcpy_d2h(ctx, h, &st->lambda, sizeof(h));
+  double h[2];
+  static_assert(offsetof(tt_dav_state, qnorm) == offsetof(tt_dav_state, last_lambda) + sizeof(double), "read at once");
+  int rc = tt_memcpy_d2h(ctx, h, &st->last_lambda, sizeof(h));
   if (rc != TT_OK) return rc;
   *eval = h[0];
-  *r_norm = h[2];
+  *r_norm = h[1];
   return TT_OK;
 }
 
@@ -753,13 +764,24 @@ int tt_dav_refill_flag(tt_dav_state* st, const int** d_flag) {
   return TT_OK;
 }
 
+int tt_dav_stamp_slots(tt_dav_state* st, int i, uint64_t** d_slots) {
+  TT_REQUIRE(st && d_slots && i >= 0 && i < TT_DAV_MAX, "tt_dav_stamp_slots: bad argument");
+  *d_slots = reinterpret_cast<uint64_t*>(st->stamps[i]);
+  return TT_OK;
+}
+
 int tt_dav_read(tt_ctx* ctx, const tt_dav_state* st, tt_dav_result* out) {
+  return tt_dav_read_stamped(ctx, st, out, nullptr);
+}
+
+int tt_dav_read_stamped(tt_ctx* ctx, const tt_dav_state* st, tt_dav_result* out, uint64_t* stamps) {
   TT_REQUIRE(ctx && st && out, "tt_dav_read: null argument");
-  // one synchronising read of the header: the flags and the Ritz value
-  constexpr size_t kHead = offsetof(tt_dav_state, lambda) + sizeof(double);
-  alignas(8) unsigned char h[kHead];
-  int rc = tt_memcpy_d2h(ctx, h, st, kHead);
+  // one synchronising read of the header: the flags, the Ritz value, the clocks
+  constexpr size_t kHead = offsetof(tt_dav_state, stamps), kAll = kHead + sizeof(tt_dav_state::stamps);
+  alignas(8) unsigned char h[kAll];
+  int rc = tt_memcpy_d2h(ctx, h, st, stamps ? kAll : kHead);
   if (rc != TT_OK) return rc;
+  if (stamps) std::memcpy(stamps, h + kHead, kAll - kHead);
   tt_dav_state head;
   std::memcpy(&head, h, kHead);
   out->done = head.done;

@@ -230,18 +230,33 @@ class ProductEngine {
   }
 
   // ev (optional): four events recorded before L*x, after it, after *mid and after *R
-  void apply(const double* v, double* y, int precision = TT_PREC_FP64, void* const* ev = nullptr) {
+  // whether the three contractions can stamp the device's clock themselves
+  bool stamps(int precision) {
+    tt_plan* p[3] = {c1_->plan_for(part_precision(precision, 0, part_flops[0]), 1),
+                     c2_->plan_for(part_precision(precision, 1, part_flops[1])),
+                     c3_->plan_for(part_precision(precision, 2, part_flops[2]), 2)};
+    return tt_plan_stamps(p[0]) && tt_plan_stamps(p[1]) && tt_plan_stamps(p[2]);
+  }
+
+  // ev: four events around the contractions; stamps: three device slots for the
+  // clock when each of them starts
+  void apply(const double* v, double* y, int precision = TT_PREC_FP64, void* const* ev = nullptr,
+             uint64_t* stamps = nullptr) {
     if (ev) check(tt_event_record(ctx(), ev[0]), "event");
     if (tt_plan* p = c1_->plan_for(part_precision(precision, 0, part_flops[0]), 1)) {  // L kept through the call
-      check(tt_contract_exec_keep(ctx(), p, L_data(), v, i1_->get(), 1.0, 1 | 8), "heff L*v");
+      check(tt_contract_exec_stamped(ctx(), p, L_data(), v, i1_->get(), 1.0, 1 | 8, stamps), "heff L*v");
       kept_.push_back(p);
     }
     if (ev) check(tt_event_record(ctx(), ev[1]), "event");
     if (tt_plan* p = c2_->plan_for(part_precision(precision, 1, part_flops[1])))
-      check(tt_contract_exec(ctx(), p, i1_->get(), A_.mid().data->get(), i2_->get(), 1.0), "heff *mid");
+      check(tt_contract_exec_stamped(ctx(), p, i1_->get(), A_.mid().data->get(), i2_->get(), 1.0, 0,
+                                     stamps ? stamps + 1 : nullptr),
+            "heff *mid");
     if (ev) check(tt_event_record(ctx(), ev[2]), "event");
     if (tt_plan* p = c3_->plan_for(part_precision(precision, 2, part_flops[2]), 2)) {  // and so is R
-      check(tt_contract_exec_keep(ctx(), p, i2_->get(), A_.right()->data->get(), y, 1.0, 2 | 4), "heff *R");
+      check(tt_contract_exec_stamped(ctx(), p, i2_->get(), A_.right()->data->get(), y, 1.0, 2 | 4,
+                                     stamps ? stamps + 2 : nullptr),
+            "heff *R");
       kept_.push_back(p);
     }
     if (ev) check(tt_event_record(ctx(), ev[3]), "event");
@@ -438,13 +453,24 @@ static bool davidson_device(big_qtensor& A, qtensor& x, int max_restart, double 
     for (size_t i = 0; i < a.size(); ++i) a[i] |= b[i];
     return a;
   };
+  // the products' device times: clocks stamped by the kernels themselves where
+  // one launch per iteration and per contraction allows it, else events
+  const bool steps = n <= TT_DAV_STEP_MAX, stamped = steps && eng.stamps(prec);
   std::vector<std::array<void*, 4>> evs;  // per product: before L*x, after L*x, after *mid, after *R
+  int products = 0;
   auto product = [&](const KVec& in) {
     KVec out = newvec();
-    std::array<void*, 4> e{nullptr, nullptr, nullptr, nullptr};
-    for (auto& x : e) check(tt_event_create(ctx(), &x), "event");
-    eng.apply(in.d->get(), out.d->get(), prec, e.data());
-    evs.push_back(e);
+    if (stamped) {
+      uint64_t* slots = nullptr;
+      check(tt_dav_stamp_slots(st, products, &slots), "stamps");
+      eng.apply(in.d->get(), out.d->get(), prec, nullptr, slots);
+    } else {
+      std::array<void*, 4> e{nullptr, nullptr, nullptr, nullptr};
+      for (auto& x : e) check(tt_event_create(ctx(), &x), "event");
+      eng.apply(in.d->get(), out.d->get(), prec, e.data());
+      evs.push_back(e);
+    }
+    ++products;
     out.p = eng.product_presence(in.p);
     return out;
   };
@@ -456,7 +482,7 @@ static bool davidson_device(big_qtensor& A, qtensor& x, int max_restart, double 
   eng.pack(x, v[0].d->get());
   v[0].p = eng.x_presence();
   va[0] = product(v[0]);
-  if (n <= TT_DAV_STEP_MAX) {
+  if (steps) {
     // one launch per iteration.  Which blocks a vector has does not depend on
     // the numbers, so the element ranges of every possible refill (the blocks of
     // the vector before) go up in one copy.
@@ -563,7 +589,9 @@ static bool davidson_device(big_qtensor& A, qtensor& x, int max_restart, double 
     }
   }
   tt_dav_result res;
-  check(tt_dav_read(ctx(), st, &res), "davidson read");  // the call's one synchronisation
+  uint64_t stamps[TT_DAV_MAX][4];
+  check(tt_dav_read_stamped(ctx(), st, &res, stamped ? &stamps[0][0] : nullptr),
+        "davidson read");  // the call's one synchronisation
   if (res.final_ii == -2 || !res.done) {
     for (auto& e : evs)
       for (void* x : e) tt_event_destroy(x);
@@ -573,19 +601,21 @@ static bool davidson_device(big_qtensor& A, qtensor& x, int max_restart, double 
   if (f >= 1) x = eng.materialize(xs[f].p, xs[f].d);
   x.normalize();
   double heff_ms = 0.0;
-  for (size_t i = 0; i < evs.size(); ++i) {
-    if ((int)i <= f) {  // products of the iterations that ran: the initial one and f more
+  for (int i = 0; i < products; ++i) {
+    if (i <= f) {  // products of the iterations that ran: the initial one and f more
       for (int k = 0; k < 3; ++k) {
         float ms = 0.f;
-        check(tt_event_elapsed_ms(evs[i][k], evs[i][k + 1], &ms), "event");
+        if (stamped) ms = (float)((double)(int64_t)(stamps[i][k + 1] - stamps[i][k]) * 1e-6);
+        else check(tt_event_elapsed_ms(evs[i][k], evs[i][k + 1], &ms), "event");
         heff_ms += ms;
         rt().heff_part_ms[k] += ms;
         rt().heff_part_flops[k] += eng.part_flops[k];
       }
       rt().heff_mid_bytes += eng.mid_bytes;
     }
-    for (void* x : evs[i]) tt_event_destroy(x);
   }
+  for (auto& e : evs)
+    for (void* x : e) tt_event_destroy(x);
   rt().last_heff_ms = heff_ms;
   double lambda = res.lambda;
   if (prec != TT_PREC_FP64 && rt().energy_fp64) {
