@@ -329,106 +329,101 @@ __device__ void tri_solve(const double* d, const double* e, int n, double lambda
   }
 }
 
-// tri_solve for a thread's column of an interleaved batch (y, u0, u1, u2 all
-// with stride st), with the global loads issued PF steps ahead: the values of
-// the next PF steps are fetched while the current PF are computed (the
-// threads of a CTA walk the same rows in lockstep, so the batch's accesses
-// coalesce and the latency of one step is the arithmetic's, not memory's).
-// The same elimination with partial pivoting as tri_solve, but each step
-// takes one reciprocal: u0 keeps 1 / pivot (the pivot clamped to +-tiny as
-// the back substitution of tri_solve clamps it), used for the multiplier
-// and again in the back substitution.  The right-hand side is y * scale
-// (the previous iterate's normalisation, applied as it is read), and the
-// return value is the squared norm of the solution, summed as it is solved.
+// Inverse iteration for one vector per thread, the arrays interleaved (entry i at
+// [i st], so that the threads of a CTA walk the same rows in lockstep and their
+// accesses coalesce; loads run PF rows ahead).  T - lambda is factored once, with
+// partial pivoting: u0 = 1 / pivot (clamped to +-tiny), u1 the next entry of the row
+// and ml the multiplier, whose last bit says whether the rows were exchanged; the
+// third entry of an exchanged row is e[i + 1].  il_factor takes the start vector
+// through the elimination as it goes, il_forward any later one.  A chain per row:
+// one division in the factorisation, two sums in a solve.  T is in shared memory (in
+// global memory no load of it could pass the stores), and a CTA is one warp, so that
+// 3072 vectors are spread over 96 SMs.  Factored anew in each of the three
+// iterations by CTAs of 128: 2.13 ms at bond dimension 3072 (n <= 1471), now 1.03.
 constexpr int PF = 8;
 __device__ __forceinline__ double clamped_rcp(double piv, double tiny) {
   return 1.0 / (fabs(piv) < tiny ? (piv < 0.0 ? -tiny : tiny) : piv);
 }
-__device__ double tri_solve_il(const double* d, const double* e, int n, double lambda, double tiny, double scale,
-                               double* y, double* u0, double* u1, double* u2, int64_t st) {
-  // forward elimination; step i reads y[i + 1]
-  double di = d[0] - lambda, si = n > 1 ? e[0] : 0.0, ti = 0.0;
+template <class Start>
+__device__ void il_factor(const double* d, const double* e, int n, double lambda, double tiny, Start start, double* y,
+                          double* u0, double* u1, double* ml, int64_t st) {
+  double di = d[0] - lambda, si = n > 1 ? e[0] : 0.0, bi = start(0);
+#pragma unroll 4
+  for (int i = 0; i + 1 < n; ++i) {
+    const double ci = e[i], an = d[i + 1] - lambda, bn = i + 2 < n ? e[i + 1] : 0.0, bnext = start(i + 1);
+    const bool sw = fabs(di) < fabs(ci);
+    if (!sw && di == 0.0) di = tiny;
+    const double piv = sw ? ci : di, r = 1.0 / piv;
+    double m = (sw ? di : ci) * r;
+    m = __hiloint2double(__double2hiint(m), (__double2loint(m) & ~1) | (sw ? 1 : 0));
+    u0[i * st] = fabs(piv) < tiny ? clamped_rcp(piv, tiny) : r;
+    u1[i * st] = sw ? an : si;
+    ml[i * st] = m;
+    y[i * st] = sw ? bnext : bi;
+    bi = sw ? bi - m * bnext : bnext - m * bi;
+    di = sw ? si - m * an : an - m * si;
+    si = sw ? -m * bn : bn;
+  }
+  u0[(n - 1) * st] = clamped_rcp(di, tiny);
+  y[(n - 1) * st] = bi;
+}
+// the elimination applied to y * scale (the iterate before, normalised as it is read)
+__device__ void il_forward(int n, double scale, double* y, const double* ml, int64_t st) {
   double bi = y[0] * scale;
-  double cur[PF], nxt[PF];
-#pragma unroll
-  for (int k = 0; k < PF; ++k) cur[k] = 1 + k < n ? y[(int64_t)(1 + k) * st] * scale : 0.0;
-  for (int i0 = 0; i0 + 1 < n; i0 += PF) {
+  double cb[PF], cm[PF], nb[PF], nm[PF];
+  auto load = [&](int i0, double (&b)[PF], double (&m)[PF]) {
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
-      const int r = i0 + PF + 1 + k;
-      nxt[k] = r < n ? y[(int64_t)r * st] * scale : 0.0;
+      const bool in = i0 + k + 1 < n;
+      b[k] = in ? y[(i0 + k + 1) * st] : 0.0;
+      m[k] = in ? ml[(i0 + k) * st] : 0.0;
     }
+  };
+  load(0, cb, cm);
+  for (int i0 = 0; i0 + 1 < n; i0 += PF) {
+    load(i0 + PF, nb, nm);
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
-      const int i = i0 + k;
-      if (i + 1 < n) {
-        double ci = e[i];
-        double an = d[i + 1] - lambda;
-        double bn = (i + 2 < n) ? e[i + 1] : 0.0;
-        double bnext = cur[k];
-        if (fabs(di) >= fabs(ci)) {
-          if (di == 0.0) di = tiny;
-          const double r = 1.0 / di;
-          const double mlt = ci * r;
-          u0[(int64_t)i * st] = fabs(di) < tiny ? clamped_rcp(di, tiny) : r;
-          u1[(int64_t)i * st] = si;
-          u2[(int64_t)i * st] = ti;
-          y[(int64_t)i * st] = bi;
-          bi = bnext - mlt * bi;
-          double nd = an - mlt * si, ns = bn - mlt * ti;
-          di = nd;
-          si = ns;
-          ti = 0.0;
-        } else {
-          const double r = 1.0 / ci;
-          const double mlt = di * r;
-          u0[(int64_t)i * st] = fabs(ci) < tiny ? clamped_rcp(ci, tiny) : r;
-          u1[(int64_t)i * st] = an;
-          u2[(int64_t)i * st] = bn;
-          y[(int64_t)i * st] = bnext;
-          bi = bi - mlt * bnext;
-          double nd = si - mlt * an, ns = ti - mlt * bn;
-          di = nd;
-          si = ns;
-          ti = 0.0;
-        }
+      if (i0 + k + 1 < n) {
+        const double bnext = cb[k] * scale, m = cm[k];
+        const bool sw = __double2loint(m) & 1;
+        y[(i0 + k) * st] = sw ? bnext : bi;
+        bi = sw ? bi - m * bnext : bnext - m * bi;
       }
     }
 #pragma unroll
-    for (int k = 0; k < PF; ++k) cur[k] = nxt[k];
+    for (int k = 0; k < PF; ++k) {
+      cb[k] = nb[k];
+      cm[k] = nm[k];
+    }
   }
-  u0[(int64_t)(n - 1) * st] = clamped_rcp(di, tiny);
-  y[(int64_t)(n - 1) * st] = bi;
-  // back substitution, i = n - 1 down to 0; step i reads y[i], u0[i], u1[i], u2[i]
-  double x1 = 0.0, x2 = 0.0;  // y[i + 1], y[i + 2] as solved
-  double ss = 0.0;
+  y[(n - 1) * st] = bi;
+}
+// back substitution; returns the squared norm of the solution
+__device__ double il_back(const double* e, int n, double* y, const double* u0, const double* u1, const double* ml,
+                          int64_t st) {
+  double x1 = 0.0, x2 = 0.0, ss = 0.0;  // x1, x2: y[i + 1], y[i + 2] as solved
   double cy[PF], c0[PF], c1[PF], c2[PF], ny[PF], n0[PF], n1[PF], n2[PF];
-#pragma unroll
-  for (int k = 0; k < PF; ++k) {
-    const int i = n - 1 - k;
-    cy[k] = i >= 0 ? y[(int64_t)i * st] : 0.0;
-    c0[k] = i >= 0 ? u0[(int64_t)i * st] : 1.0;
-    c1[k] = i >= 0 ? u1[(int64_t)i * st] : 0.0;
-    c2[k] = i >= 0 ? u2[(int64_t)i * st] : 0.0;
-  }
-  for (int b0 = n - 1; b0 >= 0; b0 -= PF) {
+  auto load = [&](int b0, double (&vy)[PF], double (&v0)[PF], double (&v1)[PF], double (&v2)[PF]) {
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
-      const int i = b0 - PF - k;
-      ny[k] = i >= 0 ? y[(int64_t)i * st] : 0.0;
-      n0[k] = i >= 0 ? u0[(int64_t)i * st] : 1.0;
-      n1[k] = i >= 0 ? u1[(int64_t)i * st] : 0.0;
-      n2[k] = i >= 0 ? u2[(int64_t)i * st] : 0.0;
+      const int i = b0 - k;
+      vy[k] = i >= 0 ? y[i * st] : 0.0;
+      v0[k] = i >= 0 ? u0[i * st] : 0.0;
+      v1[k] = i >= 0 && i + 1 < n ? u1[i * st] : 0.0;
+      v2[k] = i >= 0 && i + 2 < n ? ml[i * st] : 0.0;
     }
+  };
+  load(n - 1, cy, c0, c1, c2);
+  for (int b0 = n - 1; b0 >= 0; b0 -= PF) {
+    load(b0 - PF, ny, n0, n1, n2);
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
       const int i = b0 - k;
       if (i >= 0) {
-        double s = cy[k];
-        if (i + 1 < n) s -= c1[k] * x1;
-        if (i + 2 < n) s -= c2[k] * x2;
-        const double xi = s * c0[k];
-        y[(int64_t)i * st] = xi;
+        const double e1 = __double2loint(c2[k]) & 1 ? e[i + 1] : 0.0;  // the rows were exchanged
+        const double xi = fma(-e1, x2, fma(-c1[k], x1, cy[k])) * c0[k];
+        y[i * st] = xi;
         ss = fma(xi, xi, ss);
         x2 = x1;
         x1 = xi;
@@ -1590,13 +1585,15 @@ tridiag_eigvecs_cluster(const EigDev* __restrict__ probs, const double* G, const
 //     columnwise), then the deterministic gauge.
 // Every launch is batched over the problems; (1)-(3) use as many CTAs as
 // there are vectors, rows or tiles.
-constexpr int IV_THREADS = 128;   // vectors per CTA of the inverse iteration
+constexpr int IV_THREADS = 32;    // vectors per CTA of the inverse iteration
 constexpr int GT = 64;            // Gram tile
 constexpr int CH_PB = 32;         // Cholesky panel
+constexpr int CH_THREADS = 256;   // threads per CTA of the Cholesky: 255 registers hold a tile and all its fragments
+constexpr int CH_LD = CH_PB + 2;  // leading dimension of its triangle in shared memory
 constexpr int TS_ROWS = 32;       // rows per CTA of the triangular solve
+constexpr int TS_THREADS = 128;   // its threads: two CTAs of 255 registers per SM
 constexpr int BT_NB = 32;         // reflectors per compact-WY panel
 constexpr int BT_VB = 16;         // vectors per CTA of the back-transformation
-constexpr int BT_ROWS = 64;       // row chunk of the back-transformation
 constexpr double COLLAPSE_PIVOT2 = 1e-8;  // L_jj^2 below this: collapsed vector
 __device__ unsigned long long g_eig_redo;  // problems whose vectors the cluster kernel redid (device-wide)
 
@@ -1618,23 +1615,25 @@ __device__ double tnorm1(const double* d, const double* e, int n, double* red) {
 __global__ void __launch_bounds__(IV_THREADS)
 inv_iter_batched(const EigDev* __restrict__ probs, const VecTask* __restrict__ tasks, const double* Tg,
                  const double* W, double* Zg, double* work) {
+  extern __shared__ double de[];  // T: d and e
   __shared__ double red[33];
   const VecTask tk = tasks[blockIdx.x];
   const EigDev P = probs[tk.prob];
   const int n = P.n;
-  const double* d = Tg + 3 * P.w_off;
-  const double* e = d + n;
+  double *d = de, *e = de + n;
+  for (int i = threadIdx.x; i < 2 * n; i += IV_THREADS) de[i] = i < 2 * n - 1 ? Tg[3 * P.w_off + i] : 0.0;
+  __syncthreads();
   const double* lam = W + P.w_off;
   const double tnorm = tnorm1(d, e, n, red);
   const double tiny = tnorm > 1e-250 ? fmax(DBL_EPSILON * tnorm, DBL_MIN) : 1.0;
   const int t = threadIdx.x, j = tk.j0 + t;
   const int cnt = min(IV_THREADS, P.nvec - tk.j0);  // vectors of this CTA
   const bool active = t < cnt;  // no early return: the barrier below needs every thread
-  // the CTA's iterates and LU factors interleaved (element i of its vector t
-  // at [i cnt + t]), so that the threads' accesses coalesce: the iterates and
-  // two factor rows in the problem's work area (3 n cnt doubles from
-  // work + 3 g_off + 3 n j0), the third factor row in the CTA's own columns
-  // of Z (n cnt doubles), which receive the vectors at the end
+  // the CTA's iterates and factors interleaved (element i of its vector t at
+  // [i cnt + t]), so that the threads' accesses coalesce: the iterates, u0 and u1
+  // in the problem's work area (3 n cnt doubles from work + 3 g_off + 3 n j0), the
+  // multipliers in the CTA's own columns of Z (n cnt doubles), which receive the
+  // vectors at the end
   double* wb = work + 3 * P.g_off + (int64_t)3 * n * tk.j0;
   double* zb = Zg + P.g_off + (int64_t)n * tk.j0;
   double* y = wb + t;
@@ -1643,14 +1642,14 @@ inv_iter_batched(const EigDev* __restrict__ probs, const VecTask* __restrict__ t
   // copy) reads it; its norm is summed in the solve's back substitution
   double inv = 1.0;
   if (active) {
-    for (int i = 0; i < n; ++i)
-      y[(int64_t)i * cnt] = hash_unit(((uint64_t)P.g_off << 20) ^ ((uint64_t)j << 32) ^ (uint64_t)i);
+    const auto start = [&](int i) { return hash_unit(((uint64_t)P.g_off << 20) ^ ((uint64_t)j << 32) ^ (uint64_t)i); };
+    il_factor(d, e, n, lam[j], tiny, start, y, wb + nc + t, wb + 2 * nc + t, zb + t, cnt);
     for (int it = 0; it < INV_ITERS; ++it) {
-      const double s = tri_solve_il(d, e, n, lam[j], tiny, inv, y, wb + nc + t, wb + 2 * nc + t, zb + t, cnt);
-      inv = 1.0 / sqrt(s);
+      if (it > 0) il_forward(n, inv, y, zb + t, cnt);
+      inv = 1.0 / sqrt(il_back(e, n, y, wb + nc + t, wb + 2 * nc + t, zb + t, cnt));
     }
   }
-  __syncthreads();  // every thread's third factor row in Z is dead
+  __syncthreads();  // every thread's multipliers in Z are dead
   if (active) {
     double* z = zb + (int64_t)n * t;
     int i = 0;
@@ -1668,63 +1667,107 @@ inv_iter_batched(const EigDev* __restrict__ probs, const VecTask* __restrict__ t
 }
 
 // (2a) Gram matrix, lower 64 x 64 tiles (a >= b): G[r + m c] = sum_i Z[i, r] Z[i, c],
-// G at work + 3 g_off, leading dimension m = nvec; 256 threads, 4 x 4 outputs each
+// G at work + 3 g_off, leading dimension m = nvec.  On the FP64 tensor path, the
+// fragments straight from Z (four rows of a column are a 32-byte sector): a warp has
+// a 32 x 32 quadrant for every other group of 8 rows.  At bond dimension 3072
+// 342 -> 162 us (16-row stages through shared memory, on the FP64 pipe).
 __global__ void __launch_bounds__(256)
 gram_tiles(const EigDev* __restrict__ probs, const TileTask* __restrict__ tasks, const double* Zg, double* work,
            const int* __restrict__ flags) {
-  __shared__ double sa[16][GT + 2], sb[16][GT + 2];
+  __shared__ double half[4][32][33];
   const TileTask tk = tasks[blockIdx.x];
   if (flags[tk.prob]) return;
   const EigDev P = probs[tk.prob];
   const int n = P.n, m = P.nvec;
   const double* Z = Zg + P.g_off;
   double* Gm = work + 3 * P.g_off;
-  const int r0 = tk.a * GT, c0 = tk.b * GT;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[4][4] = {};
-  for (int i0 = 0; i0 < n; i0 += 16) {
-    __syncthreads();
-    for (int e2 = threadIdx.x; e2 < 16 * GT; e2 += blockDim.x) {
-      const int rr = e2 & 15, cc = e2 >> 4;
-      const int i = i0 + rr;
-      sa[rr][cc] = (i < n && r0 + cc < m) ? Z[i + (int64_t)n * (r0 + cc)] : 0.0;
-      sb[rr][cc] = (i < n && c0 + cc < m) ? Z[i + (int64_t)n * (c0 + cc)] : 0.0;
-    }
-    __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  const int r0 = tk.a * GT + 32 * (warp & 1), c0 = tk.b * GT + 32 * ((warp >> 1) & 1), kh = warp >> 2;
+  double acc[4][4][2] = {};
+  const double *za[4], *zb[4];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      double av[4], bv[4];
+  for (int q = 0; q < 4; ++q) {  // columns past the last repeat it; they are not stored
+    za[q] = Z + (int64_t)n * min(r0 + 8 * q + g, m - 1) + t4;
+    zb[q] = Z + (int64_t)n * min(c0 + 8 * q + g, m - 1) + t4;
+  }
+  auto load = [&](int i, double (&a)[2][4], double (&b)[2][4]) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        av[u] = sa[k][tx * 4 + u];
-        bv[u] = sb[k][ty * 4 + u];
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const bool in = i + 4 * s + t4 < n;
+        a[s][q] = in ? za[q][i + 4 * s] : 0.0;
+        b[s][q] = in ? zb[q][i + 4 * s] : 0.0;
       }
+  };
+  auto use = [&](const double (&a)[2][4], const double (&b)[2][4]) {
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int w = 0; w < 4; ++w) acc[u][w] += av[u] * bv[w];
-    }
+        for (int w = 0; w < 4; ++w) dmma_tr(acc[u][w], a[s][u], b[s][w]);
+  };
+  double a0[2][4], b0[2][4], a1[2][4], b1[2][4];
+  load(8 * kh, a0, b0);
+  for (int i = 8 * kh; i < n; i += 32) {  // one group in flight while the other is used
+    load(i + 16, a1, b1);
+    use(a0, b0);
+    load(i + 32, a0, b0);
+    use(a1, b1);
   }
+  if (kh == 1) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int w = 0; w < 4; ++w)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) half[warp & 3][8 * u + g][8 * w + 2 * t4 + x] = acc[u][w][x];
+  }
+  __syncthreads();
+  if (kh == 1) return;
 #pragma unroll
   for (int u = 0; u < 4; ++u)
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const int r = r0 + tx * 4 + u, c = c0 + ty * 4 + w;
-      if (r < m && c < m && r >= c) Gm[r + (int64_t)m * c] = acc[u][w];
+    for (int w = 0; w < 4; ++w)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const int r = r0 + 8 * u + g, c = c0 + 8 * w + 2 * t4 + x;
+        if (r < m && c < m && r >= c) Gm[r + (int64_t)m * c] = acc[u][w][x] + half[warp][8 * u + g][8 * w + 2 * t4 + x];
+      }
+}
+
+// The triangular solve both (2b) and (2c) need, one row per thread:
+// x <- x L^-T for the 32 x 32 lower triangle whose column c is lt[c][.], rd its
+// reciprocal diagonal.  Column by column, so that the chain is one product and one
+// sum each; two entries of L per load, the same for every thread of the warp.
+__device__ __forceinline__ void solve_row(double (&x)[CH_PB], const double (*lt)[CH_LD], const double* rd) {
+#pragma unroll
+  for (int c = 0; c < CH_PB; ++c) {
+    x[c] *= rd[c];
+#pragma unroll
+    for (int q = (c + 1) / 2; q < CH_PB / 2; ++q) {
+      const double2 l = *reinterpret_cast<const double2*>(&lt[c][2 * q]);
+      if (2 * q > c) x[2 * q] = fma(-x[c], l.x, x[2 * q]);
+      x[2 * q + 1] = fma(-x[c], l.y, x[2 * q + 1]);
     }
+  }
 }
 
 // (2b) Cholesky G = L L^T of the lower triangle in place, right-looking with
-// 32-column panels, one cluster per problem: CTA 0 factors the diagonal
-// block, every CTA solves its share of the panel's rows, the trailing tiles
-// are dealt out to the CTAs.  Pivots below COLLAPSE_PIVOT2 (first pass)
-// flag the problem; a flagged or non-positive pivot is replaced by 1 so the
+// 32-column panels, one cluster per problem.  Every CTA factors the diagonal block
+// for itself (a warp with a row per lane), then the panel's rows go to the cluster's
+// warps 32 at a time, then the trailing matrix 32 x 32 at a time on the FP64 tensor
+// path, the fragments straight from L2, all loads of a tile in flight (two k steps
+// at a time by twice the warps: 646 us).  A panel is a chain of L2 latencies and two
+// cluster barriers.  At bond dimension 3072 1221 -> 372 us (three barriers per
+// column of the block, divisions, 64 x 64 tiles on the FP64 pipe).
+// Pivots below COLLAPSE_PIVOT2 (first pass) flag the problem; a flagged or non-positive pivot is replaced by 1 so the
 // arithmetic stays finite (the problem is redone by the fallback).
-__global__ void __launch_bounds__(TT)
+__global__ void __launch_bounds__(CH_THREADS)
 chol_cluster(const EigDev* __restrict__ probs, double* work, int* flags, int check) {
-  __shared__ double Ld[CH_PB][CH_PB + 1];
-  __shared__ double tl[2][GT][CH_PB + 1];
-  __shared__ int s_flag;
+  __shared__ __align__(16) double lt[CH_PB][CH_LD];
+  __shared__ double rd[CH_PB];
   cgx::cluster_group cluster = cgx::this_cluster();
   const int CL = (int)cluster.num_blocks();
   const int rank = (int)cluster.block_rank();
@@ -1733,99 +1776,124 @@ chol_cluster(const EigDev* __restrict__ probs, double* work, int* flags, int che
   const EigDev P = probs[pi];
   const int m = P.nvec;
   double* A = work + 3 * P.g_off;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int unit0 = rank + CL * warp, units = CL * (CH_THREADS / 32);  // this warp's place in the cluster
   for (int p0 = 0; p0 < m; p0 += CH_PB) {
     const int pb = min(CH_PB, m - p0);
-    // (i) the diagonal block, every CTA (identical arithmetic; only CTA 0 writes)
-    for (int e2 = tid; e2 < pb * pb; e2 += blockDim.x) {
-      const int r = e2 % pb, c = e2 / pb;
-      Ld[r][c] = r >= c ? A[(p0 + r) + (int64_t)m * (p0 + c)] : 0.0;
-    }
-    if (tid == 0) s_flag = 0;
-    __syncthreads();
-    for (int k = 0; k < pb; ++k) {
-      if (tid == 0) {
-        double dk = Ld[k][k];
-        if (!(dk > (check ? COLLAPSE_PIVOT2 : 0.0))) {
-          s_flag = 1;
-          dk = 1.0;
-        }
-        Ld[k][k] = sqrt(dk);
-      }
-      __syncthreads();
-      const double piv = Ld[k][k];
-      for (int r = k + 1 + tid; r < pb; r += blockDim.x) Ld[r][k] /= piv;
-      __syncthreads();
-      for (int e2 = tid; e2 < pb * pb; e2 += blockDim.x) {
-        const int r = e2 % pb, c = e2 / pb;
-        if (c > k && r >= c) Ld[r][c] -= Ld[r][k] * Ld[c][k];
-      }
-      __syncthreads();
-    }
-    if (rank == 0) {
-      for (int e2 = tid; e2 < pb * pb; e2 += blockDim.x) {
-        const int r = e2 % pb, c = e2 / pb;
-        if (r >= c) A[(p0 + r) + (int64_t)m * (p0 + c)] = Ld[r][c];
-      }
-      if (tid == 0 && s_flag && atomicExch(&flags[pi], 1) == 0) atomicAdd(&g_eig_redo, 1ull);
-    }
-    // (ii) rows below the block: L[i, p0:p0+pb] = A[i, p0:p0+pb] L_pp^-T
-    const int rbeg = p0 + pb;
-    for (int i = rbeg + rank * (int)blockDim.x + tid; i < m; i += CL * (int)blockDim.x) {
-      double x[CH_PB];
+    // (i) the diagonal block, lane r its row r; the unit matrix past the last row
+    if (warp == 0) {
+      double a[CH_PB];
 #pragma unroll
-      for (int k = 0; k < CH_PB; ++k) x[k] = k < pb ? A[i + (int64_t)m * (p0 + k)] : 0.0;  // all loads in flight
+      for (int c = 0; c < CH_PB; ++c)
+        a[c] = lane < pb && c <= lane ? A[(p0 + lane) + (int64_t)m * (p0 + c)] : (c == lane ? 1.0 : 0.0);
+      bool bad = false;
+      double my_rd = 1.0;
 #pragma unroll
       for (int k = 0; k < CH_PB; ++k) {
-        if (k < pb) {
-          double v = x[k];
-          for (int t = 0; t < k; ++t) v -= x[t] * Ld[k][t];
-          x[k] = v / Ld[k][k];
-          A[i + (int64_t)m * (p0 + k)] = x[k];
+        double piv = __shfl_sync(0xffffffffu, a[k], k);
+        if (!(piv > (check ? COLLAPSE_PIVOT2 : 0.0)) && k < pb) {
+          bad = true;
+          piv = 1.0;
+        }
+        const double ri = rsqrt(piv);
+        if (lane == k) my_rd = ri;
+        a[k] = lane == k ? piv * ri : (lane > k ? a[k] * ri : 0.0);
+        lt[k][lane] = a[k];
+        __syncwarp();
+#pragma unroll
+        for (int q = (k + 1) / 2; q < CH_PB / 2; ++q) {
+          const double2 l = *reinterpret_cast<const double2*>(&lt[k][2 * q]);
+          if (2 * q > k) a[2 * q] = fma(-a[k], l.x, a[2 * q]);
+          a[2 * q + 1] = fma(-a[k], l.y, a[2 * q + 1]);
         }
       }
+      rd[lane] = my_rd;
+      if (rank == 0 && bad && lane == 0 && atomicExch(&flags[pi], 1) == 0) atomicAdd(&g_eig_redo, 1ull);
+    }
+    __syncthreads();
+    // (ii) rows below the block: L[i, p0:p0+pb] = A[i, p0:p0+pb] L_pp^-T
+    const int rbeg = p0 + pb;  // pb < 32 in the last panel only, which has none
+    for (int i = rbeg + 32 * unit0 + lane; i < m; i += 32 * units) {
+      double x[CH_PB];
+#pragma unroll
+      for (int k = 0; k < CH_PB; ++k) x[k] = A[i + (int64_t)m * (p0 + k)];
+      asm volatile("" : : : "memory");  // or the triangle is kept over the loop, in local memory
+      solve_row(x, lt, rd);
+#pragma unroll
+      for (int k = 0; k < CH_PB; ++k) A[i + (int64_t)m * (p0 + k)] = x[k];
     }
     __threadfence();
     cluster.sync();
-    // (iii) trailing update of the lower tiles (a >= b) of A[rbeg:, rbeg:]
-    const int nt = (m - rbeg + GT - 1) / GT;
-    const int ntiles = nt * (nt + 1) / 2;
-    for (int t = rank; t < ntiles; t += CL) {
+    if (rank == 0 && warp == 0)  // every CTA has read the block
+#pragma unroll
+      for (int c = 0; c < CH_PB; ++c)
+        if (lane < pb && c <= lane) A[(p0 + lane) + (int64_t)m * (p0 + c)] = lt[c][lane];
+    if (rbeg >= m) break;
+    // (iii) trailing update of the lower tiles (ta >= tb) of A[rbeg:, rbeg:]
+    const int nt = (m - rbeg + 31) >> 5, ntiles = nt * (nt + 1) / 2;
+    const int g = lane >> 2, t4 = lane & 3;
+    for (int t = unit0; t < ntiles; t += units) {
       int ta = 0;
       while ((ta + 1) * (ta + 2) / 2 <= t) ++ta;
       const int tb = t - ta * (ta + 1) / 2;
-      const int ra = rbeg + ta * GT, rb = rbeg + tb * GT;
-      __syncthreads();
-      for (int e2 = tid; e2 < GT * pb; e2 += blockDim.x) {
-        const int r = e2 % GT, k = e2 / GT;
-        tl[0][r][k] = ra + r < m ? A[(ra + r) + (int64_t)m * (p0 + k)] : 0.0;
-        tl[1][r][k] = rb + r < m ? A[(rb + r) + (int64_t)m * (p0 + k)] : 0.0;
+      const int ra = rbeg + 32 * ta, rb = rbeg + 32 * tb;
+      const double *la[4], *lb[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {  // rows past the last repeat it; they are not stored
+        la[q] = A + min(ra + 8 * q + g, m - 1) + (int64_t)m * (p0 + t4);
+        lb[q] = A + min(rb + 8 * q + g, m - 1) + (int64_t)m * (p0 + t4);
       }
-      __syncthreads();
-      for (int e2 = tid; e2 < GT * GT; e2 += blockDim.x) {
-        const int r = e2 % GT, c = e2 / GT;
-        const int gi = ra + r, gj = rb + c;
-        if (gi < m && gj < m && gi >= gj) {
-          double acc = 0.0;
-          for (int k = 0; k < pb; ++k) acc += tl[0][r][k] * tl[1][c][k];
-          A[gi + (int64_t)m * gj] -= acc;
+      double acc[4][4][2], a[CH_PB / 4][4], b[CH_PB / 4][4];  // all loads in flight at once
+#pragma unroll
+      for (int k = 0; k < CH_PB / 4; ++k)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          a[k][q] = -la[q][(int64_t)m * (4 * k)];
+          b[k][q] = lb[q][(int64_t)m * (4 * k)];
         }
-      }
+      auto own = [&](int r, int c) { return r < m && c <= r; };
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int r = ra + 8 * u + g, c = rb + 8 * w + 2 * t4 + x;
+            acc[u][w][x] = own(r, c) ? A[r + (int64_t)m * c] : 0.0;
+          }
+#pragma unroll
+      for (int k = 0; k < CH_PB / 4; ++k)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int w = 0; w < 4; ++w) dmma_tr(acc[u][w], a[k][u], b[k][w]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int r = ra + 8 * u + g, c = rb + 8 * w + 2 * t4 + x;
+            if (own(r, c)) A[r + (int64_t)m * c] = acc[u][w][x];
+          }
     }
     __threadfence();
     cluster.sync();
   }
 }
 
-// (2c) Z <- Z L^-T, row by row (rows are independent): TS_ROWS rows per CTA,
-// columns in 32-wide panels: the solved part enters through a small GEMM,
-// the panel's own triangle by substitution
-__global__ void __launch_bounds__(256)
+// (2c) Z <- Z L^-T, row by row (rows are independent): TS_ROWS rows per CTA, columns
+// in 32-wide panels.  The solved part enters through 32 x 32 products on the FP64
+// tensor path, a warp per 32 solved columns, the fragments straight from L2 and L1,
+// all loads of a product in flight; the panel's own triangle by substitution.  At
+// bond dimension 3072 693 -> 312 us; with eight warps of 128 registers and part of
+// the loads in flight 390 to 490.
+__global__ void __launch_bounds__(TS_THREADS, 2)
 trsm_rows(const EigDev* __restrict__ probs, const VecTask* __restrict__ tasks, double* Zg, const double* work,
           const int* __restrict__ flags) {
-  __shared__ double sx[TS_ROWS][CH_PB + 1];   // solved values, one 32-column chunk
-  __shared__ double sl[CH_PB][CH_PB + 1];     // L rows of the panel, one 32-column chunk
-  __shared__ double acc_s[TS_ROWS][CH_PB + 1];
+  __shared__ double zx[TS_ROWS][CH_PB + 1];  // the panel's columns of the rows
+  __shared__ __align__(16) double lt[CH_PB][CH_LD];
+  __shared__ double rd[CH_PB];
   const VecTask tk = tasks[blockIdx.x];
   if (flags[tk.prob]) return;
   const EigDev P = probs[tk.prob];
@@ -1833,65 +1901,75 @@ trsm_rows(const EigDev* __restrict__ probs, const VecTask* __restrict__ tasks, d
   double* Z = Zg + P.g_off;
   const double* L = work + 3 * P.g_off;
   const int i0 = tk.j0;
-  const int tid = threadIdx.x;
-  const int r = tid & 31, cg = tid >> 5;  // row in the block, column group of 4
-  // the chunks of Z (TS_ROWS x CH_PB) and L (CH_PB x CH_PB) are staged
-  // through registers one chunk ahead of the one in shared memory
-  constexpr int PER = TS_ROWS * CH_PB / 256;
-  static_assert(PER * 256 == TS_ROWS * CH_PB && TS_ROWS == CH_PB, "chunk split");
-  auto load = [&](int p0, int pb, int k0, double (&rx)[PER], double (&rl)[PER]) {
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int e2 = tid + 256 * q, rr = e2 % TS_ROWS, kk = e2 / TS_ROWS;
-      rx[q] = i0 + rr < n ? Z[(i0 + rr) + (int64_t)n * (k0 + kk)] : 0.0;
-      rl[q] = rr < pb ? L[(p0 + rr) + (int64_t)m * (k0 + kk)] : 0.0;
-    }
-  };
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
   for (int p0 = 0; p0 < m; p0 += CH_PB) {
     const int pb = min(CH_PB, m - p0);
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    double rx[PER], rl[PER];
-    __syncthreads();  // the previous panel's columns, solved by the first warp, are read below
-    if (p0 > 0) load(p0, pb, 0, rx, rl);
-    for (int k0 = 0; k0 < p0; k0 += CH_PB) {
-      __syncthreads();
+    __syncthreads();  // the columns solved before are complete; zx and lt are free
+    for (int e2 = tid; e2 < TS_ROWS * CH_PB; e2 += TS_THREADS) {
+      const int r = e2 % TS_ROWS, c = e2 / TS_ROWS;
+      zx[r][c] = i0 + r < n && c < pb ? Z[(i0 + r) + (int64_t)n * (p0 + c)] : 0.0;
+      const double l = r < pb && c <= r ? L[(p0 + r) + (int64_t)m * (p0 + c)] : 0.0;
+      lt[c][r] = l;
+      if (r == c) rd[c] = c < pb ? 1.0 / l : 0.0;
+    }
+    double acc[4][4][2] = {};
+    const bool busy = 32 * warp < p0;
+    if (busy) {
+      const double *xa[4], *lb[4];
 #pragma unroll
-      for (int q = 0; q < PER; ++q) {
-        const int e2 = tid + 256 * q, rr = e2 % TS_ROWS, kk = e2 / TS_ROWS;
-        sx[rr][kk] = rx[q];
-        sl[rr][kk] = rl[q];
+      for (int q = 0; q < 4; ++q) {  // rows past the last repeat it; they are not stored
+        xa[q] = Z + min(i0 + 8 * q + g, n - 1) + (int64_t)n * t4;
+        lb[q] = L + min(p0 + 8 * q + g, m - 1) + (int64_t)m * t4;
       }
-      if (k0 + CH_PB < p0) load(p0, pb, k0 + CH_PB, rx, rl);
-      __syncthreads();
-#pragma unroll 8
-      for (int kk = 0; kk < CH_PB; ++kk) {
-        const double xv = sx[r][kk];
+      for (int k0 = 32 * warp; k0 < p0; k0 += TS_THREADS) {
+        double a[CH_PB / 4][4], b[CH_PB / 4][4];  // all loads in flight at once
 #pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u] += xv * sl[cg * 4 + u][kk];
+        for (int k = 0; k < CH_PB / 4; ++k)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            a[k][q] = xa[q][(int64_t)n * (k0 + 4 * k)];
+            b[k][q] = lb[q][(int64_t)m * (k0 + 4 * k)];
+          }
+#pragma unroll
+        for (int k = 0; k < CH_PB / 4; ++k)
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int w = 0; w < 4; ++w) dmma_tr(acc[u][w], a[k][u], b[k][w]);
       }
     }
     __syncthreads();
+    for (int q = 0; q < TS_THREADS / 32 && 32 * q < p0; ++q) {  // one warp after the other: the same order always
+      if (warp == q) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) acc_s[r][cg * 4 + u] = acc[u];
-    for (int e2 = tid; e2 < CH_PB * CH_PB; e2 += blockDim.x) {
-      const int lr = e2 % CH_PB, lk = e2 / CH_PB;
-      sl[lr][lk] = (lr < pb && lk <= lr) ? L[(p0 + lr) + (int64_t)m * (p0 + lk)] : 0.0;
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int w = 0; w < 4; ++w)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) zx[8 * u + g][8 * w + 2 * t4 + x] -= acc[u][w][x];
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    if (tid < TS_ROWS && i0 + tid < n) {
+    if (warp == 0) {
       double x[CH_PB];
-      double* zr = Z + (i0 + tid);
 #pragma unroll
-      for (int c = 0; c < CH_PB; ++c) {
-        if (c < pb) {
-          double v = zr[(int64_t)n * (p0 + c)] - acc_s[tid][c];
-          for (int t = 0; t < c; ++t) v -= x[t] * sl[c][t];
-          x[c] = v / sl[c][c];
-          zr[(int64_t)n * (p0 + c)] = x[c];
-        }
+      for (int c = 0; c < CH_PB; ++c) x[c] = zx[lane][c];
+      solve_row(x, lt, rd);
+      if (i0 + lane < n) {
+#pragma unroll
+        for (int c = 0; c < CH_PB; ++c)
+          if (c < pb) Z[(i0 + lane) + (int64_t)n * (p0 + c)] = x[c];
       }
     }
   }
+}
+
+// entry (row i, reflector a) of the panel of mm reflectors from k0 on: the kept part
+// of column k0 + a below the subdiagonal, 1 on it, 0 above and past the ends
+__device__ __forceinline__ double reflector_entry(const double* Gp, int n, int k0, int mm, int i, int a) {
+  const int ka = k0 + a;
+  if (a >= mm || i >= n || i <= ka) return 0.0;
+  return i == ka + 1 ? 1.0 : Gp[i + (int64_t)n * ka];
 }
 
 // (3a) compact-WY factor T of the reflectors [32 b, 32 b + 32) of a problem:
@@ -1910,22 +1988,43 @@ wy_factors(const EigDev* __restrict__ probs, const TileTask* __restrict__ tasks,
   const double* tau = Tg + 3 * P.w_off + 2 * n;
   const int k0 = tk.a * BT_NB, mm = min(BT_NB, n - 2 - k0);
   double* Tout = work + 3 * P.g_off + (int64_t)P.nvec * P.nvec + (int64_t)tk.a * BT_NB * BT_NB;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  // S(a, c), a < c: v_a . v_c over rows >= k0 + c + 1 (v_c vanishes above)
-  for (int pr = warp; pr < mm * mm; pr += nw) {
-    const int a = pr % mm, c = pr / mm;
-    if (a >= c) continue;
-    const int ka = k0 + a, kc = k0 + c;
-    double acc = 0.0;
-    for (int i = kc + 1 + lane; i < n; i += 32) {
-      const double va = (i == ka + 1) ? 1.0 : Gp[i + (int64_t)n * ka];
-      const double vc = (i == kc + 1) ? 1.0 : Gp[i + (int64_t)n * kc];
-      acc += va * vc;
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) S[a][c] = acc;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  // on the FP64 tensor path: a warp takes every eighth group of 8 rows, and one
+  // fragment of V serves on both sides (at bond dimension 3072 425 -> 43 us; a warp
+  // per dot product read each reflector 31 times)
+  double acc[4][4][2] = {};
+  for (int i = k0 + 1 + 8 * warp; i < n; i += 128) {
+    double v[2][2][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          v[u][x][q] = reflector_entry(Gp, n, k0, mm, i + 64 * u + 4 * x + t4, 8 * q + g);
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) dmma_tr(acc[a][c], v[u][x][a], v[u][x][c]);
   }
-  __syncthreads();
+  for (int q = 0; q < 8; ++q) {
+    if (warp == q) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            double& s = S[8 * a + g][8 * c + 2 * t4 + x];
+            s = q == 0 ? acc[a][c][x] : s + acc[a][c][x];
+          }
+    }
+    __syncthreads();
+  }
   if (threadIdx.x < 32) {
     for (int c = 0; c < mm; ++c) {
       const double tc = tau[k0 + c];
@@ -1948,15 +2047,17 @@ wy_factors(const EigDev* __restrict__ probs, const TileTask* __restrict__ tasks,
 
 // (3b) z = Q y for the vectors [j0, j0 + BT_VB) of a problem: panels last to
 // first, Y <- Y - V (T (V^T Y)) over rows >= k0 + 1; then the gauge (largest
-// magnitude entry positive, first on ties)
+// magnitude entry positive, first on ties).  All three products are on the FP64
+// tensor path, with the fragments of V and Y straight from L2: 16 warps with some
+// 24 loads each in flight, and no barrier inside a product.  At bond dimension 3072
+// 2390 -> 890 us (64-row stages through shared memory, on the FP64 pipe); V comes
+// from L2 twice.
 __global__ void __launch_bounds__(512)
 wy_apply(const EigDev* __restrict__ probs, const VecTask* __restrict__ tasks, const double* G, double* Zg,
          const double* work, const int* __restrict__ flags) {
-  __shared__ double sv[BT_ROWS][BT_NB + 1];
-  __shared__ double sy[BT_ROWS][BT_VB + 1];
-  __shared__ double X[BT_NB][BT_VB + 1];
-  __shared__ double X2[BT_NB][BT_VB + 1];
-  __shared__ double Tm[BT_NB][BT_NB + 1];
+  constexpr int XLD = BT_VB + 4;  // a fragment's rows on different banks
+  __shared__ double part[4][BT_NB][BT_VB];
+  __shared__ double X[BT_NB][XLD], X2[BT_NB][XLD];
   const VecTask tk = tasks[blockIdx.x];
   if (flags[tk.prob]) return;
   const EigDev P = probs[tk.prob];
@@ -1964,91 +2065,105 @@ wy_apply(const EigDev* __restrict__ probs, const VecTask* __restrict__ tasks, co
   const double* Gp = G + P.g_off;
   double* Y = Zg + P.g_off + (int64_t)n * tk.j0;
   const double* Tst = work + 3 * P.g_off + (int64_t)P.nvec * P.nvec;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
   const int npan = (n - 2 + BT_NB - 1) / BT_NB;
-  const int xa = tid / BT_VB, xc = tid % BT_VB;  // the (reflector, vector) entry of X this thread sums
-  // Row chunks of V (BT_ROWS x BT_NB) and Y (BT_ROWS x BT_VB) are staged through
-  // registers one chunk ahead of the one in shared memory, so the global loads
-  // of chunk c + 1 are in flight while chunk c is being used.
-  constexpr int NV_PER = BT_ROWS * BT_NB / 512, NY_PER = BT_ROWS * BT_VB / 512;
-  static_assert(NV_PER * 512 == BT_ROWS * BT_NB && NY_PER * 512 == BT_ROWS * BT_VB, "chunk split");
-  auto load_v = [&](int k0, int mm, int i0, double (&rv)[NV_PER]) {
-#pragma unroll
-    for (int q = 0; q < NV_PER; ++q) {
-      const int e2 = tid + 512 * q, rr = e2 % BT_ROWS, a = e2 / BT_ROWS;
-      const int i = i0 + rr, ka = k0 + a;
-      rv[q] = (a < mm && i < n && i >= ka + 1) ? ((i == ka + 1) ? 1.0 : Gp[i + (int64_t)n * ka]) : 0.0;
-    }
-  };
-  auto load_y = [&](int i0, double (&ry)[NY_PER]) {
-#pragma unroll
-    for (int q = 0; q < NY_PER; ++q) {
-      const int e2 = tid + 512 * q, rr = e2 % BT_ROWS, c = e2 / BT_ROWS;
-      ry[q] = (i0 + rr < n && c < nv) ? Y[(i0 + rr) + (int64_t)n * c] : 0.0;
-    }
-  };
   for (int pnl = npan - 1; pnl >= 0; --pnl) {
     const int k0 = pnl * BT_NB, mm = min(BT_NB, n - 2 - k0);
-    __syncthreads();
-    for (int e2 = tid; e2 < BT_NB * BT_NB; e2 += blockDim.x) Tm[e2 % BT_NB][e2 / BT_NB] = Tst[(int64_t)pnl * BT_NB * BT_NB + e2];
-    double xs = 0.0;
-    double rv[NV_PER], ry[NY_PER];
-    // X = V^T Y over rows >= k0 + 1
-    load_v(k0, mm, k0 + 1, rv);
-    load_y(k0 + 1, ry);
-    for (int i0 = k0 + 1; i0 < n; i0 += BT_ROWS) {
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < NV_PER; ++q) sv[(tid + 512 * q) % BT_ROWS][(tid + 512 * q) / BT_ROWS] = rv[q];
-#pragma unroll
-      for (int q = 0; q < NY_PER; ++q) sy[(tid + 512 * q) % BT_ROWS][(tid + 512 * q) / BT_ROWS] = ry[q];
-      if (i0 + BT_ROWS < n) {
-        load_v(k0, mm, i0 + BT_ROWS, rv);
-        load_y(i0 + BT_ROWS, ry);
-      }
-      __syncthreads();
-#pragma unroll 8
-      for (int rr = 0; rr < BT_ROWS; ++rr) xs += sv[rr][xa] * sy[rr][xc];
-    }
-    X[xa][xc] = xs;
-    __syncthreads();
-    // X2 = T X (T upper triangular)
+    __syncthreads();  // Y of the panel before is complete
+    // X = V^T Y over rows >= k0 + 1, a warp every 16th group of 8 rows
     {
-      double t2 = 0.0;
-      for (int b = xa; b < BT_NB; ++b) t2 += Tm[xa][b] * X[b][xc];
-      X2[xa][xc] = t2;
-    }
-    // Y -= V X2, each thread NY_PER entries of the chunk
-    load_v(k0, mm, k0 + 1, rv);
-    load_y(k0 + 1, ry);
-    for (int i0 = k0 + 1; i0 < n; i0 += BT_ROWS) {
-      __syncthreads();
+      double acc[4][2][2] = {};
+      for (int i = k0 + 1 + 8 * warp; i < n; i += 256) {
+        double v[2][2][4], y[2][2][2];
 #pragma unroll
-      for (int q = 0; q < NV_PER; ++q) sv[(tid + 512 * q) % BT_ROWS][(tid + 512 * q) / BT_ROWS] = rv[q];
-      double yc[NY_PER];
+        for (int u = 0; u < 2; ++u)
 #pragma unroll
-      for (int q = 0; q < NY_PER; ++q) yc[q] = ry[q];
-      if (i0 + BT_ROWS < n) {
-        load_v(k0, mm, i0 + BT_ROWS, rv);
-        load_y(i0 + BT_ROWS, ry);
+          for (int x = 0; x < 2; ++x) {
+            const int r = i + 128 * u + 4 * x + t4;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[u][x][q] = reflector_entry(Gp, n, k0, mm, r, 8 * q + g);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) y[u][x][q] = r < n && 8 * q + g < nv ? Y[r + (int64_t)n * (8 * q + g)] : 0.0;
+          }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+              for (int c = 0; c < 2; ++c) dmma_tr(acc[a][c], v[u][x][a], y[u][x][c]);
       }
-      __syncthreads();
+      for (int q = 0; q < 4; ++q) {  // four warps at a time, in order
+        if (warp >> 2 == q) {
 #pragma unroll
-      for (int q = 0; q < NY_PER; ++q) {
-        const int e2 = tid + 512 * q, rr = e2 % BT_ROWS, c = e2 / BT_ROWS;
-        const int i = i0 + rr;
-        if (i < n && c < nv) {
-          double u = 0.0;
-#pragma unroll 8
-          for (int a = 0; a < BT_NB; ++a) u += sv[rr][a] * X2[a][c];
-          Y[i + (int64_t)n * c] = yc[q] - u;
+          for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int x = 0; x < 2; ++x) {
+                double& s = part[warp & 3][8 * a + g][8 * c + 2 * t4 + x];
+                s = q == 0 ? acc[a][c][x] : s + acc[a][c][x];
+              }
         }
+        __syncthreads();
+      }
+      const int a = tid / BT_VB, c = tid % BT_VB;
+      X[a][c] = (part[0][a][c] + part[1][a][c]) + (part[2][a][c] + part[3][a][c]);
+    }
+    __syncthreads();
+    // X2 = T X (T upper triangular), an 8 x 8 tile per warp
+    if (warp < 8) {
+      const int a = 8 * (warp >> 1), c = 8 * (warp & 1);
+      double tf[8], acc[2] = {};
+#pragma unroll
+      for (int k = 0; k < 8; ++k) tf[k] = Tst[(int64_t)pnl * BT_NB * BT_NB + a + g + BT_NB * (4 * k + t4)];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) dmma_tr(acc, tf[k], X[4 * k + t4][c + g]);
+      X2[a + g][c + 2 * t4] = acc[0];
+      X2[a + g][c + 2 * t4 + 1] = acc[1];
+    }
+    __syncthreads();
+    // Y -= V X2
+    double xf[8][2];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) xf[k][c] = X2[4 * k + t4][8 * c + g];
+    for (int i = k0 + 1 + 8 * warp; i < n; i += 256) {
+      double v[2][8], y[2][2][2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int r = i + 128 * u + g;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[u][k] = -reflector_entry(Gp, n, k0, mm, r, 4 * k + t4);
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int col = 8 * c + 2 * t4 + x;
+            y[u][c][x] = r < n && col < nv ? Y[r + (int64_t)n * col] : 0.0;
+          }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int r = i + 128 * u + g;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) dmma_tr(y[u][c], v[u][k], xf[k][c]);
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int col = 8 * c + 2 * t4 + x;
+            if (r < n && col < nv) Y[r + (int64_t)n * col] = y[u][c][x];
+          }
       }
     }
   }
   __syncthreads();
   // gauge, one warp per vector
-  const int lane = tid & 31, warp = tid >> 5;
   if (warp < nv) {
     double* y = Y + (int64_t)n * warp;
     double best = -1.0;
@@ -2200,8 +2315,8 @@ cudaError_t launch(tt_ctx* ctx, int grid, int block, int cl, size_t smem, bool b
 
 // One cluster of `cl` CTAs per problem; `need` doubles of dynamic shared memory.
 template <class... Args>
-cudaError_t launch_cluster(tt_ctx* ctx, int cl, int n_probs, int64_t need, const void* kernel, Args... args) {
-  return launch(ctx, cl * n_probs, TT, cl, (size_t)(need * 8), false, kernel, args...);
+cudaError_t launch_cluster(tt_ctx* ctx, int cl, int threads, int n_probs, int64_t need, const void* kernel, Args... args) {
+  return launch(ctx, cl * n_probs, threads, cl, (size_t)(need * 8), false, kernel, args...);
 }
 
 }  // namespace
@@ -2318,6 +2433,8 @@ int tt_sym_eigvecs_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
   }
   TT_REQUIRE(big.empty() || cp.cl > 0, "tt_sym_eigvecs_batched: no thread-block clusters for sectors of this size");
   const int n_small = (int)hp.size(), nbig = (int)big.size();
+  int nbig_max = 0;
+  for (const EigDev& e : big) nbig_max = std::max(nbig_max, e.n);
   hp.insert(hp.end(), big.begin(), big.end());
   std::vector<VecTask> iv, ts, ap;
   std::vector<TileTask> gm, wy;
@@ -2364,8 +2481,12 @@ int tt_sym_eigvecs_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
   }
   static thread_local uint64_t attr = 0;  // per host thread and device
   if (tt::first_on_device(attr, ctx->device))
+  {
     TT_CUDA(cudaFuncSetAttribute(eigvecs_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(double) * kVecsSmemCap)));
+    TT_CUDA(cudaFuncSetAttribute(inv_iter_batched, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double) * 2 * MAX_N)));
+  }
   if (n_small > 0) {
     eigvecs_small<<<n_small, small_threads(nsmall_max), sizeof(double) * (size_t)need, ctx->stream>>>(
         dp, G, T, w, Z, work, A, need);
@@ -2375,13 +2496,13 @@ int tt_sym_eigvecs_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
     // the GPU-wide path: inverse iteration, CholeskyQR2, compact-WY
     // back-transformation; problems it flags are redone by the cluster kernel
     if (!iv.empty())
-      TT_CUDA(launch(ctx, (int)iv.size(), IV_THREADS, 0, 0, n_small > 0, (const void*)inv_iter_batched, db, d_iv, T, w,
+      TT_CUDA(launch(ctx, (int)iv.size(), IV_THREADS, 0, sizeof(double) * 2 * (size_t)nbig_max, n_small > 0, (const void*)inv_iter_batched, db, d_iv, T, w,
                      Z, work));
     for (int pass = 0; pass < 2 && !gm.empty(); ++pass) {
       gram_tiles<<<(unsigned)gm.size(), 256, 0, ctx->stream>>>(db, d_gm, Z, work, flags);
       TT_LAUNCH_CHECK(ctx);
-      TT_CUDA(launch_cluster(ctx, cp.cl, nbig, 0, (const void*)chol_cluster, db, work, flags, pass == 0 ? 1 : 0));
-      trsm_rows<<<(unsigned)ts.size(), 256, 0, ctx->stream>>>(db, d_ts, Z, work, flags);
+      TT_CUDA(launch_cluster(ctx, cp.cl, CH_THREADS, nbig, 0, (const void*)chol_cluster, db, work, flags, pass == 0 ? 1 : 0));
+      trsm_rows<<<(unsigned)ts.size(), TS_THREADS, 0, ctx->stream>>>(db, d_ts, Z, work, flags);
       TT_LAUNCH_CHECK(ctx);
     }
     if (!wy.empty()) {
@@ -2397,7 +2518,7 @@ int tt_sym_eigvecs_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
       const int64_t full = q * e.n + extra;
       needc = std::max(needc, full <= cp.vecs_cap ? full : extra);
     }
-    TT_CUDA(launch_cluster(ctx, cp.cl, nbig, needc, (const void*)tridiag_eigvecs_cluster, db, G, T, w, Z, work,
+    TT_CUDA(launch_cluster(ctx, cp.cl, TT, nbig, needc, (const void*)tridiag_eigvecs_cluster, db, G, T, w, Z, work,
                            (int)needc, (const int*)flags));
   }
   tt::pool_free(ctx, buf);
