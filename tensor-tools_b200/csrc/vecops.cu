@@ -49,6 +49,50 @@ struct PtrPack {
   const double* p[MAXVEC];
 };
 
+// f(i, the vectors' pairs, y's pair) for this thread's pairs i, in order, with the
+// loads of U pairs in flight.  NV is the number of vectors (nv), or 16 for more than
+// 8: a load that depends on nv is a branch, and branches keep the loads apart (four
+// overlaps of 8e6 elements: 70 us or 4.6 TB/s, now 52 or 6.1; projection and norm 79
+// and now 64; a copy reaches 6.55).  The fixed grid is four blocks per SM, so up to 8
+// vectors an instance may have 64 registers: with 70 a quarter of the blocks waited
+// for the others.
+template <int NV, int U, class F>
+__device__ __forceinline__ void walk_pairs(int64_t n2, int64_t step, int nv, const PtrPack& xs, const double2* y2, F f) {
+  int64_t i = blockIdx.x * (int64_t)RT + threadIdx.x;
+  auto get = [&](int j, int64_t at) {
+    return NV <= 8 || j < nv ? reinterpret_cast<const double2*>(xs.p[j])[at] : make_double2(0.0, 0.0);
+  };
+  for (; i + (U - 1) * step < n2; i += U * step) {
+    double2 b[U], a[U][NV];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      b[u] = y2[i + u * step];
+#pragma unroll
+      for (int j = 0; j < NV; ++j) a[u][j] = get(j, i + u * step);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) f(i + u * step, a[u], b[u]);
+  }
+  if (U == 1) return;
+  for (; i < n2; i += step) {
+    double2 a[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) a[j] = get(j, i);
+    f(i, a, y2[i]);
+  }
+}
+// the instance of kernel<NV, U> for nv vectors
+#define FOR_VECTORS(kernel, nv)                                                                              \
+  ((nv) <= 1   ? kernel<1, 4>                                                                                \
+   : (nv) == 2 ? kernel<2, 3>                                                                                \
+   : (nv) == 3 ? kernel<3, 2>                                                                                \
+   : (nv) == 4 ? kernel<4, 2>                                                                                \
+   : (nv) == 5 ? kernel<5, 1>                                                                                \
+   : (nv) == 6 ? kernel<6, 1>                                                                                \
+   : (nv) == 7 ? kernel<7, 1>                                                                                \
+   : (nv) == 8 ? kernel<8, 1>                                                                                \
+               : kernel<MAXVEC, 1>)
+
 template <int NV>
 __global__ void __launch_bounds__(RT) multidot_pass1(int64_t n, PtrPack xs,
                                                      const double* __restrict__ y,
@@ -81,26 +125,22 @@ __global__ void __launch_bounds__(RT) multidot_pass1(int64_t n, PtrPack xs,
 // finish (a ticket counter, reset by that block) sums the per-block partials
 // of every vector in the same order as reduce_pass2, so the result is
 // bit-identical to the two-launch form.
-template <int NV>
-__global__ void __launch_bounds__(RT) multidot_fused(int64_t n, PtrPack xs, const double* __restrict__ y,
+template <int NV, int U>
+__global__ void __launch_bounds__(RT, NV <= 8 ? 4 : 1) multidot_fused(int64_t n, PtrPack xs, const double* __restrict__ y,
                                                      double* part, int nv, double* out, int do_sqrt,
                                                      unsigned int* ticket) {
   double acc[NV];
 #pragma unroll
   for (int j = 0; j < NV; ++j) acc[j] = 0.0;
-  const int64_t n2 = n / 2;
+  const int64_t n2 = n / 2, step = (int64_t)gridDim.x * RT;
   const double2* y2 = reinterpret_cast<const double2*>(y);
-  for (int64_t i = blockIdx.x * (int64_t)RT + threadIdx.x; i < n2; i += (int64_t)gridDim.x * RT) {
-    double2 b = y2[i];
+  walk_pairs<NV, U>(n2, step, nv, xs, y2, [&](int64_t, const double2 (&a)[NV], double2 b) {
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-      if (j < nv) {
-        double2 a = reinterpret_cast<const double2*>(xs.p[j])[i];
-        acc[j] = fma(a.x, b.x, acc[j]);
-        acc[j] = fma(a.y, b.y, acc[j]);
-      }
+      acc[j] = fma(a[j].x, b.x, acc[j]);
+      acc[j] = fma(a[j].y, b.y, acc[j]);
     }
-  }
+  });
   if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
 #pragma unroll
     for (int j = 0; j < NV; ++j)
@@ -129,7 +169,8 @@ __global__ void __launch_bounds__(RT) multidot_fused(int64_t n, PtrPack xs, cons
 // norm of its result in one launch.  The grid, the pair-wise walk and the fma
 // order are those of lincomb_kernel (per element) and of multidot_fused<1>
 // (for the norm), so both results are bit-identical to the two launches.
-__global__ void __launch_bounds__(RT) project_nrm2_kernel(int64_t n, int nv, PtrPack xs,
+template <int NV, int U>
+__global__ void __launch_bounds__(RT, NV <= 8 ? 4 : 1) project_nrm2_kernel(int64_t n, int nv, PtrPack xs,
                                                           const double* __restrict__ coef, double* y,
                                                           double* part, double* out, unsigned int* ticket,
                                                           const int* cond) {
@@ -138,19 +179,19 @@ __global__ void __launch_bounds__(RT) project_nrm2_kernel(int64_t n, int nv, Ptr
   if (threadIdx.x < nv) c[threadIdx.x] = -1.0 * coef[threadIdx.x];
   __syncthreads();
   double acc[1] = {0.0};
-  const int64_t n2 = n / 2;
+  const int64_t n2 = n / 2, step = (int64_t)gridDim.x * RT;
   double2* y2 = reinterpret_cast<double2*>(y);
-  for (int64_t i = blockIdx.x * (int64_t)RT + threadIdx.x; i < n2; i += (int64_t)gridDim.x * RT) {
-    double2 b = y2[i];
-    for (int j = 0; j < nv; ++j) {
-      const double2 a = reinterpret_cast<const double2*>(xs.p[j])[i];
-      b.x = fma(c[j], a.x, b.x);
-      b.y = fma(c[j], a.y, b.y);
-    }
+  walk_pairs<NV, U>(n2, step, nv, xs, y2, [&](int64_t i, const double2 (&a)[NV], double2 b) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (j < nv) {
+        b.x = fma(c[j], a[j].x, b.x);
+        b.y = fma(c[j], a[j].y, b.y);
+      }
     y2[i] = b;
     acc[0] = fma(b.x, b.x, acc[0]);
     acc[0] = fma(b.y, b.y, acc[0]);
-  }
+  });
   if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
     double t = y[n - 1];
     for (int j = 0; j < nv; ++j) t = fma(c[j], xs.p[j][n - 1], t);
@@ -257,6 +298,49 @@ __global__ void ritz_residual_kernel(int64_t n, int k, PtrPack vs, PtrPack vas, 
   }
 }
 
+// The same for vectors on 16-byte boundaries, two elements per load and every load of
+// a pair in flight; the element's order of sums is the one above.  k = 4 at 8e6
+// elements: 123 -> 102 us (6.3 TB/s).
+template <int NV, int>
+__global__ void __launch_bounds__(RT, NV <= 4 ? 4 : 1) ritz_residual_pairs(int64_t n, int k, PtrPack vs, PtrPack vas,
+                                                          const double* __restrict__ cx, const double* __restrict__ cq,
+                                                          double* __restrict__ x, double* __restrict__ q) {
+  __shared__ double a[MAXVEC], b[MAXVEC + 1];
+  if (threadIdx.x < k) a[threadIdx.x] = cx[threadIdx.x];
+  if (threadIdx.x <= k) b[threadIdx.x] = cq[threadIdx.x];
+  __syncthreads();
+  const int64_t n2 = n / 2;
+  for (int64_t i = blockIdx.x * (int64_t)RT + threadIdx.x; i < n2; i += (int64_t)gridDim.x * RT) {
+    double2 v[NV], w[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (NV <= 8 || j < k) {
+        v[j] = reinterpret_cast<const double2*>(vs.p[j])[i];
+        w[j] = reinterpret_cast<const double2*>(vas.p[j])[i];
+      }
+    double2 xs = make_double2(0.0, 0.0), qs = xs;
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (NV <= 8 || j < k) {
+        xs.x = fma(a[j], v[j].x, xs.x);
+        xs.y = fma(a[j], v[j].y, xs.y);
+        qs.x = fma(b[j], w[j].x, qs.x);
+        qs.y = fma(b[j], w[j].y, qs.y);
+      }
+    qs.x = fma(b[k], xs.x, qs.x);
+    qs.y = fma(b[k], xs.y, qs.y);
+    reinterpret_cast<double2*>(x)[i] = xs;
+    reinterpret_cast<double2*>(q)[i] = qs;
+  }
+  if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+    double xs = 0.0, qs = 0.0;
+    for (int j = 0; j < k; ++j) xs = fma(a[j], vs.p[j][n - 1], xs);
+    for (int j = 0; j < k; ++j) qs = fma(b[j], vas.p[j][n - 1], qs);
+    x[n - 1] = xs;
+    q[n - 1] = fma(b[k], xs, qs);
+  }
+}
+
 __device__ __forceinline__ uint64_t splitmix64(uint64_t z) {
   z += 0x9E3779B97F4A7C15ull;
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -305,12 +389,8 @@ int launch_multidot(tt_ctx* ctx, int64_t n, int nv, const double* const* xs, con
   int nb = red_blocks(ctx, n);
   double* part = tt::partials(ctx, nb * nv);
   if (!part) return tt::fail(TT_ERR_OOM, "reduction scratch");
-  if (nv <= 1)
-    multidot_fused<1><<<nb, RT, 0, ctx->stream>>>(n, pk, y, part, nv, d_out, do_sqrt, ctx->d_ticket);
-  else if (nv <= 4)
-    multidot_fused<4><<<nb, RT, 0, ctx->stream>>>(n, pk, y, part, nv, d_out, do_sqrt, ctx->d_ticket);
-  else
-    multidot_fused<MAXVEC><<<nb, RT, 0, ctx->stream>>>(n, pk, y, part, nv, d_out, do_sqrt, ctx->d_ticket);
+  const auto fn = FOR_VECTORS(multidot_fused, nv);
+  fn<<<nb, RT, 0, ctx->stream>>>(n, pk, y, part, nv, d_out, do_sqrt, ctx->d_ticket);
   TT_LAUNCH_CHECK(ctx);
   return TT_OK;
 }
@@ -477,7 +557,8 @@ int tt_vec_project_nrm2_dev_if(tt_ctx* ctx, int64_t n, int nvec, const double* c
   const int nb = red_blocks(ctx, n);
   double* part = tt::partials(ctx, nb);
   if (!part) return tt::fail(TT_ERR_OOM, "reduction scratch");
-  project_nrm2_kernel<<<nb, RT, 0, ctx->stream>>>(n, nvec, pk, d_coef, y, part, d_norm, ctx->d_ticket, d_cond);
+  const auto fn = nvec == 0 ? project_nrm2_kernel<MAXVEC, 1> : FOR_VECTORS(project_nrm2_kernel, nvec);
+  fn<<<nb, RT, 0, ctx->stream>>>(n, nvec, pk, d_coef, y, part, d_norm, ctx->d_ticket, d_cond);
   TT_LAUNCH_CHECK(ctx);
   return TT_OK;
 }
@@ -497,7 +578,12 @@ int tt_vec_ritz_residual_dev(tt_ctx* ctx, int64_t n, int k, const double* const*
     pa.p[j] = vas[j];
   }
   if (n <= 0) return TT_OK;
-  ritz_residual_kernel<<<stream_blocks(ctx, n), 256, 0, ctx->stream>>>(n, k, pv, pa, d_coef_x, d_coef_q, x, q);
+  bool pairs = aligned16(x) && aligned16(q);
+  for (int j = 0; j < k; ++j) pairs = pairs && aligned16(vs[j]) && aligned16(vas[j]);
+  const auto fn = pairs ? FOR_VECTORS(ritz_residual_pairs, k) : ritz_residual_kernel;
+  // pairs: no more blocks than are resident
+  const int nb = pairs ? std::min(stream_blocks(ctx, (n + 1) / 2), (k <= 4 ? 4 : 2) * ctx->num_sms) : stream_blocks(ctx, n);
+  fn<<<nb, 256, 0, ctx->stream>>>(n, k, pv, pa, d_coef_x, d_coef_q, x, q);
   TT_LAUNCH_CHECK(ctx);
   return TT_OK;
 }
