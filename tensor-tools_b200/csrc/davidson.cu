@@ -338,7 +338,10 @@ dav_refill_kernel(tt_dav_state* st, int ii, int ni, int maxsize, int64_t n, Refi
 // the same decisions for itself.
 //
 // At these sizes (a chain's bond) a launch that does almost nothing costs the host
-// and the device about 3 us each, and an iteration took twelve of them.
+// and the device about 3 us each, and an iteration took eleven of them.  Measured,
+// 3 and 6 basis vectors: 16384 elements 20 and 31 us (the calls: 66 and 74), 65536
+// 27 and 39 (64 and 75), 262144 46 and 70 (67 and 83), 524288 70 and 111 (79 and 94):
+// 16 SMs read more slowly than 148, hence TT_DAV_STEP_MAX.
 constexpr int DS_T = 512, DS_W = DS_T / 32, DS_CL = 16;
 
 struct DavStep {
@@ -678,11 +681,6 @@ static int launch_step(tt_ctx* ctx, tt_dav_state* st, const DavStep& P) {
                                  : (const void*)dav_step_kernel<TT_DAV_MAX, DENSE>;
   int cl = 1;
   while (cl < DS_CL && (int64_t)cl * DS_T * 2 < P.n) cl *= 2;
-  if (cl > 8) {
-    static thread_local uint64_t attr[3] = {0, 0, 0};  // per host thread and device
-    if (tt::first_on_device(attr[nv <= 4 ? 0 : nv <= 8 ? 1 : 2], ctx->device))
-      TT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -695,6 +693,25 @@ static int launch_step(tt_ctx* ctx, tt_dav_state* st, const DavStep& P) {
   cfg.stream = ctx->stream;
   cfg.attrs = at;
   cfg.numAttrs = 2;
+  if (cl > 8) {
+    // per host thread and device: whether clusters of 16 fit (8 always may)
+    static thread_local uint64_t asked[3] = {0, 0, 0}, fits[3] = {0, 0, 0};
+    const int which = nv <= 4 ? 0 : nv <= 8 ? 1 : 2;
+    const uint64_t bit = (uint64_t)1 << (ctx->device & 63);
+    if (tt::first_on_device(asked[which], ctx->device)) {
+      int nc = 0;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+          cudaOccupancyMaxActiveClusters(&nc, kernel, &cfg) == cudaSuccess && nc >= 1)
+        fits[which] |= bit;
+      else
+        cudaGetLastError();
+    }
+    if (!(fits[which] & bit)) {
+      cl = 8;
+      at[0].val.clusterDim.x = cl;
+      cfg.gridDim = dim3((unsigned)cl);
+    }
+  }
   void* argv[] = {(void*)&st, (void*)&P};
   TT_CUDA(cudaLaunchKernelExC(&cfg, kernel, argv));
   TT_LAUNCH_CHECK(ctx);
