@@ -953,26 +953,41 @@ pack_tf32_ab(const PackJob* __restrict__ jobsA, const PackTile* __restrict__ til
   const double* X = is_a ? A : B;
   const int tid = threadIdx.x;
   uint8_t* dst = (is_a ? pa : pb) + J.dst + (int64_t)(t.rt * J.kt_count + t.kt) * TC_TILE_BYTES;
+  if (J.row_unit) {  // rows are contiguous: a thread has a row, four k at a time
+    const int gr = t.rt * TC_BM + tid, row = gr < J.rows ? tab[J.row_tab + gr] : 0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = J.row_unit ? tid : (tid >> 3) + 16 * i;
-    const int q = J.row_unit ? i : (tid & 7);
-    const int gr = t.rt * TC_BM + r;
-    double x[4];
+    for (int i = 0; i < 8; ++i) {
+      double x[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int gk = t.kt * TC_BK + 4 * q + e;
-      x[e] = (gr < J.rows && gk < J.K) ? X[J.x_off + tab[J.row_tab + gr] + tab[J.k_tab + gk]] : 0.0;
+      for (int e = 0; e < 4; ++e) {
+        const int gk = t.kt * TC_BK + 4 * i + e;
+        x[e] = (gr < J.rows && gk < J.K) ? X[J.x_off + row + tab[J.k_tab + gk]] : 0.0;
+      }
+      uint32_t h[4], l[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        h[e] = to_tf32(__double2float_rn(x[e]));
+        l[e] = SPLIT ? to_tf32(__double2float_rn(x[e] - (double)__uint_as_float(h[e]))) : 0u;
+      }
+      const uint32_t o = sw128_off(tid, 4 * i);
+      *reinterpret_cast<uint4*>(st + o) = make_uint4(h[0], h[1], h[2], h[3]);
+      if (SPLIT) *reinterpret_cast<uint4*>(st + TC_TILE_BYTES / 2 + o) = make_uint4(l[0], l[1], l[2], l[3]);
     }
-    uint32_t h[4], l[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      h[e] = to_tf32(__double2float_rn(x[e]));
-      l[e] = SPLIT ? to_tf32(__double2float_rn(x[e] - (double)__uint_as_float(h[e]))) : 0u;
+  } else {
+    // a warp has a row, a lane a k: 256 contiguous bytes a load where k is contiguous
+    // (eight lanes per row with four k each took four passes over the same sectors:
+    // five products at m = 717 1121 us, now 1050; at m = 3072 16.1 ms, now 15.5)
+    const int lane = tid & 31, gk = t.kt * TC_BK + lane, col = gk < J.K ? tab[J.k_tab + gk] : 0;
+#pragma unroll 16
+    for (int i = 0; i < TC_BM / 4; ++i) {
+      const int r = (tid >> 5) + 4 * i, gr = t.rt * TC_BM + r;
+      const double x = (gr < J.rows && gk < J.K) ? X[J.x_off + tab[J.row_tab + gr] + col] : 0.0;
+      const uint32_t h = to_tf32(__double2float_rn(x));
+      const uint32_t o = sw128_off(r, lane & ~3) + 4 * (lane & 3);
+      *reinterpret_cast<uint32_t*>(st + o) = h;
+      if (SPLIT)
+        *reinterpret_cast<uint32_t*>(st + TC_TILE_BYTES / 2 + o) = to_tf32(__double2float_rn(x - (double)__uint_as_float(h)));
     }
-    const uint32_t o = sw128_off(r, 4 * q);
-    *reinterpret_cast<uint4*>(st + o) = make_uint4(h[0], h[1], h[2], h[3]);
-    if (SPLIT) *reinterpret_cast<uint4*>(st + TC_TILE_BYTES / 2 + o) = make_uint4(l[0], l[1], l[2], l[3]);
   }
   __syncthreads();
   constexpr int NV = (SPLIT ? TC_TILE_BYTES : TC_TILE_BYTES / 2) / 16;
