@@ -1435,14 +1435,19 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
       dtasks.push_back(DTask{o.c_off, o.m, o.n, o.ldc, t.m0, t.n0, t.p_begin, t.p_end, chunks[t.out]});
       longest = std::max(longest, chunks[t.out]);
     }
-    // A tile's k range is shared by a cluster while the plan has fewer than two
-    // rounds of CTAs (four fit an SM) and each keeps two chunks of the longest
-    // tile.  R at bond dimension 1400 (420 tiles, k up to 6552): 1110 us whole, 730
-    // in four; stopping at one round 860.  The products of a chain at bond
-    // dimension 128 (34 tiles of at most 12 chunks): 129 us per three products
-    // whole, 123 down to four chunks, 105 down to two.
-    while (split < SPLIT_MAX && (int64_t)dtasks.size() * split < 8 * (int64_t)ctx->num_sms &&
-           longest / (2 * split) >= 2)
+    // A tile's k range is shared by a cluster while the plan has fewer than two CTAs
+    // per SM and each keeps two chunks of the longest tile; a long k also while it
+    // has fewer than two rounds (four CTAs fit an SM) and each keeps 12.  R at bond
+    // dimension 1400 (420 tiles, k up to 6552): 1110 us whole, 730 in four; stopping
+    // at one round 860.  The products of a chain at 128 (34 tiles of at most 12
+    // chunks): 129 us per three products whole, 123 down to four chunks, 105 down to
+    // two.  Two chunks up to two rounds paid more for the exchange than for the idle
+    // SMs: environment update of the cylinder at 400 85 us, now 67, at 700 190 and
+    // 155; with 8 chunks instead of 12 a chain's at 957 130, now 120, with 16 three
+    // products of a chain at 700 350, now 296.
+    while (split < SPLIT_MAX &&
+           (((int64_t)dtasks.size() * split < 2 * (int64_t)ctx->num_sms && longest / (2 * split) >= 2) ||
+            ((int64_t)dtasks.size() * split < 8 * (int64_t)ctx->num_sms && longest / (2 * split) >= 12)))
       split *= 2;
   }
   std::vector<OutDev> ho(n_out);
