@@ -339,7 +339,9 @@ int tt_dav_step(tt_ctx* ctx, tt_dav_state* st, int ii, int maxiter, double tol, 
                 const int64_t* d_ranges, uint64_t seed);
 /* The same for step j of a restart of the dense loop (linalg/
  * tensor_davidson.cpp:74-184): writes the next basis vector to vs[j + 1], or,
- * for j = m - 1, the Ritz vector to x and, normalised, to vs[0].
+ * for j = m - 1, the Ritz vector to x and, normalised, to vs[0].  Where there is
+ * no further direction (the Ritz vector is an eigenvector, or vs[0..j] span the
+ * space) step j does what step m - 1 does, and the steps after it are no-ops.
  * tt_dav_read_dense synchronises and returns the Ritz value and the norm of
  * the residual. */
 int tt_dav_step_dense(tt_ctx* ctx, tt_dav_state* st, int j, int m, int high, int64_t n, double* const* vs,

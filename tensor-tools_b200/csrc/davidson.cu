@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(DS_T, 1) dav_step_kernel(tt_dav_state* st, con
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     st->stamps[ii][3] = t;
   }
-  if (!DENSE && ii > 0 && st->done) return;  // the whole cluster alike: written by an earlier launch
+  if (ii > 0 && st->done) return;  // the whole cluster alike: written by an earlier launch
   const double last_lambda = ii > 0 ? st->last_lambda : 1000.0;
   cgx::cluster_group cluster = cgx::this_cluster();
   cluster.sync();  // every CTA has started (and read the state) before one is written to
@@ -505,16 +505,32 @@ __global__ void __launch_bounds__(DS_T, 1) dav_step_kernel(tt_dav_state* st, con
   step_sum(acc, N, S, par, rank, CL);
   const double qnorm = sqrt(S.tot[NV]);
   double inv = 1.0;
+  // DENSE: there is no further direction.  The restart ends with the present Ritz
+  // vector in x and, normalised, in v[0]; its later steps do nothing.
+  auto end_restart = [&]() {
+    const double scale = 1.0 / sqrt(S.tot[NV + 2]);
+    walk([&](int64_t) { return 0.0; },
+         [&](int64_t i, const double (&a)[NV], double) {
+           double xs = 0.0;
+#pragma unroll
+           for (int j = 0; j < NV; ++j) xs = fma(j < nv ? coef[j] : 0.0, a[j], xs);
+           P.x[i] = xs;
+           P.v0[i] = xs * scale;
+         });
+    if (writer) st->done = 1;
+  };
   if (DENSE) {
     if (writer) {
       st->last_lambda = lambda;
       st->qnorm = qnorm;
+      st->done = 0;
     }
     if (P.last) {
       inv = 1.0 / sqrt(S.tot[NV + 2]);
       for (int64_t i = e0; i < n; i += step) P.v0[i] = P.x[i] * inv;
       return;
     }
+    if (S.tot[NV + 1] == 0.0) return end_restart();  // the Ritz vector is an eigenvector
     inv = 1.0 / sqrt(S.tot[NV + 1]);
   } else {
     const bool converged =
@@ -556,8 +572,11 @@ __global__ void __launch_bounds__(DS_T, 1) dav_step_kernel(tt_dav_state* st, con
   double g = project(inv);
   if (DENSE) {
     // q was a unit vector: a small remainder is mostly the cancellation's rounding
-    // and is projected again
-    if (g < 0.1) {
+    // and is projected again.  Rounding that lies outside the basis is as good a
+    // direction as a random one and keeps its length; of rounding that lies in it, a
+    // basis that spans the space, nothing is left time after time.
+    for (int again = 0; g < 0.1; ++again) {
+      if (again == 2 || g == 0.0) return end_restart();
       clear();
       walk([&](int64_t i) { return P.q[i]; }, [&](int64_t, const double (&a)[NV], double b) { overlaps(b, a); });
       step_sum(acc, nv, S, par, rank, CL);

@@ -511,13 +511,19 @@ double tensor_davidson(big_dtensor& A, dtensor& x, int m, int max_restart, doubl
           double alpha = v[k].inner_product(v[j]);
           v[j].add(v[k], -alpha);
         }
-        return v[j].normalize();
+        double g = v[j].norm();
+        if (g != 0.0 || j == 0) v[j] /= g;
+        return g;
       };
       // x is a unit vector: a small remainder is mostly the cancellation's
       // rounding and has to be projected again, or the projected matrix belongs
       // to a basis that is not orthonormal (a converged residual is nearly
-      // parallel to v[0]; the Ritz value then came out up to 5e-3 too high)
-      if (project() < 0.1 && j > 0) project();
+      // parallel to v[0]; the Ritz value then came out up to 5e-3 too high).
+      // Nothing is left time after time when the basis spans the space: the
+      // restart then ends with the present Ritz vector u.
+      double g = project();
+      for (int again = 0; j > 0 && g < 0.1 && g != 0.0 && again < 2; ++again) g = project();
+      if (j > 0 && g < 0.1) break;
       va[j] = A.product(v[j]);
       if (stats) stats->matvecs++;
       int l = j;
@@ -559,7 +565,9 @@ double tensor_davidson(big_dtensor& A, dtensor& x, int m, int max_restart, doubl
         // elemWiseDivide (tensor_davidson.cpp:25-36)
         DevPtr d = aligned(x, D);
         check(tt_vec_precondition(ctx(), x.size, x.data->get(), d->get(), eval), "precondition");
-        x.normalize();
+        double g = x.norm();
+        if (g == 0.0) break;  // u is an eigenvector
+        x /= g;
       }
       std::swap(M, Mnext);
     }
