@@ -329,12 +329,27 @@ __device__ void tri_solve(const double* d, const double* e, int n, double lambda
   }
 }
 
+// One step of the elimination of T - lambda with partial pivoting, rows exchanged
+// when sw: the multiplier is at most 1, so the top bit of its exponent is free, and
+// there the exchange is kept (in the last bit of its fraction the multiplier lost that
+// bit: vectors of a 4096-row chain 25 times further off).
+__device__ __forceinline__ double multiplier_of(double num, double piv, double rcp) {
+  return fabs(piv) < 0x1p-1000 ? num / piv : num * rcp;  // the reciprocal of a denormal pivot overflows
+}
+__device__ __forceinline__ double with_exchange(double m, bool sw) {
+  return __hiloint2double(__double2hiint(m) | (sw ? 0x40000000 : 0), __double2loint(m));
+}
+__device__ __forceinline__ bool exchanged(double f) { return (__double2hiint(f) & 0x40000000) != 0; }
+__device__ __forceinline__ double multiplier(double f) {
+  return __hiloint2double(__double2hiint(f) & ~0x40000000, __double2loint(f));
+}
+
 // Inverse iteration for one vector per thread, the arrays interleaved (entry i at
 // [i st], so that the threads of a CTA walk the same rows in lockstep and their
 // accesses coalesce; loads run PF rows ahead).  T - lambda is factored once, with
 // partial pivoting: u0 = 1 / pivot (clamped to +-tiny), u1 the next entry of the row
-// and ml the multiplier, whose last bit says whether the rows were exchanged; the
-// third entry of an exchanged row is e[i + 1].  il_factor takes the start vector
+// and ml the multiplier with the exchange of the rows; the third entry of an exchanged
+// row is e[i + 1].  il_factor takes the start vector
 // through the elimination as it goes, il_forward any later one.  A chain per row:
 // one division in the factorisation, two sums in a solve.  T is in shared memory (in
 // global memory no load of it could pass the stores), and a CTA is one warp, so that
@@ -354,11 +369,10 @@ __device__ void il_factor(const double* d, const double* e, int n, double lambda
     const bool sw = fabs(di) < fabs(ci);
     if (!sw && di == 0.0) di = tiny;
     const double piv = sw ? ci : di, r = 1.0 / piv;
-    double m = (sw ? di : ci) * r;
-    m = __hiloint2double(__double2hiint(m), (__double2loint(m) & ~1) | (sw ? 1 : 0));
+    const double m = multiplier_of(sw ? di : ci, piv, r);
     u0[i * st] = fabs(piv) < tiny ? clamped_rcp(piv, tiny) : r;
     u1[i * st] = sw ? an : si;
-    ml[i * st] = m;
+    ml[i * st] = with_exchange(m, sw);
     y[i * st] = sw ? bnext : bi;
     bi = sw ? bi - m * bnext : bnext - m * bi;
     di = sw ? si - m * an : an - m * si;
@@ -385,8 +399,8 @@ __device__ void il_forward(int n, double scale, double* y, const double* ml, int
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
       if (i0 + k + 1 < n) {
-        const double bnext = cb[k] * scale, m = cm[k];
-        const bool sw = __double2loint(m) & 1;
+        const double bnext = cb[k] * scale, m = multiplier(cm[k]);
+        const bool sw = exchanged(cm[k]);
         y[(i0 + k) * st] = sw ? bnext : bi;
         bi = sw ? bi - m * bnext : bnext - m * bi;
       }
@@ -421,7 +435,7 @@ __device__ double il_back(const double* e, int n, double* y, const double* u0, c
     for (int k = 0; k < PF; ++k) {
       const int i = b0 - k;
       if (i >= 0) {
-        const double e1 = __double2loint(c2[k]) & 1 ? e[i + 1] : 0.0;  // the rows were exchanged
+        const double e1 = exchanged(c2[k]) ? e[i + 1] : 0.0;
         const double xi = fma(-e1, x2, fma(-c1[k], x1, cy[k])) * c0[k];
         y[i * st] = xi;
         ss = fma(xi, xi, ss);
@@ -458,9 +472,7 @@ __device__ __forceinline__ double hash_unit(uint64_t z) {
 // Eigenvectors of the sectors with n <= SN, one CTA each.
 //
 // (a) Inverse iteration, one thread per vector: T - lambda I is factored once
-//     (one reciprocal per step; the row exchange is kept in the last bit of the
-//     multiplier, which the factorisation itself uses too), the INV_ITERS solves
-//     then are substitutions only.
+//     (one reciprocal per step), the INV_ITERS solves then are substitutions only.
 // (b) Gram-Schmidt inside clusters, right-looking and twice: once vector j is
 //     final, every warp takes it out of its share of the later members, so a
 //     vector costs one barrier.  A vector that the first pass has left less than
@@ -472,6 +484,7 @@ __device__ __forceinline__ double hash_unit(uint64_t z) {
 // Gram-Schmidt vector by vector with eight barriers each and two barriers per
 // reflector: at bond dimension 75 (n <= 36) 108 -> 52 us, at 512 (n <= 75) 282 ->
 // 116 us.
+
 // Solve with the factors of (T - lambda I): y = the solution for y * scale;
 // returns its squared norm.  Entry i of the factors is at [i * st].
 __device__ __forceinline__ double small_solve(int n, double scale, double* y, const double* u0, const double* u1,
@@ -479,8 +492,8 @@ __device__ __forceinline__ double small_solve(int n, double scale, double* y, co
   double bi = y[0] * scale;
 #pragma unroll 4
   for (int i = 0; i + 1 < n; ++i) {
-    const double bn = y[i + 1] * scale, m = ml[i * st];
-    const bool sw = __double2loint(m) & 1;
+    const double bn = y[i + 1] * scale, f = ml[i * st], m = multiplier(f);
+    const bool sw = exchanged(f);
     const double top = sw ? bn : bi, low = sw ? bi : bn;
     y[i] = top;
     bi = fma(-m, top, low);
@@ -598,12 +611,11 @@ eigvecs_small(const EigDev* __restrict__ probs, const double* G, const double* T
       const bool sw = fabs(di) < fabs(ci);
       if (!sw && di == 0.0) di = tiny;
       const double piv = sw ? ci : di, r = 1.0 / piv;
-      double m = (sw ? di : ci) * r;
-      m = __hiloint2double(__double2hiint(m), (__double2loint(m) & ~1) | (sw ? 1 : 0));
+      const double m = multiplier_of(sw ? di : ci, piv, r);
       f0[i * st] = fabs(piv) < tiny ? 1.0 / clamped(piv) : r;
       f1[i * st] = sw ? an : si;
       f2[i * st] = sw ? bn : 0.0;
-      fm[i * st] = m;
+      fm[i * st] = with_exchange(m, sw);
       di = sw ? si - m * an : an - m * si;
       si = sw ? -m * bn : bn;
     }
