@@ -211,7 +211,7 @@ void measure_sz(const qMPS& psi, std::vector<double>& sz, std::vector<double>& s
     qtensor S = with_origin(qtensor(), EL[i0]);
     for (unsigned j = i0; j < L; ++j) {
       auto cc = contract_cached(S, ZR[j], false);
-      if (tt_plan* p = cc->plan_for(rt().precision))
+      if (tt_plan* p = cc->plan_for(TT_PREC_FP64))  // an inner product, whatever operator* runs in
         check(tt_contract_exec(bound_ctx(), p, S.data->get(), ZR[j].data->get(), vals.get() + (size_t)j * row, 1.0),
               "contract exec");
       if (j + 1 == L) break;
