@@ -528,7 +528,7 @@ narrow_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const
     const double* Bp = B + E.off;
     for (int c = lane >> 3; c < E.n; c += 4)
       for (int kk = lane & 7; kk < E.k; kk += 8)
-        sb[(E.k0 + kk) * NR_LD + E.c0 + c] = Bp[(E.ks != NO_STRIDE ? kk * E.ks : tab[E.ktab + kk]) +
+        sb[(E.k0 + kk) * NR_LD + E.c0 + c] = Bp[(int64_t)(E.ks != NO_STRIDE ? kk * E.ks : tab[E.ktab + kk]) +
                                                 (E.cs != NO_STRIDE ? c * E.cs : tab[E.ctab + c])];
     q += NR_WARPS;
     if (q < ch.b_end) E = nb[q];
