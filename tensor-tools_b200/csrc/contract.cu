@@ -1279,13 +1279,14 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
       by_a[sig].push_back(o);
     }
     // the two strides (first extent d0) that a pair's row modes merge into;
-    // d0 = 0 when they do not
+    // d0 = 0 when they do not.  One stride alone fits any d0, with s1 = s0 d0.
     struct Rows {
       int64_t d0, s0, s1;
+      bool one;
     };
     auto rows_of = [&](int i) {
       const tt_block_pair& q = pairs[order[i]];
-      Rows r{1, 0, 0};
+      Rows r{1, 0, 0, true};
       int groups = 0;
       int64_t next = 0;
       for (int d = 0; d < q.n_m; ++d) {
@@ -1301,11 +1302,11 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
           r.s1 = st;
           groups = 2;
         } else {
-          return Rows{0, 0, 0};
+          return Rows{0, 0, 0, false};
         }
         next = st * e;
       }
-      if (groups <= 1) r.s1 = -1;  // any d0 will do: s1 = s0 d0
+      r.one = groups <= 1;
       return r;
     };
     std::vector<std::pair<int64_t, std::vector<int>>> groups;  // the chunks of one signature, and their cost
@@ -1334,14 +1335,14 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
         for (int i : op) {
           rw.push_back(rows_of(i));
           if (rw.back().d0 == 0) two = false;
-          if (rw.back().s1 >= 0) {
+          if (!rw.back().one) {
             two = two && (d0 == 0 || d0 == rw.back().d0);
             d0 = rw.back().d0;
           }
         }
         if (d0 == 0) d0 = c.m;
         for (size_t u = 0; u < op.size(); ++u) {
-          const int64_t s1 = rw[u].s1 < 0 ? rw[u].s0 * d0 : rw[u].s1;
+          const int64_t s1 = rw[u].one ? rw[u].s0 * d0 : rw[u].s1;
           two = two && rw[u].s0 >= 0 && rw[u].s0 <= INT_MAX && s1 >= 0 && s1 <= INT_MAX;
         }
         c.d0 = two ? (int32_t)d0 : 0;
@@ -1349,7 +1350,7 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
           const PairDev& P = hp[op[u]];
           const tt_block_pair& q = pairs[order[op[u]]];
           NrA x{P.a_off, two ? (int32_t)rw[u].s0 : P.rowA, 0, c.ktot, P.k, P.a_ks, 0};
-          if (two) x.s1 = (int32_t)(rw[u].s1 < 0 ? rw[u].s0 * d0 : rw[u].s1);
+          if (two) x.s1 = (int32_t)(rw[u].one ? rw[u].s0 * d0 : rw[u].s1);
           if (P.a_ks != NO_STRIDE) {
             nr_a.push_back(x);
           } else {  // k modes that do not merge: one entry per k

@@ -69,3 +69,35 @@ def test_offsets_beyond_31_bits(ctx):
     a = A.reshape(2, m).T
     bound = 2 * 2 * 2.0 ** -53 * (a.abs() @ b.abs())
     assert torch.all((out.reshape(2, m).T - a @ b).abs() <= bound)
+
+
+@pytest.mark.parametrize("kind", ["rows", "rows inner", "columns", "k"])
+def test_negative_strides(ctx, kind):
+    """Modes walked backwards: the second or the first row mode, B's columns, both operands' k."""
+    import torch
+    md, k, n = (40, 9), 5, 6
+    g = torch.Generator(device="cuda").manual_seed(2)
+    A, B = (torch.randn(s, dtype=torch.float64, device="cuda", generator=g) for s in (3 * 360 * k, 3 * k * n))
+    am, ak, bk, bn = [1, 40], [360], [1], [k]
+    ao = bo = 0
+    if kind == "rows":
+        am, ao = [1, -40], 320
+    elif kind == "rows inner":
+        am, ao = [-1, 40], 39
+    elif kind == "columns":
+        bn, bo = [-k], k * (n - 1)
+    else:
+        ak, ao, bk, bo = [-360], 360 * (k - 1), [-1], k - 1
+    a = A[:360 * k].reshape(k, 9, 40)
+    b = B[:k * n].reshape(n, k)
+    if kind == "rows":
+        a = a.flip(1)
+    elif kind == "rows inner":
+        a = a.flip(2)
+    elif kind == "columns":
+        b = b.flip(0)
+    a, b = a.reshape(k, 360).T, b.T
+    out = _exec(ctx, [(0, 360, n, 360)], [(0, 2, 1, 1, ao, bo, _pad(md), _pad([k]), _pad([n]), _pad(am), _pad(ak),
+                                           _pad(bk), _pad(bn))], A, B, 360 * n, alpha=-0.5)
+    bound = 2 * k * 2.0 ** -53 * 0.5 * (a.abs() @ b.abs())
+    assert torch.all((out.reshape(n, 360).T + 0.5 * (a @ b)).abs() <= bound)
