@@ -18,6 +18,7 @@
 #include <functional>
 #include <map>
 #include <numeric>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -407,9 +408,10 @@ grouped_dgemm(const DTask* __restrict__ tasks,
 // time: lane r copies row r of every k to shared memory (8-byte cp.async: 256
 // contiguous bytes per k for a unit row stride), one tile ahead of the one that
 // the m8n8k4 FP64 tensor-core products multiply with the chunk's B (staged once
-// per CTA) into all the chunk's columns.  So T1 crosses HBM once, no column or
-// k is padded by more than a fragment, and after the staging a warp needs no
-// barrier.
+// per CTA) into all the chunk's columns.  So T1 is read once per NR_N columns that
+// contract the same A blocks (an output block that shares only some of them is in a
+// chunk of its own and reads them again), no column or k is padded by more than a
+// fragment, and after the staging a warp needs no barrier.
 // Measured on the middle contraction (read T1, write T2): bond dimension 3072
 // (2.03 GB) 1131 -> 620 us (1.8 -> 3.3 TB/s), 1400 (0.42 GB) 246 -> 119 us,
 // against a thread per row with the products as FP64 FMAs, 16 columns a time.
@@ -418,8 +420,9 @@ grouped_dgemm(const DTask* __restrict__ tasks,
 // five CTAs at 96 registers 740 us; A loaded straight into the fragments 853 us.
 constexpr int NR_N = 32;          // columns of a chunk, at most
 constexpr int NR_K = 64;          // k of a pair, at most
-constexpr int NR_KTOT = 256;      // k of a chunk, at most (its B is staged whole)
-constexpr int NR_LD = NR_N + 4;   // row stride of the staged B: a fragment's 4 k on different banks
+constexpr int NR_KTOT = 256;      // k of a chunk, at most (its B is staged whole; 106 KB with 32 columns, two CTAs)
+// row stride of the staged B: a fragment's 4 k on different banks
+__host__ __device__ constexpr int narrow_ld(int cols) { return ((cols + 7) & ~7) + 4; }
 constexpr int NR_BUF = 512;       // elements of a warp's A buffer: its rows times 16 k (32 rows) or 64 k (8 rows)
 constexpr int NR_AMAX = 16;       // A blocks of a chunk staged in shared memory, at most
 constexpr int NR_WARPS = 4;
@@ -459,8 +462,28 @@ __device__ __forceinline__ void dmma_k4(double (&c)[2], double a, double b) {
 __host__ __device__ constexpr int narrow_buf(int ktot, int rw) {
   return rw * ((ktot + 3) & ~3) < NR_BUF ? rw * ((ktot + 3) & ~3) : NR_BUF;
 }
-__host__ __device__ constexpr size_t narrow_smem(int ktot, int rw) {
-  return sizeof(double) * ((size_t)NR_WARPS * 2 * narrow_buf(ktot, rw) + (size_t)((ktot + 3) & ~3) * NR_LD);
+__host__ __device__ constexpr size_t narrow_smem(int ktot, int rw, int ld) {
+  return sizeof(double) * ((size_t)NR_WARPS * 2 * narrow_buf(ktot, rw) + (size_t)((ktot + 3) & ~3) * ld);
+}
+
+// The B blocks of a chunk, its k from s0 to s1, into shared memory (row stride ld): a
+// warp per block, 8 k x 4 columns at a time.  first: the warp's first block, fetched
+// before.  Asynchronous copies, which the caller waits for: as loads they came one
+// after the other, and 160 k of 16 columns took 20 us.
+__device__ __forceinline__ void stage_b(double* sb, int ld, int s0, int s1, const double* B, const NrB* __restrict__ nb,
+                                        int b_end, int q, int warps, NrB E, const int32_t* __restrict__ tab) {
+  const int lane = threadIdx.x & 31;
+  while (q < b_end) {
+    const double* Bp = B + E.off;
+    const int lo = max(s0 - E.k0, 0), hi = min(s1 - E.k0, E.k);
+    for (int c = lane >> 3; c < E.n; c += 4)
+      for (int kk = lo + (lane & 7); kk < hi; kk += 8)
+        cp_async8(sb + (E.k0 + kk - s0) * ld + E.c0 + c, Bp + (int64_t)(E.ks != NO_STRIDE ? kk * E.ks : tab[E.ktab + kk]) +
+                                                             (E.cs != NO_STRIDE ? c * E.cs : tab[E.ctab + c]));
+    q += warps;
+    if (q < b_end) E = nb[q];
+  }
+  cp_async_commit();
 }
 
 // RW: rows of a warp's tile, 32 or 8
@@ -468,7 +491,7 @@ template <int RW>
 __global__ void __launch_bounds__(NR_THREADS, 4)
 narrow_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const NrB* __restrict__ nb,
              const int64_t* __restrict__ nc, const int32_t* __restrict__ tab, const double* __restrict__ A, const double* __restrict__ B,
-             double* __restrict__ C, double alpha, int abuf, unsigned long long* stamp) {
+             double* __restrict__ C, double alpha, int abuf, int ld, unsigned long long* stamp) {
   extern __shared__ double smem[];
   __shared__ int64_t sc[NR_N];
   __shared__ NrA sa[NR_AMAX];  // the chunk's A blocks, from the second fetch on
@@ -479,7 +502,7 @@ narrow_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const
   const int ktot = ch.ktot, kz = (ktot + 3) & ~3;
   constexpr int KB = NR_BUF / RW, MT = RW / 8, ROWS = RW * NR_WARPS, LK = 32 / RW;
   double* buf = smem + warp * 2 * abuf;      // this warp's two A buffers, [k][RW rows]
-  double* sb = smem + NR_WARPS * 2 * abuf;   // B, [kz][NR_LD]
+  double* sb = smem + NR_WARPS * 2 * abuf;   // B, [kz][ld]
   // row r of k in a buffer: a fragment's 4 k x 4 rows on different banks
   auto at = [](int k, int r) { return RW * k + (RW == 32 ? r ^ ((k & 3) << 2) : r); };
   const int nblk = ch.a_end - ch.a_begin;
@@ -518,21 +541,15 @@ narrow_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const
   if (q < ch.b_end) E = nb[q];
   after_previous(tab, stamp);
   asm volatile("" : "+l"(B) : : "memory");
+  // the chunk's B, and behind it the first k of A; zero where there is no column or k
+  stage_b(sb, ld, 0, ktot, B, nb, ch.b_end, q, NR_WARPS, E, tab);
   if (tiles > 0 && nkb > 0) fetch(0, 0, 0);
   cp_async_commit();
-
-  // the chunk's B: a warp per block, 8 k x 4 columns at a time; zero where there is no column or k
-  for (int k = warp; k < kz; k += NR_WARPS)
-    if (k >= ktot || lane >= ch.cols) sb[k * NR_LD + lane] = 0.0;
-  while (q < ch.b_end) {
-    const double* Bp = B + E.off;
-    for (int c = lane >> 3; c < E.n; c += 4)
-      for (int kk = lane & 7; kk < E.k; kk += 8)
-        sb[(E.k0 + kk) * NR_LD + E.c0 + c] = Bp[(int64_t)(E.ks != NO_STRIDE ? kk * E.ks : tab[E.ktab + kk]) +
-                                                (E.cs != NO_STRIDE ? c * E.cs : tab[E.ctab + c])];
-    q += NR_WARPS;
-    if (q < ch.b_end) E = nb[q];
-  }
+  if (tid < (kz - ktot) * ld) sb[ktot * ld + tid] = 0.0;
+  const int cpad = ch.cols + (lane & 7);
+  if (cpad < ((ch.cols + 7) & ~7))
+    for (int k = 4 * warp + (lane >> 3); k < ktot; k += 4 * NR_WARPS) sb[k * ld + cpad] = 0.0;
+  cp_async_wait<1>();
   __syncthreads();
   if (nblk <= NR_AMAX) blocks = sa;
 
@@ -552,7 +569,7 @@ narrow_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const
       __syncwarp();
       const int kn = min(KB, ktot - kb * KB);
       const double* as = buf + b * abuf;
-      const double* bs = sb + (kb * KB + t4) * NR_LD + g;
+      const double* bs = sb + (kb * KB + t4) * ld + g;
 #pragma unroll 2
       for (int k = 0; k < kn; k += 4) {
         double a[MT];
@@ -561,7 +578,7 @@ narrow_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (j < nt) {
-            const double bv = bs[k * NR_LD + 8 * j];
+            const double bv = bs[k * ld + 8 * j];
 #pragma unroll
             for (int i = 0; i < MT; ++i) dmma_k4(acc[i][j], a[i], bv);
           }
@@ -598,6 +615,95 @@ narrow_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const
       }
   }
   cp_async_wait<0>();
+}
+
+// The same chunks with a thread per row, its up to NC columns as FP64 sums in registers,
+// 16 loads of A in flight: no fragment is padded and A does not pass through shared
+// memory.  Better where a chunk has few columns, which is where the products above are
+// mostly padding and instruction issue (1e6 rows, k = 160: 1 column 190 us, 8 columns
+// 238, by fragments 521 and 529; the rule is at the plan).  B is staged whole or, beyond
+// RD_SEG bytes, in segments of kseg k, anew for every tile.
+constexpr int RD_COLS = 16;            // columns of a chunk, at most
+constexpr int RD_SEG = 96 * 1024;      // bytes of staged B, at most
+
+// SEG: more k than a segment, 256 rows to a CTA, else 128
+template <int NC, bool SEG>
+__global__ void __launch_bounds__(SEG ? 256 : 128)
+rows_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const NrB* __restrict__ nb,
+           const int64_t* __restrict__ nc, const int32_t* __restrict__ tab, const double* __restrict__ A,
+           const double* __restrict__ B, double* __restrict__ C, double alpha, int kseg, unsigned long long* stamp) {
+  extern __shared__ double smem[];  // B, [kseg][NC]
+  __shared__ int64_t sc[NC];
+  __shared__ NrA sa[NR_AMAX];
+  const NrTask task = tasks[blockIdx.x];
+  const NrChunk& ch = task.ch;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int nblk = ch.a_end - ch.a_begin, ktot = ch.ktot;
+  if (tid < ch.cols) sc[tid] = nc[ch.c_begin + tid];
+  if (tid < min(nblk, NR_AMAX)) sa[tid] = na[ch.a_begin + tid];
+  const NrA* blocks = nblk <= NR_AMAX ? sa : na + ch.a_begin;
+  after_previous(tab, stamp);
+  asm volatile("" : "+l"(A), "+l"(B) : : "memory");
+  auto stage = [&](int s0, int s1) {
+    const int q0 = ch.b_begin + warp;
+    NrB E;
+    if (q0 < ch.b_end) E = nb[q0];
+    stage_b(smem, NC, s0, s1, B, nb, ch.b_end, q0, blockDim.x >> 5, E, tab);
+    cp_async_wait<0>();
+    __syncthreads();
+  };
+  if (!SEG) stage(0, ktot);
+  const int row = task.row0 + tid, r = min(row, ch.m - 1);
+  const int r1 = ch.d0 != 0 ? r / ch.d0 : 0, r0 = r - r1 * ch.d0;
+  double acc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+  // n k at a time, their loads in flight together
+  auto run = [&](auto n, int& k, int hi, const double*& p, const double*& w, int32_t ks) {
+    constexpr int U = decltype(n)::value;
+    for (; k + U <= hi; k += U) {
+      double a[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) a[u] = p[(int64_t)u * ks];
+      p += (int64_t)U * ks;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) acc[c] = fma(a[u], w[c], acc[c]);
+        w += NC;
+      }
+    }
+  };
+  auto add = [&](const NrA& x, int s0, int s1) {
+    int k = max(s0, x.k0);
+    const int hi = min(s1, x.k0 + x.k);
+    const double* p = A + x.off + (int64_t)(k - x.k0) * x.ks + (ch.d0 != 0 ? r0 * x.s0 + r1 * x.s1 : tab[x.s0 + r]);
+    const double* w = smem + (k - s0) * NC;
+    run(std::integral_constant<int, 16>(), k, hi, p, w, x.ks);
+    run(std::integral_constant<int, 8>(), k, hi, p, w, x.ks);
+    run(std::integral_constant<int, 4>(), k, hi, p, w, x.ks);
+    run(std::integral_constant<int, 2>(), k, hi, p, w, x.ks);
+    run(std::integral_constant<int, 1>(), k, hi, p, w, x.ks);
+  };
+  if (!SEG) {
+    for (int q = 0; q < nblk; ++q) add(blocks[q], 0, ktot);
+  } else {
+    int q = 0;  // the A block that holds the next k
+    for (int s0 = 0; s0 < ktot; s0 += kseg) {
+      const int s1 = min(s0 + kseg, ktot);
+      if (s0 > 0) __syncthreads();  // the segment before is read
+      stage(s0, s1);
+      for (; q < nblk; ++q) {
+        const NrA x = blocks[q];
+        add(x, s0, s1);
+        if (x.k0 + x.k > s1) break;  // the rest of its k is in the next segment
+      }
+    }
+  }
+  if (row >= ch.m) return;
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+    if (c < ch.cols) C[sc[c] + row] = alpha * acc[c];
 }
 
 // ---------------------------------------------------------------------------
@@ -1061,6 +1167,8 @@ struct tt_plan {
   bool narrow = false;
   int nr_ktot = 0;  // the most k of a chunk
   int nr_rw = 32;   // rows of a warp's tile
+  int nr_cols = 0;  // the most columns of a chunk
+  int rd_threads = 0;  // rows_dgemm in its place: rows of a CTA
   NrTask* d_nr_tasks = nullptr;
   NrA* d_nr_a = nullptr;
   NrB* d_nr_b = nullptr;
@@ -1237,36 +1345,36 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
   lap(1);
   const bool tc = precision != TT_PREC_FP64;
   // FP64 plans whose output blocks are at most NR_N wide and whose pairs
-  // contract at most NR_K elements (NR_KTOT over a block) run on the narrow kernel
+  // contract at most NR_K elements run in chunks, on one of the narrow kernels; those
+  // with more than NR_KTOT over a block where they are narrow and many (below)
   bool narrow = !tc && n_pairs > 0;
-  for (int o = 0; o < n_out && narrow; ++o) narrow = outs[o].n <= NR_N;
-  for (int i = 0; i < n_pairs && narrow; ++i) narrow = hp[i].k <= NR_K && hp[i].n <= NR_N;
-  for (int o = 0; o < n_out && narrow; ++o) narrow = work[o] <= NR_KTOT;
+  int64_t klong = 0, rows128 = 0;  // the most k of a block; the blocks' rows in 128s
+  for (int o = 0; o < n_out; ++o) {
+    klong = std::max(klong, work[o]);
+    rows128 += outs[o].n > 0 ? (outs[o].m + 127) / 128 : 0;
+  }
+  const int most = klong <= NR_KTOT ? NR_N : RD_COLS;  // columns of a chunk
+  for (int o = 0; o < n_out && narrow; ++o) narrow = outs[o].n <= most;
+  for (int i = 0; i < n_pairs && narrow; ++i) narrow = hp[i].k <= NR_K;
+  if (klong > NR_KTOT) narrow = narrow && rows128 >= ctx->num_sms;
   for (int o = 0; o < n_out; ++o)
     TT_REQUIRE(outs[o].m >= 0 && outs[o].n >= 0 && outs[o].ldc >= outs[o].m,
                "tt_contract_plan: bad output block");
   // tile tasks, longest first (LPT) so heavy blocks start early
   const int tile_m = tc ? TC_BM : BM, tile_n = tc ? TC_BN : BN;
   std::vector<TaskDev> tsorted;
-  int nr_rw = 32;
+  int nr_rw = 32, nr_cols = 0, rd_threads = 0;
   std::vector<NrTask> nr_tasks;
   std::vector<NrChunk> nr_chunks;
   std::vector<NrA> nr_a;
   std::vector<NrB> nr_b;
   std::vector<int64_t> nr_c;
-  if (!narrow) {
-    std::vector<int> oorder(n_out);
-    std::iota(oorder.begin(), oorder.end(), 0);
-    std::stable_sort(oorder.begin(), oorder.end(), [&](int x, int y) { return work[x] > work[y]; });
-    for (int o : oorder)
-      for (int m0 = 0; m0 < outs[o].m; m0 += tile_m)
-        for (int n0 = 0; n0 < outs[o].n; n0 += tile_n) tsorted.push_back(TaskDev{o, m0, n0, first[o], first[o + 1]});
-  } else {
-    // chunks: output blocks whose pairs read the same A blocks the same way
-    // (an offset table stands for its modes and strides), so that every k of a
-    // chunk belongs to every one of its columns
-    std::map<std::vector<int64_t>, std::vector<int>> by_a;  // (rows, A blocks in order) -> output blocks
-    std::vector<std::vector<int>> opairs(n_out);             // an output block's pairs in that order
+  // chunks: output blocks whose pairs read the same A blocks the same way (an offset
+  // table stands for its modes and strides), so that every k of a chunk belongs to every
+  // one of its columns
+  std::map<std::vector<int64_t>, std::vector<int>> by_a;  // (rows, A blocks in order) -> output blocks
+  std::vector<std::vector<int>> opairs(narrow ? n_out : 0);  // an output block's pairs in that order
+  if (narrow) {
     std::vector<int64_t> sig;
     for (int o = 0; o < n_out; ++o) {
       if (outs[o].m == 0 || outs[o].n == 0) continue;
@@ -1278,6 +1386,53 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
       for (int i : op) sig.insert(sig.end(), {hp[i].a_off, hp[i].rowA, hp[i].colA, hp[i].k});
       by_a[sig].push_back(o);
     }
+    int64_t all = 0;  // the chunks' rows in 128s
+    for (const auto& kv : by_a) {
+      int cols = 0;
+      for (int o : kv.second) {
+        if (cols == 0 || cols + outs[o].n > most) {
+          all += (outs[o].m + 127) / 128;
+          cols = 0;
+        }
+        cols += outs[o].n;
+        nr_cols = std::max(nr_cols, cols);
+      }
+    }
+    // A thread per row or fragments?  Measured over 1e3 to 1e6 rows (in 128s per SM: 0.05
+    // to 50), 1 to 32 columns, k of 5 to 1200, each against both and against 64 x 64 tiles:
+    // up to 8 columns a thread per row is better at any k once half of the SMs have rows
+    // (30000 rows, k = 128, 1 and 8 columns: 7.9 and 10.7 us, fragments 17 and 18; 8000
+    // rows, k = 56: 6.4 and 7.8, fragments 5.6 and 6.2); up to 16 columns until the
+    // FP64 sums of one row outweigh its loads (16 columns, k = 56: 60000 rows 14.5 and
+    // 16.3 us, 250000 54 and 48, 1e6 196 and 149; k = 14: 9.1 and 12.7 at 120000, 72 and
+    // 71 at 1e6).  With more k than fragments take, tiles are better while there are few
+    // rows (16 columns, k = 640: 30000 rows 134 and 86 us, 250000 494 and 480), unless
+    // their pairs' k are mostly padding to 16 (200000 rows, 100 pairs of 6: 455 and 810).
+    const int64_t sms = ctx->num_sms;
+    int64_t kpad = 0, ksum = 0;
+    for (int o = 0; o < n_out; ++o) {
+      kpad += (int64_t)chunks[o] * BK;
+      ksum += work[o];
+    }
+    bool per_row;
+    if (nr_cols <= 8) per_row = klong <= NR_KTOT ? 2 * all >= sms : all >= sms;
+    else if (nr_cols > RD_COLS) per_row = false;
+    else if (klong <= NR_KTOT) per_row = all >= sms && (all < 20 * sms || klong <= 16);
+    else per_row = all >= 2 * sms && 5 * kpad >= 7 * ksum;
+    if (per_row) rd_threads = klong <= NR_KTOT ? 128 : 256;
+    else narrow = klong <= NR_KTOT;
+    // Fragments: 8 rows to a warp, all of their k in flight at once, where 32 would leave
+    // SMs idle (8000 rows, k = 56, 32 columns: 7.3 and 9.8 us; 30000 rows: 15.0 and 11.9)
+    nr_rw = all < sms ? 8 : 32;
+  }
+  if (!narrow) {
+    std::vector<int> oorder(n_out);
+    std::iota(oorder.begin(), oorder.end(), 0);
+    std::stable_sort(oorder.begin(), oorder.end(), [&](int x, int y) { return work[x] > work[y]; });
+    for (int o : oorder)
+      for (int m0 = 0; m0 < outs[o].m; m0 += tile_m)
+        for (int n0 = 0; n0 < outs[o].n; n0 += tile_n) tsorted.push_back(TaskDev{o, m0, n0, first[o], first[o + 1]});
+  } else {
     // the two strides (first extent d0) that a pair's row modes merge into;
     // d0 = 0 when they do not.  One stride alone fits any d0, with s1 = s0 d0.
     struct Rows {
@@ -1317,7 +1472,7 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
       for (size_t x = 0; x < os.size();) {
         NrChunk c{(int32_t)nr_a.size(), 0, 0, (int32_t)nr_b.size(), 0, (int32_t)nr_c.size(), 0, outs[os[x]].m, 0};
         size_t y = x;
-        for (; y < os.size() && c.cols + outs[os[y]].n <= NR_N; ++y) {
+        for (; y < os.size() && c.cols + outs[os[y]].n <= most; ++y) {
           int32_t k0 = 0;
           for (int i : opairs[os[y]]) {
             const PairDev& P = hp[i];
@@ -1380,15 +1535,11 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
     // rows per CTA: enough tiles to pay for staging B, but eight CTAs per SM and
     // more while there are rows (at bond dimension 1400 2857 us per two products
     // with this bound, 2894 with sixteen tiles as soon as there are four CTAs)
-    // (of 128 rows).  With fewer than four of them per SM the kernel is a chain of
-    // latencies: 8 rows to a warp then, all of their k in flight at once (a sweep
-    // of 48 sites at bond dimension 200: 220 -> 210 ms, with the bound at one, two,
-    // four or eight per SM)
     int64_t all = 0;
     for (const NrChunk& c : nr_chunks) all += (c.m + 127) / 128;
-    nr_rw = all < 4 * (int64_t)ctx->num_sms ? 8 : 32;
-    const int rows = nr_rw * NR_WARPS;
-    const int tiles = (int)std::max<int64_t>(1, std::min<int64_t>(16, all / (8 * (int64_t)ctx->num_sms)));
+    const int rows = rd_threads > 0 ? rd_threads : nr_rw * NR_WARPS;
+    const int tiles =
+        rd_threads > 0 ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(16, all / (8 * (int64_t)ctx->num_sms)));
     for (const auto& gr : groups) {
       const int m = nr_chunks[gr.second[0]].m;
       for (int row0 = 0; row0 < m; row0 += tiles * rows)
@@ -1493,6 +1644,8 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
   plan->precision = precision;
   plan->narrow = narrow;
   plan->nr_rw = nr_rw;
+  plan->nr_cols = nr_cols;
+  plan->rd_threads = rd_threads;
   for (const NrChunk& c : nr_chunks) plan->nr_ktot = std::max(plan->nr_ktot, c.ktot);
   plan->n_tilesA = (int)ta.size();
   plan->n_tilesB = (int)tb.size();
@@ -1606,9 +1759,12 @@ int tt_contract_exec_stamped(tt_ctx* ctx, const tt_plan* plan, const double* A, 
     TT_CUDA(cudaFuncSetAttribute(grouped_dgemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)SMEM_BYTES));
     TT_CUDA(cudaFuncSetAttribute(narrow_dgemm<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)narrow_smem(NR_KTOT, 8)));
+                                 (int)narrow_smem(NR_KTOT, 8, narrow_ld(NR_N))));
     TT_CUDA(cudaFuncSetAttribute(narrow_dgemm<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)narrow_smem(NR_KTOT, 32)));
+                                 (int)narrow_smem(NR_KTOT, 32, narrow_ld(NR_N))));
+    TT_CUDA(cudaFuncSetAttribute(rows_dgemm<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RD_SEG));
+    TT_CUDA(cudaFuncSetAttribute(rows_dgemm<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RD_SEG));
+    TT_CUDA(cudaFuncSetAttribute(rows_dgemm<RD_COLS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RD_SEG));
     TT_CUDA(cudaFuncSetAttribute(grouped_tc_persist<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)TC_BULK_SMEM));
     TT_CUDA(cudaFuncSetAttribute(grouped_tc_persist<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1626,14 +1782,33 @@ int tt_contract_exec_stamped(tt_ctx* ctx, const tt_plan* plan, const double* A, 
     cfg.stream = ctx->stream;
     cfg.attrs = at;
     cfg.numAttrs = !plan->narrow && plan->split > 1 ? 2 : 1;
-    if (plan->narrow) {
+    if (plan->narrow && plan->rd_threads > 0) {
+      const int nc = plan->nr_cols <= 4 ? 4 : plan->nr_cols <= 8 ? 8 : RD_COLS;
+      // segments of equal length
+      const int kmax = RD_SEG / (8 * nc), segs = std::max(1, (plan->nr_ktot + kmax - 1) / kmax);
+      const int kseg = std::max(1, (plan->nr_ktot + segs - 1) / segs);
+      cfg.gridDim = dim3((unsigned)plan->n_tasks);
+      cfg.blockDim = dim3((unsigned)plan->rd_threads);
+      cfg.dynamicSmemBytes = sizeof(double) * (size_t)kseg * nc;
+      const auto fn = plan->rd_threads == 128
+                          ? (nc == 4   ? rows_dgemm<4, false>
+                             : nc == 8 ? rows_dgemm<8, false>
+                                       : rows_dgemm<RD_COLS, false>)
+                          : (nc == 4   ? rows_dgemm<4, true>
+                             : nc == 8 ? rows_dgemm<8, true>
+                                       : rows_dgemm<RD_COLS, true>);
+      TT_CUDA(cudaLaunchKernelEx(&cfg, fn,
+                                 (const NrTask*)plan->d_nr_tasks, (const NrA*)plan->d_nr_a, (const NrB*)plan->d_nr_b,
+                                 (const int64_t*)plan->d_nr_c, (const int32_t*)plan->d_tab, A, B, C, alpha, kseg,
+                                 (unsigned long long*)d_stamp));
+    } else if (plan->narrow) {
       cfg.gridDim = dim3((unsigned)plan->n_tasks);
       cfg.blockDim = dim3(NR_THREADS);
-      cfg.dynamicSmemBytes = narrow_smem(plan->nr_ktot, plan->nr_rw);
+      cfg.dynamicSmemBytes = narrow_smem(plan->nr_ktot, plan->nr_rw, narrow_ld(plan->nr_cols));
       TT_CUDA(cudaLaunchKernelEx(&cfg, plan->nr_rw == 8 ? narrow_dgemm<8> : narrow_dgemm<32>,
                                  (const NrTask*)plan->d_nr_tasks, (const NrA*)plan->d_nr_a, (const NrB*)plan->d_nr_b,
                                  (const int64_t*)plan->d_nr_c, (const int32_t*)plan->d_tab, A, B, C, alpha,
-                                 narrow_buf(plan->nr_ktot, plan->nr_rw), (unsigned long long*)d_stamp));
+                                 narrow_buf(plan->nr_ktot, plan->nr_rw), narrow_ld(plan->nr_cols), (unsigned long long*)d_stamp));
     } else {
       cfg.gridDim = dim3((unsigned)plan->n_tasks * (unsigned)plan->split);
       cfg.blockDim = dim3(THREADS);

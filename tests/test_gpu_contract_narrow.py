@@ -101,3 +101,97 @@ def test_negative_strides(ctx, kind):
                                            _pad(bk), _pad(bn))], A, B, 360 * n, alpha=-0.5)
     bound = 2 * k * 2.0 ** -53 * 0.5 * (a.abs() @ b.abs())
     assert torch.all((out.reshape(n, 360).T + 0.5 * (a @ b)).abs() <= bound)
+
+
+def _strides(dims, gap):
+    st, run = [], 1
+    for d in dims:
+        st.append(run)
+        run = run * d + gap
+    return st, run
+
+
+def _offsets(dims, st):
+    import torch
+    r = torch.zeros(1, dtype=torch.int64, device="cuda")
+    for d, s in zip(dims, st):
+        r = (r[None, :] + (torch.arange(d, device="cuda") * s)[:, None]).reshape(-1)
+    return r
+
+
+def _check(ctx, rows, blocks, alpha=1.0, gap=0, seed=0):
+    """blocks: per output block its column modes and the (k modes, key) of its pairs; pairs of one key share their A.
+    A holds its row modes (`rows`) first, B its k modes; `gap` unused elements after every mode."""
+    import torch
+    m, (am, msize) = int(np.prod(rows)), _strides(rows, gap)
+    outs, pairs, place, a, b, c = [], [], {}, 0, 0, 0
+    for o, (cols, ks) in enumerate(blocks):
+        n = int(np.prod(cols))
+        outs.append((c, m, n, m + o))
+        c += (m + o) * n
+        for kd, key in ks:
+            ak = [msize * s for s in _strides(kd, gap)[0]]
+            if key is None or (key, kd) not in place:
+                place[(key, kd)] = a
+                a += msize * _strides(kd, gap)[1] + 1
+            bk, ksize = _strides(kd, gap)
+            bn = [ksize * s for s in _strides(cols, gap)[0]]
+            pairs.append((o, len(rows), len(kd), len(cols), place[(key, kd)], b, _pad(rows), _pad(kd), _pad(cols),
+                          _pad(am), _pad(ak), _pad(bk), _pad(bn)))
+            b += ksize * _strides(cols, gap)[1] + 1
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    A, B = (torch.randn(s, dtype=torch.float64, device="cuda", generator=g) for s in (a, b))
+    got = _exec(ctx, outs, pairs, A, B, c, alpha)
+    ro = _offsets(rows, am)
+    for o, (off, _, n, ld) in enumerate(outs):
+        want, bound = (torch.zeros((m, n), dtype=torch.float64, device="cuda") for _ in range(2))
+        k = 0
+        for q in pairs:
+            if q[0] == o:
+                x = A[q[4] + ro[:, None] + _offsets(q[7][:q[2]], q[10])[None, :]]
+                y = B[q[5] + _offsets(q[7][:q[2]], q[11])[:, None] + _offsets(q[8][:q[3]], q[12])[None, :]]
+                want += x @ y
+                bound += x.abs() @ y.abs()
+                k += x.shape[1]
+        at = off + torch.arange(m, device="cuda")[:, None] + ld * torch.arange(n, device="cuda")[None, :]
+        assert torch.all((got[at] - alpha * want).abs() <= 2 * max(k, 1) * 2.0 ** -53 * abs(alpha) * bound), (o, k)
+        assert torch.all(got[off + ld * torch.arange(n, device="cuda")[:, None] + torch.arange(m, ld, device="cuda")] == 7.0)
+
+
+FEW, MANY = 148 * 128 + 77, 16 * 148 * 128 + 301  # rows: one tile of 128 per SM, and several tiles per block of threads
+
+
+def _shared(widths, ks):
+    return [((w,), [((k,), i) for i, k in enumerate(ks)]) for w in widths]
+
+
+@pytest.mark.parametrize("rows", [1, 130, FEW // 2 - 300, FEW // 2 + 300, FEW, MANY])
+@pytest.mark.parametrize("widths", [(1,), (4,), (3, 2), (8,), (9,), (7, 9), (7, 10), (20, 12), (17, 17, 9)])
+def test_rows_and_columns(ctx, rows, widths):
+    """A thread per row (4, 8, 16 columns) and fragments of 8 and 32 rows, one chunk and several; k of several buffers."""
+    _check(ctx, (rows,), _shared(widths, (14, 5, 16, 2)), alpha=-0.5)
+
+
+@pytest.mark.parametrize("rows", [1000, FEW])
+@pytest.mark.parametrize("n", [3, 13, 25])
+@pytest.mark.parametrize("ks", [(1,), (15,), (16,), (17,), (64, 1), (64, 64, 64, 64), (3,) * 25, (0, 5, 0), ()])
+def test_k(ctx, rows, n, ks):
+    """k around the buffers' 16 and 64 and the staged 256; more A blocks than are kept in shared memory; no k."""
+    _check(ctx, (rows,), _shared((n,), ks))
+
+
+@pytest.mark.parametrize("rows,n,ks", [(FEW, 2, (64,) * 5), (FEW, 7, (64,) * 25), (FEW, 8, (61,) * 26),
+                                       (2 * FEW, 5, (64,) * 49), (2 * FEW, 16, (6,) * 140), (2 * FEW, 11, (20,) * 40),
+                                       (900, 5, (64,) * 5), (FEW, 16, (64,) * 5), (FEW, 31, (33,) * 9)])
+def test_long_k(ctx, rows, n, ks):
+    """More k than fragments take: a thread per row with B staged whole or in segments, and tiles."""
+    _check(ctx, (rows,), _shared((n,), ks), alpha=3.0)
+
+
+@pytest.mark.parametrize("rows", [(7, 5, 11), (40, 30, 33)])
+@pytest.mark.parametrize("cols", [(2, 3), (4, 5)])
+@pytest.mark.parametrize("gap", [0, 3])
+def test_tables(ctx, rows, cols, gap):
+    """Modes that do not merge: rows, k (one A entry each, more than 16) and B's both directions through tables."""
+    _check(ctx, rows, [(cols, [((3, 6), 0), ((2, 5), 1)]), (cols, [((3, 6), 0), ((2, 5), 1)]), ((3,), [((4,), 0)])],
+           gap=gap)
