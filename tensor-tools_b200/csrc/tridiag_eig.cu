@@ -35,8 +35,8 @@ constexpr int INV_ITERS = 3;
 
 struct EigDev {
   int64_t g_off, w_off, a_off;
-  int32_t n, flags, nvec, pad;
-  int64_t s_off;               // its columns in the scratch of the cluster reduction
+  int32_t n, flags, nvec, nb;  // nb: panel width of the blocked reduction
+  int64_t s_off;               // its place in the scratch of the cluster reductions
 };
 
 __device__ double block_reduce(double v, double* red, bool is_max) {
@@ -800,8 +800,7 @@ eigvecs_small(const EigDev* __restrict__ probs, const double* G, const double* T
 // barrier (v is complete) before the next products.  When nb reflectors are
 // pending, the products' pass over the own columns applies them on the way.
 // What a CTA pushes for column k + 1 may arrive while another still reads what it
-// got for column k, so the arrays pushed to are double (by parity); where two do
-// not fit (n above about 3300) a second barrier per column follows instead.
+// got for column k, so the arrays pushed to are double (by parity).
 //
 // Phase 2: CTA r owns eigenvectors [r q, r q + q), q = ceil(nvec / CL).
 // Inverse iteration runs one thread per vector.  Gram-Schmidt (twice, inside
@@ -832,30 +831,47 @@ __device__ __host__ __forceinline__ int first_owned(int from, int rank, int CL) 
   return from <= rank ? 0 : (from - rank + CL - 1) / CL;
 }
 
+constexpr int PNB_MAX = 32;      // widest panel of the blocked reduction
+
+// doubles of dynamic shared memory of the blocked cluster reduction
+__host__ __device__ inline int64_t blocked_smem(int n, int nb, int CL) {
+  const int64_t nloc = (n + CL - 1) / CL;
+  return 2 * (int64_t)nb * nloc        // V, W of the panel on the own rows
+         + 2 * nloc                    // the own rows of the current and the next column
+         + (int64_t)CL * nloc          // the pushed column, then v, owner-major
+         + (int64_t)CL * nloc          // this CTA's row sums of A22 v, owner-major
+         + (int64_t)CL * nloc          // pushed row sums of A22 v on the own rows, per sender
+         + (int64_t)NWARP * nloc       // per-warp column dots
+         + CL_MAX * 2 * (int64_t)nb    // pushed V^T v, W^T v partials
+         + CL_MAX                      // pushed v^T A22 v partials
+         + CL_MAX * (int64_t)nb        // pushed row sums on the panel's rows
+         + nb                          // pushed column dots of the panel's rows
+         + 2 * (int64_t)nb * nb        // V, W on the panel's rows
+         + 2 * (int64_t)nb;            // V^T v, W^T v
+}
+
 // Shared memory of the cluster reduction, in doubles, for the n rows and columns
 // that are left: nb pending reflectors (v, w) on all rows and (w, v) on the own
-// columns, the current v, the pushed pairs (once or twice), the pushed partial
-// sums, and the own columns when they are resident.
+// columns, the current v, the pushed pairs (twice), the pushed partial sums, and the
+// own columns when they are resident.
 constexpr int CLR_MISC = 2 * CL_MAX * 2 * NB_MAX + 2 * CL_MAX * NWARP + NWARP * 2 * NB_MAX;
 struct ClusterLayout {
   int nb;           // pending reflectors (0: does not fit)
   bool resident;    // own columns in shared memory
-  bool twice;       // double push buffers
   int64_t doubles;  // in all
 };
 __host__ __device__ inline int cl_ld(int n) { return (n + 2) & ~1; }  // rows of a column: even, at least one of padding
 __host__ __device__ inline ClusterLayout cluster_layout(int n, int CL, int64_t cap) {
   const int64_t ld = cl_ld(n), nloc = (n + CL - 1) / CL;
-  for (int form = 0; form < 3; ++form) {  // resident; in L2; in L2 with single push buffers
-    const bool resident = form == 0, twice = form < 2;
-    const int64_t fixed = CLR_MISC + ld + (twice ? 4 : 2) * ld + (resident ? nloc * ld : 0);
+  for (const bool resident : {true, false}) {
+    const int64_t fixed = CLR_MISC + 5 * ld + (resident ? nloc * ld : 0);
     int64_t nb = fixed < cap ? (cap - fixed) / (2 * (ld + nloc)) : 0;
     if (nb > NB_MAX) nb = NB_MAX;
     // resident columns pay when a few reflectors still fit beside them
     if (nb < (resident ? 6 : 1)) continue;
-    return ClusterLayout{(int)nb, resident, twice, fixed + nb * 2 * (ld + nloc)};
+    return ClusterLayout{(int)nb, resident, fixed + nb * 2 * (ld + nloc)};
   }
-  return ClusterLayout{0, false, false, 0};
+  return ClusterLayout{0, false, 0};
 }
 
 // D += A B for one m8n8k4 FP64 tile (DMMA): A 8x4 row fragment (lane L holds
@@ -1036,21 +1052,20 @@ tridiag_eigvals_cluster(const EigDev* __restrict__ probs, double* G, double* Tg,
   // be pending, until the own columns fit as well.  All pointers take the absolute
   // row r or own column l.
   int o = 0, nb = 0, ldv = 0, ldw = 0, ldc = rend;
-  bool resident = false, twice = true;
+  bool resident = false;
   double2 *vw = nullptr, *push = nullptr, *part = nullptr, *ab = nullptr, *wv = nullptr;
   double *vcur = nullptr, *vav = nullptr, *cols = nullptr;
   auto lay_out = [&](int from) {
     const ClusterLayout L = cluster_layout(n - from, CL, cap);
     o = from;
     nb = L.nb;
-    twice = L.twice;
     resident = L.resident;
     ldv = rend - o;
     ldw = nloc - o / CL;
     vw = reinterpret_cast<double2*>(sm) - o;                     // [nb][ldv]: (v, w)
     vcur = sm + (int64_t)nb * 2 * ldv - o;                       // [ldv]
-    push = reinterpret_cast<double2*>(vcur + o + ldv) - o;       // [1 or 2][ldv]: (A0 v, A0[:, k + 1])
-    part = push + o + (twice ? 2 : 1) * ldv;                     // [2][CL_MAX][NB_MAX]: shares of (W^T v, V^T v)
+    push = reinterpret_cast<double2*>(vcur + o + ldv) - o;       // [2][ldv]: (A0 v, A0[:, k + 1])
+    part = push + o + 2 * ldv;                                   // [2][CL_MAX][NB_MAX]: shares of (W^T v, V^T v)
     vav = reinterpret_cast<double*>(part + 2 * CL_MAX * NB_MAX);  // [2][CL_MAX][NW]: shares of v^T A0 v
     ab = reinterpret_cast<double2*>(vav + 2 * CL_MAX * NWARP) + warp * NB_MAX;  // this warp's (W^T v, V^T v)
     wv = reinterpret_cast<double2*>(reinterpret_cast<double*>(part) + CLR_MISC) - o / CL;  // [nb][ldw]: (w, v) on the own columns
@@ -1132,7 +1147,7 @@ tridiag_eigvals_cluster(const EigDev* __restrict__ probs, double* G, double* Tg,
     __syncthreads();
     // ---- the shares of the pending V^T v and W^T v, and A0 v on the own columns ----
     const bool flush = np == nb;
-    double2* pushed = push + (twice ? par * ldv : 0);
+    double2* pushed = push + par * ldv;
     double2* mypart = part + par * CL_MAX * NB_MAX;
     double* myvav = vav + par * CL_MAX * NWARP;
     const int lf = first_owned(k + 1, rank, CL), rs = (k + 1) & ~1;
@@ -1223,7 +1238,6 @@ tridiag_eigvals_cluster(const EigDev* __restrict__ probs, double* G, double* Tg,
     }
     ++np;
     par ^= 1;
-    if (!twice) cluster.sync();  // the pushed pairs are read before the next ones arrive
   }
   // T: the last 2 x 2 block
   __syncthreads();
@@ -1251,6 +1265,441 @@ tridiag_eigvals_cluster(const EigDev* __restrict__ probs, double* G, double* Tg,
   cluster.sync();  // the last access of another CTA's shared memory
   // launched alongside tridiag_small: complete only when that is
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// The largest sectors: the blocked reduction of LAPACK's dsytrd / dlatrd (Golub & Van
+// Loan, ibid., with the panel form of sec. 5.1.7).  The reflectors of a panel of nb
+// columns are formed one by one against the matrix as it stood at the start of the
+// panel, corrected on the fly by the panel's V and W (A22 v - V W^T v - W V^T v), and
+// the trailing matrix receives the rank-2nb update A -= V W^T + W V^T once per panel.
+// Only the lower triangle is read or updated, in place.  Index c (row or column)
+// belongs to CTA c % CL.  Per column j, two cluster barriers:
+//   1. the owners of rows >= j bring column j up to date and push it to every CTA;
+//   2. every CTA forms the same reflector from the whole column (same data, same
+//      reduction order), keeps v, and pushes its partial V^T v, W^T v;
+//   3. every CTA runs A22 v over the lower triangle of its own columns: one warp per
+//      block of 64 rows, each lane two rows, columns 16 at a time; an element A[i,c]
+//      (i >= c) adds A[i,c] v_i to the dot of column c and, below the diagonal,
+//      A[i,c] v_c to row i.  The column dots are summed across the lanes by a butterfly
+//      reduce-scatter, the row sums go to the row's owner (a slot per sender), and the
+//      CTA's share of v^T A22 v to every CTA;
+//   4. every CTA completes p = A22 v on its own rows (own dot + the pushed row sums, in
+//      CTA order), w' = tau (p - V W^T v - W V^T v) and w = w' - (tau/2)(w'.v) v; the
+//      panel's rows, which every CTA needs, have their sums pushed to every CTA.
+// Every CTA sums pushed partials in CTA order, so every decision and scalar is the same
+// in every CTA.  The trailing update goes through a global n x 2nb scratch.
+//
+// The reduction above holds its pending reflectors on all rows in every CTA, so the
+// larger the sector the fewer it can hold (6 at n = 1471, 3 at 2048, 1 at 3000) and the
+// more often both triangles go through L2; here a CTA holds 8 to 32 on its own rows
+// only, and half of the matrix moves.  Measured (this / that, ms): one sector of 1750
+// 31.4 / 27.2, 2048 45.3 / 40.5, 2200 46.9 / 55.3, 3000 91.9 / 158, 4096 219 / 573; four
+// of 1750 32.5 / 29.5, 1900 37.3 / 40.6, 2048 48.0 / 53.5: the rule is blocked_sectors.
+// acc[k] (k < 16) summed over the 32 lanes of the warp, lane L receiving the
+// sum of index L % 16: a butterfly sum across the half-warps, then a
+// reduce-scatter (31 shuffles for 16 sums)
+__device__ __forceinline__ double warp_reduce_scatter16(double (&acc)[16], int lane) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 16);
+#pragma unroll
+  for (int s = 8; s >= 1; s >>= 1) {
+    const bool up = (lane & s) != 0;
+#pragma unroll
+    for (int k = 0; k < s; ++k) {
+      const double send = up ? acc[k] : acc[k + s];
+      const double keep = up ? acc[k + s] : acc[k];
+      acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+    }
+  }
+  return acc[0];
+}
+
+__global__ void __launch_bounds__(TT)
+tridiag_blocked_cluster(const EigDev* __restrict__ probs, double* G, double* Tg, double* VWg) {
+  extern __shared__ double sm[];
+  __shared__ double red[33];
+  __shared__ double s_K;
+  __shared__ double vw_part[NWARP * 2 * PNB_MAX];  // per-warp V^T v, W^T v sums
+
+  cgx::cluster_group cluster = cgx::this_cluster();
+  const int CL = (int)cluster.num_blocks();
+  const int rank = (int)cluster.block_rank();
+  const EigDev P = probs[blockIdx.x / CL];
+  const int n = P.n;
+  const int tid = threadIdx.x;
+  if (n <= 0) return;  // the same problem for the whole cluster
+  const int nb = P.nb;
+  double* Gp = G + P.g_off;
+  double* dg = Tg + 3 * P.w_off;
+  double* eg = dg + n;
+  double* tg = eg + n;
+  double* VW = VWg + P.s_off;  // n x 2nb, row-major: [i][t] = V(i, t), [i][nb + t] = W(i, t)
+  const int warp = tid >> 5, lane = tid & 31;
+  const int nloc = (n + CL - 1) / CL;
+  int lown = 0;  // own indices c = rank + CL l, l < lown
+  while (lown < nloc && rank + CL * lown < n) ++lown;
+  double* Vl = sm;                            // [nb][nloc]
+  double* Wl = Vl + (int64_t)nb * nloc;       // [nb][nloc]
+  double* xc = Wl + (int64_t)nb * nloc;       // [2][nloc]: own rows of a column, by parity of jj
+  // Vectors over all rows are kept owner-major: row i = r + CL l at [r nloc + l],
+  // so what one CTA pushes to another is contiguous on both sides
+  const int lg = __ffs(CL) - 1;  // CL is a power of two
+  auto om = [&](int i) { return ((i & (CL - 1)) * nloc) + (i >> lg); };
+  double* xo = xc + 2 * nloc;                 // [CL][nloc]: column j as pushed, then v
+  double* yl = xo + (int64_t)CL * nloc;       // [CL][nloc]: this CTA's row sums of A22 v
+  double* yb = yl + (int64_t)CL * nloc;       // [CL][nloc]: row sums of A22 v on the own rows, by sender
+  double* dw = yb + (int64_t)CL * nloc;       // [NWARP][nloc]: column dots by warp
+  double* r2 = dw + (int64_t)NWARP * nloc;    // [CL_MAX][2nb]: V^T v, W^T v partials by sender
+  double* r3 = r2 + CL_MAX * 2 * nb;          // [CL_MAX]: v^T A22 v partials by sender
+  double* yp = r3 + CL_MAX;                   // [CL_MAX][nb]: row sums on the panel's rows by sender
+  double* dp = yp + CL_MAX * nb;              // [nb]: column dots of the panel's rows
+  double* Vp = dp + nb;                       // [nb][nb]: Vp[t nb + s] = v_t[k0 + s]
+  double* Wq = Vp + nb * nb;                  // [nb][nb]: Wq[t nb + s] = w_t[k0 + s]
+  double* cvt = Wq + nb * nb;                 // [nb]: V^T v
+  double* cwt = cvt + nb;                     // [nb]: W^T v
+  for (int k0 = 0; k0 + 2 < n; k0 += nb) {
+    const int nbe = min(nb, n - 2 - k0);  // reflector columns k0 .. k0 + nbe - 1
+    for (int jj = 0; jj < nbe; ++jj) {
+      const int j = k0 + jj;
+      double* xcur = xc + (jj & 1) * nloc;
+      // ---- 1: column j on the own rows >= j, pushed to every CTA ----
+      const int l1 = first_owned(j, rank, CL);
+      {
+        // four threads per row, each summing a quarter of the panel's terms
+        // (the loop bound is the same for the whole warp: the shuffles need it)
+        const int sub = tid & 3;
+        for (int base = l1 + (warp << 3); base < lown; base += blockDim.x >> 2) {
+          const int l = base + (lane >> 2);
+          const bool act = l < lown;
+          double corr = 0.0;
+          if (act)
+#pragma unroll 1
+            for (int t = sub; t < jj; t += 4)
+              corr += Vl[t * nloc + l] * Wq[t * nb + jj] + Wl[t * nloc + l] * Vp[t * nb + jj];
+          corr += __shfl_xor_sync(0xffffffffu, corr, 1);
+          corr += __shfl_xor_sync(0xffffffffu, corr, 2);
+          if (act && sub == 0) xcur[l] = (jj == 0 ? Gp[(rank + CL * l) + (int64_t)n * j] : xcur[l]) - corr;
+        }
+      }
+      __syncthreads();
+      for (int e = tid; e < (lown - l1) * CL; e += blockDim.x) {
+        const int q = e / (lown - l1), l = l1 + e % (lown - l1);
+        *cluster.map_shared_rank(xo + rank * nloc + l, q) = xcur[l];
+      }
+      cluster.sync();  // A
+      // ---- 2: the reflector (same in every CTA), v kept, V^T v and W^T v partials ----
+      const double alpha = xo[om(j + 1)];  // read before the reduction's barriers, overwritten below
+      double part = 0.0;
+      for (int i = j + 2 + tid; i < n; i += blockDim.x) part += xo[om(i)] * xo[om(i)];
+      const double sigma = block_reduce(part, red, false);
+      double tau = 0.0, beta = alpha, scale = 0.0;
+      if (sigma != 0.0) {
+        const double mu = sqrt(alpha * alpha + sigma);
+        beta = alpha <= 0.0 ? mu : -mu;
+        tau = (beta - alpha) / beta;
+        scale = 1.0 / (alpha - beta);
+      }
+      if (rank == j % CL && tid == 0) {
+        dg[j] = xo[om(j)];
+        tg[j] = tau;
+        eg[j] = beta;
+      }
+      for (int i = j + 1 + tid; i < n; i += blockDim.x) xo[om(i)] = i == j + 1 ? 1.0 : xo[om(i)] * scale;
+      __syncthreads();
+      for (int l = tid; l < lown; l += blockDim.x) {
+        const int i = rank + CL * l;
+        const double vi = i >= j + 1 ? xo[rank * nloc + l] : 0.0;
+        Vl[jj * nloc + l] = vi;
+        Wl[jj * nloc + l] = 0.0;
+        if (i >= j + 2) Gp[i + (int64_t)n * j] = vi;  // reflector kept below the subdiagonal for phase 2
+      }
+      for (int s = tid; s < nb; s += blockDim.x) {
+        const int row = k0 + s;
+        Vp[jj * nb + s] = row >= j + 1 && row < n ? xo[om(row)] : 0.0;
+      }
+      __syncthreads();
+      const int lf = first_owned(j + 1, rank, CL);
+      // V^T v and W^T v partials over the own rows >= j + 1: lane t of each
+      // warp sums column t over every NWARP-th row, the warps' sums are added
+      // in warp order and pushed to every CTA
+      if (jj > 0) {
+        double sv = 0.0, sw = 0.0;
+        if (lane < jj)
+          for (int l = lf + warp; l < lown; l += NWARP) {
+            const double v = Vl[jj * nloc + l];
+            sv += Vl[lane * nloc + l] * v;
+            sw += Wl[lane * nloc + l] * v;
+          }
+        vw_part[warp * 2 * PNB_MAX + lane] = sv;
+        vw_part[warp * 2 * PNB_MAX + PNB_MAX + lane] = sw;
+        __syncthreads();
+        if (tid < 2 * PNB_MAX) {
+          const int t = tid & (PNB_MAX - 1);
+          if (t < jj) {
+            double a = 0.0;
+            for (int w = 0; w < NWARP; ++w) a += vw_part[w * 2 * PNB_MAX + tid];
+            const int slot = rank * 2 * nb + (tid < PNB_MAX ? t : nb + t);
+            for (int q = 0; q < CL; ++q) *cluster.map_shared_rank(r2 + slot, q) = a;
+          }
+        }
+      }
+      // ---- 3: p = A22 v from the lower triangle of the own columns ----
+      if (jj + 1 < nbe)  // the next column's own rows: unchanged until its step 1
+        for (int l = lf + tid; l < lown; l += blockDim.x)
+          xc[((jj + 1) & 1) * nloc + l] = Gp[(rank + CL * l) + (int64_t)n * (j + 1)];
+      double kp = 0.0;  // this thread's share of v^T A22 v
+      if (tau != 0.0) {
+        for (int l = lf + lane; l < lown; l += 32) dw[warp * nloc + l] = 0.0;
+        __syncwarp();
+        // blocks of 64 rows from row j + 1, two rows per lane (i0 = rb + lane,
+        // i1 = i0 + 32); the longest (last) blocks are dealt first and back and
+        // forth, so the warps' shares come out even
+        const int nrb = (n - j - 1 + 63) / 64;
+        const int64_t cstep = (int64_t)n * CL;  // from one own column to the next
+        for (int round = 0; round * NWARP < nrb; ++round) {
+          const int o = round * NWARP + ((round & 1) ? NWARP - 1 - warp : warp);
+          if (o >= nrb) continue;
+          const int rb = j + 1 + 64 * (nrb - 1 - o);
+          const int i0 = rb + lane, i1 = i0 + 32;
+          const double v0 = i0 < n ? xo[om(i0)] : 0.0, v1 = i1 < n ? xo[om(i1)] : 0.0;
+          // rows past the end read row n - 1 (weighted by v = 0, sums discarded)
+          const double* g0 = Gp + min(i0, n - 1) + (int64_t)n * rank;
+          const double* g1 = Gp + min(i1, n - 1) + (int64_t)n * rank;
+          const int le = first_owned(min(n, rb + 64), rank, CL);  // own columns c < the block's end
+          const int lfull = min(le, first_owned(rb, rank, CL));   // own columns c < rb: no masking
+          double y0 = 0.0, y1 = 0.0;
+          int lt = lf;
+          for (; lt + 16 <= lfull; lt += 16) {
+            double acc[16];
+#pragma unroll
+            for (int h = 0; h < 16; h += 8) {  // eight columns' loads in flight at a time
+              double a0[8], a1[8];
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                a0[k] = g0[(lt + h + k) * cstep];
+                a1[k] = g1[(lt + h + k) * cstep];
+              }
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const double vc = xo[rank * nloc + lt + h + k];
+                y0 = fma(a0[k], vc, y0);
+                y1 = fma(a1[k], vc, y1);
+                acc[h + k] = fma(a1[k], v1, a0[k] * v0);
+              }
+            }
+            const double d = warp_reduce_scatter16(acc, lane);
+            if (lane < 16) dw[warp * nloc + lt + lane] += d;
+          }
+          for (; lt < le; lt += 16) {  // the rest, masked: the block's diagonal part and a short tail
+            double acc[16];
+#pragma unroll
+            for (int h = 0; h < 16; h += 8) {
+              double a0[8], a1[8];
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const int c = rank + CL * (lt + h + k);
+                const bool cv = lt + h + k < le;
+                a0[k] = cv && i0 >= c ? g0[(lt + h + k) * cstep] : 0.0;
+                a1[k] = cv && i1 >= c ? g1[(lt + h + k) * cstep] : 0.0;
+              }
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const int c = rank + CL * (lt + h + k);
+                const double vc = lt + h + k < le ? xo[rank * nloc + lt + h + k] : 0.0;
+                y0 = fma(i0 > c ? a0[k] : 0.0, vc, y0);
+                y1 = fma(i1 > c ? a1[k] : 0.0, vc, y1);
+                acc[h + k] = fma(a1[k], v1, a0[k] * v0);
+              }
+            }
+            const double d = warp_reduce_scatter16(acc, lane);
+            if (lane < 16 && lt + lane < le) dw[warp * nloc + lt + lane] += d;
+          }
+          if (i0 < n) {
+            yl[om(i0)] = y0;
+            kp += v0 * y0;
+          }
+          if (i1 < n) {
+            yl[om(i1)] = y1;
+            kp += v1 * y1;
+          }
+        }
+      }
+      __syncthreads();
+      if (tau != 0.0) {
+        // the row sums to their owners (rows below j + 1 and beyond n ride
+        // along unread), those of the panel's rows to every CTA
+        const int lmin = (j + 1) >> lg, cnt = nloc - lmin;
+        for (int e = tid; e < CL * cnt; e += blockDim.x) {
+          const int d = e / cnt, l = lmin + e % cnt;
+          *cluster.map_shared_rank(yb + rank * nloc + l, d) = yl[d * nloc + l];
+        }
+        for (int e = tid; e < CL * nb; e += blockDim.x) {
+          const int q = e / nb, s = e % nb, row = k0 + s;
+          if (row >= j + 1 && row < n) *cluster.map_shared_rank(yp + rank * nb + s, q) = yl[om(row)];
+        }
+      }
+      if (tau != 0.0)
+        for (int l = lf + tid; l < lown; l += blockDim.x) {
+          double d = 0.0;
+          for (int w = 0; w < NWARP; ++w) d += dw[w * nloc + l];
+          dw[l] = d;  // the column's dot, kept in warp 0's row
+          const int c = rank + CL * l;
+          kp += xo[rank * nloc + l] * d;
+          if (c < k0 + nb)
+            for (int q = 0; q < CL; ++q) *cluster.map_shared_rank(dp + (c - k0), q) = d;
+        }
+      const double vav_part = block_reduce(kp, red, false);
+      if (tid < CL) *cluster.map_shared_rank(r3 + rank, tid) = vav_part;
+      cluster.sync();  // B
+      // ---- 4: w on the own rows and on the panel's rows ----
+      if (warp == 0) {  // V^T v, W^T v and the scalar K = (tau/2) w'.v, one lane per panel column
+        double a = 0.0, b = 0.0;
+        if (lane < jj)
+          for (int q = 0; q < CL; ++q) {
+            a += r2[q * 2 * nb + lane];
+            b += r2[q * 2 * nb + nb + lane];
+          }
+        if (lane < jj) {
+          cvt[lane] = a;
+          cwt[lane] = b;
+        }
+        const double cc = warp_sum(a * b);
+        if (lane == 0) {
+          double vav = 0.0;
+          for (int q = 0; q < CL; ++q) vav += r3[q];
+          s_K = 0.5 * tau * tau * (vav - 2.0 * cc);
+        }
+      }
+      __syncthreads();
+      if (tau != 0.0) {
+        const double K = s_K;
+        // own rows: four threads per row, each summing a quarter of the terms
+        // (the loop bound is the same for the whole warp: the shuffles need it)
+        const int sub = tid & 3;
+        for (int base = lf + (warp << 3); base < lown; base += blockDim.x >> 2) {
+          const int l = base + (lane >> 2);
+          const bool act = l < lown;
+          double p = 0.0, corr = 0.0;
+          if (act) {
+#pragma unroll 1
+            for (int q = sub; q < CL; q += 4) p += yb[q * nloc + l];
+#pragma unroll 1
+            for (int t = sub; t < jj; t += 4) corr += Vl[t * nloc + l] * cwt[t] + Wl[t * nloc + l] * cvt[t];
+          }
+          p += __shfl_xor_sync(0xffffffffu, p, 1);
+          p += __shfl_xor_sync(0xffffffffu, p, 2);
+          corr += __shfl_xor_sync(0xffffffffu, corr, 1);
+          corr += __shfl_xor_sync(0xffffffffu, corr, 2);
+          if (act && sub == 0) Wl[jj * nloc + l] = tau * (dw[l] + p - corr) - K * Vl[jj * nloc + l];
+        }
+        // the panel's rows: sixteen threads per row
+        const int s = tid >> 4, sub16 = tid & 15;
+        if (s < nb) {
+          const int row = k0 + s;
+          const bool live = row >= j + 1 && row < n;
+          double p = 0.0, corr = 0.0;
+          if (live) {
+            for (int q = sub16; q < CL; q += 16) p += yp[q * nb + s];
+            for (int t = sub16; t < jj; t += 16) corr += Vp[t * nb + s] * cwt[t] + Wq[t * nb + s] * cvt[t];
+          }
+#pragma unroll
+          for (int o = 1; o < 16; o <<= 1) {
+            p += __shfl_xor_sync(0xffffffffu, p, o);
+            corr += __shfl_xor_sync(0xffffffffu, corr, o);
+          }
+          if (sub16 == 0) Wq[jj * nb + s] = live ? tau * (dp[s] + p - corr) - K * Vp[jj * nb + s] : 0.0;
+        }
+      } else {
+        for (int s = tid; s < nb; s += blockDim.x) Wq[jj * nb + s] = 0.0;
+      }
+      __syncthreads();
+    }
+    // ---- trailing update A[k1:, k1:] -= V W^T + W V^T (lower triangle) through the global scratch ----
+    const int k1 = k0 + nbe;
+    for (int e = tid; e < lown * 2 * nbe; e += blockDim.x) {
+      const int l = e / (2 * nbe), t2 = e - l * 2 * nbe;
+      const int i = rank + CL * l;
+      if (i < k1) continue;
+      const int t = t2 < nbe ? t2 : t2 - nbe;
+      VW[(int64_t)i * 2 * nb + (t2 < nbe ? t : nb + t)] = (t2 < nbe ? Vl : Wl)[t * nloc + l];
+    }
+    __threadfence();
+    cluster.sync();
+    // DMMA (m8n8k4 f64) tiles: a warp takes 32 rows x 16 own columns and runs
+    // P = V W^T + W V^T over the panel's k, the rows' [V W] fragments read
+    // straight from the scratch (no shared staging, no barrier per tile); the
+    // lower triangle of its block then receives A -= P
+    const int lf = first_owned(k1, rank, CL);
+    const int nbe4 = (nbe + 3) & ~3;
+    const int gr = lane >> 2, gk = lane & 3;
+    const int nrt = (n - k1 + 31) >> 5;                 // 32-row tiles
+    const int ncb = (first_owned(n, rank, CL) - lf + 15) >> 4;  // 16-column blocks
+    for (int task = warp; task < nrt * ncb; task += NWARP) {
+      const int i0 = k1 + 32 * (task / ncb), lb = lf + 16 * (task % ncb);
+      if (rank + CL * lb > i0 + 31) continue;  // the block lies above the diagonal
+      const int le = min(first_owned(min(n, i0 + 32), rank, CL), lb + 16);
+      double acc[4][2][2];
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        // part 0: V (rows) x W (columns); part 1: W x V
+        const int xo0 = part ? nb : 0;
+        const double* Y = part ? Vl : Wl;
+#pragma unroll 1
+        for (int t = 0; t < nbe4; t += 4) {
+          const int k = t + gk;
+          const bool kv = k < nbe;
+          double af[4], bf[2];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            const int i = i0 + 8 * a + gr;
+            af[a] = kv && i < n ? VW[(int64_t)i * 2 * nb + xo0 + k] : 0.0;
+          }
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            const int l = lb + 8 * b + gr;
+            bf[b] = kv && l < le ? Y[k * nloc + l] : 0.0;
+          }
+#pragma unroll
+          for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) dmma_tr(acc[a][b], af[a], bf[b]);
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const int i = i0 + 8 * a + gr;
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int l = lb + 8 * b + 2 * gk + e;
+            const int c = rank + CL * l;
+            if (i < n && l < le && i >= c) Gp[(int64_t)n * c + i] -= acc[a][b][e];
+          }
+      }
+    }
+    __threadfence();
+    cluster.sync();
+  }
+  // T: the last two diagonal entries and the last off-diagonal A[n-1, n-2]
+  if (tid == 0) {
+    if (rank == (n - 2) % CL) {
+      dg[n - 2] = Gp[(n - 2) + (int64_t)n * (n - 2)];
+      eg[n - 2] = Gp[(n - 1) + (int64_t)n * (n - 2)];
+    }
+    if (rank == (n - 1) % CL) dg[n - 1] = Gp[(n - 1) + (int64_t)n * (n - 1)];
+    if (rank == 0) {
+      eg[n - 1] = 0.0;
+      tg[n - 1] = 0.0;
+      tg[n - 2] = 0.0;
+    }
+  }
+  __threadfence();
+  cluster.sync();  // also the last access of another CTA's shared memory
 }
 
 // Bisection for every sector after its tridiagonalisation, spread over the
@@ -2210,22 +2659,35 @@ constexpr int64_t kVecsSmemCap = 28 * 1024;  // doubles (224 KB) of dynamic shar
 // Sectors above the size of the one-CTA kernels go to the cluster kernels.
 bool is_big(const EigDev& e) { return e.n > SN && !(e.flags & TT_EIG_ROW_1X2); }
 
-// Cluster size and shared-memory caps of the cluster kernels on this thread's
-// device: 16 CTAs per cluster when the device can co-schedule that many with
-// the full shared-memory carve-out, else 8, else none (an error for sectors that
-// need them).
 // The cluster reduction for sectors of up to n states
 const void* vals_kernel(int n) {
   return n <= 2 * CR_THREADS   ? (const void*)tridiag_eigvals_cluster<2>
          : n <= 4 * CR_THREADS ? (const void*)tridiag_eigvals_cluster<4>
-         : n <= 8 * CR_THREADS ? (const void*)tridiag_eigvals_cluster<8>
-                               : (const void*)tridiag_eigvals_cluster<16>;
+                               : (const void*)tridiag_eigvals_cluster<8>;
+}
+constexpr int CR_MAX = 8 * CR_THREADS;  // states of a sector that it takes, at most
+
+// Whether a batch of cluster-sized sectors goes to the blocked reduction: its largest
+// has more states than the other takes, or is one of those (1800 up) for which both
+// triangles of all sectors together must stay in L2.
+bool blocked_sectors(const std::vector<EigDev>& big) {
+  int n = 0;
+  int64_t bytes = 0;
+  for (const EigDev& e : big) {
+    n = std::max(n, e.n);
+    bytes += (int64_t)sizeof(double) * e.n * e.n;
+  }
+  return n > CR_MAX || (n > 1800 && bytes > 100000000);
 }
 
+// Cluster size and shared-memory caps of the cluster kernels on this thread's
+// device: 16 CTAs per cluster when the device can co-schedule that many with
+// the full shared-memory carve-out, else 8, else none (an error for sectors that
+// need them).
 struct ClusterPlan {
   int device = -1;
   int cl = 0;
-  int64_t vals_cap = 0, vecs_cap = 0;  // doubles of dynamic shared memory per CTA
+  int64_t vals_cap = 0, blocked_cap = 0, vecs_cap = 0;  // doubles of dynamic shared memory per CTA
 };
 
 const ClusterPlan& cluster_plan(tt_ctx* ctx) {
@@ -2238,19 +2700,20 @@ const ClusterPlan& cluster_plan(tt_ctx* ctx) {
     cudaGetLastError();
     return cp;
   }
-  cudaFuncAttributes fa, fb;
-  if (cudaFuncGetAttributes(&fa, vals_kernel(MAX_N)) != cudaSuccess ||
-      cudaFuncGetAttributes(&fb, tridiag_eigvecs_cluster) != cudaSuccess) {
-    cudaGetLastError();
-    return cp;
-  }
-  const int64_t va = ((int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024) / 8;
-  const int64_t vb = ((int64_t)optin - (int64_t)fb.sharedSizeBytes - 1024) / 8;
-  if (vb < 6 * MAX_N) return cp;
   constexpr int NK = 5;
-  const void* kernels[NK] = {vals_kernel(1), vals_kernel(4 * CR_THREADS), vals_kernel(8 * CR_THREADS), vals_kernel(MAX_N),
-                             (const void*)tridiag_eigvecs_cluster};
-  const int64_t caps[NK] = {va, va, va, va, vb};
+  const void* kernels[NK] = {vals_kernel(1), vals_kernel(4 * CR_THREADS), vals_kernel(CR_MAX),
+                             (const void*)tridiag_blocked_cluster, (const void*)tridiag_eigvecs_cluster};
+  int64_t caps[NK];
+  for (int k = 0; k < NK; ++k) {
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, kernels[k]) != cudaSuccess) {
+      cudaGetLastError();
+      return cp;
+    }
+    caps[k] = ((int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024) / 8;
+  }
+  const int64_t va = std::min({caps[0], caps[1], caps[2]}), vc = caps[3], vb = caps[4];
+  if (vb < 6 * MAX_N) return cp;
   for (int k = 0; k < NK; ++k) {
     if (cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(caps[k] * 8)) !=
             cudaSuccess ||
@@ -2264,7 +2727,8 @@ const ClusterPlan& cluster_plan(tt_ctx* ctx) {
     return cp;
   }
   for (int cl : {CL_MAX, 8}) {
-    bool ok = cluster_layout(MAX_N, cl, va).nb > 0;  // the largest sector fits
+    // the largest sectors fit, the blocked reduction's at the narrowest panel
+    bool ok = cluster_layout(CR_MAX, cl, va).nb > 0 && blocked_smem(MAX_N, 8, cl) <= vc;
     for (int k = 0; k < NK && ok; ++k) {
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute at[1];
@@ -2273,7 +2737,7 @@ const ClusterPlan& cluster_plan(tt_ctx* ctx) {
       at[0].val.clusterDim.y = 1;
       at[0].val.clusterDim.z = 1;
       cfg.gridDim = dim3(cl);
-      cfg.blockDim = dim3(k + 1 < NK ? CR_THREADS : TT);
+      cfg.blockDim = dim3(k < 3 ? CR_THREADS : TT);
       cfg.dynamicSmemBytes = (size_t)(caps[k] * 8);
       cfg.attrs = at;
       cfg.numAttrs = 1;
@@ -2290,6 +2754,7 @@ const ClusterPlan& cluster_plan(tt_ctx* ctx) {
     }
   }
   cp.vals_cap = va;
+  cp.blocked_cap = vc;
   cp.vecs_cap = vb;
   return cp;
 }
@@ -2355,9 +2820,19 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
   const int n_small = (int)hp.size();
   int64_t need = 0, scratch = 0;
   int nbig_max = 0;
+  const bool blocked = blocked_sectors(big);
   if (!big.empty()) {
     TT_REQUIRE(cp.cl > 0, "tt_sym_eigvals_batched: no thread-block clusters for sectors of this size");
     for (EigDev& e : big) {
+      if (blocked) {  // the widest panel whose shared memory fits
+        e.nb = PNB_MAX;
+        while (e.nb > 8 && blocked_smem(e.n, e.nb, cp.cl) > cp.blocked_cap) e.nb /= 2;
+        need = std::max(need, blocked_smem(e.n, e.nb, cp.cl));
+        TT_REQUIRE(need <= cp.blocked_cap, "tt_sym_eigvals_batched: sector too large for the cluster eigensolver");
+        e.s_off = scratch;
+        scratch += (int64_t)e.n * 2 * e.nb;
+        continue;
+      }
       const ClusterLayout L = cluster_layout(e.n, cp.cl, cp.vals_cap);
       TT_REQUIRE(L.nb > 0, "tt_sym_eigvals_batched: sector too large for the cluster eigensolver");
       // the layouts of later stages take what there is
@@ -2376,7 +2851,7 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
     nmax = std::max(nmax, hp[p].n);
     for (int j0 = 0; j0 < hp[p].n; j0 += BS_PER) bt.push_back(VecTaskB{p, j0});
   }
-  // problems, bisection tasks and the columns' scratch in one buffer
+  // problems, bisection tasks and the reductions' scratch in one buffer
   const size_t pb = sizeof(EigDev) * hp.size(), tb = (sizeof(VecTaskB) * bt.size() + 15) & ~(size_t)15;
   std::vector<char> host(pb + tb);
   std::memcpy(host.data(), hp.data(), pb);
@@ -2386,7 +2861,7 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
   TT_CUDA(tt::h2d_async(ctx, buf, host.data(), host.size()));
   const EigDev* dp = reinterpret_cast<const EigDev*>(buf);
   const VecTaskB* d_bt = reinterpret_cast<const VecTaskB*>(buf + pb);
-  double* cols = reinterpret_cast<double*>(buf + pb + tb);
+  double* sc = reinterpret_cast<double*>(buf + pb + tb);
   static thread_local uint64_t attr = 0;  // per host thread and device
   if (tt::first_on_device(attr, ctx->device)) {
     TT_CUDA(cudaFuncSetAttribute(tridiag_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2400,9 +2875,12 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
         dp, G, T, w, A);
     TT_LAUNCH_CHECK(ctx);
   }
-  if (!big.empty()) {
+  if (blocked) {
+    TT_CUDA(launch_cluster(ctx, cp.cl, TT, (int)big.size(), need, (const void*)tridiag_blocked_cluster, dp + n_small, G,
+                           T, sc));
+  } else if (!big.empty()) {
     TT_CUDA(launch(ctx, cp.cl * (int)big.size(), CR_THREADS, cp.cl, (size_t)(need * 8), n_small > 0,
-                   vals_kernel(nbig_max), dp + n_small, G, T, cols, need));
+                   vals_kernel(nbig_max), dp + n_small, G, T, sc, need));
   }
   if (!bt.empty()) {
     const size_t bs_smem = sizeof(double2) * (size_t)((nmax + 7) & ~7);
