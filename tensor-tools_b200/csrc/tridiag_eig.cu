@@ -2821,8 +2821,17 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
   int64_t need = 0, scratch = 0;
   int nbig_max = 0;
   const bool blocked = blocked_sectors(big);
+  int cl = cp.cl;
   if (!big.empty()) {
     TT_REQUIRE(cp.cl > 0, "tt_sym_eigvals_batched: no thread-block clusters for sectors of this size");
+    for (const EigDev& e : big) nbig_max = std::max(nbig_max, e.n);
+    // More clusters than run at once: smaller ones, as long as their CTAs hold the
+    // columns in shared memory.  In clusters of 16, 20 sectors of 130 took 1291 us and
+    // 100 of 160 7.73 ms (one CTA each, before: 937 us and 1.35 ms), so 469 us and 1.48
+    // ms; 74 of 220 8.0 -> 2.6 ms, 36 of 260 5.3 -> 2.2.
+    while (!blocked && cl > 2 && (int64_t)big.size() * cl > ctx->num_sms &&
+           cluster_layout(nbig_max, cl / 2, cp.vals_cap).resident)
+      cl /= 2;
     for (EigDev& e : big) {
       if (blocked) {  // the widest panel whose shared memory fits
         e.nb = PNB_MAX;
@@ -2833,13 +2842,12 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
         scratch += (int64_t)e.n * 2 * e.nb;
         continue;
       }
-      const ClusterLayout L = cluster_layout(e.n, cp.cl, cp.vals_cap);
+      const ClusterLayout L = cluster_layout(e.n, cl, cp.vals_cap);
       TT_REQUIRE(L.nb > 0, "tt_sym_eigvals_batched: sector too large for the cluster eigensolver");
       // the layouts of later stages take what there is
       need = std::max(need, L.resident ? L.doubles : cp.vals_cap);
       e.s_off = scratch;
-      nbig_max = std::max(nbig_max, e.n);
-      scratch += (int64_t)cp.cl * ((e.n + cp.cl - 1) / cp.cl) * cl_ld(e.n);
+      scratch += (int64_t)cl * ((e.n + cl - 1) / cl) * cl_ld(e.n);
     }
   }
   hp.insert(hp.end(), big.begin(), big.end());
@@ -2879,7 +2887,7 @@ int tt_sym_eigvals_batched(tt_ctx* ctx, const tt_eig_problem* probs, int n_probs
     TT_CUDA(launch_cluster(ctx, cp.cl, TT, (int)big.size(), need, (const void*)tridiag_blocked_cluster, dp + n_small, G,
                            T, sc));
   } else if (!big.empty()) {
-    TT_CUDA(launch(ctx, cp.cl * (int)big.size(), CR_THREADS, cp.cl, (size_t)(need * 8), n_small > 0,
+    TT_CUDA(launch(ctx, cl * (int)big.size(), CR_THREADS, cl, (size_t)(need * 8), n_small > 0,
                    vals_kernel(nbig_max), dp + n_small, G, T, sc, need));
   }
   if (!bt.empty()) {

@@ -23,7 +23,8 @@ def _reflect(G, v):
     return G - 2.0 * np.outer(v, g) - 2.0 * np.outer(g, v) + 4.0 * (v @ g) * np.outer(v, v)
 
 
-@pytest.mark.parametrize("ns", [[1900] * 4 + [130, 40], [2049, 700]])
+@pytest.mark.parametrize("ns", [[1900] * 4 + [130, 40], [2049, 700], [129 + 3 * (i % 11) for i in range(12)],
+                                [160, 131, 20] * 9, [129 + i % 32 for i in range(80)], [300] * 18 + [129]])
 def test_batch(ns):
     import torch
     import tt_b200
