@@ -197,16 +197,16 @@ void measure_sz(const qMPS& psi, std::vector<double>& sz, std::vector<double>& s
     ZR[i] = D * zket[i];
     if (i > 0) ER = D * psi.A[i];
   }
-  // 64 sites at a time, fewer where that would be more than 2^26 numbers
-  const unsigned chunk =
+  // 64 sites at a time, fewer where that would be more than 2^26 numbers, or more than
+  // the device has room for
+  unsigned chunk =
       (unsigned)std::max<int64_t>(1, std::min<int64_t>(std::min(L, 64u), ((int64_t)1 << 26) / largest));
   const unsigned row = chunk + 1;
   sz.assign(L, 0.0);
   szsz.assign((size_t)L * L, 0.0);
   DevBuf vals((int64_t)L * row);
   std::vector<double> h((size_t)L * row);
-  for (unsigned i0 = 0; i0 < L; i0 += chunk) {
-    const unsigned i1 = std::min(L, i0 + chunk);
+  auto group = [&](unsigned i0, unsigned i1) {  // the sites i0 <= i < i1
     vals.zero();
     qtensor S = with_origin(qtensor(), EL[i0]);
     for (unsigned j = i0; j < L; ++j) {
@@ -226,6 +226,16 @@ void measure_sz(const qMPS& psi, std::vector<double>& sz, std::vector<double>& s
       }
       for (unsigned i = i0; i < std::min(i1, j); ++i)
         szsz[(size_t)i * L + j] = szsz[(size_t)j * L + i] = h[(size_t)j * row + 1 + i - i0] / nrm2;
+    }
+  };
+  for (unsigned i0 = 0; i0 < L;) {
+    const unsigned i1 = std::min(L, i0 + chunk);
+    try {
+      group(i0, i1);
+      i0 = i1;
+    } catch (const tt_error& e) {
+      if (e.code != TT_ERR_OOM || chunk == 1) throw;
+      chunk = (chunk + 1) / 2;
     }
   }
 }
