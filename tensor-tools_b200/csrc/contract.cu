@@ -1400,9 +1400,11 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
     }
     // A thread per row or fragments?  Measured over 1e3 to 1e6 rows (in 128s per SM: 0.05
     // to 50), 1 to 32 columns, k of 5 to 1200, each against both and against 64 x 64 tiles:
-    // up to 8 columns a thread per row is better at any k once half of the SMs have rows
-    // (30000 rows, k = 128, 1 and 8 columns: 7.9 and 10.7 us, fragments 17 and 18; 8000
-    // rows, k = 56: 6.4 and 7.8, fragments 5.6 and 6.2); up to 16 columns until the
+    // up to 8 columns a thread per row is better once half of the SMs have rows (30000
+    // rows, k = 128, 1 and 8 columns: 7.9 and 10.7 us, fragments 17 and 18; 8000 rows, k =
+    // 56: 6.4 and 7.8, fragments 5.6 and 6.2), with k of up to 28 four per SM (three
+    // products of a chain, k = 8 over many short chunks, 0.8 to 3.8 of them: 82.5 and 112
+    // us, fragments 78.5 and 110, 5.1: 135 and 141); up to 16 columns until the
     // FP64 sums of one row outweigh its loads (16 columns, k = 56: 60000 rows 14.5 and
     // 16.3 us, 250000 54 and 48, 1e6 196 and 149; k = 14: 9.1 and 12.7 at 120000, 72 and
     // 71 at 1e6).  With more k than fragments take, tiles are better while there are few
@@ -1415,9 +1417,10 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
       ksum += work[o];
     }
     bool per_row;
-    if (nr_cols <= 8) per_row = klong <= NR_KTOT ? 2 * all >= sms : all >= sms;
-    else if (nr_cols > RD_COLS) per_row = false;
-    else if (klong <= NR_KTOT) per_row = all >= sms && (all < 20 * sms || klong <= 16);
+    if (nr_cols > RD_COLS) per_row = false;
+    else if (klong <= 28) per_row = all >= 4 * sms && (nr_cols <= 8 || all < 20 * sms || klong <= 16);
+    else if (nr_cols <= 8) per_row = klong <= NR_KTOT ? 2 * all >= sms : all >= sms;
+    else if (klong <= NR_KTOT) per_row = all >= sms && all < 20 * sms;
     else per_row = all >= 2 * sms && 5 * kpad >= 7 * ksum;
     if (per_row) rd_threads = klong <= NR_KTOT ? 128 : 256;
     else narrow = klong <= NR_KTOT;
