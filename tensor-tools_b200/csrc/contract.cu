@@ -1102,60 +1102,97 @@ pack_tf32_ab(const PackJob* __restrict__ jobsA, const PackTile* __restrict__ til
     reinterpret_cast<uint4*>(dst)[v] = reinterpret_cast<const uint4*>(st)[v];
 }
 
-// Cost model of the *_AUTO precisions: predicted device time (microseconds)
-// of one exec of a contraction in `prec` (FP64 DMMA, or a tcgen05 kind with
-// its two packing launches).  Work is counted on padded tiles (an output tile
-// runs every pair of its block over k rounded up to the k-step); the grid is
-// bound by the total at the full-chip rate, by its longest tile at one SM's
-// rate, and by its DRAM bytes.  The tensor-core form moves each operand
-// element three more times (read by the packer, written packed, read packed),
-// so a contraction with a small k -- the bandwidth-bound middle contraction
-// of H_eff*x and of the environment update -- stays in FP64, which is exact
-// to more digits and faster there (measured at bond dimension 1024 on the
-// J1-J2 cylinder: 354 us FP64 against 685 us packed tensor-core form, while
-// L*x and *R take 141 and 161 us on the tensor cores against 301 and 473 us
-// in FP64).  Rates are the measured single-block throughputs of the two
-// kernels on B200 (4096^3: DMMA 26 TFLOP/s, tcgen05 690 TFLOP/s of TF32
-// products).
+// CTAs that share a tile's k range in grouped_dgemm, for plans of `tiles` tiles of at
+// most `longest` chunks.  While there are fewer than two CTAs per SM, each keeps two
+// chunks of the longest tile; a long k is shared also while there are fewer than two
+// rounds (four CTAs fit an SM) and each keeps 12.  R at bond dimension 1400 (420 tiles, k
+// up to 6552): 1110 us whole, 730 in four; stopping at one round 860.  The products of a
+// chain at 128 (34 tiles of at most 12 chunks): 129 us per three products whole, 123 down
+// to four chunks, 105 down to two.  Two chunks up to two rounds paid more for the
+// exchange than for the idle SMs: environment update of the cylinder at 400 85 us, now
+// 67, at 700 190 and 155; with 8 chunks instead of 12 a chain's at 957 130, now 120, with
+// 16 three products of a chain at 700 350, now 296.
+int dgemm_split(int64_t tiles, int longest, int num_sms) {
+  int split = 1;
+  while (split < SPLIT_MAX && ((tiles * split < 2 * (int64_t)num_sms && longest / (2 * split) >= 2) ||
+                               (tiles * split < 8 * (int64_t)num_sms && longest / (2 * split) >= 12)))
+    split *= 2;
+  return split;
+}
+
+// Cost model of the *_AUTO precisions: predicted device time (microseconds) of one exec
+// of a contraction in `prec` (FP64, or a tcgen05 kind with its two packing launches).
+// Fitted to 242 contractions (1 to 40 blocks of 40 x 40 to 20000 x 40, k of 64 to 6000, and
+// blocks of mixed sizes as a bond has): FP64 0.79 to 1.15 and 3xTF32 0.77 to 1.02 of the
+// measured time (tenth to ninetieth per cent).  The choice that it leads to cost more than
+// 1.15 of the better one in 8 of them, at most 1.41, all but one by staying in FP64.
+//   FP64 tiles: c CTAs of an SM take 0.6 + 0.58 c us per chunk of 16 k together (1.2 us
+//     alone, the latencies of one chunk; 0.73 each where four share the SM), a tile 1.5
+//     chunks more for its start and end; CTAs come in rounds of four per SM, and a tile's k
+//     range is shared as the plan shares it.
+//   FP64 narrow chunks: bound by their bytes.
+//   Tensor cores: 0.57 us per chunk of 32 k and tile in 3xTF32, a tile at a time per SM;
+//     the packed operands and C pass through memory, and before that every operand is read
+//     and written packed (kept operands once for kKeptUses execs).
 double predict_us(const tt_out_block* outs, int n_out, const std::vector<PairDev>& hp,
                   const std::vector<int>& first, int prec, int num_sms, int keep = 0) {
-  constexpr double kDmmaRate = 27e12, kTcRate = 650e12, kHbm = 6.0e12, kLaunchUs = 2.5;
+  constexpr double kHbm = 5.0e6, kKeptUses = 4.0;  // bytes per us
+  const double sms = std::max(1, num_sms);
   const bool tc = prec != TT_PREC_FP64;
-  // the DMMA kernel stops at k rounded up to its k-step of 4; the tcgen05
-  // kernel runs whole 32-wide k-chunks
-  const int tm = tc ? TC_BM : BM, tn = tc ? TC_BN : BN, tk = tc ? TC_BK : 4;
-  const double rate = tc ? (prec == TT_PREC_TF32X3 ? kTcRate / 3.0 : kTcRate) : kDmmaRate;
+  const int tm = tc ? TC_BM : BM, tn = tc ? TC_BN : BN;
   auto up = [](int x, int t) { return (double)((x + t - 1) / t) * t; };
-  double total = 0.0, longest = 0.0, bytes = 0.0;
+  // a pair's k in chunks: of 32, or of 16, whose last one costs less where 8 or fewer are left
+  auto cost = [&](int k) { return tc ? up(k, TC_BK) / TC_BK : k / BK + (k % BK == 0 ? 0.0 : k % BK <= 8 ? 0.7 : 1.0); };
+  double tiles = 0.0, total = 0.0, longest = 0.0, c_bytes = 0.0;
+  int chunks = 0;  // of the longest tile, as the plan counts them
+  bool narrow = !tc;
   std::map<int64_t, std::pair<double, double>> ua, ub;  // distinct operand blocks: (elements, padded elements)
   for (int o = 0; o < n_out; ++o) {
-    double kpad = 0.0;
+    double task = 0.0;
+    int whole = 0;
+    int64_t k = 0;
     for (int i = first[o]; i < first[o + 1]; ++i) {
       const PairDev& P = hp[i];
-      kpad += up(P.k, tk);
-      ua.emplace(P.a_off, std::make_pair((double)P.m * P.k, up(P.m, tm) * up(P.k, tk)));
-      ub.emplace(P.b_off, std::make_pair((double)P.n * P.k, up(P.n, tn) * up(P.k, tk)));
+      task += cost(P.k);
+      whole += (P.k + BK - 1) / BK;
+      k += P.k;
+      narrow = narrow && P.k <= NR_K;
+      ua.emplace(P.a_off, std::make_pair((double)P.m * P.k, up(P.m, tm) * up(P.k, TC_BK)));
+      ub.emplace(P.b_off, std::make_pair((double)P.n * P.k, up(P.n, tn) * up(P.k, TC_BK)));
     }
-    const double tiles = up(outs[o].m, tm) / tm * (up(outs[o].n, tn) / tn);
-    const double task = 2.0 * tm * tn * kpad;
-    total += tiles * task;
-    if (tiles > 0) longest = std::max(longest, task);
-    bytes += 8.0 * outs[o].m * outs[o].n;  // C
+    narrow = narrow && outs[o].n <= NR_N && k <= NR_KTOT;
+    const double t = up(outs[o].m, tm) / tm * (up(outs[o].n, tn) / tn);
+    tiles += t;
+    total += t * task;
+    if (t > 0) {
+      longest = std::max(longest, task);
+      chunks = std::max(chunks, whole);
+    }
+    c_bytes += 8.0 * outs[o].m * outs[o].n;
   }
-  // FP64 reads every operand element once from DRAM; the tensor-core form
-  // also writes the packed tiles (hi + lo: 8 bytes per padded element, TF32:
-  // 4) and reads them back
-  const double packed = prec == TT_PREC_TF32X3 ? 8.0 : 4.0;
-  // an operand kept packed across execs (keep bit 0: A, bit 1: B) is packed
-  // once for kKeptUses of them
-  constexpr double kKeptUses = 4.0;
+  double read = 0.0, pack = 0.0, packed = 0.0;
+  const double per = prec == TT_PREC_TF32X3 ? 8.0 : 4.0;  // bytes of a packed element
   for (int w = 0; w < 2; ++w) {
     const double share = ((keep >> w) & 1) ? 1.0 / kKeptUses : 1.0;
-    for (const auto& kv : (w == 0 ? ua : ub))
-      bytes += 8.0 * kv.second.first + (tc ? 2.0 * packed * kv.second.second * share : 0.0);
+    for (const auto& kv : (w == 0 ? ua : ub)) {
+      read += 8.0 * kv.second.first;
+      pack += (8.0 * kv.second.first + per * kv.second.second) * share;
+      packed += per * kv.second.second;
+    }
   }
-  const double t = std::max({total / rate, longest / (rate / std::max(1, num_sms)), bytes / kHbm});
-  return t * 1e6 + (tc ? 3 : 1) * kLaunchUs;
+  if (narrow) return 3.0 + (read + c_bytes) / 3.0e6;
+  if (tc) {
+    const double tau = prec == TT_PREC_TF32X3 ? 0.57 : 0.25;
+    const double rounds = tiles <= 4 * sms ? std::ceil(tiles / sms) : tiles / sms;
+    const double mma = std::max(longest, tiles > 0 ? rounds * total / tiles : 0.0) * tau;
+    return 12.0 + pack / kHbm + std::max(mma, (packed + c_bytes) / kHbm);
+  }
+  const int split = dgemm_split((int64_t)tiles, chunks, num_sms);
+  const double ctas = tiles * split, avg = ctas > 0 ? total / ctas + 1.5 : 0.0;
+  auto tau = [](double c) { return c > 0 ? 0.6 + 0.58 * c : 0.0; };  // c CTAs of an SM, a chunk each
+  const double full = std::floor(ctas / (4 * sms)), rest = std::ceil((ctas - full * 4 * sms) / sms);
+  const double math = std::max((longest / split + 1.5) * tau(1), avg * (full * tau(4) + tau(rest)));
+  return 2.5 + (split > 1 ? 1.5 : 0.0) + std::max(math, (read + c_bytes) / 6.0e6);
 }
 
 }  // namespace
@@ -1590,20 +1627,7 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
       dtasks.push_back(DTask{o.c_off, o.m, o.n, o.ldc, t.m0, t.n0, t.p_begin, t.p_end, chunks[t.out]});
       longest = std::max(longest, chunks[t.out]);
     }
-    // A tile's k range is shared by a cluster while the plan has fewer than two CTAs
-    // per SM and each keeps two chunks of the longest tile; a long k also while it
-    // has fewer than two rounds (four CTAs fit an SM) and each keeps 12.  R at bond
-    // dimension 1400 (420 tiles, k up to 6552): 1110 us whole, 730 in four; stopping
-    // at one round 860.  The products of a chain at 128 (34 tiles of at most 12
-    // chunks): 129 us per three products whole, 123 down to four chunks, 105 down to
-    // two.  Two chunks up to two rounds paid more for the exchange than for the idle
-    // SMs: environment update of the cylinder at 400 85 us, now 67, at 700 190 and
-    // 155; with 8 chunks instead of 12 a chain's at 957 130, now 120, with 16 three
-    // products of a chain at 700 350, now 296.
-    while (split < SPLIT_MAX &&
-           (((int64_t)dtasks.size() * split < 2 * (int64_t)ctx->num_sms && longest / (2 * split) >= 2) ||
-            ((int64_t)dtasks.size() * split < 8 * (int64_t)ctx->num_sms && longest / (2 * split) >= 12)))
-      split *= 2;
+    split = dgemm_split((int64_t)dtasks.size(), longest, ctx->num_sms);
   }
   std::vector<OutDev> ho(n_out);
   for (int o = 0; o < n_out; ++o) ho[o] = OutDev{outs[o].c_off, outs[o].m, outs[o].n, outs[o].ldc};
