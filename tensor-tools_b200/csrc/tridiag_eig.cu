@@ -2233,7 +2233,9 @@ chol_cluster(const EigDev* __restrict__ probs, double* work, int* flags, int che
   const int CL = (int)cluster.num_blocks();
   const int rank = (int)cluster.block_rank();
   const int pi = blockIdx.x / CL;
-  if (flags[pi]) return;  // the whole cluster alike
+  const bool redo = flags[pi] != 0;
+  cluster.sync();  // read by every CTA before CTA 0 may raise it: the whole cluster goes on or returns
+  if (redo) return;
   const EigDev P = probs[pi];
   const int m = P.nvec;
   double* A = work + 3 * P.g_off;

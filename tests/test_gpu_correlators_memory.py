@@ -1,11 +1,10 @@
 """The Sz correlators on a device with little room left.
 
 ``measure_sz`` takes the environments of many sites through the chain together; where the
-device has no room for them it takes fewer, down to one at a time.
-A 26-site chain with bonds up to 1800 takes about 130
-MB that way and 420 MB together; with 200 MB left it has to give what it gave with the
-device empty.  In a process of its own: a pool that an earlier context has grown would
-serve it.
+device has no room for them it takes fewer, down to one at a time.  A 26-site chain with
+bonds up to 1800 takes about 130 MB that way and 420 MB together; with 200 MB left it has
+to give what it gave with the device empty.  In a process of its own: a pool that an
+earlier context has grown would serve it.
 """
 import os
 import subprocess
