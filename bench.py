@@ -127,6 +127,7 @@ def parse():
     p.add_argument("--breakdown", action="store_true", help="one further step per precision with phase times")
     p.add_argument("--env-prec", default=ENV_PREC, help="environment-update precision of the chosen form")
     p.add_argument("--no-clock-sampler", action="store_true", help="diagnostic: no nvidia-smi sampling")
+    p.add_argument("--detail", help="file for the whole result: per-step times, phases and host load of both arms")
     p.add_argument("--gemm-size", type=int, default=4096)
     p.add_argument("--precisions", default="fp64,tf32x3,tf32")
     p.add_argument("--chains", type=int, default=64)
@@ -669,6 +670,30 @@ def c5_arm(prec, ck, H, args, ctx, stream, flush, torch, tt_b200, sampler=None, 
     return res
 
 
+def _rounded(x):
+    if isinstance(x, dict):
+        return {k: _rounded(v) for k, v in x.items()}
+    if isinstance(x, (list, tuple)):
+        return [_rounded(v) for v in x]
+    return float("%.7g" % x) if isinstance(x, float) else x
+
+
+def compact(out):
+    """The result line of what --detail writes: of the two arms what their comparison needs, numbers with seven digits
+    (energies in full)."""
+    line = {k: _rounded(v) for k, v in out.items() if k not in ("mixed", "fp64")}
+    short = ("value", "ms_per_step", "heff_share_of_step", "heff_tflops", "launches_per_step", "speedup_vs_fp64")
+    full = ("energy", "dE_per_site_vs_fp64", "szsz_max_abs_err_vs_fp64", "full_sweep")
+    for name in ("mixed", "fp64"):
+        arm = out[name]
+        line[name] = {k: _rounded(arm[k]) for k in short if k in arm}
+        line[name].update({k: arm[k] for k in full if k in arm})
+        if "step_seconds" in arm:
+            line[name]["step_seconds_min_max"] = _rounded([min(arm["step_seconds"]), max(arm["step_seconds"])])
+        line[name]["kernel_fracs"] = {k: _rounded(r["frac"]) for k, r in arm.get("kernel_rooflines", {}).items()}
+    return line
+
+
 def run_c5(args):
     import torch
     import tt_b200
@@ -779,7 +804,10 @@ def run_c5(args):
             "fp64": fp64,
             "peaks_measured": peaks,
         }
-        print(json.dumps(out))
+        if args.detail:
+            with open(args.detail, "w") as f:
+                json.dump(out, f)
+        print(json.dumps(compact(out)))
     ctx.close()
     if dist is not None:
         dist.destroy_process_group()
