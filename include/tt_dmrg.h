@@ -92,9 +92,10 @@ int tt_dmrg_unbind(void);
 int tt_dmrg_set_profiling(int on);
 /* Per-thread totals over the device-resident Davidson calls' H_eff*x
  * products: device milliseconds and algorithmic flops of L*x, *mid and *R
- * (ms[0..2], flops[0..2], event-timed on the library stream) and the
- * algorithmic bytes of the *mid contractions (distinct operand blocks read
- * once, the output written once). */
+ * (ms[0..2], flops[0..2]; timed by events on the library stream, or by the
+ * contractions' own clock stamps where all three run in FP64 on vectors of up
+ * to TT_DAV_STEP_MAX elements) and the algorithmic bytes of the *mid
+ * contractions (distinct operand blocks read once, the output written once). */
 int tt_dmrg_heff_parts(double* ms, double* flops, double* mid_bytes);
 /* host-side planning counters of this thread: seconds and calls spent in
  * block-structure computation and in contraction-plan creation */

@@ -212,6 +212,23 @@ __device__ __forceinline__ void load_chunk(double* st, const double* __restrict_
   }
 }
 
+// A contraction is one of a chain of small launches.  It is launched so that it may
+// start when the blocks of the kernel before it have ended; it waits here for that
+// kernel's memory before it touches anything but its own plan, which an earlier copy
+// wrote.  (A kernel that let the next one in from its own start lost 5 % at
+// m = 1400.)  The pointers to what plain loads read pass through the wait: no read
+// through a __restrict__ argument is moved above it (asynchronous copies are not
+// moved; rows_dgemm's loads of A have a line of their own).  The stamp is the device's clock at that point.  Nine
+// launches of three products at a chain's m = 128: 86 -> 68 us.
+__device__ __forceinline__ void after_previous(const int32_t* __restrict__& tab, unsigned long long* stamp) {
+  asm volatile("griddepcontrol.wait;" : "+l"(tab) : : "memory");
+  if (stamp && blockIdx.x == 0 && threadIdx.x == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    *stamp = t;
+  }
+}
+
 // A cluster of CTAs (one, where the plan has tiles enough to fill the GPU)
 // takes one output tile; its CTAs share the tile's k chunks evenly, in order,
 // and add their partial tiles through distributed shared memory, CTA 0's
@@ -228,23 +245,6 @@ __device__ __forceinline__ void load_chunk(double* st, const double* __restrict_
 // for every element, padded stages and m8n8k4 fragments: env update at bond
 // dimension 2048 1154 -> 975 us per product; R product at 1400 1110 -> 730 us,
 // where the tile's k range is now shared.
-// A contraction is one of a chain of small launches.  It is launched so that it may
-// start when the blocks of the kernel before it have ended; it waits here for that
-// kernel's memory before it touches anything but its own plan, which an earlier copy
-// wrote.  (A kernel that let the next one in from its own start lost 5 % at
-// m = 1400.)  The pointers to what plain loads read pass through the wait: no read
-// through a __restrict__ argument is moved above it (A, and grouped_dgemm's B, are
-// read by cp.async only).  The stamp is the device's clock at that point.  Nine
-// launches of three products at a chain's m = 128: 86 -> 68 us.
-__device__ __forceinline__ void after_previous(const int32_t* __restrict__& tab, unsigned long long* stamp) {
-  asm volatile("griddepcontrol.wait;" : "+l"(tab) : : "memory");
-  if (stamp && blockIdx.x == 0 && threadIdx.x == 0) {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    *stamp = t;
-  }
-}
-
 __global__ void __launch_bounds__(THREADS, 4)
 grouped_dgemm(const DTask* __restrict__ tasks,
               const PairDev* __restrict__ pairs, const int32_t* __restrict__ tab,

@@ -229,7 +229,6 @@ class ProductEngine {
     return precision;
   }
 
-  // ev (optional): four events recorded before L*x, after it, after *mid and after *R
   // whether the three contractions can stamp the device's clock themselves
   bool stamps(int precision) {
     tt_plan* p[3] = {c1_->plan_for(part_precision(precision, 0, part_flops[0]), 1),
@@ -238,8 +237,8 @@ class ProductEngine {
     return tt_plan_stamps(p[0]) && tt_plan_stamps(p[1]) && tt_plan_stamps(p[2]);
   }
 
-  // ev: four events around the contractions; stamps: three device slots for the
-  // clock when each of them starts
+  // ev (optional): four events recorded before L*x, after it, after *mid and after *R;
+  // stamps (optional): three device slots for the clock when each of them starts
   void apply(const double* v, double* y, int precision = TT_PREC_FP64, void* const* ev = nullptr,
              uint64_t* stamps = nullptr) {
     if (ev) check(tt_event_record(ctx(), ev[0]), "event");

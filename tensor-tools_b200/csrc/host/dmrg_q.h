@@ -122,7 +122,7 @@ struct DmrgLog {
   std::vector<double> entropy;
   double initial_energy = 0.0;
   double heff_flops = 0.0;
-  double heff_seconds = 0.0;  // device time of the H_eff*x launches (event-timed)
+  double heff_seconds = 0.0;  // device time of the H_eff*x launches (events or clock stamps)
 };
 
 // One environment step ((A^dag' env) W) A, for a left or a right environment

@@ -197,8 +197,9 @@ void measure_sz(const qMPS& psi, std::vector<double>& sz, std::vector<double>& s
     ZR[i] = D * zket[i];
     if (i > 0) ER = D * psi.A[i];
   }
-  // 64 sites at a time, fewer where that would be more than 2^26 numbers, or more than
-  // the device has room for
+  // 64 sites at a time (100 sites, bond dimension 40: 16 sites 35 ms, 64 25, all 24; 160
+  // sites at 20: 55, 34, 29), fewer where that would be more than 2^26 numbers, 0.5 GB in
+  // each of the four stacks that are alive at once, or more than the device has room for
   unsigned chunk =
       (unsigned)std::max<int64_t>(1, std::min<int64_t>(std::min(L, 64u), ((int64_t)1 << 26) / largest));
   const unsigned row = chunk + 1;

@@ -116,6 +116,7 @@ __device__ __forceinline__ int sturm_count(const double2* de, int npad, double x
 // stops at 128: its working arrays and a 128 x 128 matrix take 197 KB.
 // doubles of shared memory
 __host__ __device__ constexpr int64_t small_smem(int n, int nw) { return (int64_t)n * n + 4 * (int64_t)nw * n + n; }
+// six sectors of 20 and of 32 states: 58 and 74 us with 256 threads, 64 and 85 with 512
 constexpr int small_threads(int nmax) { return nmax <= 32 ? 256 : 512; }
 
 __global__ void __launch_bounds__(TT, 1)
@@ -867,7 +868,9 @@ __host__ __device__ inline ClusterLayout cluster_layout(int n, int CL, int64_t c
     const int64_t fixed = CLR_MISC + 5 * ld + (resident ? nloc * ld : 0);
     int64_t nb = fixed < cap ? (cap - fixed) / (2 * (ld + nloc)) : 0;
     if (nb > NB_MAX) nb = NB_MAX;
-    // resident columns pay when a few reflectors still fit beside them
+    // resident columns pay when a few reflectors still fit beside them (n = 470, 6 and
+    // in L2 16 pending: 1.88 and 2.04 ms; from 2 on 540 would take 2.29 ms for 2.43, 700 as
+    // long)
     if (nb < (resident ? 6 : 1)) continue;
     return ClusterLayout{(int)nb, resident, fixed + nb * 2 * (ld + nloc)};
   }
@@ -2222,9 +2225,9 @@ __device__ __forceinline__ void solve_row(double (&x)[CH_PB], const double (*lt)
 // path, the fragments straight from L2, all loads of a tile in flight (two k steps
 // at a time by twice the warps: 646 us).  A panel is a chain of L2 latencies and two
 // cluster barriers.  At bond dimension 3072 1221 -> 372 us (three barriers per
-// column of the block, divisions, 64 x 64 tiles on the FP64 pipe).
-// Pivots below COLLAPSE_PIVOT2 (first pass) flag the problem; a flagged or non-positive pivot is replaced by 1 so the
-// arithmetic stays finite (the problem is redone by the fallback).
+// column of the block, divisions, 64 x 64 tiles on the FP64 pipe).  Pivots below
+// COLLAPSE_PIVOT2 (first pass) flag the problem; a flagged or non-positive pivot is
+// replaced by 1 so the arithmetic stays finite (the problem is redone by the fallback).
 __global__ void __launch_bounds__(CH_THREADS)
 chol_cluster(const EigDev* __restrict__ probs, double* work, int* flags, int check) {
   __shared__ __align__(16) double lt[CH_PB][CH_LD];
