@@ -473,7 +473,11 @@ __device__ __forceinline__ double hash_unit(uint64_t z) {
 // Eigenvectors of the sectors with n <= SN, one CTA each.
 //
 // (a) Inverse iteration, one thread per vector: T - lambda I is factored once
-//     (one reciprocal per step), the INV_ITERS solves then are substitutions only.
+//     (one reciprocal per step; the row exchange is kept in the last bit of the
+//     multiplier, which the factorisation itself uses too), the INV_ITERS solves
+//     then are substitutions only.  Up to 128 rows that bit was seen to move
+//     a vector by 2e-14 at most, and a U(1) sweep's single Gram-Schmidt pass can carry any change of a last
+//     bit here to 5e-9 in <Sz>, so it stays as it is.
 // (b) Gram-Schmidt inside clusters, right-looking and twice: once vector j is
 //     final, every warp takes it out of its share of the later members, so a
 //     vector costs one barrier.  A vector that the first pass has left less than
@@ -493,8 +497,8 @@ __device__ __forceinline__ double small_solve(int n, double scale, double* y, co
   double bi = y[0] * scale;
 #pragma unroll 4
   for (int i = 0; i + 1 < n; ++i) {
-    const double bn = y[i + 1] * scale, f = ml[i * st], m = multiplier(f);
-    const bool sw = exchanged(f);
+    const double bn = y[i + 1] * scale, m = ml[i * st];
+    const bool sw = __double2loint(m) & 1;
     const double top = sw ? bn : bi, low = sw ? bi : bn;
     y[i] = top;
     bi = fma(-m, top, low);
@@ -612,11 +616,12 @@ eigvecs_small(const EigDev* __restrict__ probs, const double* G, const double* T
       const bool sw = fabs(di) < fabs(ci);
       if (!sw && di == 0.0) di = tiny;
       const double piv = sw ? ci : di, r = 1.0 / piv;
-      const double m = multiplier_of(sw ? di : ci, piv, r);
+      double m = (sw ? di : ci) * r;
+      m = __hiloint2double(__double2hiint(m), (__double2loint(m) & ~1) | (sw ? 1 : 0));
       f0[i * st] = fabs(piv) < tiny ? 1.0 / clamped(piv) : r;
       f1[i * st] = sw ? an : si;
       f2[i * st] = sw ? bn : 0.0;
-      fm[i * st] = with_exchange(m, sw);
+      fm[i * st] = m;
       di = sw ? si - m * an : an - m * si;
       si = sw ? -m * bn : bn;
     }
