@@ -626,7 +626,8 @@ narrow_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const
 constexpr int RD_COLS = 16;            // columns of a chunk, at most
 constexpr int RD_SEG = 96 * 1024;      // bytes of staged B, at most
 
-// SEG: more k than a segment, 256 rows to a CTA, else 128
+// SEG: more k than a segment, 256 rows to a CTA, else 128.  Block (x, y) has tile y of
+// task x.
 template <int NC, bool SEG>
 __global__ void __launch_bounds__(SEG ? 256 : 128)
 rows_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const NrB* __restrict__ nb,
@@ -639,10 +640,12 @@ rows_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const N
   const NrChunk& ch = task.ch;
   const int tid = threadIdx.x, warp = tid >> 5;
   const int nblk = ch.a_end - ch.a_begin, ktot = ch.ktot;
+  const int row = task.row0 + (int)(blockDim.x * blockIdx.y) + tid, r = min(row, ch.m - 1);
   if (tid < ch.cols) sc[tid] = nc[ch.c_begin + tid];
   if (tid < min(nblk, NR_AMAX)) sa[tid] = na[ch.a_begin + tid];
   const NrA* blocks = nblk <= NR_AMAX ? sa : na + ch.a_begin;
-  after_previous(tab, stamp);
+  after_previous(tab, blockIdx.y == 0 ? stamp : nullptr);
+  if ((int)blockIdx.y >= task.tiles) return;
   asm volatile("" : "+l"(A), "+l"(B) : : "memory");
   auto stage = [&](int s0, int s1) {
     const int q0 = ch.b_begin + warp;
@@ -652,8 +655,7 @@ rows_dgemm(const NrTask* __restrict__ tasks, const NrA* __restrict__ na, const N
     cp_async_wait<0>();
     __syncthreads();
   };
-  if (!SEG) stage(0, ktot);
-  const int row = task.row0 + tid, r = min(row, ch.m - 1);
+  if (!SEG || ktot == 0) stage(0, ktot);
   const int r1 = ch.d0 != 0 ? r / ch.d0 : 0, r0 = r - r1 * ch.d0;
   double acc[NC];
 #pragma unroll
@@ -1205,7 +1207,8 @@ struct tt_plan {
   int nr_ktot = 0;  // the most k of a chunk
   int nr_rw = 32;   // rows of a warp's tile
   int nr_cols = 0;  // the most columns of a chunk
-  int rd_threads = 0;  // rows_dgemm in its place: rows of a CTA
+  int rd_threads = 0;  // rows_dgemm in its place: rows of a CTA,
+  int rd_tiles = 1;    // and its tiles of a task, at most
   NrTask* d_nr_tasks = nullptr;
   NrA* d_nr_a = nullptr;
   NrB* d_nr_b = nullptr;
@@ -1400,7 +1403,7 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
   // tile tasks, longest first (LPT) so heavy blocks start early
   const int tile_m = tc ? TC_BM : BM, tile_n = tc ? TC_BN : BN;
   std::vector<TaskDev> tsorted;
-  int nr_rw = 32, nr_cols = 0, rd_threads = 0;
+  int nr_rw = 32, nr_cols = 0, rd_threads = 0, rd_tiles = 1;
   std::vector<NrTask> nr_tasks;
   std::vector<NrChunk> nr_chunks;
   std::vector<NrA> nr_a;
@@ -1577,9 +1580,12 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
     // with this bound, 2894 with sixteen tiles as soon as there are four CTAs)
     int64_t all = 0;
     for (const NrChunk& c : nr_chunks) all += (c.m + 127) / 128;
+    // (a thread per row: its tiles are blocks of their own, so that is how many a task
+    // describes; one each, they were 24000 for an environment update at 2048, which took
+    // 1 ms longer to plan)
     const int rows = rd_threads > 0 ? rd_threads : nr_rw * NR_WARPS;
-    const int tiles =
-        rd_threads > 0 ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(16, all / (8 * (int64_t)ctx->num_sms)));
+    const int tiles = (int)std::max<int64_t>(1, std::min<int64_t>(16, all / (8 * (int64_t)ctx->num_sms)));
+    if (rd_threads > 0) rd_tiles = tiles;
     for (const auto& gr : groups) {
       const int m = nr_chunks[gr.second[0]].m;
       for (int row0 = 0; row0 < m; row0 += tiles * rows)
@@ -1673,6 +1679,7 @@ int tt_contract_plan_keep(tt_ctx* ctx, const tt_out_block* outs, int n_out, cons
   plan->nr_rw = nr_rw;
   plan->nr_cols = nr_cols;
   plan->rd_threads = rd_threads;
+  plan->rd_tiles = rd_tiles;
   for (const NrChunk& c : nr_chunks) plan->nr_ktot = std::max(plan->nr_ktot, c.ktot);
   plan->n_tilesA = (int)ta.size();
   plan->n_tilesB = (int)tb.size();
@@ -1789,9 +1796,6 @@ int tt_contract_exec_stamped(tt_ctx* ctx, const tt_plan* plan, const double* A, 
                                  (int)narrow_smem(NR_KTOT, 8, narrow_ld(NR_N))));
     TT_CUDA(cudaFuncSetAttribute(narrow_dgemm<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)narrow_smem(NR_KTOT, 32, narrow_ld(NR_N))));
-    TT_CUDA(cudaFuncSetAttribute(rows_dgemm<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RD_SEG));
-    TT_CUDA(cudaFuncSetAttribute(rows_dgemm<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RD_SEG));
-    TT_CUDA(cudaFuncSetAttribute(rows_dgemm<RD_COLS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RD_SEG));
     TT_CUDA(cudaFuncSetAttribute(grouped_tc_persist<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)TC_BULK_SMEM));
     TT_CUDA(cudaFuncSetAttribute(grouped_tc_persist<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1814,7 +1818,7 @@ int tt_contract_exec_stamped(tt_ctx* ctx, const tt_plan* plan, const double* A, 
       // segments of equal length
       const int kmax = RD_SEG / (8 * nc), segs = std::max(1, (plan->nr_ktot + kmax - 1) / kmax);
       const int kseg = std::max(1, (plan->nr_ktot + segs - 1) / segs);
-      cfg.gridDim = dim3((unsigned)plan->n_tasks);
+      cfg.gridDim = dim3((unsigned)plan->n_tasks, (unsigned)plan->rd_tiles);
       cfg.blockDim = dim3((unsigned)plan->rd_threads);
       cfg.dynamicSmemBytes = sizeof(double) * (size_t)kseg * nc;
       const auto fn = plan->rd_threads == 128
@@ -1824,6 +1828,9 @@ int tt_contract_exec_stamped(tt_ctx* ctx, const tt_plan* plan, const double* A, 
                           : (nc == 4   ? rows_dgemm<4, true>
                              : nc == 8 ? rows_dgemm<8, true>
                                        : rows_dgemm<RD_COLS, true>);
+      static thread_local uint64_t rd_set[3] = {0, 0, 0};  // as attr_set, per instance that may need it
+      if (plan->rd_threads != 128 && tt::first_on_device(rd_set[nc == 4 ? 0 : nc == 8 ? 1 : 2], ctx->device))
+        TT_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, RD_SEG));
       TT_CUDA(cudaLaunchKernelEx(&cfg, fn,
                                  (const NrTask*)plan->d_nr_tasks, (const NrA*)plan->d_nr_a, (const NrB*)plan->d_nr_b,
                                  (const int64_t*)plan->d_nr_c, (const int32_t*)plan->d_tab, A, B, C, alpha, kseg,

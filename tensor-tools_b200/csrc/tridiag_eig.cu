@@ -475,9 +475,9 @@ __device__ __forceinline__ double hash_unit(uint64_t z) {
 // (a) Inverse iteration, one thread per vector: T - lambda I is factored once
 //     (one reciprocal per step; the row exchange is kept in the last bit of the
 //     multiplier, which the factorisation itself uses too), the INV_ITERS solves
-//     then are substitutions only.  Up to 128 rows that bit was seen to move
-//     a vector by 2e-14 at most, and a U(1) sweep's single Gram-Schmidt pass can carry any change of a last
-//     bit here to 5e-9 in <Sz>, so it stays as it is.
+//     then are substitutions only.  Up to 128 rows that bit was seen to move a
+//     vector by 2e-14 at most, and a U(1) sweep's single Gram-Schmidt pass can
+//     carry any change of a last bit here to 5e-9 in <Sz>, so it stays.
 // (b) Gram-Schmidt inside clusters, right-looking and twice: once vector j is
 //     final, every warp takes it out of its share of the later members, so a
 //     vector costs one barrier.  A vector that the first pass has left less than
