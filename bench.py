@@ -679,9 +679,14 @@ def _rounded(x):
 
 
 def compact(out):
-    """The result line of what --detail writes: of the two arms what their comparison needs, numbers with seven digits
-    (energies in full)."""
+    """The result line of what --detail writes: without the texts that explain a number, of the two arms what their
+    comparison needs, numbers with seven digits (energies in full)."""
     line = {k: _rounded(v) for k, v in out.items() if k not in ("mixed", "fp64")}
+    for name, keys in (("config", ("ramp_seconds", "ramp_energies", "start_bond_dims_mid", "setup", "value_definition")),
+                       ("roofline", ("peak_source", "tf32_products_frac")), ("e2e", ("includes",)),
+                       ("cpu_baseline", ("sample",))):
+        for k in keys:
+            (line.get(name) or {}).pop(k, None)
     short = ("value", "ms_per_step", "heff_share_of_step", "heff_tflops", "launches_per_step", "speedup_vs_fp64")
     full = ("energy", "dE_per_site_vs_fp64", "szsz_max_abs_err_vs_fp64", "full_sweep")
     for name in ("mixed", "fp64"):

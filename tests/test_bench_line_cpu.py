@@ -27,8 +27,11 @@ def _arm(steps):
 def test_line_is_short_and_complete():
     out = {"metric": bench.METRIC, "value": 10.71012345678901, "unit": "s/sweep", "n_gpus": 1, "steps": 200,
            "warmup": 5, "ms_per_step": 450.9512345678, "higher_is_better": False, "scaling": "weak",
-           "vs_baseline": None, "dtype": "tf32x3+f64", "data": "synthetic", "config": {"workload": "x" * 900},
-           "heff_tflops": 120.1, "roofline": {"frac": 0.48123456789, "peak_source": "x" * 120}, "cpu_baseline": None,
+           "vs_baseline": None, "dtype": "tf32x3+f64", "data": "synthetic",
+           "config": {"workload": "x" * 260, "precision": "x" * 160, "l2": "x" * 100, "step": "x" * 90, "setup": "x" * 240,
+                      "value_definition": "x" * 80, "ramp_energies": [-47.95547901582197] * 7, "ramp_seconds": 26.5},
+           "heff_tflops": 120.1, "roofline": {"frac": 0.48123456789, "kernel": "x" * 120, "peak_source": "x" * 140},
+           "cpu_baseline": None,
            "e2e": {"value": 11.0, "unit": "s/sweep", "h2d_bytes_per_step": 1, "d2h_bytes_per_step": 1},
            "gpu_launches": 123456, "clocks": {"sm_mhz": 1965.0, "sm_max_mhz": 1965.0, "reasons": []},
            "mixed": _arm(200), "fp64": _arm(200), "peaks_measured": {"fp64": 35.4563323726006, "tf32": 753.5856}}
