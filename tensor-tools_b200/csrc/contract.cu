@@ -415,7 +415,8 @@ grouped_dgemm(const DTask* __restrict__ tasks,
 // Measured on the middle contraction (read T1, write T2): bond dimension 3072
 // (2.03 GB) 1131 -> 620 us (1.8 -> 3.3 TB/s), 1400 (0.42 GB) 246 -> 119 us,
 // against a thread per row with the products as FP64 FMAs, 16 columns a time.
-// What is left is instruction issue (IPC 1.7, the tensor pipe 39 % active).
+// What is left is instruction issue (at 1400: IPC 1.8, the tensor pipe active for
+// 41 % of the launch, DRAM at 40 % of its peak).
 // Buffers of 16 k with four CTAs per SM measured best: 32 k (three CTAs) 662 us,
 // five CTAs at 96 registers 740 us; A loaded straight into the fragments 853 us.
 constexpr int NR_N = 32;          // columns of a chunk, at most
