@@ -767,7 +767,7 @@ def run_c5(args):
                                                               fp64["full_sweep"]["energy"]) / C5_N
         chosen["roofline"] = {
             "bound": "tensor", "kernel": "H_eff*x: grouped_tc_persist (3xTF32 tcgen05) for L*x and *R, "
-                                         "grouped_dgemm (FP64) for the middle contraction",
+                                         "narrow_dgemm (FP64) for the middle contraction",
             "achieved": chosen["heff_tflops"], "peak": peaks["tf32"] / 3.0, "unit": "TFLOP/s",
             "frac": chosen["heff_tflops"] / (peaks["tf32"] / 3.0),
             "peak_source": "cuBLAS TF32 GEMM 8192^3 measured in this run (%.1f TFLOP/s) / 3: each algorithmic "
